@@ -25,6 +25,9 @@
 #define NC_MAX_BATCHES 64u
 #define NC_YARN_SLOTS 4u
 #define NC_MAX_PAIRS 2016u
+#define NC_PAIR_SLOTS 4u    /* near fruit pairs a lane of the pair sweep's warp takes */
+#define NC_PAIR_NEAR (32u * NC_PAIR_SLOTS)
+#define NC_PAIR_COLOURS 24u /* pair colours from which the sweep runs its near pairs as wavefronts */
 #define NC_TRACE_SLOTS 128u
 #define NC_HASH_CAP 8u      /* particles one self-contact bucket holds */
 #define NC_FRICTION_STAGE 128u   /* recorded segments the staged friction sweep holds */
@@ -309,6 +312,12 @@ struct FruitShared {
     float4 v[NC_MAX_FRUITS];               // velocity xyz, inverse mass
     float4 o[NC_MAX_FRUITS];               // spin xyz, radius
     unsigned long long loaded;             // pair colours with an impulse this substep
+    // the pair sweep's wavefronts: near pairs as bits and as a list, the near
+    // pairs of every fruit, every fruit's path
+    uint32_t near_bits[(NC_MAX_PAIRS + 31u) / 32u];
+    unsigned short near[NC_PAIR_NEAR];
+    uint32_t member[NC_MAX_FRUITS][NC_PAIR_SLOTS];
+    float path[NC_MAX_FRUITS];
 };
 
 // The fruit/yarn friction sweep's recorded segments, staged by the fruit CTA

@@ -651,11 +651,139 @@ __device__ void fruit_air(FruitState& f, const SubCfg& c) {
     f.omega = f.omega * ratt;
 }
 
-// Sphere/sphere separation (tools/cloth_bag.cpp:1897-1919).
-// All fruit-pair colours, in the fruit CTA: fruit positions staged in
-// shared memory, one warp walks the colours (a colour's pairs are disjoint,
-// so its lanes never touch the same fruit); pair impulses accumulate in
-// shared memory.
+// Sphere/sphere separation (tools/cloth_bag.cpp:1897-1919) of one pair on the
+// staged fruit positions: true where the pair touched, with the positions
+// moved, the normal and the impulse.
+__device__ __forceinline__ bool fruit_pair_core(FruitShared& fs, uint32_t ab, float dt, V3& normal, float& imp) {
+    const uint32_t ia = ab & 0xffu;
+    const uint32_t ib = ab >> 8;
+    const float4 A = fs.fx[ia];
+    const float4 B = fs.fx[ib];
+    const V3 diff = xyz(B) - xyz(A);
+    const float L = len3(diff);
+    const float target = fs.fr[ia] + fs.fr[ib];
+    if (L >= target || L < 1.0e-12f) return false;
+    const float den = A.w + B.w;
+    const float lambda = (target - L) / den;
+    normal = vdiv(diff, L);
+    const V3 corr = normal * lambda;
+    fs.fx[ia] = with_xyz(A, xyz(A) - corr * A.w);
+    fs.fx[ib] = with_xyz(B, xyz(B) + corr * B.w);
+    imp = lambda / dt;
+    return true;
+}
+
+// A pair's contact record with an impulse along a normal added.
+__device__ __forceinline__ float4 pair_contact(const float4& c, V3 normal, float imp) {
+    const V3 wn = xyz(c) + normal * imp;
+    return make_float4(wn.x, wn.y, wn.z, c.w + imp);
+}
+
+// The pair sweep as wavefronts, one warp (all 32 lanes): the candidate pairs
+// (fs.near, colour order) each run as soon as the earlier candidates that
+// share one of their fruits have run, so every fruit sees its pairs in colour
+// order and the result is the colour walk's bit for bit.  A pair that is no
+// candidate starts at least `margin` from contact, and no pair can act
+// before the sweep's motion has closed that gap: where no fruit's path
+// exceeds just under half of it, the other pairs did nothing.  False where
+// the proof fails (nothing but fs.fx has changed then).
+__device__ __forceinline__ bool fruit_pair_waves(const DeviceCloth& d, FruitShared& fs, float dt, uint32_t count,
+                                                 float margin) {
+    const uint32_t lane = threadIdx.x;
+    uint32_t ab[NC_PAIR_SLOTS], wait[NC_PAIR_SLOTS][NC_PAIR_SLOTS], done[NC_PAIR_SLOTS];
+    float4 contact[NC_PAIR_SLOTS];
+    float path = 0.0f;
+#pragma unroll
+    for (uint32_t q = 0; q < NC_PAIR_SLOTS; ++q) {
+        const uint32_t c = q * 32u + lane;
+        const uint32_t k = c < count ? fs.near[c] : 0u;
+        ab[q] = fs.ab[k];
+        contact[q] = fs.contact[k];
+        done[q] = q * 32u < count ? (count - q * 32u >= 32u ? 0u : ~0u << (count - q * 32u)) : ~0u;
+        if (c < count) {
+            atomicOr(&fs.member[ab[q] & 0xffu][q], 1u << lane);
+            atomicOr(&fs.member[ab[q] >> 8][q], 1u << lane);
+        }
+    }
+    __syncwarp();
+    // the earlier candidates of either fruit
+#pragma unroll
+    for (uint32_t q = 0; q < NC_PAIR_SLOTS; ++q)
+#pragma unroll
+        for (uint32_t w = 0; w < NC_PAIR_SLOTS; ++w) {
+            const uint32_t below = w < q ? ~0u : w == q ? (1u << lane) - 1u : 0u;
+            wait[q][w] = (fs.member[ab[q] & 0xffu][w] | fs.member[ab[q] >> 8][w]) & below;
+        }
+    // at least the lowest open candidate runs in every round
+    for (uint32_t round = 0; round < count; ++round) {
+        uint32_t open = 0u;
+#pragma unroll
+        for (uint32_t q = 0; q < NC_PAIR_SLOTS; ++q) open |= ~done[q];
+        if (open == 0u) break;
+        uint32_t ran[NC_PAIR_SLOTS];
+#pragma unroll
+        for (uint32_t q = 0; q < NC_PAIR_SLOTS; ++q) {
+            uint32_t left = 0u;
+#pragma unroll
+            for (uint32_t w = 0; w < NC_PAIR_SLOTS; ++w) left |= wait[q][w] & ~done[w];
+            const bool go = ((done[q] >> lane) & 1u) == 0u && left == 0u;
+            if (go) {
+                const uint32_t ia = ab[q] & 0xffu, ib = ab[q] >> 8;
+                const V3 a0 = xyz(fs.fx[ia]), b0 = xyz(fs.fx[ib]);
+                V3 normal;
+                float imp;
+                if (fruit_pair_core(fs, ab[q], dt, normal, imp)) {
+                    contact[q] = pair_contact(contact[q], normal, imp);
+                    fs.path[ia] += len3(xyz(fs.fx[ia]) - a0);
+                    fs.path[ib] += len3(xyz(fs.fx[ib]) - b0);
+                }
+            }
+            ran[q] = __ballot_sync(0xffffffffu, go);
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t q = 0; q < NC_PAIR_SLOTS; ++q) done[q] |= ran[q];
+    }
+    for (uint32_t f = lane; f < d.f_count; f += 32u) {
+        const float p = fs.path[f];
+        path = p > path || !(p == p) ? p : path;
+    }
+    // two fruits' paths against the margin; 2 % covers the rounding of the
+    // distances and of the path sums
+    if (__any_sync(0xffffffffu, !(2.0f * path <= 0.98f * margin))) return false;
+#pragma unroll
+    for (uint32_t q = 0; q < NC_PAIR_SLOTS; ++q) {
+        const uint32_t c = q * 32u + lane;
+        if (c >= count) continue;
+        const uint32_t k = fs.near[c];
+        const float before = fs.contact[k].w;
+        fs.contact[k] = contact[q];
+        if (contact[q].w > 0.0f && contact[q].w != before) {
+            // the pair's colour: the last batch that starts at or before it
+            uint32_t lo = 0u, hi = d.n_pair_batches;
+            while (hi - lo > 1u) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (d.pair_batches[mid].first <= k) lo = mid;
+                else hi = mid;
+            }
+            atomicOr(&fs.loaded, 1ull << lo);
+        }
+    }
+    return true;
+}
+
+// All fruit-pair colours, in the fruit CTA, on the fruit positions staged in
+// shared memory; pair impulses accumulate in shared memory.  Spheres resting
+// on each other touch in most of the 63 colours of 64 fruits, but a fruit
+// has few near pairs, so the near pairs in dependence order (a handful of
+// rounds) replace the walk of every colour: 64 spheres resting on a cloth
+// took 19.2 us for the walk of 63 colours (0.3 us a colour, its quotients
+// and roots one after the other) and take 6.6 us.  Below NC_PAIR_COLOURS the
+// walk is shorter than building the wavefronts (the bag's 12 fruits have 11
+// colours: 1 % of its frame), and it stays for more than NC_PAIR_NEAR near
+// pairs and for sweeps that move a fruit too far for the proof.  One warp
+// walks the colours (a colour's pairs are disjoint, so its lanes never touch
+// the same fruit).
 __device__ void fruit_pair_sweep(const DeviceCloth& d, FruitShared& fs, float dt) {
     for (uint32_t f = threadIdx.x; f < d.f_count; f += blockDim.x) {
         const NumiClothFruit& fr = d.fruits[f];
@@ -663,44 +791,78 @@ __device__ void fruit_pair_sweep(const DeviceCloth& d, FruitShared& fs, float dt
                                fr.positionAndInverseMass.z, fr.positionAndInverseMass.w);
         fs.fr[f] = fr.previousAndRadius.w;
     }
+    const bool waves = d.n_pair_batches >= NC_PAIR_COLOURS;
+    if (waves)
+        for (uint32_t e = threadIdx.x; e < d.f_count * NC_PAIR_SLOTS; e += blockDim.x) {
+            (&fs.member[0][0])[e] = 0u;
+            fs.path[e / NC_PAIR_SLOTS] = 0.0f;
+        }
     __syncthreads();
     // Fruits move only through pair contacts, so when no pair touches at the
     // start of the sweep none touches at any point of it: skip the walk.
+    // Near: within 0.4 of the smallest radius of contact (8 mm for the 2 cm
+    // sphere; a sphere landing at 4 m/s moves 1.4 mm in a substep).
     bool touching = false;
-    for (uint32_t k = threadIdx.x; k < d.p_count; k += blockDim.x) {
-        const uint32_t ia = fs.ab[k] & 0xffu;
-        const uint32_t ib = fs.ab[k] >> 8;
-        const float L = len3(xyz(fs.fx[ib]) - xyz(fs.fx[ia]));
-        touching = touching || !(L >= fs.fr[ia] + fs.fr[ib] || L < 1.0e-12f);
+    const uint32_t lane = threadIdx.x & 31u;
+    float smallest = INFINITY;
+    for (uint32_t f = lane; waves && f < d.f_count; f += 32u) smallest = fminf(smallest, fs.fr[f]);
+    for (int o = 16; o > 0; o >>= 1) smallest = fminf(smallest, __shfl_xor_sync(0xffffffffu, smallest, o));
+    const float margin = 0.4f * smallest;
+    for (uint32_t base = threadIdx.x - lane; base < d.p_count; base += blockDim.x) {
+        const uint32_t k = base + lane;
+        bool near = false;
+        if (k < d.p_count) {
+            const uint32_t ia = fs.ab[k] & 0xffu;
+            const uint32_t ib = fs.ab[k] >> 8;
+            const float L = len3(xyz(fs.fx[ib]) - xyz(fs.fx[ia]));
+            const float target = fs.fr[ia] + fs.fr[ib];
+            touching = touching || !(L >= target || L < 1.0e-12f);
+            near = !(L >= target + margin);
+        }
+        if (!waves) continue;
+        const uint32_t bits = __ballot_sync(0xffffffffu, near);
+        if (lane == 0u) fs.near_bits[base >> 5] = bits;
     }
     if (!__syncthreads_or(touching)) return;
     if (threadIdx.x < 32u) {
-        for (uint32_t b = 0; b < d.n_pair_batches; ++b) {
-            const Batch bt = d.pair_batches[b];
-            bool loaded = false;
-            for (uint32_t k = bt.first + threadIdx.x; k < bt.first + bt.count; k += 32u) {
-                const uint32_t ia = fs.ab[k] & 0xffu;
-                const uint32_t ib = fs.ab[k] >> 8;
-                const float4 A = fs.fx[ia];
-                const float4 B = fs.fx[ib];
-                const V3 diff = xyz(B) - xyz(A);
-                const float L = len3(diff);
-                const float target = fs.fr[ia] + fs.fr[ib];
-                if (L >= target || L < 1.0e-12f) continue;
-                const float den = A.w + B.w;
-                const float lambda = (target - L) / den;
-                const V3 normal = vdiv(diff, L);
-                const V3 corr = normal * lambda;
-                fs.fx[ia] = with_xyz(A, xyz(A) - corr * A.w);
-                fs.fx[ib] = with_xyz(B, xyz(B) + corr * B.w);
-                const float imp = lambda / dt;
-                const float4 c = fs.contact[k];
-                const V3 wn = xyz(c) + normal * imp;
-                fs.contact[k] = make_float4(wn.x, wn.y, wn.z, c.w + imp);
-                loaded = loaded || c.w + imp > 0.0f;
+        // the near pairs in colour order
+        uint32_t count = 0u;
+        for (uint32_t w0 = 0; waves && w0 * 32u < d.p_count; w0 += 32u) {
+            uint32_t bits = (w0 + lane) * 32u < d.p_count ? fs.near_bits[w0 + lane] : 0u;
+            uint32_t at = __popc(bits);
+            for (uint32_t o = 1; o < 32u; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, at, o);
+                if (lane >= o) at += v;
             }
-            if (__any_sync(0xffffffffu, loaded) && threadIdx.x == 0) fs.loaded |= 1ull << b;
+            const uint32_t total = __shfl_sync(0xffffffffu, at, 31);
+            at += count - __popc(bits);
+            for (; bits != 0u; bits &= bits - 1u, ++at)
+                if (at < NC_PAIR_NEAR)
+                    fs.near[at] = static_cast<unsigned short>((w0 + lane) * 32u + __ffs(static_cast<int>(bits)) - 1);
+            count += total;
+        }
+        __syncwarp();
+        if (!waves || count > NC_PAIR_NEAR || !fruit_pair_waves(d, fs, dt, count, margin)) {
+            for (uint32_t f = lane; f < d.f_count; f += 32u) {
+                const NumiClothFruit& fr = d.fruits[f];
+                fs.fx[f] = make_float4(fr.positionAndInverseMass.x, fr.positionAndInverseMass.y,
+                                       fr.positionAndInverseMass.z, fr.positionAndInverseMass.w);
+            }
             __syncwarp();
+            for (uint32_t b = 0; b < d.n_pair_batches; ++b) {
+                const Batch bt = d.pair_batches[b];
+                bool loaded = false;
+                for (uint32_t k = bt.first + threadIdx.x; k < bt.first + bt.count; k += 32u) {
+                    V3 normal;
+                    float imp;
+                    if (!fruit_pair_core(fs, fs.ab[k], dt, normal, imp)) continue;
+                    const float4 c = pair_contact(fs.contact[k], normal, imp);
+                    fs.contact[k] = c;
+                    loaded = loaded || c.w > 0.0f;
+                }
+                if (__any_sync(0xffffffffu, loaded) && threadIdx.x == 0) fs.loaded |= 1ull << b;
+                __syncwarp();
+            }
         }
     }
     __syncthreads();
