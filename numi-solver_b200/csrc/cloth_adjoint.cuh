@@ -2,11 +2,10 @@
 // reference calibrates with external finite-difference sensitivities,
 // docs/CLOTH_SPECIMEN_CALIBRATION.md:52-82).
 //
-// The forward runs a segment of substeps on one CTA and records a tape: the
-// positions at the start of every substep and after every phase barrier,
-// and the velocities at the start of every substep.  This kernel walks the
-// segment's substeps and each substep's phases in reverse and applies the
-// vector-Jacobian product of every projection.  Branch decisions are
+// The forward records a tape: the positions at the start of every substep
+// and after every phase barrier, and the velocities at the start of every
+// substep.  This kernel walks the taped substeps and each substep's phases in
+// reverse and applies the vector-Jacobian product of every projection.  Branch decisions are
 // recomputed in FP32 from the tape exactly as the forward made them; the
 // derivatives are evaluated in FP64 at the FP32 state, and adjoints and
 // parameter gradients are accumulated in FP64.
@@ -48,8 +47,9 @@ struct AdjointArgs {
     const NumiClothConfig* cfg;      // the segment's Configs
     const float4* tape;              // [substeps][slots][n]
     const float4* tape_v;            // [substeps][n]
-    const uint2* phases;             // [slots - 1] (type, batch) per barrier
+    const uint4* phases;             // [slots - 1] (type, first record, records, 0) per barrier
     uint32_t slots;
+    uint32_t shift;                  // log2 of the particles each CTA of the cluster owns
     uint32_t substeps;               // substeps of the segment
     uint32_t first_substep;          // rollout index of the segment's first substep
     float damping;                   // the schedule's (or the cloth's) damping
@@ -89,27 +89,105 @@ __device__ __forceinline__ D3v crossd(D3v a, D3v b) {
 }
 __device__ __forceinline__ void put(double4* g, uint32_t i, D3v v) { g[i] = make_double4(v.x, v.y, v.z, 0.0); }
 
+// Adjoint of the positions during a segment.  kShared: CTA r of the cloth's
+// cluster holds particles [r << shift, (r + 1) << shift) in its shared
+// memory (three doubles each: an odd stride, so neighbouring particles fall
+// in different banks), the others' through distributed shared memory.
+// Otherwise (clouds too large for that) the global array, past L1.
+template <bool kShared>
+struct AdjointX {
+    double* own;
+    double4* all;
+    uint32_t rank, shift;
+
+    __device__ __forceinline__ double* at(uint32_t i) const {
+        const uint32_t r = i >> shift;
+        double* p = own + 3u * (i & ((1u << shift) - 1u));
+        return r == rank ? p : static_cast<double*>(__cluster_map_shared_rank(p, r));
+    }
+    __device__ __forceinline__ D3v get(uint32_t i) const {
+        if constexpr (kShared) {
+            const double* p = at(i);
+            return D3v{p[0], p[1], p[2]};
+        } else {
+            const double2* p = reinterpret_cast<const double2*>(all + i);
+            const double2 xy = __ldcg(p);
+            return D3v{xy.x, xy.y, __ldcg(&p[1].x)};
+        }
+    }
+    __device__ __forceinline__ void put(uint32_t i, D3v v) const {
+        if constexpr (kShared) {
+            double* p = at(i);
+            p[0] = v.x;
+            p[1] = v.y;
+            p[2] = v.z;
+        } else {
+            all[i] = make_double4(v.x, v.y, v.z, 0.0);
+        }
+    }
+};
+
 // VJP of x_a' = x_a - w_a dl n, x_b' = x_b + w_b dl n with
 // dl = -(L - rest) / (w_a + w_b + alpha) (lambda from zero), n = (x_b - x_a)/L,
 // at the FP32 state a, b (derivatives in FP64).  Returns d loss / d alpha.
-__device__ __forceinline__ double distance_vjp(double4* gx, uint32_t ia, uint32_t ib, const float4& a, const float4& b,
+template <class X>
+__device__ __forceinline__ double distance_vjp(const X& gx, uint32_t ia, uint32_t ib, const float4& a, const float4& b,
                                                double rest, double alpha) {
     const D3v dd = subd(d4f(b), d4f(a));
     const double L = sqrt(dotd(dd, dd));
     const D3v n = muld(dd, 1.0 / L);
     const double den = (static_cast<double>(a.w) + b.w) + alpha;
     const double dl = -(L - rest) / den;
-    const D3v ga = d3(gx[ia]), gb = d3(gx[ib]);
+    const D3v ga = gx.get(ia), gb = gx.get(ib);
     const D3v u = subd(muld(gb, b.w), muld(ga, a.w));
     const double un = dotd(u, n);
     const D3v gd = addd(muld(n, -un / den), muld(subd(u, muld(n, un)), dl / L));
-    put(gx, ia, subd(ga, gd));
-    put(gx, ib, addd(gb, gd));
+    gx.put(ia, subd(ga, gd));
+    gx.put(ib, addd(gb, gd));
     return -un * dl / den;
 }
 
-// Forward-mode dual number (value, one tangent) for the knot projection,
-// whose Jacobian involves the derivatives of its own gradients.
+// VJP of the knot projection (nc::solve_knot with lambda from zero) at the
+// positions p with inverse masses p.w: g[4], the adjoints of the moved
+// positions, become those of p.  Returns d loss / d alpha.  Reverse mode by
+// hand: one pass over the projection's steps (two square roots, five
+// quotients), against thirteen of them for a tangent per input.
+__device__ __forceinline__ double knot_vjp(const float4 p[4], double alpha, double rest, D3v g[4]) {
+    const double w0 = p[0].w, w1 = p[1].w, w2 = p[2].w, w3 = p[3].w;
+    const D3v e = subd(d4f(p[1]), d4f(p[0])), f = subd(d4f(p[3]), d4f(p[2]));
+    const double el = 1.0 / sqrt(dotd(e, e)), fl = 1.0 / sqrt(dotd(f, f));
+    const D3v u = muld(e, el), v = muld(f, fl);
+    double c = dotd(u, v);
+    const bool clamped = c > 1.0 || c < -1.0;
+    c = c > 1.0 ? 1.0 : c < -1.0 ? -1.0 : c;
+    // gradients of the cosine, the step along them
+    const D3v gw = muld(subd(v, muld(u, c)), el), gf = muld(subd(u, muld(v, c)), fl);
+    const double we = w0 + w1, wf = w2 + w3;
+    const double iden = 1.0 / (alpha + we * dotd(gw, gw) + wf * dotd(gf, gf));
+    const double dl = -(c - rest) * iden;
+    // reverse: p1 + gw w1 dl, p0 - gw w0 dl, p3 + gf w3 dl, p2 - gf w2 dl
+    const D3v A = subd(muld(g[1], w1), muld(g[0], w0)), B = subd(muld(g[3], w3), muld(g[2], w2));
+    const double bdl = dotd(A, gw) + dotd(B, gf);
+    const double bden = -bdl * dl * iden;
+    const D3v bgw = addd(muld(A, dl), muld(gw, 2.0 * we * bden));
+    const D3v bgf = addd(muld(B, dl), muld(gf, 2.0 * wf * bden));
+    const D3v q = muld(bgw, el), r = muld(bgf, fl);
+    double bc = -bdl * iden - dotd(q, u) - dotd(r, v);
+    if (clamped) bc = 0.0;
+    const D3v bu = addd(subd(r, muld(q, c)), muld(v, bc));
+    const D3v bv = addd(subd(q, muld(r, c)), muld(u, bc));
+    // u = e / |e| and the 1 / |e| of gw: along e, then across it
+    const D3v be = muld(subd(bu, muld(u, dotd(bu, u) + dotd(bgw, gw))), el);
+    const D3v bf = muld(subd(bv, muld(v, dotd(bv, v) + dotd(bgf, gf))), fl);
+    g[0] = subd(g[0], be);
+    g[1] = addd(g[1], be);
+    g[2] = subd(g[2], bf);
+    g[3] = addd(g[3], bf);
+    return bden;
+}
+
+// Forward-mode dual number (value, one tangent) for the bend projection on
+// the ground, whose branches a hand-written reverse pass would repeat.
 struct Dual {
     double v, d;
 };
@@ -129,33 +207,6 @@ struct DV {
 __device__ __forceinline__ DV operator-(DV a, DV b) { return DV{a.x - b.x, a.y - b.y, a.z - b.z}; }
 __device__ __forceinline__ DV operator*(DV a, Dual s) { return DV{a.x * s, a.y * s, a.z * s}; }
 __device__ __forceinline__ Dual ddot(DV a, DV b) { return (a.x * b.x + a.y * b.y) + a.z * b.z; }
-
-// Knot projection (nc::solve_knot with lambda from zero) on dual numbers:
-// positions p[4], inverse masses w[4], compliance alpha; writes out[4].
-__device__ __forceinline__ void knot_dual(const DV p[4], const double w[4], Dual alpha, double rest, DV out[4]) {
-    const DV warpv = p[1] - p[0];
-    const DV weftv = p[3] - p[2];
-    const Dual wl = dsqrt(ddot(warpv, warpv));
-    const Dual fl = dsqrt(ddot(weftv, weftv));
-    const Dual one{1.0, 0.0};
-    const DV warp = warpv * (one / wl);
-    const DV weft = weftv * (one / fl);
-    Dual cosine = ddot(warp, weft);
-    if (cosine.v > 1.0) cosine = Dual{1.0, 0.0};
-    if (cosine.v < -1.0) cosine = Dual{-1.0, 0.0};
-    const Dual value = cosine - Dual{rest, 0.0};
-    const DV gw = (weft - warp * cosine) * (one / wl);
-    const DV gf = (warp - weft * cosine) * (one / fl);
-    const Dual W[4] = {{w[0], 0.0}, {w[1], 0.0}, {w[2], 0.0}, {w[3], 0.0}};
-    const Dual den = alpha + W[0] * ddot(gw, gw) + W[1] * ddot(gw, gw) + W[2] * ddot(gf, gf) + W[3] * ddot(gf, gf);
-    const Dual dl = Dual{0.0, 0.0} - value / den;
-    const Dual zero{0.0, 0.0};
-    const DV g[4] = {DV{zero, zero, zero} - gw, gw, DV{zero, zero, zero} - gf, gf};
-    for (int q = 0; q < 4; ++q) {
-        const Dual s = W[q] * dl;
-        out[q] = DV{p[q].x + g[q].x * s, p[q].y + g[q].y * s, p[q].z + g[q].z * s};
-    }
-}
 
 // Branches the forward bend projection took (nc::bend_core): active[s]
 // when the ground holds particle s's normal motion; frac_src the particle
@@ -259,16 +310,133 @@ __device__ __forceinline__ void bend_dual(const DV p[2], const double w[2], Dual
 
 }  // namespace adj
 
-__device__ __forceinline__ void adjoint_segment(const AdjointArgs& A) {
+// One item of a constraint colour: the record's points at the positions the
+// phase started from, its material and compliance group.
+struct AdjointItem {
+    uint32_t k;
+    uint32_t idx[4];
+    float4 p[4];
+    float4 m;
+    uint32_t group;
+};
+
+#define ADJ_THREADS 512u
+#define ADJ_PHASES 256u   /* phase records kept in shared memory */
+#define ADJ_CLUSTER_MAX 16u
+
+// The reverse sweep of one cloth's taped segment on its cluster of CTAs.
+//
+// A substep is some twenty dependent phases of at most a few thousand items,
+// so the sweep is bound by the latency of a phase: barrier, gather, a chain
+// of FP64 quotients and roots.  On one CTA of 256 threads with the adjoint in
+// global memory a phase of the 64 x 64 cloth's 2,000 items took eight rounds
+// of dependent L2 loads (22.9 ms for 96 substeps).  Here a cluster gives every
+// item its own thread, the adjoint lives in the cluster's shared memory, and a
+// thread loads its next item (indices, material, taped positions: nothing the
+// sweep writes) before the barrier in front of it.  Phases that touch only a
+// particle's own adjoint (finalize, ground, contact counts, predict) run on
+// its owner, one after the other without barriers.
+template <bool kShared>
+__device__ __forceinline__ void adjoint_segment(const AdjointArgs& A, uint32_t rank, uint32_t ranks, double* smem) {
     using namespace adj;
     const DeviceCloth& d = *A.cloth;
     const uint32_t n = d.n;
+    const uint32_t bottom = A.slots - 1u;   // phases of a substep
+    __shared__ uint4 s_phase[ADJ_PHASES];
+    for (uint32_t b = threadIdx.x; b < min(bottom, ADJ_PHASES); b += blockDim.x) s_phase[b] = A.phases[b];
+    auto phase = [&](uint32_t b) { return b < ADJ_PHASES ? s_phase[b] : A.phases[b]; };
+    auto sync = [&]() {
+        if (ranks > 1u)
+            cooperative_groups::this_cluster().sync();
+        else
+            __syncthreads();
+    };
+    const AdjointX<kShared> gx{smem, A.gx, rank, A.shift};
+    const uint32_t own = min(rank << A.shift, n), own_end = min(own + (1u << A.shift), n);
+    if constexpr (kShared)
+        for (uint32_t i = own + threadIdx.x; i < own_end; i += blockDim.x) {
+            const double4 v = A.gx[i];
+            gx.put(i, D3v{v.x, v.y, v.z});
+        }
     double acc[ADJ_MAX_GROUPS + 1u];
     for (uint32_t e = 0; e <= ADJ_MAX_GROUPS; ++e) acc[e] = 0.0;
     const uint32_t damp_slot = A.groups;
     double loss = 0.0;
     unsigned int rough = 0u;
     __shared__ double s_grip[NC_MAX_GRIPS][6];
+
+    // item r of a colour phase, at the positions `pre` the phase started from
+    auto load = [&](const uint4& ph, uint32_t r, const float4* pre, AdjointItem& it) {
+        const uint32_t k = ph.y + r;
+        it.k = k;
+        if (ph.x == ADJ_KNOT) {
+            const uint4 q = __ldg(d.k_ij + k);
+            const float2 m = __ldg(d.k_mat + k);
+            it.m = make_float4(m.x, m.y, 0.0f, 0.0f);
+            it.idx[0] = q.x;
+            it.idx[1] = q.y;
+            it.idx[2] = q.z;
+            it.idx[3] = q.w;
+            it.group = __ldg(A.k_group + k);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) it.p[e] = __ldg(pre + it.idx[e]);
+            return;
+        }
+        if (ph.x == ADJ_BEND) {
+            const uint4 q = __ldg(d.b_ij + k);
+            const float2 m = __ldg(d.b_mat + k);
+            it.m = make_float4(m.x, m.y, 0.0f, 0.0f);
+            it.idx[0] = q.x;
+            it.idx[1] = q.z;
+            it.group = __ldg(A.b_group + k);
+        } else {
+            const uint2 q = __ldg(d.d_ij + k);
+            it.m = __ldg(d.d_mat + k);
+            it.idx[0] = q.x;
+            it.idx[1] = q.y;
+            it.group = __ldg(A.d_group + k);
+        }
+        it.p[0] = __ldg(pre + it.idx[0]);
+        it.p[1] = __ldg(pre + it.idx[1]);
+    };
+    // this CTA's slice of a phase's items
+    auto slice = [&](uint32_t count, uint32_t& lo, uint32_t& hi) {
+        lo = static_cast<uint32_t>(static_cast<unsigned long long>(count) * rank / ranks);
+        hi = static_cast<uint32_t>(static_cast<unsigned long long>(count) * (rank + 1u) / ranks);
+    };
+    // this thread's first item of the next colour phase below (si, b)
+    AdjointItem next{};
+    auto fetch = [&](uint32_t si, uint32_t b) {
+        for (;;) {
+            if (b == 0u) {
+                if (si == 0u) return;
+                --si;
+                b = bottom;
+            }
+            --b;
+            const uint4 ph = phase(b);
+            if (ph.x != ADJ_DIST && ph.x != ADJ_STRAIN && ph.x != ADJ_BEND && ph.x != ADJ_KNOT) continue;
+            uint32_t lo, hi;
+            slice(ph.z, lo, hi);
+            if (lo + threadIdx.x < hi)
+                load(ph, lo + threadIdx.x, A.tape + (static_cast<size_t>(si) * A.slots + b) * n, next);
+            return;
+        }
+    };
+    // the sweep of one colour phase's items: each loaded before the one in
+    // front of it is computed
+    auto colour = [&](const uint4& ph, const float4* pre, auto&& apply) {
+        uint32_t lo, hi;
+        slice(ph.z, lo, hi);
+        for (uint32_t r = lo + threadIdx.x; r < hi; r += blockDim.x) {
+            const AdjointItem it = next;
+            if (r + blockDim.x < hi) load(ph, r + blockDim.x, pre, next);
+            apply(it);
+        }
+    };
+    sync();
+    fetch(A.substeps, 0u);
+    bool loose = false;   // own-particle phases ran since the last barrier
     for (uint32_t si = A.substeps; si-- > 0u;) {
         const NumiClothConfig& cf = A.cfg[si];
         const float dt = cf.gravityAndTimestep.w;
@@ -278,30 +446,36 @@ __device__ __forceinline__ void adjoint_segment(const AdjointArgs& A) {
         const bool ground = cf.constraintCounts.z != 0u;
         const float4* T = A.tape + static_cast<size_t>(si) * A.slots * n;
         const uint32_t step = A.first_substep + si;
-        // loss seed at the end of the substep
+        // loss seed at the end of the substep, by the tracked particles' owners
         if (A.loss_every != 0u && (step + 1u) % A.loss_every == 0u) {
             const uint32_t li = (step + 1u) / A.loss_every - 1u;
-            const float4* xe = T + static_cast<size_t>(A.slots - 1u) * n;
-            for (uint32_t t = threadIdx.x; t < A.n_tracked; t += blockDim.x) {
-                const uint32_t i = A.tracked[t];
+            const float4* xe = T + static_cast<size_t>(bottom) * n;
+            for (uint32_t t = 0; t < A.n_tracked; ++t) {
+                const uint32_t i = __ldg(A.tracked + t);
+                if (i < own || i >= own_end || (i - own) % blockDim.x != threadIdx.x) continue;
                 const double* tg = A.targets + (static_cast<size_t>(li) * A.n_tracked + t) * 3u;
                 const D3v diff{static_cast<double>(xe[i].x) - tg[0], static_cast<double>(xe[i].y) - tg[1],
                                static_cast<double>(xe[i].z) - tg[2]};
                 loss += dotd(diff, diff);
-                put(A.gx, i, addd(d3(A.gx[i]), muld(diff, 2.0)));
+                gx.put(i, addd(gx.get(i), muld(diff, 2.0)));
             }
-            __syncthreads();
+            loose = true;
         }
-        for (uint32_t b = A.slots - 1u; b-- > 0u;) {
-            const uint2 ph = A.phases[b];
+        for (uint32_t b = bottom; b-- > 0u;) {
+            const uint4 ph = phase(b);
             const float4* pre = T + static_cast<size_t>(b) * n;     // positions before the phase
             const float4* post = pre + n;                            // after its barrier
+            bool crossed = true;   // the phase touches particles of other threads
+            if (loose && (ph.x == ADJ_STRAIN || ph.x == ADJ_DIST || ph.x == ADJ_BEND || ph.x == ADJ_KNOT ||
+                          ph.x == ADJ_GRIP)) {
+                sync();
+                loose = false;
+            }
             switch (ph.x) {
-            case ADJ_TAIL:
-                break;
             case ADJ_YARN:
                 // fruit/yarn contact moved the cloth: not differentiated
-                for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
+                crossed = false;
+                for (uint32_t i = own + threadIdx.x; i < own_end; i += blockDim.x)
                     if (pre[i].x != post[i].x || pre[i].y != post[i].y || pre[i].z != post[i].z) ++rough;
                 break;
             case ADJ_FINAL: {
@@ -312,13 +486,14 @@ __device__ __forceinline__ void adjoint_segment(const AdjointArgs& A) {
                 // sliding removes mu (v_end.z - v_pred.z) along the slip.
                 // The adjoint of the predicted normal velocity goes to
                 // gprev.w for the predict step.
+                crossed = false;
                 const float4* xs = T;
                 const float4* vs = A.tape_v + static_cast<size_t>(si) * n;
                 const float inv_dt = 1.0f / dt;
                 const float mu = cf.clothMaterial.z;
-                for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+                for (uint32_t i = own + threadIdx.x; i < own_end; i += blockDim.x) {
                     if (pre[i].w == 0.0f) {
-                        A.gx[i] = make_double4(0, 0, 0, 0);
+                        gx.put(i, D3v{0.0, 0.0, 0.0});
                         A.gv[i] = make_double4(0, 0, 0, 0);
                         A.gprev[i] = make_double4(0, 0, 0, 0);
                         continue;
@@ -355,7 +530,7 @@ __device__ __forceinline__ void adjoint_segment(const AdjointArgs& A) {
                             }
                         }
                     }
-                    put(A.gx, i, addd(d3(A.gx[i]), muld(gvv, 1.0 / dtd)));
+                    gx.put(i, addd(gx.get(i), muld(gvv, 1.0 / dtd)));
                     const D3v gp = muld(gvv, -1.0 / dtd);
                     A.gprev[i] = make_double4(gp.x, gp.y, gp.z, gvpz);
                     A.gv[i] = make_double4(0, 0, 0, 0);
@@ -363,118 +538,72 @@ __device__ __forceinline__ void adjoint_segment(const AdjointArgs& A) {
                 break;
             }
             case ADJ_STRAIN:
-            case ADJ_DIST: {
-                const Batch bt = d.dist_batches[ph.y];
-                const uint32_t count = ph.x == ADJ_STRAIN ? bt.limited : bt.count;
-                for (uint32_t r = threadIdx.x; r < count; r += blockDim.x) {
-                    const uint32_t k = bt.first + r;
-                    const uint2 ij = d.d_ij[k];
-                    const float4 m = d.d_mat[k];
-                    const float4 a = pre[ij.x], bb = pre[ij.y];
-                    const V3 diff = xyz(bb) - xyz(a);
-                    const float L = len3(diff);
-                    if (ph.x == ADJ_STRAIN) {
-                        if (!(m.w > 0.0f)) continue;
-                        const float maxL = m.x * (1.0f + m.w);
-                        if (L <= maxL || L < 1.0e-12f) continue;
-                        if (a.w + bb.w <= 0.0f) continue;
-                        // x_a += dir w_a (L - maxL)/den: the distance form with rest maxL, alpha 0
-                        distance_vjp(A.gx, ij.x, ij.y, a, bb, static_cast<double>(maxL), 0.0);
-                    } else {
-                        if (L < 1.0e-12f) continue;
-                        const float alpha = m.y / dt2;
-                        if ((a.w + bb.w) + alpha <= 0.0f) continue;
-                        const double alphad = static_cast<double>(m.y) / (dtd * dtd);
-                        const double galpha =
-                            distance_vjp(A.gx, ij.x, ij.y, a, bb, static_cast<double>(m.x), alphad);
-                        acc[A.d_group[k]] += galpha * alphad;
-                    }
-                }
+                colour(ph, pre, [&](const AdjointItem& it) {
+                    const float4 a = it.p[0], bb = it.p[1], m = it.m;
+                    if (!(m.w > 0.0f)) return;
+                    const float L = len3(xyz(bb) - xyz(a));
+                    const float maxL = m.x * (1.0f + m.w);
+                    if (L <= maxL || L < 1.0e-12f) return;
+                    if (a.w + bb.w <= 0.0f) return;
+                    // x_a += dir w_a (L - maxL)/den: the distance form with rest maxL, alpha 0
+                    distance_vjp(gx, it.idx[0], it.idx[1], a, bb, static_cast<double>(maxL), 0.0);
+                });
                 break;
-            }
-            case ADJ_KNOT: {
-                const Batch bt = d.knot_batches[ph.y];
-                for (uint32_t r = threadIdx.x; r < bt.count; r += blockDim.x) {
-                    const uint32_t k = bt.first + r;
-                    const uint4 q = d.k_ij[k];
-                    const float2 m = d.k_mat[k];
-                    const uint32_t idx[4] = {q.x, q.y, q.z, q.w};
-                    float4 p[4];
-                    for (int e = 0; e < 4; ++e) p[e] = pre[idx[e]];
+            case ADJ_DIST:
+                colour(ph, pre, [&](const AdjointItem& it) {
+                    const float4 a = it.p[0], bb = it.p[1];
+                    if (len3(xyz(bb) - xyz(a)) < 1.0e-12f) return;
+                    const float alpha = it.m.y / dt2;
+                    if ((a.w + bb.w) + alpha <= 0.0f) return;
+                    const double alphad = static_cast<double>(it.m.y) / (dtd * dtd);
+                    acc[it.group] +=
+                        distance_vjp(gx, it.idx[0], it.idx[1], a, bb, static_cast<double>(it.m.x), alphad) * alphad;
+                });
+                break;
+            case ADJ_KNOT:
+                colour(ph, pre, [&](const AdjointItem& it) {
                     // the forward's own skip tests, in FP32
+                    const float4* p = it.p;
                     const float wl = len3(xyz(p[1]) - xyz(p[0]));
                     const float fl = len3(xyz(p[3]) - xyz(p[2]));
-                    if (wl < 1.0e-12f || fl < 1.0e-12f) continue;
+                    if (wl < 1.0e-12f || fl < 1.0e-12f) return;
                     const V3 warp = vdiv(xyz(p[1]) - xyz(p[0]), wl);
                     const V3 weft = vdiv(xyz(p[3]) - xyz(p[2]), fl);
                     const float cosine = fminf(fmaxf(dot3(warp, weft), -1.0f), 1.0f);
                     const V3 gw = vdiv(weft - warp * cosine, wl);
                     const V3 gf = vdiv(warp - weft * cosine, fl);
-                    const float alpha = m.y / dt2;
-                    float den = alpha;
+                    float den = it.m.y / dt2;
                     den = den + p[0].w * lsq(gw * -1.0f);
                     den = den + p[1].w * lsq(gw);
                     den = den + p[2].w * lsq(gf * -1.0f);
                     den = den + p[3].w * lsq(gf);
-                    if (den <= 0.0f) continue;
-                    // VJP by forward mode: one tangent per input (12 coordinates, alpha)
-                    double u[12];
-                    for (int e = 0; e < 4; ++e) {
-                        const double4 ge = A.gx[idx[e]];
-                        u[3 * e] = ge.x;
-                        u[3 * e + 1] = ge.y;
-                        u[3 * e + 2] = ge.z;
-                    }
-                    const double w[4] = {p[0].w, p[1].w, p[2].w, p[3].w};
-                    const double alphad = static_cast<double>(m.y) / (dtd * dtd);
-                    double gin[13];
-                    for (int dir = 0; dir < 13; ++dir) {
-                        DV pd[4];
-                        for (int e = 0; e < 4; ++e) {
-                            pd[e] = DV{Dual{p[e].x, dir == 3 * e ? 1.0 : 0.0}, Dual{p[e].y, dir == 3 * e + 1 ? 1.0 : 0.0},
-                                       Dual{p[e].z, dir == 3 * e + 2 ? 1.0 : 0.0}};
-                        }
-                        DV out[4];
-                        knot_dual(pd, w, Dual{alphad, dir == 12 ? 1.0 : 0.0}, static_cast<double>(m.x), out);
-                        double acc_dir = 0.0;
-                        for (int e = 0; e < 4; ++e)
-                            acc_dir += u[3 * e] * out[e].x.d + u[3 * e + 1] * out[e].y.d + u[3 * e + 2] * out[e].z.d;
-                        gin[dir] = acc_dir;
-                    }
-                    for (int e = 0; e < 4; ++e)
-                        A.gx[idx[e]] = make_double4(gin[3 * e], gin[3 * e + 1], gin[3 * e + 2], 0.0);
-                    acc[A.k_group[k]] += gin[12] * alphad;
-                }
+                    if (den <= 0.0f) return;
+                    const double alphad = static_cast<double>(it.m.y) / (dtd * dtd);
+                    D3v g[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) g[e] = gx.get(it.idx[e]);
+                    acc[it.group] += knot_vjp(p, alphad, static_cast<double>(it.m.x), g) * alphad;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) gx.put(it.idx[e], g[e]);
+                });
                 break;
-            }
-            case ADJ_BEND: {
-                const Batch bt = d.bend_batches[ph.y];
-                for (uint32_t r = threadIdx.x; r < bt.count; r += blockDim.x) {
-                    const uint32_t k = bt.first + r;
-                    const uint4 q = d.b_ij[k];
-                    const float2 m = d.b_mat[k];
-                    const float4 p0 = pre[q.x], p2 = pre[q.z];
+            case ADJ_BEND:
+                colour(ph, pre, [&](const AdjointItem& it) {
+                    const float4 p0 = it.p[0], p2 = it.p[1];
+                    const float2 m = make_float2(it.m.x, it.m.y);
                     BendBranches br;
-                    if (!bend_branches(p0, p2, m, dt2, radius, ground, br)) continue;
+                    if (!bend_branches(p0, p2, m, dt2, radius, ground, br)) return;
                     const double alphad = static_cast<double>(m.y) / (dtd * dtd);
                     if (!br.active[0] && !br.active[1] && br.frac_src < 0 && !br.clamp[0] && !br.clamp[1]) {
                         // clear of the ground: the distance form
-                        const double galpha =
-                            distance_vjp(A.gx, q.x, q.z, p0, p2, static_cast<double>(m.x), alphad);
-                        acc[A.b_group[k]] += galpha * alphad;
-                        continue;
+                        acc[it.group] +=
+                            distance_vjp(gx, it.idx[0], it.idx[1], p0, p2, static_cast<double>(m.x), alphad) * alphad;
+                        return;
                     }
                     // on the ground: VJP by forward mode along the forward's
                     // branches, one tangent per input (6 coordinates, alpha)
-                    const uint32_t idx[2] = {q.x, q.z};
                     const float4 pp[2] = {p0, p2};
-                    double u[6];
-                    for (int e = 0; e < 2; ++e) {
-                        const double4 ge = A.gx[idx[e]];
-                        u[3 * e] = ge.x;
-                        u[3 * e + 1] = ge.y;
-                        u[3 * e + 2] = ge.z;
-                    }
+                    const D3v u0 = gx.get(it.idx[0]), u1 = gx.get(it.idx[1]);
                     const double w[2] = {p0.w, p2.w};
                     double gin[7];
                     for (int dir = 0; dir < 7; ++dir) {
@@ -485,22 +614,24 @@ __device__ __forceinline__ void adjoint_segment(const AdjointArgs& A) {
                         DV out[2];
                         bend_dual(pd, w, Dual{alphad, dir == 6 ? 1.0 : 0.0}, static_cast<double>(m.x),
                                   static_cast<double>(radius), br, out);
-                        double acc_dir = 0.0;
-                        for (int e = 0; e < 2; ++e)
-                            acc_dir += u[3 * e] * out[e].x.d + u[3 * e + 1] * out[e].y.d + u[3 * e + 2] * out[e].z.d;
-                        gin[dir] = acc_dir;
+                        gin[dir] = (u0.x * out[0].x.d + u0.y * out[0].y.d + u0.z * out[0].z.d) +
+                                   (u1.x * out[1].x.d + u1.y * out[1].y.d + u1.z * out[1].z.d);
                     }
-                    for (int e = 0; e < 2; ++e)
-                        A.gx[idx[e]] = make_double4(gin[3 * e], gin[3 * e + 1], gin[3 * e + 2], 0.0);
-                    acc[A.b_group[k]] += gin[6] * alphad;
-                }
+                    gx.put(it.idx[0], D3v{gin[0], gin[1], gin[2]});
+                    gx.put(it.idx[1], D3v{gin[3], gin[4], gin[5]});
+                    acc[it.group] += gin[6] * alphad;
+                });
                 break;
-            }
             case ADJ_GRIP: {
-                const bool active = cf.gripTargetAndActive.w > 0.0f;
+                // the first CTA, one thread per grip
+                if (!(cf.gripTargetAndActive.w > 0.0f) || d.g_count == 0u) {
+                    crossed = false;
+                    break;
+                }
+                if (rank != 0u) break;
                 const uint32_t g = threadIdx.x;
                 double gg[6] = {0, 0, 0, 0, 0, 0};
-                if (active && g < d.g_count) {
+                if (g < d.g_count) {
                     const NumiClothGrip grip = d.grips[g];
                     if (grip.particle.y == cf.gripControl.x) {
                         const uint32_t i = grip.particle.x;
@@ -515,12 +646,12 @@ __device__ __forceinline__ void adjoint_segment(const AdjointArgs& A) {
                             const D3v target = addd(D3v{cf.gripTargetAndActive.x, cf.gripTargetAndActive.y,
                                                         cf.gripTargetAndActive.z},
                                                     d3f(ro));
-                            const D3v gout = d3(A.gx[i]);
+                            const D3v gout = gx.get(i);
                             const double w = p.w;
                             const double al = static_cast<double>(grip.targetOffsetAndCompliance.w) / (dtd * dtd);
                             const double dn = w + al;
                             // x' = (alpha x + w T) / (w + alpha)
-                            put(A.gx, i, muld(gout, al / dn));
+                            gx.put(i, muld(gout, al / dn));
                             const D3v gT = muld(gout, w / dn);
                             const D3v xm = subd(d4f(p), target);
                             acc[A.g_group[g]] += dotd(gout, muld(xm, w / (dn * dn))) * al;
@@ -545,73 +676,90 @@ __device__ __forceinline__ void adjoint_segment(const AdjointArgs& A) {
                 break;
             }
             case ADJ_GROUND:
+                crossed = false;
                 if (ground)
-                    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-                        if (radius - pre[i].z > 0.0f) A.gx[i].z = 0.0;
+                    for (uint32_t i = own + threadIdx.x; i < own_end; i += blockDim.x)
+                        if (radius - pre[i].z > 0.0f) {
+                            D3v v = gx.get(i);
+                            v.z = 0.0;
+                            gx.put(i, v);
+                        }
                 break;
             case ADJ_BEGIN: {
                 // x' = x_s + v' dt, v' = (v_s + g dt) / (1 + c dt)
+                crossed = false;
                 const float4* vs = A.tape_v + static_cast<size_t>(si) * n;
                 const double c = A.damping;
                 const double kf = c != 0.0 ? 1.0 / (1.0 + c * dtd) : 1.0;
                 const double dk = -dtd / ((1.0 + c * dtd) * (1.0 + c * dtd));
                 const D3v grav{cf.gravityAndTimestep.x, cf.gravityAndTimestep.y, cf.gravityAndTimestep.z};
-                for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+                for (uint32_t i = own + threadIdx.x; i < own_end; i += blockDim.x) {
                     if (pre[i].w == 0.0f) {
-                        A.gx[i] = make_double4(0, 0, 0, 0);
+                        gx.put(i, D3v{0.0, 0.0, 0.0});
                         A.gv[i] = make_double4(0, 0, 0, 0);
                         continue;
                     }
-                    D3v gpos = d3(A.gx[i]);
+                    D3v gpos = gx.get(i);
                     // swept ground clamp: the predicted z is set to the radius
                     if (ground && pre[i].z >= radius && post[i].z == radius) gpos.z = 0.0;
                     // v' feeds x' and, through friction, the finalize step
+                    const double4 gp = A.gprev[i];
                     D3v gvp = muld(gpos, dtd);
-                    gvp.z += A.gprev[i].w;
+                    gvp.z += gp.w;
                     const D3v v0 = addd(D3v{vs[i].x, vs[i].y, vs[i].z}, muld(grav, dtd));
                     acc[damp_slot] += dotd(gvp, v0) * dk;
                     put(A.gv, i, muld(gvp, kf));
-                    put(A.gx, i, addd(gpos, d3(A.gprev[i])));
+                    gx.put(i, addd(gpos, d3(gp)));
                     A.gprev[i] = make_double4(0, 0, 0, 0);
                 }
                 break;
             }
-            default:
+            default:   // ADJ_TAIL
+                crossed = false;
                 break;
             }
-            __syncthreads();
+            if (crossed) {
+                if (ph.x != ADJ_GRIP) fetch(si, b);
+                sync();
+            } else if (ph.x != ADJ_TAIL) {
+                loose = true;
+            }
         }
     }
-    // fixed-order block reductions
-    __shared__ double s_red[NC_THREADS];
-    __shared__ unsigned int s_rough;
-    if (threadIdx.x == 0) s_rough = 0u;
-    __syncthreads();
-    if (rough) atomicAdd(&s_rough, rough);
+    if constexpr (kShared)
+        for (uint32_t i = own + threadIdx.x; i < own_end; i += blockDim.x) put(A.gx, i, gx.get(i));
+    // fixed-order reductions: each CTA's threads, then the cluster's CTAs
+    __shared__ double s_red[ADJ_THREADS];
+    __shared__ double s_part[ADJ_CLUSTER_MAX][ADJ_MAX_GROUPS + 2u];
+    double* parts = &s_part[rank][0];
+    if (ranks > 1u) parts = static_cast<double*>(__cluster_map_shared_rank(parts, 0u));
     for (uint32_t e = 0; e <= A.groups + 1u; ++e) {
+        __syncthreads();
         s_red[threadIdx.x] = e <= A.groups ? acc[e] : loss;
         __syncthreads();
         for (uint32_t st = blockDim.x / 2u; st > 0u; st >>= 1u) {
             if (threadIdx.x < st) s_red[threadIdx.x] += s_red[threadIdx.x + st];
             __syncthreads();
         }
-        if (threadIdx.x == 0) {
-            if (e <= A.groups)
-                A.grads[e] += s_red[0];
-            else
-                *A.loss += s_red[0];
-        }
-        __syncthreads();
+        if (threadIdx.x == 0) parts[e] = s_red[0];
     }
-    if (threadIdx.x == 0) *A.nonsmooth += s_rough;
+    if (rough) atomicAdd(A.nonsmooth, rough);
+    sync();
+    if (rank == 0u && threadIdx.x <= A.groups + 1u) {
+        double sum = 0.0;
+        for (uint32_t r = 0; r < ranks; ++r) sum += s_part[r][threadIdx.x];
+        if (threadIdx.x <= A.groups)
+            A.grads[threadIdx.x] += sum;
+        else
+            *A.loss += sum;
+    }
 }
 
-// One cloth's segment on one CTA.
-__global__ void __launch_bounds__(NC_THREADS) numi_cloth_adjoint_kernel(AdjointArgs A) { adjoint_segment(A); }
-
-// Many cloths' segments, one CTA each.
-__global__ void __launch_bounds__(NC_THREADS) numi_cloth_adjoint_batch_kernel(const AdjointArgs* args) {
-    adjoint_segment(args[blockIdx.x]);
+// Many cloths' segments, a cluster of CTAs each.
+template <bool kShared>
+__global__ void __launch_bounds__(ADJ_THREADS, 1) numi_cloth_adjoint_kernel(const AdjointArgs* args, uint32_t ranks) {
+    extern __shared__ __align__(16) double nc_adjoint_smem[];
+    adjoint_segment<kShared>(args[blockIdx.x / ranks], blockIdx.x % ranks, ranks, nc_adjoint_smem);
 }
 
 // Device-to-device copies of many regions in one launch, one CTA per

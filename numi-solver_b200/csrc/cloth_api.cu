@@ -2451,24 +2451,108 @@ namespace {
 // Barrier sequence of one substep for the schedules the adjoint supports
 // (one iteration, no reconciliation / final / certificate passes, no air
 // load, no self contact): mirrors nc::substep.
-std::vector<uint2> adjoint_phases(const DeviceCloth& d, const Schedule& s) {
-    std::vector<uint2> ph;
-    ph.push_back(make_uint2(ADJ_BEGIN, 0u));
-    for (uint32_t b = 0; b < d.n_dist_batches; ++b) ph.push_back(make_uint2(ADJ_DIST, b));
-    for (uint32_t b = 0; b < d.n_knot_batches; ++b) ph.push_back(make_uint2(ADJ_KNOT, b));
-    for (uint32_t b = 0; b < d.n_bend_batches; ++b) ph.push_back(make_uint2(ADJ_BEND, b));
-    ph.push_back(make_uint2(ADJ_GRIP, 0u));
+std::vector<uint4> adjoint_phases(const DeviceCloth& d, const Schedule& s) {
+    std::vector<uint4> ph;
+    auto add = [&](uint32_t type, uint32_t first, uint32_t count) { ph.push_back(make_uint4(type, first, count, 0u)); };
+    add(ADJ_BEGIN, 0u, 0u);
+    for (uint32_t b = 0; b < d.n_dist_batches; ++b) add(ADJ_DIST, d.dist_batches[b].first, d.dist_batches[b].count);
+    for (uint32_t b = 0; b < d.n_knot_batches; ++b) add(ADJ_KNOT, d.knot_batches[b].first, d.knot_batches[b].count);
+    for (uint32_t b = 0; b < d.n_bend_batches; ++b) add(ADJ_BEND, d.bend_batches[b].first, d.bend_batches[b].count);
+    add(ADJ_GRIP, 0u, 0u);
     if (d.f_count > 0u)
         for (uint32_t b = 0; b < d.n_dist_batches; ++b)
-            if (d.dist_batches[b].yarn != 0u) ph.push_back(make_uint2(ADJ_YARN, b));
-    ph.push_back(make_uint2(ADJ_GROUND, 0u));
+            if (d.dist_batches[b].yarn != 0u) add(ADJ_YARN, 0u, 0u);
+    add(ADJ_GROUND, 0u, 0u);
     for (uint32_t sw = 0; sw < s.strain_sweeps; ++sw)
         for (uint32_t b = 0; b < d.n_dist_batches; ++b)
-            if (d.dist_batches[b].limited != 0u) ph.push_back(make_uint2(ADJ_STRAIN, b));
-    ph.push_back(make_uint2(ADJ_FINAL, 0u));
+            if (d.dist_batches[b].limited != 0u)
+                add(ADJ_STRAIN, d.dist_batches[b].first, d.dist_batches[b].limited);
+    add(ADJ_FINAL, 0u, 0u);
     // fruit/yarn friction and the fruit tail share the substep's last phase
-    ph.push_back(make_uint2(ADJ_TAIL, 0u));
+    add(ADJ_TAIL, 0u, 0u);
     return ph;
+}
+
+// Launch shape of the reverse sweep of `count` cloths: a cluster of `ranks`
+// CTAs per cloth.  More CTAs shorten a phase until each of its items has a
+// thread of its own (256 items a CTA leave half of its threads for the FP64
+// units to switch between), as long as every cloth keeps its own SMs: one
+// 64 x 64 cloth takes 8, sixteen take 8 each, 96 bags one each.
+struct AdjointShape {
+    uint32_t ranks = 1;
+    bool shared = true;
+    size_t smem = 0;
+};
+
+uint32_t adjoint_shift(uint32_t n, uint32_t ranks) {
+    uint32_t shift = 0;
+    while ((static_cast<uint64_t>(ranks) << shift) < n) ++shift;
+    return shift;
+}
+
+int adjoint_shape(int device, const std::vector<const DeviceCloth*>& cloths, AdjointShape& out) {
+    int optin = 0, sms = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    uint32_t items = 0;
+    for (const DeviceCloth* d : cloths) {
+        for (uint32_t b = 0; b < d->n_dist_batches; ++b) items = std::max(items, d->dist_batches[b].count);
+        for (uint32_t b = 0; b < d->n_knot_batches; ++b) items = std::max(items, d->knot_batches[b].count);
+        for (uint32_t b = 0; b < d->n_bend_batches; ++b) items = std::max(items, d->bend_batches[b].count);
+    }
+    uint32_t ranks = 1;
+    while (ranks < ADJ_CLUSTER_MAX && 256u * ranks < items &&
+           cloths.size() * 2u * ranks <= static_cast<size_t>(std::max(sms, 1)))
+        ranks *= 2u;
+    const void* fns[2] = {reinterpret_cast<const void*>(numi_cloth_adjoint_kernel<true>),
+                          reinterpret_cast<const void*>(numi_cloth_adjoint_kernel<false>)};
+    for (;; ranks /= 2u) {
+        size_t smem = 0;
+        for (const DeviceCloth* d : cloths) {
+            const size_t chunk = static_cast<size_t>(1) << adjoint_shift(d->n, ranks);
+            smem = std::max(smem, std::min<size_t>(chunk, d->n) * 3u * sizeof(double));
+        }
+        cudaFuncAttributes fa{};
+        if (cudaFuncGetAttributes(&fa, fns[0]) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+        out.ranks = ranks;
+        out.shared = smem + fa.sharedSizeBytes <= static_cast<size_t>(optin);
+        out.smem = out.shared ? smem : 0u;
+        const void* fn = fns[out.shared ? 0 : 1];
+        if (out.shared && raise_smem(fn, smem) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+        if (ranks == 1u) return NUMI_CLOTH_OK;
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = ranks;
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(ranks);
+        cfg.blockDim = dim3(ADJ_THREADS);
+        cfg.dynamicSmemBytes = out.smem;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters >= 1) return NUMI_CLOTH_OK;
+        cudaGetLastError();
+    }
+}
+
+cudaError_t adjoint_launch(const AdjointShape& shape, const AdjointArgs* args, uint32_t count, cudaStream_t stream) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = shape.ranks;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(count * shape.ranks);
+    cfg.blockDim = dim3(ADJ_THREADS);
+    cfg.dynamicSmemBytes = shape.smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = shape.ranks > 1u ? 1u : 0u;
+    return shape.shared ? cudaLaunchKernelEx(&cfg, numi_cloth_adjoint_kernel<true>, args, shape.ranks)
+                        : cudaLaunchKernelEx(&cfg, numi_cloth_adjoint_kernel<false>, args, shape.ranks);
 }
 
 // Device allocations of one rollout, freed on scope exit.
@@ -2623,7 +2707,7 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         cudaSuccess)
         return NUMI_CLOTH_ECUDA;
     const Schedule s = device_schedule(sc);
-    const std::vector<uint2> phases = adjoint_phases(h->d, s);
+    const std::vector<uint4> phases = adjoint_phases(h->d, s);
     const uint32_t slots = static_cast<uint32_t>(phases.size()) + 1u;
     const uint32_t n = h->d.n;
     const uint32_t segs = (substeps + checkpoint_every - 1u) / checkpoint_every;
@@ -2641,8 +2725,9 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
     char* ckpt = mem.get<char>((segs + 1u) * state_bytes);
     float4* tape = mem.get<float4>(static_cast<size_t>(checkpoint_every) * slots * n);
     float4* tape_v = mem.get<float4>(static_cast<size_t>(checkpoint_every) * n);
-    uint2* d_phases = mem.get<uint2>(phases.size());
+    uint4* d_phases = mem.get<uint4>(phases.size());
     DeviceCloth* d_cloth = mem.get<DeviceCloth>(1);
+    AdjointArgs* d_args = mem.get<AdjointArgs>(1);
     uint32_t* d_tracked = mem.get<uint32_t>(n_tracked);
     double* d_targets = mem.get<double>(static_cast<size_t>(losses) * n_tracked * 3u);
     double4* gx = mem.get<double4>(n);
@@ -2655,10 +2740,10 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
     uint8_t* gg = mem.get<uint8_t>(groups.g.size());
     double* d_grip = mem.get<double>(static_cast<size_t>(substeps) * 6u);
     unsigned int* d_rough = mem.get<unsigned int>(1);
-    if (!ckpt || !tape || !tape_v || !d_phases || !d_cloth || !d_tracked || !d_targets || !gx || !gv || !gprev ||
+    if (!ckpt || !tape || !tape_v || !d_phases || !d_cloth || !d_args || !d_tracked || !d_targets || !gx || !gv || !gprev ||
         !d_out || !d_grip || !d_rough || !gd || !gk || !gb || !gg)
         return NUMI_CLOTH_ENOMEM;
-    cudaError_t e = cudaMemcpyAsync(d_phases, phases.data(), phases.size() * sizeof(uint2), cudaMemcpyHostToDevice,
+    cudaError_t e = cudaMemcpyAsync(d_phases, phases.data(), phases.size() * sizeof(uint4), cudaMemcpyHostToDevice,
                                     h->stream);
     if (e == cudaSuccess && n_tracked)
         e = cudaMemcpyAsync(d_tracked, tracked, n_tracked * sizeof(uint32_t), cudaMemcpyHostToDevice, h->stream);
@@ -2714,6 +2799,11 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
     // backward: replay each segment on one CTA with the tape, then reverse it
     const float damping = h->d.damping >= 0.0f ? h->d.damping : s.damping;
     const bool resident_one = h->d.resident != 0u && h->grid == 1u;
+    AdjointShape shape;
+    {
+        const int rc = adjoint_shape(h->device, {&h->d}, shape);
+        if (rc != NUMI_CLOTH_OK) return rc;
+    }
     for (uint32_t g = segs; g-- > 0u;) {
         const uint32_t first = g * checkpoint_every;
         const uint32_t count = std::min(checkpoint_every, substeps - first);
@@ -2739,6 +2829,7 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         A.tape_v = tape_v;
         A.phases = d_phases;
         A.slots = slots;
+        A.shift = adjoint_shift(n, shape.ranks);
         A.substeps = count;
         A.first_substep = first;
         A.damping = damping;
@@ -2759,8 +2850,9 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         A.loss = d_out + ngroups + 1u;
         A.grip_grads = d_grip;
         A.nonsmooth = d_rough;
-        numi_cloth_adjoint_kernel<<<1, NC_THREADS, 0, h->stream>>>(A);
-        if (cudaGetLastError() != cudaSuccess) {
+        e = cudaMemcpyAsync(d_args, &A, sizeof(A), cudaMemcpyHostToDevice, h->stream);
+        if (e == cudaSuccess) e = adjoint_launch(shape, d_args, 1u, h->stream);
+        if (e != cudaSuccess || cudaGetLastError() != cudaSuccess) {
             h->poisoned = true;
             return NUMI_CLOTH_ECUDA;
         }
@@ -2796,7 +2888,7 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
 // Batched rollout gradients (numi_cloth_batch_rollout_grad): the forward of
 // every cloth in one persistent launch per segment, the taped replays in one
 // launch per segment, and the adjoint of every cloth's segment in one grid
-// (a CTA per cloth).  Checkpoints are moved by one copy kernel per segment.
+// (a cluster per cloth).  Checkpoints are moved by one copy kernel per segment.
 
 extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiClothConfig* configs, uint32_t substeps,
                                              const NumiClothSchedule* schedule, uint32_t checkpoint_every,
@@ -2834,7 +2926,14 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
     Scratch mem;
     // per cloth: groups, phase list, tape, checkpoints, adjoint arrays
     std::vector<Groups> groups(count);
-    std::vector<std::vector<uint2>> phases(count);
+    std::vector<std::vector<uint4>> phases(count);
+    AdjointShape shape;
+    {
+        std::vector<const DeviceCloth*> all;
+        for (numi_cloth* h : b->cloths) all.push_back(&h->d);
+        const int rc = adjoint_shape(b->device, all, shape);
+        if (rc != NUMI_CLOTH_OK) return rc;
+    }
     std::vector<size_t> state_bytes(count), tape_off(count), ckpt_off(count);
     size_t tape_total = 0, ckpt_total = 0;
     uint32_t max_slots = 0;
@@ -2871,7 +2970,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
     auto round256 = [](size_t v) { return (v + 255u) & ~size_t(255u); };
     size_t arena_bytes = 0;
     for (uint32_t k = 0; k < count; ++k)
-        arena_bytes += round256(phases[k].size() * sizeof(uint2)) + round256(3u * sizeof(double4) * b->cloths[k]->d.n) +
+        arena_bytes += round256(phases[k].size() * sizeof(uint4)) + round256(3u * sizeof(double4) * b->cloths[k]->d.n) +
                        round256(groups[k].d.size() + 1u) + round256(groups[k].k.size() + 1u) +
                        round256(groups[k].b.size() + 1u) + round256(groups[k].g.size() + 1u);
     char* arena = mem.get<char>(arena_bytes);
@@ -2886,13 +2985,13 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         numi_cloth* h = b->cloths[k];
         const uint32_t n = h->d.n;
         const uint32_t slots = static_cast<uint32_t>(phases[k].size()) + 1u;
-        uint2* ph = reinterpret_cast<uint2*>(carve(phases[k].size() * sizeof(uint2)));
+        uint4* ph = reinterpret_cast<uint4*>(carve(phases[k].size() * sizeof(uint4)));
         double4* gx = reinterpret_cast<double4*>(carve(3u * sizeof(double4) * n));
         uint8_t* gd = reinterpret_cast<uint8_t*>(carve(groups[k].d.size() + 1u));
         uint8_t* gk = reinterpret_cast<uint8_t*>(carve(groups[k].k.size() + 1u));
         uint8_t* gb = reinterpret_cast<uint8_t*>(carve(groups[k].b.size() + 1u));
         uint8_t* gg = reinterpret_cast<uint8_t*>(carve(groups[k].g.size() + 1u));
-        e = cudaMemcpyAsync(ph, phases[k].data(), phases[k].size() * sizeof(uint2), cudaMemcpyHostToDevice, b->stream);
+        e = cudaMemcpyAsync(ph, phases[k].data(), phases[k].size() * sizeof(uint4), cudaMemcpyHostToDevice, b->stream);
         const std::vector<uint8_t>* lists[4] = {&groups[k].d, &groups[k].k, &groups[k].b, &groups[k].g};
         uint8_t* dst[4] = {gd, gk, gb, gg};
         for (int f = 0; f < 4 && e == cudaSuccess; ++f)
@@ -2906,6 +3005,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         A.tape_v = A.tape + static_cast<size_t>(checkpoint_every) * slots * n;
         A.phases = ph;
         A.slots = slots;
+        A.shift = adjoint_shift(n, shape.ranks);
         A.damping = h->d.damping >= 0.0f ? h->d.damping : s.damping;
         A.frictions = s.frictions;
         A.tracked = d_tracked;
@@ -3017,7 +3117,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         }
         e = cudaMemcpyAsync(d_args, args.data(), count * sizeof(AdjointArgs), cudaMemcpyHostToDevice, b->stream);
         if (e != cudaSuccess) return NUMI_CLOTH_ECUDA;
-        numi_cloth_adjoint_batch_kernel<<<count, NC_THREADS, 0, b->stream>>>(d_args);
+        if (adjoint_launch(shape, d_args, count, b->stream) != cudaSuccess) return NUMI_CLOTH_ECUDA;
         // args is rewritten next segment: wait for this copy to be consumed
         if (cudaStreamSynchronize(b->stream) != cudaSuccess) {
             for (numi_cloth* h : b->cloths) h->poisoned = true;
