@@ -85,6 +85,73 @@ bool env_u32(const char* name, uint32_t& out) {
 
 }  // namespace
 
+// Typed pieces of one allocation, 256-byte aligned (with a null base the
+// walk only measures).
+struct Carver {
+    char* base;
+    size_t used = 0;
+    template <class T>
+    T* get(size_t count) {
+        T* p = reinterpret_cast<T*>(base + used);
+        used += (count * sizeof(T) + 255u) & ~size_t(255u);
+        return p;
+    }
+};
+
+// Device memory of the rollout gradients of one handle or batch: kept from
+// call to call up to `keep` bytes (an allocation and its release cost more
+// than a small rollout), and freed with its owner; a call that needs more
+// gives it back at its end.
+struct Workspace {
+    size_t keep = size_t(1) << 30;
+    void* mem = nullptr;
+    size_t bytes = 0;
+    Workspace() = default;
+    Workspace(const Workspace&) = delete;
+    Workspace& operator=(const Workspace&) = delete;
+    ~Workspace() { release(); }
+    void release() {
+        if (mem != nullptr) cudaFree(mem);
+        mem = nullptr;
+        bytes = 0;
+    }
+    // One call's use of it.
+    struct Lease {
+        Workspace& w;
+        cudaStream_t stream;
+        Lease(Workspace& space, cudaStream_t s) : w(space), stream(s) {}
+        ~Lease() {
+            if (w.bytes <= w.keep) return;
+            cudaStreamSynchronize(stream);
+            w.release();
+        }
+        // False where the device has no room for the pieces; with `quarter`
+        // also where they would take more than a quarter of what is free.
+        template <class F>
+        bool layout(F&& pieces, bool quarter = false) {
+            Carver measure{nullptr};
+            pieces(measure);
+            if (measure.used > w.bytes) {
+                size_t room = 0, total = 0;
+                if (quarter && cudaMemGetInfo(&room, &total) == cudaSuccess && measure.used > (room + w.bytes) / 4u)
+                    return false;
+                // whatever ran on the old memory has ended
+                if (w.mem != nullptr && cudaStreamSynchronize(stream) != cudaSuccess) return false;
+                w.release();
+                if (cudaMalloc(&w.mem, measure.used) != cudaSuccess) {
+                    cudaGetLastError();
+                    w.mem = nullptr;
+                    return false;
+                }
+                w.bytes = measure.used;
+            }
+            Carver c{static_cast<char*>(w.mem)};
+            pieces(c);
+            return true;
+        }
+    };
+};
+
 struct numi_cloth {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -129,6 +196,8 @@ struct numi_cloth {
     // device staging of particle records for the host copies (one transfer
     // each way, transposed to and from the state arrays on the device)
     NumiClothParticle* io = nullptr;
+    Workspace grad;   // rollout gradients
+    bool rollout_touched = false;   // a fruit touched the cloth in the last rollout
 };
 
 namespace {
@@ -633,12 +702,32 @@ bool tile_schedule(const numi_cloth* h, const Schedule& s) {
            s.primitive_self == 0u && s.reconcile_passes == 0u && s.final_passes == 0u && s.certificate_passes == 0u;
 }
 
-cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t cfg_offset = 0) {
+// Adjoint tape of a launch: [substep][slots][n] positions, [substep][n]
+// velocities.
+struct Tape {
+    float4* x = nullptr;      // null: the launch is not taped
+    float4* v = nullptr;
+    uint32_t slots = 0;
+    uint32_t first = 0;       // substep of the tape the launch starts at
+    uint32_t* touched = nullptr;   // set where a fruit touched the cloth
+};
+
+cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t cfg_offset = 0,
+                   const Tape& tape = {}) {
     DeviceCloth d = h->d;
     d.cfg = h->d_cfg + cfg_offset;
     d.epoch_base = h->epoch;
+    const bool taped = tape.x != nullptr;
+    d.yarn_touched = tape.touched;
+    if (taped) {
+        d.tape = tape.x;
+        d.tape_v = tape.v;
+        d.tape_slots = tape.slots;
+        d.trace = nullptr;
+    }
     Schedule sc = s;
     sc.substeps = substeps;
+    sc.tape_first = tape.first;
     void* args[] = {&d, &sc};
     const bool edge = sc.primitive_self != 0u && d.edge_count != nullptr;
     if (d.trace != nullptr && substeps > h->trace_capacity) d.trace = nullptr;
@@ -679,7 +768,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
         e = cudaLaunchKernelExC(&cfg, frame_fn(edge, h->self_exact), args);
     } else if (h->grid == 1) {
         e = cudaLaunchKernel(frame_fn(edge, h->self_exact), dim3(1), dim3(h->block), args, smem, h->stream);
-    } else if (tile_schedule(h, sc)) {
+    } else if (!taped && tile_schedule(h, sc)) {   // the tape follows the colour-by-colour barriers
         if (h->tiles_dirty) {
             if (!rebuild_tiles(h)) return cudaErrorUnknown;
             h->tiles_dirty = false;
@@ -699,7 +788,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     } else {
         // neighbour syncs between colours (the kernel without the edge/edge
         // phases; its flags start at zero in every launch)
-        if (h->neighbours && !edge) {
+        if (h->neighbours && !edge && !taped) {
             d.nbr_on = 1u;
             e = cudaMemsetAsync(d.nbr_flag, 0, NC_NBR_FLAG_STRIDE * h->grid * sizeof(unsigned int), h->stream);
             if (e != cudaSuccess) return e;
@@ -2066,6 +2155,8 @@ struct numi_cloth_batch {
     bool edge_room = true;             // the shape leaves room for the box tree's sort keys
     uint32_t ctas = 0;
     size_t smem = 0;
+    Workspace grad;   // rollout gradients
+    bool rollout_touched = false;   // a fruit touched a cloth in the last rollout
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     const NumiClothConfig* graph_cfg = nullptr;
@@ -2448,6 +2539,26 @@ int numi_cloth_batch_replay(numi_cloth_batch_t* b) {
 
 namespace {
 
+// Substeps a rollout tapes at once: all of them where the tape fits
+// kTapeBytes, which needs no replay; else as many whole checkpoint intervals
+// as fit, at least one.
+//
+// Where a fruit touches the cloth, the gradient is taken along replays from
+// checkpoints at the caller's interval, as it has always been: a replay meets
+// the forward's contact records of the same substeps and resolves the fruits'
+// friction by them, so its trajectory, and the loss and gradient on it, are
+// not quite the forward's.  Whether one touches shows only as the forward
+// runs.  So a cloth with fruits is taped and checkpointed, and the tape is
+// used where nothing was recorded; a rollout after one that did record does
+// not tape.
+constexpr size_t kTapeBytes = size_t(8) << 30;
+uint32_t taped_substeps(uint32_t substeps, uint32_t checkpoint_every, size_t bytes_per_substep) {
+    const size_t fit = kTapeBytes / std::max<size_t>(bytes_per_substep, 1u);
+    if (substeps <= fit) return substeps;
+    const size_t whole = std::max<size_t>(fit / checkpoint_every, 1u) * checkpoint_every;
+    return static_cast<uint32_t>(std::min<size_t>(whole, substeps));
+}
+
 // Barrier sequence of one substep for the schedules the adjoint supports
 // (one iteration, no reconciliation / final / certificate passes, no air
 // load, no self contact): mirrors nc::substep.
@@ -2554,22 +2665,6 @@ cudaError_t adjoint_launch(const AdjointShape& shape, const AdjointArgs* args, u
     return shape.shared ? cudaLaunchKernelEx(&cfg, numi_cloth_adjoint_kernel<true>, args, shape.ranks)
                         : cudaLaunchKernelEx(&cfg, numi_cloth_adjoint_kernel<false>, args, shape.ranks);
 }
-
-// Device allocations of one rollout, freed on scope exit.
-struct Scratch {
-    std::vector<void*> owned;
-    template <class T>
-    T* get(size_t count) {
-        void* p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) return nullptr;
-        cudaMemset(p, 0, std::max<size_t>(count, 1) * sizeof(T));
-        owned.push_back(p);
-        return static_cast<T*>(p);
-    }
-    ~Scratch() {
-        for (void* p : owned) cudaFree(p);
-    }
-};
 
 // Compliance groups: the distinct compliance values of each constraint
 // family (distance, knot, bend, grip), ascending, numbered family by family.
@@ -2710,7 +2805,6 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
     const std::vector<uint4> phases = adjoint_phases(h->d, s);
     const uint32_t slots = static_cast<uint32_t>(phases.size()) + 1u;
     const uint32_t n = h->d.n;
-    const uint32_t segs = (substeps + checkpoint_every - 1u) / checkpoint_every;
     const uint32_t losses = substeps / loss_every;
 
     Groups groups;
@@ -2719,30 +2813,64 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         if (rc != NUMI_CLOTH_OK) return rc;
     }
     const uint32_t ngroups = static_cast<uint32_t>(groups.value.size());
-    Scratch mem;
     size_t state_bytes = 0;
     for (const auto& r : h->dynamic) state_bytes += (r.bytes + 255u) & ~size_t(255u);
-    char* ckpt = mem.get<char>((segs + 1u) * state_bytes);
-    float4* tape = mem.get<float4>(static_cast<size_t>(checkpoint_every) * slots * n);
-    float4* tape_v = mem.get<float4>(static_cast<size_t>(checkpoint_every) * n);
-    uint4* d_phases = mem.get<uint4>(phases.size());
-    DeviceCloth* d_cloth = mem.get<DeviceCloth>(1);
-    AdjointArgs* d_args = mem.get<AdjointArgs>(1);
-    uint32_t* d_tracked = mem.get<uint32_t>(n_tracked);
-    double* d_targets = mem.get<double>(static_cast<size_t>(losses) * n_tracked * 3u);
-    double4* gx = mem.get<double4>(n);
-    double4* gv = mem.get<double4>(n);
-    double4* gprev = mem.get<double4>(n);
-    double* d_out = mem.get<double>(ngroups + 2u);   // group gradients, damping, loss
-    uint8_t* gd = mem.get<uint8_t>(groups.d.size());
-    uint8_t* gk = mem.get<uint8_t>(groups.k.size());
-    uint8_t* gb = mem.get<uint8_t>(groups.b.size());
-    uint8_t* gg = mem.get<uint8_t>(groups.g.size());
-    double* d_grip = mem.get<double>(static_cast<size_t>(substeps) * 6u);
-    unsigned int* d_rough = mem.get<unsigned int>(1);
-    if (!ckpt || !tape || !tape_v || !d_phases || !d_cloth || !d_args || !d_tracked || !d_targets || !gx || !gv || !gprev ||
-        !d_out || !d_grip || !d_rough || !gd || !gk || !gb || !gg)
-        return NUMI_CLOTH_ENOMEM;
+    // the taped segment, and without a tape of the whole rollout the
+    // checkpoints of the segments before it
+    const size_t tape_step = static_cast<size_t>(slots + 1u) * n * sizeof(float4);
+    uint32_t every = taped_substeps(substeps, checkpoint_every, tape_step);   // substeps on the tape
+    const bool fruits = h->d.f_count > 0u;
+    const uint32_t interval = std::min(checkpoint_every, substeps);
+    if (fruits && (h->rollout_touched || every < substeps)) every = interval;
+    uint32_t seg = 0, segs = 0;   // substeps of a forward launch, their number
+    float4 *tape_x = nullptr, *tape_v = nullptr;
+    char* ckpt = nullptr;
+    uint4* d_phases = nullptr;
+    DeviceCloth* d_cloth = nullptr;
+    AdjointArgs* d_args = nullptr;
+    uint32_t* d_tracked = nullptr;
+    double* d_targets = nullptr;
+    double4 *gx = nullptr, *gv = nullptr, *gprev = nullptr;
+    double *d_out = nullptr, *d_grip = nullptr;   // d_out: group gradients, damping, loss
+    uint8_t *gd = nullptr, *gk = nullptr, *gb = nullptr, *gg = nullptr;
+    unsigned int* d_rough = nullptr;
+    uint32_t* d_touched = nullptr;
+    char* zero_end = nullptr;
+    auto layout = [&](Carver& c) {
+        seg = fruits ? interval : every;
+        segs = (substeps + seg - 1u) / seg;
+        // zeroed
+        gx = c.get<double4>(n);
+        gv = c.get<double4>(n);
+        gprev = c.get<double4>(n);
+        d_out = c.get<double>(ngroups + 2u);
+        d_grip = c.get<double>(static_cast<size_t>(substeps) * 6u);
+        d_rough = c.get<unsigned int>(1);
+        d_touched = c.get<uint32_t>(1);
+        zero_end = c.get<char>(0);
+        // written before they are read
+        d_phases = c.get<uint4>(phases.size());
+        d_cloth = c.get<DeviceCloth>(1);
+        d_args = c.get<AdjointArgs>(1);
+        d_tracked = c.get<uint32_t>(n_tracked);
+        d_targets = c.get<double>(static_cast<size_t>(losses) * n_tracked * 3u);
+        gd = c.get<uint8_t>(groups.d.size());
+        gk = c.get<uint8_t>(groups.k.size());
+        gb = c.get<uint8_t>(groups.b.size());
+        gg = c.get<uint8_t>(groups.g.size());
+        tape_x = c.get<float4>(static_cast<size_t>(every) * slots * n);
+        tape_v = c.get<float4>(static_cast<size_t>(every) * n);
+        if (fruits || segs > 1u) ckpt = c.get<char>((segs + 1u) * state_bytes);
+    };
+    Workspace::Lease mem(h->grad, h->stream);
+    if (!mem.layout(layout, every > checkpoint_every)) {
+        every = interval;
+        if (!mem.layout(layout)) return NUMI_CLOTH_ENOMEM;
+    }
+    if (cudaMemsetAsync(gx, 0, static_cast<size_t>(zero_end - reinterpret_cast<char*>(gx)), h->stream) != cudaSuccess)
+        return NUMI_CLOTH_ECUDA;
+    // the whole rollout on the tape (with fruits only while none touched)
+    bool whole = every == substeps && !(fruits && h->rollout_touched);
     cudaError_t e = cudaMemcpyAsync(d_phases, phases.data(), phases.size() * sizeof(uint4), cudaMemcpyHostToDevice,
                                     h->stream);
     if (e == cudaSuccess && n_tracked)
@@ -2779,14 +2907,20 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         return true;
     };
 
-    // forward in the handle's own launch shape, checkpointing every segment
+    // forward in the handle's own launch shape: taped where the tape holds
+    // it, else checkpointed (the last segment of a cloth without fruits is
+    // taped as it runs)
     std::vector<uint32_t> seg_epoch(segs);
+    auto last_taped = [&](uint32_t g) { return whole || (!fruits && g + 1u == segs); };
     for (uint32_t g = 0; g < segs; ++g) {
-        const uint32_t first = g * checkpoint_every;
-        const uint32_t count = std::min(checkpoint_every, substeps - first);
+        const uint32_t first = g * seg;
+        const uint32_t count = std::min(seg, substeps - first);
         seg_epoch[g] = h->epoch;
-        if (!save(g)) return NUMI_CLOTH_ECUDA;
-        e = launch(h, count, s, first);
+        if ((fruits || g + 1u < segs) && !save(g)) return NUMI_CLOTH_ECUDA;
+        Tape tape;
+        if (last_taped(g)) tape = Tape{tape_x, tape_v, slots, whole ? first : 0u};
+        tape.touched = d_touched;
+        e = launch(h, count, s, first, tape);
         h->epoch += count;
         if (e != cudaSuccess) {
             h->poisoned = true;
@@ -2794,38 +2928,45 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         }
     }
     const uint32_t end_epoch = h->epoch;
-    if (!save(segs)) return NUMI_CLOTH_ECUDA;
-
-    // backward: replay each segment on one CTA with the tape, then reverse it
+    if ((fruits || segs > 1u) && !save(segs)) return NUMI_CLOTH_ECUDA;
+    if (fruits) {
+        uint32_t touched = 0u;
+        if (cudaMemcpyAsync(&touched, d_touched, sizeof(touched), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
+            cudaStreamSynchronize(h->stream) != cudaSuccess) {
+            h->poisoned = true;
+            return NUMI_CLOTH_ECUDA;
+        }
+        h->rollout_touched = touched != 0u;
+        if (touched != 0u) whole = false;
+    }
+    // backward: reverse the tape, or segment by segment after a taped replay
+    // from its checkpoint
     const float damping = h->d.damping >= 0.0f ? h->d.damping : s.damping;
-    const bool resident_one = h->d.resident != 0u && h->grid == 1u;
+    const uint32_t launches = h->launches;
     AdjointShape shape;
     {
         const int rc = adjoint_shape(h->device, {&h->d}, shape);
         if (rc != NUMI_CLOTH_OK) return rc;
     }
-    for (uint32_t g = segs; g-- > 0u;) {
-        const uint32_t first = g * checkpoint_every;
-        const uint32_t count = std::min(checkpoint_every, substeps - first);
-        if (!load(g)) return NUMI_CLOTH_ECUDA;
-        DeviceCloth d = h->d;
-        d.cfg = h->d_cfg + first;
-        d.epoch_base = seg_epoch[g];
-        d.trace = nullptr;
-        d.trace_cta = nullptr;
-        d.cluster_barrier = 0u;
-        d.resident = resident_one ? 1u : 0u;
-        d.tape = tape;
-        d.tape_v = tape_v;
-        d.tape_slots = slots;
-        Schedule st = s;
-        st.substeps = count;
-        const size_t smem = resident_one ? h->smem : nc_resident_offset();
-        numi_cloth_frame_kernel<<<1, h->block, smem, h->stream>>>(d, st);
+    bool replayed = false;
+    for (uint32_t g = whole ? 1u : segs; g-- > 0u;) {
+        const uint32_t first = g * seg;
+        const uint32_t count = whole ? substeps : std::min(seg, substeps - first);
+        if (!last_taped(g)) {
+            replayed = true;
+            if (!load(g)) return NUMI_CLOTH_ECUDA;
+            h->epoch = seg_epoch[g];
+            e = launch(h, count, s, first, Tape{tape_x, tape_v, slots});
+            h->epoch = end_epoch;
+            if (e != cudaSuccess) {
+                h->poisoned = true;
+                return NUMI_CLOTH_ECUDA;
+            }
+        }
         AdjointArgs A{};
         A.cloth = d_cloth;
         A.cfg = h->d_cfg + first;
-        A.tape = tape;
+        A.tape = tape_x;
         A.tape_v = tape_v;
         A.phases = d_phases;
         A.slots = slots;
@@ -2856,16 +2997,18 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
             h->poisoned = true;
             return NUMI_CLOTH_ECUDA;
         }
-        uint32_t barriers = 0;
-        if (cudaMemcpyAsync(&barriers, h->d.stats, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
-            cudaStreamSynchronize(h->stream) != cudaSuccess) {
-            h->poisoned = true;
-            return NUMI_CLOTH_ECUDA;
-        }
-        if (barriers + 1u != slots) return NUMI_CLOTH_ESTATE;   // the phase list does not match the kernel
     }
-    if (!load(segs)) return NUMI_CLOTH_ECUDA;
+    if (replayed && !load(segs)) return NUMI_CLOTH_ECUDA;
     h->epoch = end_epoch;
+    h->launches = launches;
+    h->last_substeps = substeps;
+    uint32_t barriers = 0;
+    if (cudaMemcpyAsync(&barriers, h->d.stats, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess ||
+        cudaStreamSynchronize(h->stream) != cudaSuccess) {
+        h->poisoned = true;
+        return NUMI_CLOTH_ECUDA;
+    }
+    if (barriers + 1u != slots) return NUMI_CLOTH_ESTATE;   // the phase list does not match the kernel
     std::vector<double> out(ngroups + 2u);
     unsigned int rough = 0;
     e = cudaMemcpyAsync(out.data(), d_out, out.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
@@ -2920,10 +3063,8 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
                                     cudaMemcpyHostToDevice, b->stream);
     if (e != cudaSuccess) return NUMI_CLOTH_ECUDA;
     const Schedule s = device_schedule(sc);
-    const uint32_t segs = (substeps + checkpoint_every - 1u) / checkpoint_every;
     const uint32_t losses = substeps / loss_every;
 
-    Scratch mem;
     // per cloth: groups, phase list, tape, checkpoints, adjoint arrays
     std::vector<Groups> groups(count);
     std::vector<std::vector<uint4>> phases(count);
@@ -2934,48 +3075,79 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         const int rc = adjoint_shape(b->device, all, shape);
         if (rc != NUMI_CLOTH_OK) return rc;
     }
-    std::vector<size_t> state_bytes(count), tape_off(count), ckpt_off(count);
-    size_t tape_total = 0, ckpt_total = 0;
-    uint32_t max_slots = 0;
+    std::vector<size_t> state_bytes(count);
+    size_t tape_step = 0, state_total = 0;   // float4s a substep tapes, bytes of a checkpoint
+    uint32_t regions = 0;
     for (uint32_t k = 0; k < count; ++k) {
         numi_cloth* h = b->cloths[k];
         const int rc = compliance_groups(h, groups[k]);
         if (rc != NUMI_CLOTH_OK) return rc;
         phases[k] = adjoint_phases(h->d, s);
-        const uint32_t slots = static_cast<uint32_t>(phases[k].size()) + 1u;
-        max_slots = std::max(max_slots, slots);
-        tape_off[k] = tape_total;
-        tape_total += static_cast<size_t>(checkpoint_every) * (slots + 1u) * h->d.n;   // positions + velocities
-        size_t bytes = 0;
-        for (const auto& r : h->dynamic) bytes += (r.bytes + 255u) & ~size_t(255u);
-        state_bytes[k] = bytes;
-        ckpt_off[k] = ckpt_total;
-        ckpt_total += (segs + 1u) * bytes;
+        tape_step += (phases[k].size() + 2u) * h->d.n;   // positions + velocities
+        for (const auto& r : h->dynamic) state_bytes[k] += (r.bytes + 255u) & ~size_t(255u);
+        state_total += state_bytes[k];
+        regions += static_cast<uint32_t>(h->dynamic.size());
     }
-    float4* tape = mem.get<float4>(tape_total);
-    char* ckpt = mem.get<char>(ckpt_total);
-    uint32_t* d_tracked = mem.get<uint32_t>(n_tracked);
-    double* d_targets = mem.get<double>(static_cast<size_t>(count) * losses * n_tracked * 3u);
-    double* d_out = mem.get<double>(static_cast<size_t>(count) * (NUMI_CLOTH_MAX_GROUPS + 2u));
-    unsigned int* d_rough = mem.get<unsigned int>(count);
-    DeviceCloth* d_replay = mem.get<DeviceCloth>(count);   // launch order, tape set
-    DeviceCloth* d_plain = mem.get<DeviceCloth>(count);    // caller order, for the adjoint
-    AdjointArgs* d_args = mem.get<AdjointArgs>(count);
-    CopyOp* d_save = mem.get<CopyOp>(static_cast<size_t>(count) * 16u);
-    if (!tape || !ckpt || !d_tracked || !d_targets || !d_out || !d_rough || !d_replay || !d_plain || !d_args || !d_save)
-        return NUMI_CLOTH_ENOMEM;
-    std::vector<AdjointArgs> args(count);
-    std::vector<DeviceCloth> replay(count), plain(count);
-    // one arena for every cloth's phase list, adjoint arrays and group ids
+    uint32_t every = taped_substeps(substeps, checkpoint_every, tape_step * sizeof(float4));   // substeps on the tape
+    bool fruits = false;
+    for (numi_cloth* h : b->cloths) fruits = fruits || h->d.f_count > 0u;
+    const uint32_t interval = std::min(checkpoint_every, substeps);
+    if (fruits && (b->rollout_touched || every < substeps)) every = interval;
+    uint32_t seg = 0, segs = 0;   // substeps of a forward launch, their number
+    uint32_t* d_touched = nullptr;
+    float4* tape = nullptr;
+    char *ckpt = nullptr, *arena = nullptr, *zero = nullptr, *zero_end = nullptr;
+    uint32_t* d_tracked = nullptr;
+    double *d_targets = nullptr, *d_out = nullptr;
+    unsigned int* d_rough = nullptr;
+    DeviceCloth *d_replay = nullptr, *d_plain = nullptr;   // launch order with the tape; caller order for the adjoint
+    AdjointArgs* d_args = nullptr;
+    CopyOp* d_ops = nullptr;
+    std::vector<double4*> adjoint(count);   // a cloth's gx, gv and gprev
+    // one arena for every cloth's phase list and group ids
     auto round256 = [](size_t v) { return (v + 255u) & ~size_t(255u); };
     size_t arena_bytes = 0;
     for (uint32_t k = 0; k < count; ++k)
-        arena_bytes += round256(phases[k].size() * sizeof(uint4)) + round256(3u * sizeof(double4) * b->cloths[k]->d.n) +
-                       round256(groups[k].d.size() + 1u) + round256(groups[k].k.size() + 1u) +
-                       round256(groups[k].b.size() + 1u) + round256(groups[k].g.size() + 1u);
-    char* arena = mem.get<char>(arena_bytes);
-    if (!arena) return NUMI_CLOTH_ENOMEM;
+        arena_bytes += round256(phases[k].size() * sizeof(uint4)) + round256(groups[k].d.size() + 1u) +
+                       round256(groups[k].k.size() + 1u) + round256(groups[k].b.size() + 1u) +
+                       round256(groups[k].g.size() + 1u);
+    auto layout = [&](Carver& c) {
+        seg = fruits ? interval : every;
+        segs = (substeps + seg - 1u) / seg;
+        // zeroed
+        zero = c.get<char>(0);
+        for (uint32_t k = 0; k < count; ++k) adjoint[k] = c.get<double4>(3u * static_cast<size_t>(b->cloths[k]->d.n));
+        d_out = c.get<double>(static_cast<size_t>(count) * (NUMI_CLOTH_MAX_GROUPS + 2u));
+        d_rough = c.get<unsigned int>(count);
+        d_touched = c.get<uint32_t>(1);
+        zero_end = c.get<char>(0);
+        // written before they are read
+        arena = c.get<char>(arena_bytes);
+        d_tracked = c.get<uint32_t>(n_tracked);
+        d_targets = c.get<double>(static_cast<size_t>(count) * losses * n_tracked * 3u);
+        d_replay = c.get<DeviceCloth>(count);
+        d_plain = c.get<DeviceCloth>(count);
+        d_args = c.get<AdjointArgs>(count);
+        tape = c.get<float4>(tape_step * every);
+        if (fruits || segs > 1u) {
+            d_ops = c.get<CopyOp>(2u * static_cast<size_t>(segs + 1u) * regions);
+            ckpt = c.get<char>((segs + 1u) * state_total);
+        }
+    };
+    b->grad.keep = kTapeBytes + (kTapeBytes >> 3);
+    Workspace::Lease mem(b->grad, b->stream);
+    if (!mem.layout(layout, every > checkpoint_every)) {
+        every = interval;
+        if (!mem.layout(layout)) return NUMI_CLOTH_ENOMEM;
+    }
+    // the whole rollout on the tape (with fruits only while none touched)
+    bool whole = every == substeps && !(fruits && b->rollout_touched);
+    if (cudaMemsetAsync(zero, 0, static_cast<size_t>(zero_end - zero), b->stream) != cudaSuccess)
+        return NUMI_CLOTH_ECUDA;
+    std::vector<AdjointArgs> args(count);
+    std::vector<DeviceCloth> replay(count), plain(count);
     size_t cursor = 0;
+    float4* tape_at = tape;
     auto carve = [&](size_t bytes) {
         char* p = arena + cursor;
         cursor += round256(bytes);
@@ -2986,7 +3158,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         const uint32_t n = h->d.n;
         const uint32_t slots = static_cast<uint32_t>(phases[k].size()) + 1u;
         uint4* ph = reinterpret_cast<uint4*>(carve(phases[k].size() * sizeof(uint4)));
-        double4* gx = reinterpret_cast<double4*>(carve(3u * sizeof(double4) * n));
+        double4* gx = adjoint[k];
         uint8_t* gd = reinterpret_cast<uint8_t*>(carve(groups[k].d.size() + 1u));
         uint8_t* gk = reinterpret_cast<uint8_t*>(carve(groups[k].k.size() + 1u));
         uint8_t* gb = reinterpret_cast<uint8_t*>(carve(groups[k].b.size() + 1u));
@@ -3001,8 +3173,9 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         plain[k] = h->d;
         AdjointArgs& A = args[k];
         A.cloth = d_plain + k;
-        A.tape = tape + tape_off[k];
-        A.tape_v = A.tape + static_cast<size_t>(checkpoint_every) * slots * n;
+        A.tape = tape_at;
+        A.tape_v = A.tape + static_cast<size_t>(every) * slots * n;
+        tape_at += static_cast<size_t>(every) * (slots + 1u) * n;
         A.phases = ph;
         A.slots = slots;
         A.shift = adjoint_shift(n, shape.ranks);
@@ -3036,6 +3209,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
             replay[j].tape = const_cast<float4*>(args[k].tape);
             replay[j].tape_v = const_cast<float4*>(args[k].tape_v);
             replay[j].tape_slots = args[k].slots;
+        replay[j].yarn_touched = d_touched;
         }
     }
     e = cudaMemcpyAsync(d_replay, replay.data(), count * sizeof(DeviceCloth), cudaMemcpyHostToDevice, b->stream);
@@ -3050,24 +3224,18 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
     // one copy kernel per checkpoint move: op tables for save (state ->
     // checkpoint) and load (checkpoint -> state) of every slot
     std::vector<CopyOp> save_ops, load_ops;
-    uint32_t regions = 0;
-    for (numi_cloth* h : b->cloths) regions += static_cast<uint32_t>(h->dynamic.size());
-    CopyOp* d_ops = mem.get<CopyOp>(2u * static_cast<size_t>(segs + 1u) * regions);
-    if (!d_ops) return NUMI_CLOTH_ENOMEM;
-    for (uint32_t g = 0; g <= segs; ++g) {
-        for (uint32_t k = 0; k < count; ++k) {
-            numi_cloth* h = b->cloths[k];
-            size_t off = 0;
+    const bool checkpoints = fruits || segs > 1u;
+    for (uint32_t g = 0; checkpoints && g <= segs; ++g) {
+        char* slot = ckpt + g * state_total;
+        for (numi_cloth* h : b->cloths)
             for (const auto& r : h->dynamic) {
-                char* slot = ckpt + ckpt_off[k] + g * state_bytes[k] + off;
                 save_ops.push_back(CopyOp{r.ptr, slot, r.bytes});
                 load_ops.push_back(CopyOp{slot, r.ptr, r.bytes});
-                off += (r.bytes + 255u) & ~size_t(255u);
+                slot += (r.bytes + 255u) & ~size_t(255u);
             }
-        }
     }
-    e = cudaMemcpyAsync(d_ops, save_ops.data(), save_ops.size() * sizeof(CopyOp), cudaMemcpyHostToDevice, b->stream);
-    if (e == cudaSuccess)
+    if (checkpoints) e = cudaMemcpyAsync(d_ops, save_ops.data(), save_ops.size() * sizeof(CopyOp), cudaMemcpyHostToDevice, b->stream);
+    if (checkpoints && e == cudaSuccess)
         e = cudaMemcpyAsync(d_ops + save_ops.size(), load_ops.data(), load_ops.size() * sizeof(CopyOp),
                             cudaMemcpyHostToDevice, b->stream);
     if (e != cudaSuccess) return NUMI_CLOTH_ECUDA;
@@ -3080,36 +3248,51 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
                cudaStreamSynchronize(b->stream) == cudaSuccess;
     };
 
-    // forward
-    std::vector<uint32_t> seg_epoch(segs);
+    // one segment of every cloth, taped (from tape_first on) or not
+    auto step = [&](uint32_t g, bool taped, uint32_t tape_first) {
+        const uint32_t first = g * seg;
+        Schedule st = s;
+        st.substeps = std::min(seg, substeps - first);
+        st.cfg_offset = first;
+        st.epoch_ptr = b->epoch;
+        st.tape_first = tape_first;
+        cudaMemsetAsync(b->queue, 0, sizeof(unsigned int), b->stream);
+        numi_cloth_batch_kernel<<<b->ctas, b->block, b->smem, b->stream>>>(taped ? d_replay : b->d_cloths, count, st,
+                                                                         b->queue);
+        return cudaGetLastError() == cudaSuccess;
+    };
+    // forward: taped where the tape holds it, else checkpointed (the last
+    // segment of cloths without fruits is taped as it runs)
     const uint32_t epoch0 = b->epoch_host;
     if (!set_epoch(epoch0)) return NUMI_CLOTH_ECUDA;
+    auto last_taped = [&](uint32_t g) { return whole || (!fruits && g + 1u == segs); };
     for (uint32_t g = 0; g < segs; ++g) {
-        const uint32_t first = g * checkpoint_every;
-        const uint32_t cnt = std::min(checkpoint_every, substeps - first);
-        seg_epoch[g] = epoch0 + first;
-        move(true, g);
-        Schedule st = s;
-        st.substeps = cnt;
-        st.cfg_offset = first;
-        st.epoch_ptr = b->epoch;
-        cudaMemsetAsync(b->queue, 0, sizeof(unsigned int), b->stream);
-        numi_cloth_batch_kernel<<<b->ctas, b->block, b->smem, b->stream>>>(b->d_cloths, count, st, b->queue);
-        numi_cloth_epoch_kernel<<<1, 1, 0, b->stream>>>(b->epoch, cnt);
+        if (fruits || g + 1u < segs) move(true, g);
+        if (!step(g, last_taped(g), whole ? g * seg : 0u)) return NUMI_CLOTH_ECUDA;
+        numi_cloth_epoch_kernel<<<1, 1, 0, b->stream>>>(b->epoch, std::min(seg, substeps - g * seg));
     }
-    move(true, segs);
-    // backward
-    for (uint32_t g = segs; g-- > 0u;) {
-        const uint32_t first = g * checkpoint_every;
-        const uint32_t cnt = std::min(checkpoint_every, substeps - first);
-        move(false, g);
-        if (!set_epoch(seg_epoch[g])) return NUMI_CLOTH_ECUDA;
-        Schedule st = s;
-        st.substeps = cnt;
-        st.cfg_offset = first;
-        st.epoch_ptr = b->epoch;
-        cudaMemsetAsync(b->queue, 0, sizeof(unsigned int), b->stream);
-        numi_cloth_batch_kernel<<<b->ctas, b->block, b->smem, b->stream>>>(d_replay, count, st, b->queue);
+    if (checkpoints) move(true, segs);
+    if (fruits && whole) {
+        uint32_t touched = 0u;
+        if (cudaMemcpyAsync(&touched, d_touched, sizeof(touched), cudaMemcpyDeviceToHost, b->stream) != cudaSuccess ||
+            cudaStreamSynchronize(b->stream) != cudaSuccess) {
+            for (numi_cloth* h : b->cloths) h->poisoned = true;
+            return NUMI_CLOTH_ECUDA;
+        }
+        b->rollout_touched = touched != 0u;
+        if (touched != 0u) whole = false;
+    }
+    // backward: reverse the tape, or segment by segment after a taped replay
+    // from its checkpoint
+    bool replayed = false;
+    for (uint32_t g = whole ? 1u : segs; g-- > 0u;) {
+        const uint32_t first = g * seg;
+        const uint32_t cnt = whole ? substeps : std::min(seg, substeps - first);
+        if (!last_taped(g)) {
+            replayed = true;
+            move(false, g);
+            if (!set_epoch(epoch0 + first) || !step(g, true, 0u)) return NUMI_CLOTH_ECUDA;
+        }
         for (uint32_t k = 0; k < count; ++k) {
             args[k].cfg = b->d_cfg + static_cast<size_t>(k) * substeps + first;
             args[k].substeps = cnt;
@@ -3124,7 +3307,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
             return NUMI_CLOTH_ECUDA;
         }
     }
-    move(false, segs);
+    if (replayed) move(false, segs);
     const uint32_t end_epoch = epoch0 + substeps;
     if (!set_epoch(end_epoch)) return NUMI_CLOTH_ECUDA;
     b->epoch_host = end_epoch;
@@ -3134,6 +3317,9 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
     }
     std::vector<double> out(static_cast<size_t>(count) * (NUMI_CLOTH_MAX_GROUPS + 2u));
     std::vector<unsigned int> rough(count);
+    uint32_t touched = 0u;
+    e = cudaMemcpyAsync(&touched, d_touched, sizeof(touched), cudaMemcpyDeviceToHost, b->stream);
+    if (e != cudaSuccess) return NUMI_CLOTH_ECUDA;
     e = cudaMemcpyAsync(out.data(), d_out, out.size() * sizeof(double), cudaMemcpyDeviceToHost, b->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(rough.data(), d_rough, count * sizeof(unsigned int), cudaMemcpyDeviceToHost, b->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
@@ -3141,6 +3327,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         for (numi_cloth* h : b->cloths) h->poisoned = true;
         return NUMI_CLOTH_ECUDA;
     }
+    b->rollout_touched = touched != 0u;   // (replays see the forward's contacts too)
     for (uint32_t k = 0; k < count; ++k) {
         const double* o = out.data() + static_cast<size_t>(k) * (NUMI_CLOTH_MAX_GROUPS + 2u);
         for (uint32_t q = 0; q <= NUMI_CLOTH_MAX_GROUPS; ++q) grads[static_cast<size_t>(k) * (NUMI_CLOTH_MAX_GROUPS + 1u) + q] = o[q];

@@ -250,12 +250,14 @@ struct DeviceCloth {
     // largest displacement since the build, [2 CTAs, 3 CTAs) largest motion
     // over the substep
     double* edge_red;
-    // adjoint tape (one-CTA launches only): positions at the start of every
+    // adjoint tape: positions at the start of every
     // substep and after every barrier, [substep][tape_slots][n], and
     // velocities at the start of every substep, [substep][n]
     float4* tape;
     float4* tape_v;
     uint32_t tape_slots;
+    // set to 1 by a segment that records a fruit/yarn contact (null: not asked)
+    uint32_t* yarn_touched;
     // tile mode of the cooperative grid (cloth_tile.cuh): CTA r's plan is
     // tile_words[tile_off[r] .. tile_off[r + 1]); tile_owner[i] = (owning
     // CTA << 16) | local index of particle i; positions and velocities
@@ -293,6 +295,8 @@ struct Schedule {
     const uint32_t* epoch_ptr;
     // first Config of the launch within DeviceCloth::cfg
     uint32_t cfg_offset;
+    // place of the launch's first substep on DeviceCloth::tape
+    uint32_t tape_first;
     // 1: the launch runs in tile mode (cloth_tile.cuh)
     uint32_t tiles;
     // edge/edge launches: byte offset in dynamic shared memory of the box

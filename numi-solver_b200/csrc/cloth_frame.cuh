@@ -20,41 +20,16 @@ namespace {   // internal linkage: the edge kernels' unit includes these too
 // ends with a CTA barrier, so they share one array.
 __shared__ __align__(16) double nc_red_smem[3][NC_BLOCK_MAX];
 
-// Grid-wide barrier with a bounded wait.  Arrival is a release-add of 1 to
-// a counter the host zeroes before each launch; barrier number s of the
-// launch completes when an acquire load sees s times the number of CTAs on
-// the cloth.  A CTA that waits past the limit
-// raises TIMEOUT and the abort flag, and every CTA leaves at its next
-// barrier (or as soon as it sees the flag while waiting).
-__device__ bool grid_sync(Ctx& ctx) {
+// Arrival and bounded wait of one barrier of the cooperative grid.  Arrival
+// is a release-add of 1 to a counter the host zeroes before each launch;
+// barrier number s of the launch completes when an acquire load sees s times
+// the number of CTAs on the cloth.  A CTA that waits past the limit raises
+// TIMEOUT and the abort flag, and every CTA leaves at its next barrier (or as
+// soon as it sees the flag while waiting).
+__device__ __forceinline__ bool grid_wait(Ctx& ctx) {
     const DeviceCloth& d = ctx.d;
-    ++ctx.barriers;
-    ++ctx.seq;
-    if (d.trace_cta && ctx.barriers <= NC_TRACE_SLOTS) {
-        __syncthreads();
-        if (threadIdx.x == 0)
-            d.trace_cta[(static_cast<size_t>(ctx.sub) * NC_TRACE_SLOTS + ctx.barriers - 1u) * ctx.ranks + ctx.rank] =
-                globaltimer();
-    }
-    if (d.cluster_barrier) {
-        cooperative_groups::this_cluster().sync();
-        if (d.trace && ctx.rank == 0 && threadIdx.x == 0 && ctx.barriers <= NC_TRACE_SLOTS)
-            d.trace[static_cast<size_t>(ctx.sub) * NC_TRACE_SLOTS + ctx.barriers - 1u] = globaltimer();
-        return true;
-    }
-    if (ctx.ranks == 1) {
-        __syncthreads();
-        if (d.tape != nullptr && ctx.barriers < d.tape_slots) {
-            // adjoint tape: positions after this barrier
-            float4* slot = d.tape + (static_cast<size_t>(ctx.sub) * d.tape_slots + ctx.barriers) * d.n;
-            for (uint32_t i = threadIdx.x; i < d.n; i += blockDim.x) slot[i] = px(ctx, i);
-            __syncthreads();
-        }
-        if (d.trace && threadIdx.x == 0 && ctx.barriers <= NC_TRACE_SLOTS)
-            d.trace[static_cast<size_t>(ctx.sub) * NC_TRACE_SLOTS + ctx.barriers - 1u] = globaltimer();
-        return true;
-    }
     __shared__ unsigned s_abort;
+    ++ctx.seq;
     __syncthreads();
     if (threadIdx.x == 0) {
         const unsigned long long target = ctx.seq * (ctx.ranks + d.bar_phantom);
@@ -82,11 +57,46 @@ __device__ bool grid_sync(Ctx& ctx) {
         // orders the CTA's other threads after this thread
         if (!ab) (void)ld_acquire_u64(d.bar_count);
         s_abort = ab;
-        if (d.trace && ctx.rank == 0 && ctx.barriers <= NC_TRACE_SLOTS)
-            d.trace[static_cast<size_t>(ctx.sub) * NC_TRACE_SLOTS + ctx.barriers - 1u] = globaltimer();
     }
     __syncthreads();
     return s_abort == 0u;
+}
+
+// Adjoint tape: the CTA's particles after barrier ctx.barriers of the
+// substep (0: at its start).
+__device__ __forceinline__ void tape_store(const Ctx& ctx) {
+    const DeviceCloth& d = ctx.d;
+    if (ctx.barriers >= d.tape_slots) return;
+    float4* slot = d.tape + (static_cast<size_t>(ctx.s.tape_first + ctx.sub) * d.tape_slots + ctx.barriers) * d.n;
+    for (Range r = particle_range(ctx); r.i < r.end; r.i += r.stride) slot[r.i] = px(ctx, r.i);
+}
+
+// Barrier between two phases, over whatever the cloth runs on: one CTA, one
+// cluster (the hardware barrier) or the cooperative grid.  A taped launch
+// passes it twice, with the tape's stores between, since a CTA's particles
+// may be another's to move in the next phase.
+__device__ __forceinline__ bool grid_sync(Ctx& ctx) {
+    const DeviceCloth& d = ctx.d;
+    ++ctx.barriers;
+    if (d.trace_cta && ctx.barriers <= NC_TRACE_SLOTS) {
+        __syncthreads();
+        if (threadIdx.x == 0)
+            d.trace_cta[(static_cast<size_t>(ctx.sub) * NC_TRACE_SLOTS + ctx.barriers - 1u) * ctx.ranks + ctx.rank] =
+                globaltimer();
+    }
+    for (bool taped = d.tape != nullptr;; taped = false) {
+        if (d.cluster_barrier)
+            cooperative_groups::this_cluster().sync();
+        else if (ctx.ranks == 1)
+            __syncthreads();
+        else if (!grid_wait(ctx))
+            return false;
+        if (!taped) break;
+        tape_store(ctx);
+    }
+    if (d.trace && ctx.rank == 0 && threadIdx.x == 0 && ctx.barriers <= NC_TRACE_SLOTS)
+        d.trace[static_cast<size_t>(ctx.sub) * NC_TRACE_SLOTS + ctx.barriers - 1u] = globaltimer();
+    return true;
 }
 
 #define NC_SYNC(ctx) \
@@ -557,6 +567,7 @@ struct SegRecords {
 
     __device__ void finish(const Ctx& ctx) const {
         if (!recorded) return;
+        if (ctx.d.yarn_touched != nullptr) *ctx.d.yarn_touched = 1u;
         ctx.d.yarn_live[seg] = ctx.epoch;
         // first record of the substep: the segment joins the friction list
         if (!was_live) ctx.d.yarn_list[atomicAdd(ctx.d.yarn_list_n, 1u)] = seg;
@@ -684,7 +695,7 @@ __device__ __forceinline__ bool yarn_warp_contacts(const Ctx& ctx, bool valid, b
 // colour stages them in shared memory for all colours, the CTA's
 // displacement sums accumulate over the sweep, and the last colour adds
 // them to the global sums.
-__device__ void yarn_contact_batch(Ctx& ctx, uint32_t slot, const Batch& bt, bool first, bool last) {
+__device__ __forceinline__ void yarn_contact_batch(Ctx& ctx, uint32_t slot, const Batch& bt, bool first, bool last) {
     const DeviceCloth& d = ctx.d;
     __shared__ float4 s_fruit[NC_MAX_FRUITS];   // xyz position, w radius
     __shared__ float s_fw[NC_MAX_FRUITS];
@@ -735,7 +746,7 @@ __device__ void yarn_contact_batch(Ctx& ctx, uint32_t slot, const Batch& bt, boo
 // segment visiting the fruits in ascending order, fruit displacements summed.
 // A fruit whose swept box is farther than the contact distance from the
 // segment's swept box cannot be found by the advancement and is skipped.
-__device__ void swept_contact_batch(Ctx& ctx, const Batch& bt, bool first, bool last) {
+__device__ __forceinline__ void swept_contact_batch(Ctx& ctx, const Batch& bt, bool first, bool last) {
     const DeviceCloth& d = ctx.d;
     const SubCfg& c = ctx.c;
     __shared__ float4 s_fx[NC_MAX_FRUITS];   // position xyz, radius
@@ -828,7 +839,7 @@ __device__ void swept_contact_batch(Ctx& ctx, const Batch& bt, bool first, bool 
     if (last) cta_sums_flush(s_sum, acc, 3u * nf);
 }
 
-__device__ bool yarn_sweep(Ctx& ctx) {
+__device__ __forceinline__ bool yarn_sweep(Ctx& ctx) {
     if (ctx.d.f_count == 0u) return true;
     fruit_flush(ctx);
     uint32_t first = NC_MAX_BATCHES, last = 0;
@@ -1928,7 +1939,7 @@ __device__ void fruit_ground(Ctx& ctx) {
 }
 
 template <bool kIlp>
-__device__ bool strain_sweeps(Ctx& ctx) {
+__device__ __forceinline__ bool strain_sweeps(Ctx& ctx) {
     const DeviceCloth& d = ctx.d;
     for (uint32_t sw = 0; sw < ctx.s.strain_sweeps; ++sw) {
         if constexpr (kIlp) {
@@ -2051,7 +2062,7 @@ __device__ bool residuals_converged(Ctx& ctx) {
 }
 
 template <bool kIlp>
-__device__ bool contacts_pass(Ctx& ctx, bool with_strain) {
+__device__ __forceinline__ bool contacts_pass(Ctx& ctx, bool with_strain) {
     // fruit pairs (fruit CTA) -> fruit/yarn -> [strain] -> ground
     if (ctx.fruit_cta && ctx.d.p_count > 0u) {
         fruit_flush(ctx);
@@ -2954,13 +2965,12 @@ __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule
         ctx.c = nc::load_cfg(d.cfg + s.cfg_offset + sub);
         ctx.epoch = epoch_base + sub;
         ctx.barriers = 0;
-        if (d.tape != nullptr && ranks == 1u) {
-            // adjoint tape: state at the start of the substep
-            float4* slot = d.tape + static_cast<size_t>(sub) * d.tape_slots * d.n;
-            for (uint32_t i = threadIdx.x; i < d.n; i += blockDim.x) {
-                slot[i] = px(ctx, i);
-                d.tape_v[static_cast<size_t>(sub) * d.n + i] = pv(ctx, i);
-            }
+        if (d.tape != nullptr) {
+            // adjoint tape: state at the start of the substep (its first
+            // phase moves a CTA's own particles, thread by thread as here)
+            nc::tape_store(ctx);
+            for (nc::Range r = nc::particle_range(ctx); r.i < r.end; r.i += r.stride)
+                d.tape_v[static_cast<size_t>(s.tape_first + sub) * d.n + r.i] = pv(ctx, r.i);
             __syncthreads();
         }
         if constexpr (!kEdge && !kIlp) {
