@@ -463,7 +463,10 @@ int numi_cloth_batch_step(numi_cloth_batch_t* batch, const NumiClothConfig* conf
 
 /* Launch shape: out[0] resident particle chunk (cloths with at most that
  * many particles keep them in shared memory; 0 = none), out[1] threads per
- * CTA, out[2] CTAs of the persistent launch. */
+ * CTA, out[2] CTAs of the persistent launch.  The shape of a new batch is
+ * fitted to its cloths (particles in shared memory as far as they fit, a
+ * cluster of CTAs per cloth where there are SMs to spare); set_shape and
+ * tune replace it. */
 int numi_cloth_batch_shape(numi_cloth_batch_t* batch, uint32_t out[3]);
 /* A shape whose resident chunk leaves no shared memory for the edge/edge
  * family's box-tree sort keys (32 KB) serves only schedules with
@@ -471,8 +474,8 @@ int numi_cloth_batch_shape(numi_cloth_batch_t* batch, uint32_t out[3]);
  * on it, and the tuner skips it for such schedules. */
 int numi_cloth_batch_set_shape(numi_cloth_batch_t* batch, uint32_t resident_chunk, uint32_t threads);
 
-/* Autotuner: times one step of every candidate shape (resident chunk 0,
- * 256 ... 4096; 256 or 512 threads) on the current state, restores the
+/* Autotuner: times one step of every candidate shape (the fitted one;
+ * resident chunk 0, 256 ... 4096 with 256 or 512 threads) on the current state, restores the
  * state after each, and keeps the fastest; out (optional) receives it. */
 int numi_cloth_batch_tune(numi_cloth_batch_t* batch, const NumiClothConfig* configs, uint32_t substeps,
                           const NumiClothSchedule* schedule, uint32_t out[3]);

@@ -2155,6 +2155,14 @@ struct numi_cloth_batch {
     bool edge_room = true;             // the shape leaves room for the box tree's sort keys
     uint32_t ctas = 0;
     size_t smem = 0;
+    // the default shape (batch_fit): residency cloth by cloth, a cluster of
+    // `ranks` CTAs per cloth; its launches with the edge/edge family run one
+    // CTA per cloth
+    bool fitted = false;
+    uint32_t ranks = 1;
+    uint32_t edge_ctas = 0;
+    size_t edge_smem = 0;
+    bool layout_edge = false;          // which of the two the descriptors are laid out for
     Workspace grad;   // rollout gradients
     bool rollout_touched = false;   // a fruit touched a cloth in the last rollout
     cudaGraph_t graph = nullptr;
@@ -2207,13 +2215,156 @@ int batch_shape(numi_cloth_batch* b, uint32_t chunk, uint32_t block) {
     b->block = block;
     b->smem = smem;
     b->ctas = std::min<uint32_t>(static_cast<uint32_t>(b->cloths.size()), static_cast<uint32_t>(sms * per_sm));
+    b->fitted = false;
+    b->ranks = 1u;
     b->layout_valid = false;
     return NUMI_CLOTH_OK;
 }
 
+// How a cloth of n particles lives in `room` bytes of the shared memory of
+// each of its cluster's CTAs: positions and velocities where both fit (1),
+// else the positions (2: every colour gathers them, velocities are read
+// twice a substep), else neither (0).
+struct Residency {
+    uint32_t mode = 0, shift = 0;
+    size_t bytes = 0;
+};
+
+Residency batch_residency(uint32_t n, uint32_t ranks, size_t room) {
+    Residency r;
+    r.shift = 4u;
+    while ((static_cast<uint64_t>(ranks) << r.shift) < n) ++r.shift;
+    const size_t one = std::min<size_t>(static_cast<size_t>(1) << r.shift, n) * sizeof(float4);
+    r.mode = 2u * one <= room ? 1u : one <= room ? 2u : 0u;
+    r.bytes = r.mode == 1u ? 2u * one : r.mode == 2u ? one : 0u;
+    return r;
+}
+
+// Shared memory a CTA of the batch kernel has left for particles.
+size_t batch_room(const numi_cloth_batch* b, bool edge) {
+    int optin = 0;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
+    cudaFuncAttributes fa{};
+    if (cudaFuncGetAttributes(&fa, batch_fn(edge)) != cudaSuccess) return 0;
+    const size_t fixed = nc_resident_offset() + fa.sharedSizeBytes + (edge ? NC_EDGE_TREE_KEY_BYTES + 256u : 0u);
+    return static_cast<size_t>(optin) > fixed ? static_cast<size_t>(optin) - fixed : 0u;
+}
+
+// The default launch shape: 512 threads (a cloth's frame is latency-bound on
+// its SM: 192 square cloths of 16 to 96 particles a side take 10.6 ms a frame,
+// 15.6 with 256 threads and global particles), particles in shared memory as
+// far as they fit, and where there are
+// SMs to spare a cluster of up to 8 CTAs per cloth, until each CTA holds 256
+// particles (the single cloth's resident cluster).
+int batch_fit(numi_cloth_batch* b) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+    const uint32_t count = static_cast<uint32_t>(b->cloths.size());
+    uint32_t largest = 0;
+    for (numi_cloth* h : b->cloths) largest = std::max(largest, h->d.n);
+    b->block = NC_BLOCK_MAX;
+    uint32_t ranks = 1;
+    while (ranks < 8u && static_cast<uint64_t>(count) * 2u * ranks <= static_cast<uint64_t>(std::max(sms, 1)) &&
+           256u * ranks < largest)
+        ranks *= 2u;
+    for (bool edge : {false, true}) {
+        const size_t room = batch_room(b, edge);
+        for (;;) {
+            const uint32_t r = edge ? 1u : ranks;
+            size_t bytes = 0;
+            b->chunk = edge ? b->chunk : 0u;
+            for (numi_cloth* h : b->cloths) {
+                const Residency res = batch_residency(h->d.n, r, room);
+                bytes = std::max(bytes, res.bytes);
+                if (!edge && res.mode != 0u) b->chunk = std::max(b->chunk, h->d.n);
+            }
+            const size_t smem = nc_resident_offset() + bytes;
+            const size_t launch = edge ? nc_round256(smem) + NC_EDGE_TREE_KEY_BYTES : smem;
+            if (raise_smem(batch_fn(edge), launch) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+            int fit = 0;
+            if (r > 1u) {
+                cudaLaunchAttribute attr{};
+                attr.id = cudaLaunchAttributeClusterDimension;
+                attr.val.clusterDim.x = r;
+                attr.val.clusterDim.y = 1;
+                attr.val.clusterDim.z = 1;
+                cudaLaunchConfig_t cfg{};
+                cfg.gridDim = dim3(r);
+                cfg.blockDim = dim3(b->block);
+                cfg.dynamicSmemBytes = launch;
+                cfg.attrs = &attr;
+                cfg.numAttrs = 1;
+                if (cudaOccupancyMaxActiveClusters(&fit, batch_fn(edge), &cfg) != cudaSuccess ||
+                    static_cast<uint32_t>(std::max(fit, 0)) < count) {
+                    // not every cloth would have a cluster: fewer CTAs each
+                    cudaGetLastError();
+                    ranks /= 2u;
+                    continue;
+                }
+            } else {
+                int k = 0;
+                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, batch_fn(edge), static_cast<int>(b->block), launch) !=
+                        cudaSuccess ||
+                    k < 1)
+                    return NUMI_CLOTH_EINVAL;
+                fit = k * sms;
+            }
+            const uint32_t ctas = r * std::min<uint32_t>(count, static_cast<uint32_t>(fit));
+            if (edge) {
+                b->edge_smem = smem;
+                b->edge_ctas = ctas;
+            } else {
+                b->smem = smem;
+                b->ctas = ctas;
+            }
+            break;
+        }
+    }
+    b->ranks = ranks;
+    b->fitted = true;
+    b->edge_room = true;
+    b->layout_valid = false;
+    return NUMI_CLOTH_OK;
+}
+
+// Launch of the batch kernel over `cloths` (launch order) in the batch's
+// shape; the work queue starts at zero.
+cudaError_t batch_kernel(numi_cloth_batch* b, const DeviceCloth* cloths, const Schedule& s) {
+    const bool edge = s.primitive_self != 0u;
+    const bool fit_edge = b->fitted && edge;
+    uint32_t ranks = fit_edge ? 1u : b->ranks;
+    uint32_t count = static_cast<uint32_t>(b->cloths.size());
+    Schedule sc = s;
+    size_t smem = fit_edge ? b->edge_smem : b->smem;
+    if (edge) {   // the box tree's sort keys (the shape has room for them)
+        sc.tree_keys = static_cast<uint32_t>(nc_round256(smem));
+        smem = nc_round256(smem) + NC_EDGE_TREE_KEY_BYTES;
+    }
+    cudaError_t e = cudaMemsetAsync(b->queue, 0, sizeof(unsigned int), b->stream);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = ranks;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(fit_edge ? b->edge_ctas : b->ctas);
+    cfg.blockDim = dim3(b->block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = b->stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = ranks > 1u ? 1u : 0u;
+    unsigned int* queue = b->queue;
+    void* args[] = {&cloths, &count, &sc, &queue, &ranks};
+    return cudaLaunchKernelExC(&cfg, batch_fn(edge), args);
+}
+
 // Descriptors of every cloth for a launch of `substeps` Configs each.
-int batch_layout(numi_cloth_batch* b, uint32_t substeps) {
-    if (b->layout_valid && b->layout_substeps == substeps) return NUMI_CLOTH_OK;
+int batch_layout(numi_cloth_batch* b, uint32_t substeps, bool edge) {
+    if (b->layout_valid && b->layout_substeps == substeps && (!b->fitted || b->layout_edge == edge))
+        return NUMI_CLOTH_OK;
+    const uint32_t ranks = b->fitted && !edge ? b->ranks : 1u;
+    const size_t room = b->fitted ? batch_room(b, edge) : 0u;
     const uint32_t count = static_cast<uint32_t>(b->cloths.size());
     std::vector<DeviceCloth> host(count);
     for (uint32_t j = 0; j < count; ++j) {
@@ -2222,9 +2373,14 @@ int batch_layout(numi_cloth_batch* b, uint32_t substeps) {
         d.cfg = b->d_cfg + static_cast<size_t>(k) * substeps;
         d.trace = nullptr;
         d.trace_cta = nullptr;
-        d.cluster_barrier = 0u;
+        d.cluster_barrier = ranks > 1u ? 1u : 0u;
         d.resident = (b->chunk != 0u && d.n <= b->chunk) ? 1u : 0u;
         d.resident_shift = b->chunk ? log2_pow2(b->chunk) : 0u;
+        if (b->fitted) {
+            const Residency res = batch_residency(d.n, ranks, room);
+            d.resident = res.mode;
+            d.resident_shift = res.shift;
+        }
         host[j] = d;
     }
     if (cudaMemcpyAsync(b->d_cloths, host.data(), count * sizeof(DeviceCloth), cudaMemcpyHostToDevice, b->stream) !=
@@ -2232,6 +2388,7 @@ int batch_layout(numi_cloth_batch* b, uint32_t substeps) {
         return NUMI_CLOTH_ECUDA;
     if (cudaStreamSynchronize(b->stream) != cudaSuccess) return NUMI_CLOTH_ECUDA;
     b->layout_substeps = substeps;
+    b->layout_edge = edge;
     b->layout_valid = true;
     return NUMI_CLOTH_OK;
 }
@@ -2274,27 +2431,17 @@ int batch_prepare(numi_cloth_batch* b, const NumiClothConfig* configs, uint32_t 
         if (h->stream != b->stream && h->stream != nullptr && cudaStreamSynchronize(h->stream) != cudaSuccess)
             return NUMI_CLOTH_ECUDA;
     }
-    return batch_layout(b, substeps);
+    return batch_layout(b, substeps, sched.primitiveSelf != 0u);
 }
 
 cudaError_t batch_launch(numi_cloth_batch* b, const NumiClothConfig* configs, uint32_t substeps, const Schedule& s) {
     const uint32_t count = static_cast<uint32_t>(b->cloths.size());
     cudaError_t e = cudaMemcpyAsync(b->d_cfg, configs, static_cast<size_t>(count) * substeps * sizeof(NumiClothConfig),
                                     cudaMemcpyHostToDevice, b->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b->queue, 0, sizeof(unsigned int), b->stream);
-    if (e != cudaSuccess) return e;
     Schedule sc = s;
     sc.substeps = substeps;
     sc.epoch_ptr = b->epoch;
-    unsigned int* queue = b->queue;
-    const DeviceCloth* cloths = b->d_cloths;
-    void* args[] = {&cloths, const_cast<uint32_t*>(&count), &sc, &queue};
-    size_t smem = b->smem;
-    if (sc.primitive_self != 0u) {   // the box tree's sort keys (batch_shape checked the room)
-        sc.tree_keys = static_cast<uint32_t>(nc_round256(smem));
-        smem = nc_round256(smem) + NC_EDGE_TREE_KEY_BYTES;
-    }
-    e = cudaLaunchKernel(batch_fn(sc.primitive_self != 0u), dim3(b->ctas), dim3(b->block), args, smem, b->stream);
+    if (e == cudaSuccess) e = batch_kernel(b, b->d_cloths, sc);
     if (e != cudaSuccess) return e;
     numi_cloth_epoch_kernel<<<1, 1, 0, b->stream>>>(b->epoch, substeps);
     return cudaGetLastError();
@@ -2356,8 +2503,7 @@ int numi_cloth_batch_create(numi_cloth_t* const* cloths, uint32_t count, numi_cl
         delete b;
         return NUMI_CLOTH_ENOMEM;
     }
-    // default shape: particles from global memory, 256 threads per CTA
-    const int rc = batch_shape(b, 0u, NC_THREADS);
+    const int rc = batch_fit(b);
     if (rc != NUMI_CLOTH_OK) {
         delete b;
         return rc;
@@ -2432,15 +2578,18 @@ int numi_cloth_batch_tune(numi_cloth_batch_t* b, const NumiClothConfig* configs,
     cudaEventCreate(&t0);
     cudaEventCreate(&t1);
     float best_ms = INFINITY;
-    uint32_t best_chunk = 0, best_block = NC_THREADS;
-    const uint32_t chunks[] = {0u, 256u, 512u, 1024u, 2048u, 4096u};
+    constexpr uint32_t kFit = ~0u;   // the default shape
+    uint32_t best_chunk = kFit, best_block = NC_BLOCK_MAX;
+    auto shape = [&](uint32_t chunk, uint32_t block) { return chunk == kFit ? batch_fit(b) : batch_shape(b, chunk, block); };
+    const uint32_t chunks[] = {kFit, 0u, 256u, 512u, 1024u, 2048u, 4096u};
     const uint32_t blocks[] = {NC_THREADS, NC_BLOCK_MAX};
     const Schedule s = device_schedule(*schedule);
     int rc = NUMI_CLOTH_OK;
     for (uint32_t chunk : chunks) {
-        if (chunk > 0u && chunk / 2u >= largest) continue;   // same as a smaller chunk
+        if (chunk != kFit && chunk > 0u && chunk / 2u >= largest) continue;   // same as a smaller chunk
         for (uint32_t block : blocks) {
-            if (batch_shape(b, chunk, block) != NUMI_CLOTH_OK) continue;
+            if (chunk == kFit && block != NC_BLOCK_MAX) continue;   // it has its own
+            if (shape(chunk, block) != NUMI_CLOTH_OK) continue;
             if (schedule->primitiveSelf != 0u && !b->edge_room) continue;
             rc = batch_prepare(b, configs, substeps, *schedule);
             if (rc != NUMI_CLOTH_OK) break;
@@ -2470,7 +2619,7 @@ int numi_cloth_batch_tune(numi_cloth_batch_t* b, const NumiClothConfig* configs,
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
     if (rc != NUMI_CLOTH_OK) return rc;
-    rc = batch_shape(b, best_chunk, best_block);
+    rc = shape(best_chunk, best_block);
     if (rc == NUMI_CLOTH_OK && out != nullptr) numi_cloth_batch_shape(b, out);
     return rc;
 }
@@ -3256,10 +3405,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         st.cfg_offset = first;
         st.epoch_ptr = b->epoch;
         st.tape_first = tape_first;
-        cudaMemsetAsync(b->queue, 0, sizeof(unsigned int), b->stream);
-        numi_cloth_batch_kernel<<<b->ctas, b->block, b->smem, b->stream>>>(taped ? d_replay : b->d_cloths, count, st,
-                                                                         b->queue);
-        return cudaGetLastError() == cudaSuccess;
+        return batch_kernel(b, taped ? d_replay : b->d_cloths, st) == cudaSuccess;
     };
     // forward: taped where the tape holds it, else checkpointed (the last
     // segment of cloths without fruits is taped as it runs)

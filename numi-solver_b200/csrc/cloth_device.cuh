@@ -153,7 +153,8 @@ struct DeviceCloth {
     unsigned int* nbr_flag;        // [32 * grid]
     // resident mode: 1 when particle positions and velocities live in the
     // (distributed) shared memory of the grid's CTAs for the whole launch;
-    // CTA r owns particles [r << resident_shift, (r + 1) << resident_shift)
+    // CTA r owns particles [r << resident_shift, (r + 1) << resident_shift);
+    // 2 when only the positions do (velocities are read twice a substep)
     uint32_t resident;
     uint32_t resident_shift;
     double* red;          // [blocks * 8] reduction partials

@@ -12,6 +12,7 @@ __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_frame_edge_kernel(
 }
 
 __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_batch_edge_kernel(const DeviceCloth* cloths, uint32_t count,
-                                                                              Schedule s, unsigned int* queue) {
+                                                                              Schedule s, unsigned int* queue,
+                                                                              uint32_t ranks) {
     NC_BATCH_BODY(true)
 }

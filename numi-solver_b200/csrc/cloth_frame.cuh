@@ -2908,6 +2908,7 @@ __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule
     ctx.seq = 0;
     ctx.nseq = 0;
     ctx.resident = d.resident != 0u;
+    ctx.resident_v = d.resident == 1u;
     ctx.rank = rank;
     ctx.ranks = ranks;
     ctx.shift = d.resident_shift;
@@ -2916,12 +2917,12 @@ __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule
         // Stage this CTA's particles into shared memory for the whole launch
         // (bulk copies of its slices of x and v).
         ctx.xs = reinterpret_cast<float4*>(dynamic_smem + nc_resident_offset());
-        ctx.vs = ctx.xs + (1u << ctx.shift);
+        ctx.vs = ctx.xs + min(1u << ctx.shift, d.n);
         own_first = min(ctx.rank << ctx.shift, d.n);
         own_end = min(own_first + (1u << ctx.shift), d.n);
         const uint32_t bytes = (own_end - own_first) * static_cast<uint32_t>(sizeof(float4));
         const nc::BulkJob jobs[2] = {{ctx.xs, d.x + own_first, bytes}, {ctx.vs, d.v + own_first, bytes}};
-        const bool staged = nc::bulk_load(d, jobs, 2u);
+        const bool staged = nc::bulk_load(d, jobs, ctx.resident_v ? 2u : 1u);
         // a cluster's CTAs all pass its barrier; a copy that timed out has
         // raised TIMEOUT and the abort flag for the host
         if (ranks > 1u)
@@ -2996,7 +2997,7 @@ __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule
         // particles back (bulk copies).
         const uint32_t bytes = (own_end - own_first) * static_cast<uint32_t>(sizeof(float4));
         const nc::BulkJob jobs[2] = {{ctx.xs, d.x + own_first, bytes}, {ctx.vs, d.v + own_first, bytes}};
-        nc::bulk_store(jobs, 2u);
+        nc::bulk_store(jobs, ctx.resident_v ? 2u : 1u);
     }
 }
 
@@ -3006,7 +3007,7 @@ __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule
 // and the default kernels grow a call frame.
 __global__ void numi_cloth_frame_edge_kernel(DeviceCloth d, Schedule s);
 __global__ void numi_cloth_batch_edge_kernel(const DeviceCloth* cloths, uint32_t count, Schedule s,
-                                             unsigned int* queue);
+                                             unsigned int* queue, uint32_t ranks);
 // The frame kernels whose point self contact keeps the reference's
 // Gauss-Seidel order are likewise in cloth_self_order_kernels.cu: its
 // out-of-line ordered pass would otherwise cost the default kernels
@@ -3014,19 +3015,35 @@ __global__ void numi_cloth_batch_edge_kernel(const DeviceCloth* cloths, uint32_t
 __global__ void numi_cloth_frame_exact_kernel(DeviceCloth d, Schedule s);
 __global__ void numi_cloth_frame_edge_exact_kernel(DeviceCloth d, Schedule s);
 
-// Many independent cloths in one persistent launch: every CTA takes the
-// next cloth from a device work queue (cloths ordered by work, largest
-// first) and runs its whole frame alone, until the queue is empty.
-#define NC_BATCH_BODY(kEdge)                                                  \
-    extern __shared__ __align__(16) unsigned char nc_dynamic_smem[];          \
-    __shared__ uint32_t s_next;                                               \
-    for (;;) {                                                                \
-        if (threadIdx.x == 0) s_next = atomicAdd(queue, 1u);                  \
-        __syncthreads();                                                      \
-        const uint32_t k = s_next;                                            \
-        if (k >= count) break;                                                \
-        run_frame<kEdge, true>(cloths[k], s, 0u, 1u, nc_dynamic_smem);        \
-        __syncthreads();                                                      \
+// Many independent cloths in one persistent launch: every cluster of `ranks`
+// CTAs takes the next cloth from a device work queue (cloths ordered by work,
+// largest first) and runs its whole frame alone, until the queue is empty.
+// The cluster's first CTA draws for all of them; the barrier after the draw
+// also keeps a CTA from staging the next cloth over particles another CTA of
+// the cluster still reads.
+#define NC_BATCH_BODY(kEdge)                                                                        \
+    extern __shared__ __align__(16) unsigned char nc_dynamic_smem[];                                \
+    __shared__ uint32_t s_next;                                                                     \
+    const uint32_t rank = blockIdx.x % ranks;                                                       \
+    if (ranks > 1u) cooperative_groups::this_cluster().sync(); /* every CTA's shared memory is up */ \
+    for (;;) {                                                                                      \
+        if (rank == 0u && threadIdx.x == 0) {                                                       \
+            const uint32_t drawn = atomicAdd(queue, 1u);                                            \
+            s_next = drawn;                                                                         \
+            for (uint32_t r = 1; r < ranks; ++r)                                                    \
+                *static_cast<uint32_t*>(__cluster_map_shared_rank(&s_next, r)) = drawn;             \
+        }                                                                                           \
+        if (ranks > 1u)                                                                             \
+            cooperative_groups::this_cluster().sync();                                              \
+        else                                                                                        \
+            __syncthreads();                                                                        \
+        const uint32_t k = s_next;                                                                  \
+        if (k >= count) break;                                                                      \
+        run_frame<kEdge, true>(cloths[k], s, rank, ranks, nc_dynamic_smem);                         \
+        if (ranks > 1u)                                                                             \
+            cooperative_groups::this_cluster().sync();                                              \
+        else                                                                                        \
+            __syncthreads();                                                                        \
     }
 
 #ifndef NC_EDGE_KERNELS
@@ -3036,7 +3053,8 @@ __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_frame_kernel(Devic
     run_frame<false, false>(d, s, blockIdx.x, gridDim.x, nc_dynamic_smem);
 }
 __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_batch_kernel(const DeviceCloth* cloths, uint32_t count,
-                                                                         Schedule s, unsigned int* queue) {
+                                                                         Schedule s, unsigned int* queue,
+                                                                         uint32_t ranks) {
     NC_BATCH_BODY(false)
 }
 

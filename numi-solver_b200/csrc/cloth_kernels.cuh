@@ -152,6 +152,7 @@ struct Ctx {
     unsigned nseq;            // colour syncs passed in this launch
     FruitShared* fs;          // fruit-CTA shared state (valid in the fruit CTA)
     bool resident;
+    bool resident_v;          // velocities too
     uint32_t rank;            // cluster rank (resident) or 0
     uint32_t ranks;           // CTAs that own particles (resident) or 1
     uint32_t shift;           // log2 of the particles each CTA owns
@@ -188,10 +189,10 @@ __device__ __forceinline__ void px_set(const Ctx& c, uint32_t i, float4 v) {
         c.gx[i] = v;
 }
 __device__ __forceinline__ float4 pv(const Ctx& c, uint32_t i) {
-    return c.resident ? *resident_ptr(c, c.vs, i) : __ldcg(c.gv + i);
+    return c.resident_v ? *resident_ptr(c, c.vs, i) : __ldcg(c.gv + i);
 }
 __device__ __forceinline__ void pv_set(const Ctx& c, uint32_t i, float4 v) {
-    if (c.resident)
+    if (c.resident_v)
         *resident_ptr(c, c.vs, i) = v;
     else
         c.gv[i] = v;
