@@ -170,7 +170,7 @@ struct DeviceCloth {
     // buckets of older passes read as empty and nothing is cleared between
     // passes
     unsigned long long* hash_head;
-    HashSlot* hash;       // [buckets * NC_HASH_CAP]
+    HashSlot* hash;       // [buckets * NC_HASH_CAP], eight buckets' slots interleaved (hash_slot)
     // particles whose bucket was full: (pass tag << 32) | count, and [n]
     // slots, so no particle is ever dropped
     unsigned long long* hash_over_head;
