@@ -450,9 +450,9 @@ bool prepare_neighbours(numi_cloth* h, const NumiClothScene* scene) {
 // colour before touching an owned particle or a particle of an item found,
 // and so on.  Local particles are ordered own, then the fruit/yarn and
 // strain chains' other particles, then the constraint chain's, so every
-// chain reads a prefix.  Returns false (tile mode off) when a plan would not
-// fit the shared memory of one CTA per SM or a closure holds 65,536
-// particles or more.
+// chain reads a prefix.  Returns false (tile mode off) when a plan's
+// particles would not fit the shared memory of one CTA per SM or a closure
+// holds 65,536 particles or more.
 struct TileColour {
     uint32_t family, first, count;
 };
@@ -526,7 +526,7 @@ bool build_tiles(numi_cloth* h, uint32_t grid_width, const std::vector<uint2>& d
     std::vector<int32_t> lidx(n, -1);
     uint32_t stamp = 0;
     std::vector<std::vector<uint32_t>> plans(R);
-    size_t widest = 0;
+    size_t widest = 0, widest_stream = 0;   // bytes of a plan and its particles, without and with streamed items
     std::vector<std::vector<uint32_t>> own_of(tiles);
     for (uint32_t i = 0; i < n; ++i) own_of[tile_of[i]].push_back(i);
     for (uint32_t t = 0; t < R; ++t) {
@@ -643,9 +643,15 @@ bool build_tiles(numi_cloth* h, uint32_t grid_width, const std::vector<uint2>& d
         for (uint32_t l = 0; l < local.size(); ++l) w[list_at + l] = local[l];
         for (uint32_t p : local) lidx[p] = -1;
         widest = std::max(widest, w.size() * 4u + local.size() * sizeof(float4));
+        widest_stream = std::max(widest_stream, items_at * 4u + local.size() * sizeof(float4));
     }
-    // the fruit CTA holds its fruit state and the staged friction sweep
-    const size_t smem = std::max(nc_resident_offset() + sizeof(FrictionStage), nc_fruit_offset() + widest);
+    // the fruit CTA holds its fruit state and the staged friction sweep.
+    // Plans that do not fit keep their items in global memory: the
+    // 512 x 512 cloth's are 25,000 items a CTA, 59 MB in all, which the L2
+    // holds (a substep 158 us colour by colour, 101 with streamed items).
+    const size_t fruit = nc_resident_offset() + sizeof(FrictionStage);
+    const bool stream = std::max(fruit, nc_fruit_offset() + widest) > smem_budget;
+    const size_t smem = std::max(fruit, nc_fruit_offset() + (stream ? widest_stream : widest));
     if (smem > smem_budget) return false;
     std::vector<uint32_t> off(R + 1u, 0u), words;
     for (uint32_t t = 0; t < R; ++t) {
@@ -671,6 +677,7 @@ bool build_tiles(numi_cloth* h, uint32_t grid_width, const std::vector<uint2>& d
         cudaMemcpy(dw, words.data(), words.size() * sizeof(uint32_t), cudaMemcpyHostToDevice) != cudaSuccess)
         return false;
     dd.tile_words = dw;
+    dd.tile_stream = stream ? 1u : 0u;
     h->tile_smem = smem;
     return true;
 }
@@ -773,6 +780,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
             if (!rebuild_tiles(h)) return cudaErrorUnknown;
             h->tiles_dirty = false;
             d.tile_words = h->d.tile_words;
+            d.tile_stream = h->d.tile_stream;
         }
         sc.tiles = 1u;
         if (h->tile_grid > h->grid) d.trace_cta = nullptr;

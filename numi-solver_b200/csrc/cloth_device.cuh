@@ -266,6 +266,7 @@ struct DeviceCloth {
     const uint32_t* tile_off;
     const uint32_t* tile_words;
     const uint32_t* tile_owner;
+    uint32_t tile_stream;          // 1: the plans' items stay in global memory
     float4* x_alt;
     float4* v_alt;
     // allocation-free launches: [n + NC_MAX_FRUITS] words of scratch; when

@@ -2963,12 +2963,9 @@ __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule
         // tile mode: the CTA's plan and its local particles after the
         // descriptor (the fruit CTA keeps its fruit state there instead)
         uint32_t* plan = reinterpret_cast<uint32_t*>(dynamic_smem + nc_fruit_offset());
-        ctx.tp = plan;
         if (ctx.fruit_cta) ctx.fst = reinterpret_cast<FrictionStage*>(dynamic_smem + nc_resident_offset());
         if (!ctx.fruit_cta) {
             if (!nc::tile_stage(ctx, plan)) return;
-            ctx.tx = reinterpret_cast<float4*>(
-                dynamic_smem + nc_fruit_offset() + 4u * (d.tile_off[rank + 1u] - d.tile_off[rank]));
             ctx.tile_box = nc::tile_closure_box(ctx);
         }
     } else {

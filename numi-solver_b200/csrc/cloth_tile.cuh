@@ -44,7 +44,8 @@
 // waits for the fruit CTA's flag, and the others go on.
 //
 // Plan of one CTA (host-built, 16-byte aligned words, staged into shared
-// memory once per launch with a bulk copy):
+// memory once per launch with a bulk copy; the items of a plan too large for
+// that are streamed from global memory in every substep):
 //   [0] local particles, [1] owned particles (the first ones),
 //   [2] word offset of the particle list, [3] word offset of the items,
 //   [4 + k] local particles chain k reads (a prefix of the list),
@@ -68,18 +69,23 @@ namespace {
 #define NC_TILE_LIMIT 2u
 #define NC_TILE_SEGMENT 3u
 // Stage this CTA's plan into shared memory: one bulk load (nc::bulk_load,
-// bounded wait).
-__device__ bool tile_stage(const Ctx& ctx, uint32_t* plan) {
+// bounded wait).  Where the items would not fit beside the particles they
+// stay in global memory (DeviceCloth::tile_stream) and only the words in
+// front of them are staged.  Sets the plan, the items and the room for the
+// local particles after the staged words.
+__device__ bool tile_stage(Ctx& ctx, uint32_t* plan) {
     const DeviceCloth& d = ctx.d;
-    const uint32_t w0 = d.tile_off[ctx.rank], w1 = d.tile_off[ctx.rank + 1u];
-    const BulkJob job{plan, d.tile_words + w0, (w1 - w0) * 4u};
+    const uint32_t w0 = d.tile_off[ctx.rank];
+    const uint32_t items = __ldg(d.tile_words + w0 + 3u);
+    const uint32_t staged = d.tile_stream != 0u ? items : d.tile_off[ctx.rank + 1u] - w0;
+    ctx.tp = plan;
+    ctx.ti = reinterpret_cast<const uint4*>(d.tile_stream != 0u ? d.tile_words + w0 + items : plan + items);
+    ctx.tx = reinterpret_cast<float4*>(plan + staged);
+    const BulkJob job{plan, d.tile_words + w0, staged * 4u};
     return bulk_load(d, &job, 1u);
 }
 
 __device__ __forceinline__ const uint32_t* tile_list(const Ctx& ctx) { return ctx.tp + ctx.tp[2]; }
-__device__ __forceinline__ const uint4* tile_items(const Ctx& ctx) {
-    return reinterpret_cast<const uint4*>(ctx.tp + ctx.tp[3]);
-}
 __device__ __forceinline__ float4* other_x(const Ctx& ctx) { return ctx.gx == ctx.d.x ? ctx.d.x_alt : ctx.d.x; }
 __device__ __forceinline__ float4* other_v(const Ctx& ctx) { return ctx.gv == ctx.d.v ? ctx.d.v_alt : ctx.d.v; }
 
@@ -129,52 +135,67 @@ __device__ void tile_predict(const Ctx& ctx, float4* v_next) {
     __syncthreads();
 }
 
-// A chain's colours in order, CTA barriers between them.  Distances and
-// bends start from zero multipliers (one iteration per substep), and the
-// owner publishes every multiplier it computes (zero when the projection
-// changes nothing, as after the reset of the substep start).
-__device__ void tile_chain(const Ctx& ctx, uint32_t chain, float dt2) {
+// One item of the constraint and strain chains on the local particles.
+// Distances and bends start from zero multipliers (one iteration per
+// substep), and the owner publishes every multiplier it computes (zero when
+// the projection changes nothing, as after the reset of the substep start).
+__device__ __forceinline__ void tile_item(const Ctx& ctx, uint32_t family, const uint4& it, float dt2) {
     const DeviceCloth& d = ctx.d;
+    float4* tx = ctx.tx;
+    const uint32_t al = it.x & 0xffffu, bl = it.x >> 16;
+    const uint32_t rec = it.y & 0x7fffffffu;
+    const bool owner = (it.y >> 31) != 0u;
+    if (family == NC_TILE_DISTANCE) {
+        float4 a = tx[al], b = tx[bl];
+        const float4 m = make_float4(__uint_as_float(it.z), __uint_as_float(it.w), 0.0f, 0.0f);
+        float lam = 0.0f;
+        if (distance_core(a, b, m, lam, dt2)) {
+            tx[al] = a;
+            tx[bl] = b;
+        }
+        if (owner) d.d_lambda[rec] = lam;
+    } else if (family == NC_TILE_BEND) {
+        float4 p[2] = {tx[al], tx[bl]};
+        const float2 m = make_float2(__uint_as_float(it.z), __uint_as_float(it.w));
+        float lam = 0.0f;
+        if (bend_core(p, m, lam, dt2, ctx.c.radius, ctx.c.ground)) {
+            tx[al] = p[0];
+            tx[bl] = p[1];
+        }
+        if (owner) d.b_lambda[rec] = lam;
+    } else {
+        float4 a = tx[al], b = tx[bl];
+        const float4 m = make_float4(__uint_as_float(it.z), 0.0f, 0.0f, __uint_as_float(it.w));
+        if (strain_core(a, b, m)) {
+            tx[al] = a;
+            tx[bl] = b;
+        }
+    }
+}
+
+// Streamed items of a chain's colour c into L1, a line per thread: issued a
+// colour ahead, so that the colour's loads do not wait for the L2.
+__device__ __forceinline__ void tile_prefetch(const Ctx& ctx, uint32_t chain, uint32_t c) {
+    if (ctx.d.tile_stream == 0u || c >= ctx.tp[9u + 2u * chain]) return;
+    const uint32_t* table = ctx.tp + ctx.tp[8u + 2u * chain];
+    const uint4* first = ctx.ti + table[2u * c];
+    const uint32_t count = table[2u * c + 1u] & 0x0fffffffu;
+    for (uint32_t k = 8u * threadIdx.x; k < count; k += 8u * blockDim.x)   // 128 bytes
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(first + k));
+}
+
+// A chain's colours in order, CTA barriers between them.
+__device__ void tile_chain(const Ctx& ctx, uint32_t chain, float dt2) {
     const uint32_t* table = ctx.tp + ctx.tp[8u + 2u * chain];
     const uint32_t colours = ctx.tp[9u + 2u * chain];
-    const uint4* items = tile_items(ctx);
-    float4* tx = ctx.tx;
+    const uint4* staged = reinterpret_cast<const uint4*>(ctx.tp + ctx.tp[3]);
     for (uint32_t c = 0; c < colours; ++c) {
         const uint32_t first = table[2u * c];
         const uint32_t count = table[2u * c + 1u] & 0x0fffffffu;
         const uint32_t family = table[2u * c + 1u] >> 28;
-        for (uint32_t k = threadIdx.x; k < count; k += blockDim.x) {
-            const uint4 it = items[first + k];
-            const uint32_t al = it.x & 0xffffu, bl = it.x >> 16;
-            const uint32_t rec = it.y & 0x7fffffffu;
-            const bool owner = (it.y >> 31) != 0u;
-            if (family == NC_TILE_DISTANCE) {
-                float4 a = tx[al], b = tx[bl];
-                const float4 m = make_float4(__uint_as_float(it.z), __uint_as_float(it.w), 0.0f, 0.0f);
-                float lam = 0.0f;
-                if (distance_core(a, b, m, lam, dt2)) {
-                    tx[al] = a;
-                    tx[bl] = b;
-                }
-                if (owner) d.d_lambda[rec] = lam;
-            } else if (family == NC_TILE_BEND) {
-                float4 p[2] = {tx[al], tx[bl]};
-                const float2 m = make_float2(__uint_as_float(it.z), __uint_as_float(it.w));
-                float lam = 0.0f;
-                if (bend_core(p, m, lam, dt2, ctx.c.radius, ctx.c.ground)) {
-                    tx[al] = p[0];
-                    tx[bl] = p[1];
-                }
-                if (owner) d.b_lambda[rec] = lam;
-            } else {
-                float4 a = tx[al], b = tx[bl];
-                const float4 m = make_float4(__uint_as_float(it.z), 0.0f, 0.0f, __uint_as_float(it.w));
-                if (strain_core(a, b, m)) {
-                    tx[al] = a;
-                    tx[bl] = b;
-                }
-            }
-        }
+        tile_prefetch(ctx, chain, c + 1u);
+        for (uint32_t k = threadIdx.x; k < count; k += blockDim.x)
+            tile_item(ctx, family, ctx.d.tile_stream != 0u ? __ldg(ctx.ti + first + k) : staged[first + k], dt2);
         __syncthreads();
     }
 }
@@ -218,11 +239,12 @@ __device__ void tile_yarn(const Ctx& ctx) {
     __syncthreads();
     const uint32_t* table = ctx.tp + ctx.tp[8u + 2u * NC_TILE_YARN];
     const uint32_t colours = ctx.tp[9u + 2u * NC_TILE_YARN];
-    const uint4* items = tile_items(ctx);
+    const uint4* items = ctx.ti;
     const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t c = 0; c < colours; ++c) {
         const uint32_t first = table[2u * c];
         const uint32_t count = table[2u * c + 1u] & 0x0fffffffu;
+        tile_prefetch(ctx, NC_TILE_YARN, c + 1u);
         for (uint32_t base = threadIdx.x - lane; base < count; base += blockDim.x) {
             const uint32_t k = base + lane;
             const bool valid = k < count;
@@ -426,6 +448,7 @@ __device__ bool substep_tiles(Ctx& ctx, bool last) {
             if (ctx.fruit_wait && !tile_wait_fruit(ctx, ctx.sub)) return false;
             ctx.fruit_wait = false;
             tile_mark(ctx, 0u);
+            tile_prefetch(ctx, NC_TILE_CONSTRAINTS, 0u);
             tile_predict(ctx, v_next);
             tile_mark(ctx, 1u);
             tile_chain(ctx, NC_TILE_CONSTRAINTS, dt2);
@@ -447,6 +470,7 @@ __device__ bool substep_tiles(Ctx& ctx, bool last) {
         float4* x_next = other_x(ctx);
         if (!ctx.fruit_cta) {
             tile_mark(ctx, 4u);
+            tile_prefetch(ctx, NC_TILE_YARN, 0u);
             tile_load(ctx, NC_TILE_YARN);
             tile_mark(ctx, 5u);
             tile_yarn(ctx);
@@ -526,6 +550,7 @@ __device__ bool substep_tiles(Ctx& ctx, bool last) {
             }
         } else {
             if (!split) tile_mark(ctx, 9u);
+            if (s.strain_sweeps > 0u) tile_prefetch(ctx, NC_TILE_STRAIN, 0u);
             tile_load(ctx, NC_TILE_STRAIN);
             if (!split) tile_mark(ctx, 10u);
             if (sw == 0u && !split) tile_self_ground(ctx, false, ctx.tp[4u + NC_TILE_STRAIN]);
