@@ -179,6 +179,8 @@ struct numi_cloth {
     // changed (its items carry the materials)
     bool tiles = false;
     bool tiles_dirty = false;
+    bool tiles_wanted = false;   // small cloth: its plan is built once it has stepped kTilePlanSubsteps
+    uint32_t tile_substeps = 0;  // substeps it has stepped (or is about to) that a plan covers
     uint32_t tile_grid = 0, tile_block = 0;
     size_t tile_smem = 0;
     uint32_t last_grid = 0, last_block = 0;
@@ -704,10 +706,13 @@ bool rebuild_tiles(numi_cloth* h) {
 
 // A launch runs in tile mode when the cloth has tile plans and the
 // schedule is one the tile substep covers.
-bool tile_schedule(const numi_cloth* h, const Schedule& s) {
-    return h->tiles && s.iterations == 1u && s.aerodynamics == 0u && s.swept_fruit_yarn == 0u &&
+bool tile_covers(const Schedule& s) {
+    return s.iterations == 1u && s.aerodynamics == 0u && s.swept_fruit_yarn == 0u &&
            s.primitive_self == 0u && s.reconcile_passes == 0u && s.final_passes == 0u && s.certificate_passes == 0u;
 }
+bool tile_schedule(const numi_cloth* h, const Schedule& s) { return h->tiles && tile_covers(s); }
+bool configure_tiles(numi_cloth* h, uint32_t grid);
+constexpr uint32_t kTilePlanSubsteps = 48;
 
 // Adjoint tape of a launch: [substep][slots][n] positions, [substep][n]
 // velocities.
@@ -743,6 +748,21 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     if (e != cudaSuccess) return e;
     h->last_substeps = substeps;
     size_t smem = h->smem;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (h->tiles_wanted && !taped && tile_covers(sc))
+        h->tile_substeps = std::min(h->tile_substeps + std::min(substeps, kTilePlanSubsteps), kTilePlanSubsteps);
+    if (h->tiles_wanted && !taped && tile_covers(sc) && h->tile_substeps == kTilePlanSubsteps &&
+        cudaStreamIsCapturing(h->stream, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone) {
+        h->tiles_wanted = false;
+        configure_tiles(h, h->tile_grid);
+        d.tile_off = h->d.tile_off;
+        d.tile_words = h->d.tile_words;
+        d.tile_owner = h->d.tile_owner;
+        d.tile_stream = h->d.tile_stream;
+        d.x_alt = h->d.x_alt;
+        d.v_alt = h->d.v_alt;
+    }
+    const bool tiled = !taped && tile_schedule(h, sc);
     if (edge) {
         // the edge/edge phases' box-tree sort keys after the launch's own
         // shared memory, where the device has room
@@ -758,7 +778,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
         }
         cudaGetLastError();
     }
-    if (h->cluster > 0) {
+    if (h->cluster > 0 && !tiled) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(h->cluster);
         cfg.blockDim = dim3(h->block);
@@ -773,9 +793,9 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
         cfg.numAttrs = 1;
         d.cluster_barrier = 1u;
         e = cudaLaunchKernelExC(&cfg, frame_fn(edge, h->self_exact), args);
-    } else if (h->grid == 1) {
+    } else if (h->grid == 1 && !tiled) {
         e = cudaLaunchKernel(frame_fn(edge, h->self_exact), dim3(1), dim3(h->block), args, smem, h->stream);
-    } else if (!taped && tile_schedule(h, sc)) {   // the tape follows the colour-by-colour barriers
+    } else if (tiled) {   // not a taped launch: the tape follows the colour-by-colour barriers
         if (h->tiles_dirty) {
             if (!rebuild_tiles(h)) return cudaErrorUnknown;
             h->tiles_dirty = false;
@@ -783,6 +803,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
             d.tile_stream = h->d.tile_stream;
         }
         sc.tiles = 1u;
+        d.resident = 0u;   // a small cloth's other launches keep it in a cluster's shared memory
         if (h->tile_grid > h->grid) d.trace_cta = nullptr;
         e = raise_frame_smem(h->tile_smem);
         if (e == cudaSuccess)
@@ -1432,6 +1453,23 @@ int numi_cloth_create(const NumiClothScene* scene, numi_cloth_t** out) {
     // on by default; NUMI_CLOTH_TILES=0 keeps the colour-by-colour schedule.
     uint32_t want_tiles = 1;
     env_u32("NUMI_CLOTH_TILES", want_tiles);
+    // A small cloth that runs resident on a cluster of its own choice takes
+    // tile mode too, on as many CTAs as the cluster has and one for the
+    // fruits (the same share of the GPU when several cloths step at once):
+    // five grid barriers a substep instead of 26 cluster barriers (a frame of
+    // a 61 x 61 cloth: 3.6 -> 2.2 ms).  Its plan is built once it has stepped
+    // a frame's substeps: a 24 x 24 cloth's takes 0.5 ms, about what it then
+    // saves in as many substeps again, and a cloth that only joins batches or
+    // rollouts never needs one.  The reference-order kernels
+    // stay on the cluster, whose barrier has no bound for the ordered
+    // pass's serial fallback to outlast.
+    if (want_tiles != 0u && h->cluster > 1u && d.resident != 0u && K == 0u && !h->self_exact && forced == 0u &&
+        !forced_block && std::getenv("NUMI_CLOTH_CLUSTER") == nullptr && std::getenv("NUMI_CLOTH_RESIDENT") == nullptr &&
+        std::getenv("NUMI_CLOTH_RESIDENT_CHUNK") == nullptr) {
+        h->tile_grid = std::max(h->cluster + 1u, 3u);
+        h->tile_block = NC_BLOCK_MAX;
+        h->tiles_wanted = true;
+    }
     if (want_tiles != 0u && h->grid > 1u && h->cluster == 0u && d.resident == 0u && K == 0u) {
         int max_optin = 0;
         cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
