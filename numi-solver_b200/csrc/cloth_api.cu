@@ -58,6 +58,7 @@ struct Snapshot {
     bool valid = false;
     void* mem = nullptr;
     size_t bytes = 0;
+    std::vector<float> grip_compliance;   // the grips' at the snapshot
 };
 
 struct DeviceBuffers {
@@ -189,6 +190,15 @@ struct numi_cloth {
     std::vector<uint2> host_yarn;
     std::vector<uint32_t> host_local_off, host_local_idx;
     Snapshot snaps[kSnapshotSlots + 1u];   // the callers' slots, then the tuners' own
+    // Host copy of what the compliance groups are made of: per family
+    // (distance, knot, bend) the distinct values, ascending, and every
+    // record's index among them (read from the device when first asked for,
+    // then kept in step by numi_cloth_replace_compliance, the only writer);
+    // and every grip's compliance, which a restore brings back with the grips.
+    bool compliance_known = false;
+    std::vector<float> compliance[3];
+    std::vector<uint8_t> compliance_id[3];
+    std::vector<float> grip_compliance;
     // dynamic state regions copied by snapshot/restore
     struct Region {
         void* ptr;
@@ -1490,6 +1500,7 @@ int numi_cloth_create(const NumiClothScene* scene, numi_cloth_t** out) {
         }
         cudaGetLastError();
     }
+    for (uint32_t g = 0; g < G; ++g) h->grip_compliance.push_back(scene->grips[g].targetOffsetAndCompliance.w);
     h->dynamic = {{d.x, n * sizeof(float4)},
                   {d.xp, n * sizeof(float4)},
                   {d.v, n * sizeof(float4)},
@@ -1757,6 +1768,46 @@ int numi_cloth_restore(numi_cloth_t* h, uint32_t slot) {
 }  // extern "C"
 
 namespace {
+
+// The dynamic state's regions (each a whole number of 4-byte words, 16-byte
+// aligned) to or from one block, every region at a multiple of 256 bytes:
+// one launch in place of ten copies of 2 us of host time each.
+constexpr uint32_t kStateRegions = 16;
+struct StateCopy {
+    struct Op {
+        const char* src;
+        char* dst;
+        uint32_t words;
+    } op[kStateRegions];
+};
+
+__global__ void numi_cloth_state_copy_kernel(StateCopy c) {
+    const StateCopy::Op op = c.op[blockIdx.y];
+    const uint32_t quads = op.words / 4u;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < quads; k += gridDim.x * blockDim.x)
+        reinterpret_cast<uint4*>(op.dst)[k] = __ldcg(reinterpret_cast<const uint4*>(op.src) + k);
+    if (blockIdx.x == 0u && threadIdx.x < op.words % 4u) {
+        const uint32_t k = 4u * quads + threadIdx.x;
+        reinterpret_cast<uint32_t*>(op.dst)[k] = __ldcg(reinterpret_cast<const uint32_t*>(op.src) + k);
+    }
+}
+
+cudaError_t copy_state(numi_cloth* h, char* block, bool save) {
+    StateCopy c{};
+    uint32_t regions = 0, most = 0;
+    for (const auto& r : h->dynamic) {
+        if (regions == kStateRegions || r.bytes % 4u != 0u || r.bytes / 4u > 0xffffffffull) return cudaErrorInvalidValue;
+        char* live = static_cast<char*>(r.ptr);
+        const uint32_t words = static_cast<uint32_t>(r.bytes / 4u);
+        c.op[regions++] = {save ? live : block, save ? block : live, words};
+        most = std::max(most, words);
+        block += (r.bytes + 255u) & ~size_t(255u);
+    }
+    const uint32_t blocks = std::max(1u, std::min(most / 4u / 256u, 148u));
+    numi_cloth_state_copy_kernel<<<dim3(blocks, regions), 256, 0, h->stream>>>(c);
+    return cudaGetLastError();
+}
+
 int snapshot_slot(numi_cloth_t* h, uint32_t slot) {
     cudaSetDevice(h->device);
     size_t total = 0;
@@ -1766,26 +1817,16 @@ int snapshot_slot(numi_cloth_t* h, uint32_t slot) {
         if (cudaMalloc(&s.mem, total) != cudaSuccess) return NUMI_CLOTH_ENOMEM;
         s.bytes = total;
     }
-    size_t off = 0;
-    for (const auto& r : h->dynamic) {
-        if (cudaMemcpyAsync(static_cast<char*>(s.mem) + off, r.ptr, r.bytes, cudaMemcpyDeviceToDevice, h->stream) !=
-            cudaSuccess)
-            return NUMI_CLOTH_ECUDA;
-        off += (r.bytes + 255u) & ~size_t(255u);
-    }
+    if (copy_state(h, static_cast<char*>(s.mem), true) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+    s.grip_compliance = h->grip_compliance;
     s.valid = true;
     return NUMI_CLOTH_OK;
 }
 
 int restore_slot(numi_cloth_t* h, uint32_t slot) {
     cudaSetDevice(h->device);
-    size_t off = 0;
-    for (const auto& r : h->dynamic) {
-        if (cudaMemcpyAsync(r.ptr, static_cast<char*>(h->snaps[slot].mem) + off, r.bytes, cudaMemcpyDeviceToDevice,
-                            h->stream) != cudaSuccess)
-            return NUMI_CLOTH_ECUDA;
-        off += (r.bytes + 255u) & ~size_t(255u);
-    }
+    if (copy_state(h, static_cast<char*>(h->snaps[slot].mem), false) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+    h->grip_compliance = h->snaps[slot].grip_compliance;
     return NUMI_CLOTH_OK;
 }
 }  // namespace
@@ -2189,6 +2230,7 @@ struct numi_cloth_batch {
     std::vector<uint32_t> order;       // launch position -> caller index
     DeviceBuffers buf;
     DeviceCloth* d_cloths = nullptr;   // launch order
+    std::vector<DeviceCloth> host_cloths;   // the same on the host, as last laid out
     NumiClothConfig* d_cfg = nullptr;  // caller order, cloth-major
     uint32_t cfg_capacity = 0;         // substeps per cloth d_cfg holds
     uint32_t layout_substeps = 0;      // substeps the uploaded descriptors assume
@@ -2412,7 +2454,8 @@ int batch_layout(numi_cloth_batch* b, uint32_t substeps, bool edge) {
     const uint32_t ranks = b->fitted && !edge ? b->ranks : 1u;
     const size_t room = b->fitted ? batch_room(b, edge) : 0u;
     const uint32_t count = static_cast<uint32_t>(b->cloths.size());
-    std::vector<DeviceCloth> host(count);
+    std::vector<DeviceCloth>& host = b->host_cloths;
+    host.resize(count);
     for (uint32_t j = 0; j < count; ++j) {
         const uint32_t k = b->order[j];
         DeviceCloth d = b->cloths[k]->d;
@@ -2869,46 +2912,80 @@ struct Groups {
     std::vector<uint8_t> d, k, b, g;   // per record
 };
 
-int compliance_groups(numi_cloth* h, Groups& out) {
+// Distinct values, ascending, and every value's index among them.
+void distinct_values(const std::vector<float>& values, std::vector<float>& distinct, std::vector<uint8_t>& ids) {
+    distinct = values;
+    std::sort(distinct.begin(), distinct.end());
+    distinct.erase(std::unique(distinct.begin(), distinct.end()), distinct.end());
+    ids.resize(values.size());
+    for (size_t r = 0; r < values.size(); ++r)
+        ids[r] = static_cast<uint8_t>(std::lower_bound(distinct.begin(), distinct.end(), values[r]) - distinct.begin());
+}
+
+int read_compliance(numi_cloth* h) {
+    if (h->compliance_known) return NUMI_CLOTH_OK;
     const DeviceCloth& d = h->d;
     std::vector<float4> dm(d.d_count);
     std::vector<float2> km(d.k_count), bm(d.b_count);
-    std::vector<NumiClothGrip> gr(d.g_count);
     cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess && d.d_count) e = cudaMemcpy(dm.data(), d.d_mat, d.d_count * sizeof(float4), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && d.k_count) e = cudaMemcpy(km.data(), d.k_mat, d.k_count * sizeof(float2), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && d.b_count) e = cudaMemcpy(bm.data(), d.b_mat, d.b_count * sizeof(float2), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && d.g_count)
-        e = cudaMemcpy(gr.data(), d.grips, d.g_count * sizeof(NumiClothGrip), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return NUMI_CLOTH_ECUDA;
-    auto assign = [&](uint32_t family, const std::vector<float>& values, std::vector<uint8_t>& ids) {
-        std::vector<float> distinct = values;
-        std::sort(distinct.begin(), distinct.end());
-        distinct.erase(std::unique(distinct.begin(), distinct.end()), distinct.end());
+    std::vector<float> v;
+    for (const float4& m : dm) v.push_back(m.y);
+    distinct_values(v, h->compliance[0], h->compliance_id[0]);
+    v.clear();
+    for (const float2& m : km) v.push_back(m.y);
+    distinct_values(v, h->compliance[1], h->compliance_id[1]);
+    v.clear();
+    for (const float2& m : bm) v.push_back(m.y);
+    distinct_values(v, h->compliance[2], h->compliance_id[2]);
+    // more values than groups can be: read again when asked again
+    h->compliance_known = h->compliance[0].size() + h->compliance[1].size() + h->compliance[2].size() <= NUMI_CLOTH_MAX_GROUPS;
+    return NUMI_CLOTH_OK;
+}
+
+int compliance_groups(numi_cloth* h, Groups& out) {
+    const int rc = read_compliance(h);
+    if (rc != NUMI_CLOTH_OK) return rc;
+    auto assign = [&](uint32_t family, const std::vector<float>& distinct, const std::vector<uint8_t>& id,
+                      std::vector<uint8_t>& ids) {
         const uint32_t base = static_cast<uint32_t>(out.value.size());
         for (float v : distinct) {
             out.family.push_back(family);
             out.value.push_back(v);
         }
-        ids.resize(values.size());
-        for (size_t r = 0; r < values.size(); ++r)
-            ids[r] = static_cast<uint8_t>(
-                base + (std::lower_bound(distinct.begin(), distinct.end(), values[r]) - distinct.begin()));
+        ids.resize(id.size());
+        for (size_t r = 0; r < id.size(); ++r) ids[r] = static_cast<uint8_t>(base + id[r]);
     };
-    std::vector<float> v;
-    v.clear();
-    for (const float4& m : dm) v.push_back(m.y);
-    assign(0u, v, out.d);
-    v.clear();
-    for (const float2& m : km) v.push_back(m.y);
-    assign(1u, v, out.k);
-    v.clear();
-    for (const float2& m : bm) v.push_back(m.y);
-    assign(2u, v, out.b);
-    v.clear();
-    for (const NumiClothGrip& g : gr) v.push_back(g.targetOffsetAndCompliance.w);
-    assign(3u, v, out.g);
+    std::vector<float> grip;
+    std::vector<uint8_t> grip_id;
+    distinct_values(h->grip_compliance, grip, grip_id);
+    assign(0u, h->compliance[0], h->compliance_id[0], out.d);
+    assign(1u, h->compliance[1], h->compliance_id[1], out.k);
+    assign(2u, h->compliance[2], h->compliance_id[2], out.b);
+    assign(3u, grip, grip_id, out.g);
     return out.value.size() <= NUMI_CLOTH_MAX_GROUPS ? NUMI_CLOTH_OK : NUMI_CLOTH_EINVAL;
+}
+
+// The host copy after every record of `family` with compliance `from` took
+// `to`: the values stay distinct and ascending.
+void replaced_compliance(numi_cloth* h, uint32_t family, float from, float to) {
+    if (family == 3u) {
+        for (float& v : h->grip_compliance)
+            if (v == from) v = to;
+        return;
+    }
+    if (!h->compliance_known) return;
+    std::vector<float>& values = h->compliance[family];
+    std::vector<float> moved = values, distinct;
+    for (float& v : moved)
+        if (v == from) v = to;
+    std::vector<uint8_t> at;   // old index -> new index
+    distinct_values(moved, distinct, at);
+    for (uint8_t& id : h->compliance_id[family]) id = at[id];
+    values = distinct;
 }
 
 __global__ void numi_cloth_replace_compliance_kernel(DeviceCloth d, uint32_t family, float from, float to) {
@@ -2960,7 +3037,9 @@ extern "C" int numi_cloth_replace_compliance(numi_cloth_t* h, uint32_t family, f
     cudaSetDevice(h->device);
     h->tiles_dirty = h->tiles;   // the tile plan's items carry the materials
     numi_cloth_replace_compliance_kernel<<<64, 256, 0, h->stream>>>(h->d, family, from, to);
-    return cudaGetLastError() == cudaSuccess ? NUMI_CLOTH_OK : NUMI_CLOTH_ECUDA;
+    if (cudaGetLastError() != cudaSuccess) return NUMI_CLOTH_ECUDA;
+    replaced_compliance(h, family, from, to);
+    return NUMI_CLOTH_OK;
 }
 
 extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* configs, uint32_t substeps,
@@ -3081,26 +3160,8 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
             e = cudaMemcpyAsync(dst[f], lists[f]->data(), lists[f]->size(), cudaMemcpyHostToDevice, h->stream);
     if (e != cudaSuccess) return NUMI_CLOTH_ECUDA;
 
-    auto save = [&](uint32_t slot) {
-        size_t off = 0;
-        for (const auto& r : h->dynamic) {
-            if (cudaMemcpyAsync(ckpt + slot * state_bytes + off, r.ptr, r.bytes, cudaMemcpyDeviceToDevice, h->stream) !=
-                cudaSuccess)
-                return false;
-            off += (r.bytes + 255u) & ~size_t(255u);
-        }
-        return true;
-    };
-    auto load = [&](uint32_t slot) {
-        size_t off = 0;
-        for (const auto& r : h->dynamic) {
-            if (cudaMemcpyAsync(r.ptr, ckpt + slot * state_bytes + off, r.bytes, cudaMemcpyDeviceToDevice, h->stream) !=
-                cudaSuccess)
-                return false;
-            off += (r.bytes + 255u) & ~size_t(255u);
-        }
-        return true;
-    };
+    auto save = [&](uint32_t slot) { return copy_state(h, ckpt + slot * state_bytes, true) == cudaSuccess; };
+    auto load = [&](uint32_t slot) { return copy_state(h, ckpt + slot * state_bytes, false) == cudaSuccess; };
 
     // forward in the handle's own launch shape: taped where the tape holds
     // it, else checkpointed (the last segment of a cloth without fruits is
@@ -3341,30 +3402,29 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         return NUMI_CLOTH_ECUDA;
     std::vector<AdjointArgs> args(count);
     std::vector<DeviceCloth> replay(count), plain(count);
+    std::vector<char> host_arena(arena_bytes);   // filled cloth by cloth, uploaded once
     size_t cursor = 0;
     float4* tape_at = tape;
-    auto carve = [&](size_t bytes) {
+    auto carve = [&](const void* from, size_t bytes, size_t room) {
         char* p = arena + cursor;
-        cursor += round256(bytes);
+        if (bytes != 0u) std::memcpy(host_arena.data() + cursor, from, bytes);
+        cursor += round256(room);
         return p;
     };
     for (uint32_t k = 0; k < count; ++k) {
         numi_cloth* h = b->cloths[k];
         const uint32_t n = h->d.n;
         const uint32_t slots = static_cast<uint32_t>(phases[k].size()) + 1u;
-        uint4* ph = reinterpret_cast<uint4*>(carve(phases[k].size() * sizeof(uint4)));
         double4* gx = adjoint[k];
-        uint8_t* gd = reinterpret_cast<uint8_t*>(carve(groups[k].d.size() + 1u));
-        uint8_t* gk = reinterpret_cast<uint8_t*>(carve(groups[k].k.size() + 1u));
-        uint8_t* gb = reinterpret_cast<uint8_t*>(carve(groups[k].b.size() + 1u));
-        uint8_t* gg = reinterpret_cast<uint8_t*>(carve(groups[k].g.size() + 1u));
-        e = cudaMemcpyAsync(ph, phases[k].data(), phases[k].size() * sizeof(uint4), cudaMemcpyHostToDevice, b->stream);
-        const std::vector<uint8_t>* lists[4] = {&groups[k].d, &groups[k].k, &groups[k].b, &groups[k].g};
-        uint8_t* dst[4] = {gd, gk, gb, gg};
-        for (int f = 0; f < 4 && e == cudaSuccess; ++f)
-            if (!lists[f]->empty())
-                e = cudaMemcpyAsync(dst[f], lists[f]->data(), lists[f]->size(), cudaMemcpyHostToDevice, b->stream);
-        if (e != cudaSuccess) return NUMI_CLOTH_ECUDA;
+        const size_t ph_bytes = phases[k].size() * sizeof(uint4);
+        const uint4* ph = reinterpret_cast<const uint4*>(carve(phases[k].data(), ph_bytes, ph_bytes));
+        auto ids = [&](const std::vector<uint8_t>& list) {
+            return reinterpret_cast<const uint8_t*>(carve(list.data(), list.size(), list.size() + 1u));
+        };
+        const uint8_t* gd = ids(groups[k].d);
+        const uint8_t* gk = ids(groups[k].k);
+        const uint8_t* gb = ids(groups[k].b);
+        const uint8_t* gg = ids(groups[k].g);
         plain[k] = h->d;
         AdjointArgs& A = args[k];
         A.cloth = d_plain + k;
@@ -3394,20 +3454,17 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         A.nonsmooth = d_rough + k;
     }
     // replay descriptors: the batch's launch-order descriptors with tapes
-    {
-        std::vector<DeviceCloth> base(count);
-        e = cudaMemcpy(base.data(), b->d_cloths, count * sizeof(DeviceCloth), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return NUMI_CLOTH_ECUDA;
-        for (uint32_t j = 0; j < count; ++j) {
-            const uint32_t k = b->order[j];
-            replay[j] = base[j];
-            replay[j].tape = const_cast<float4*>(args[k].tape);
-            replay[j].tape_v = const_cast<float4*>(args[k].tape_v);
-            replay[j].tape_slots = args[k].slots;
+    for (uint32_t j = 0; j < count; ++j) {
+        const uint32_t k = b->order[j];
+        replay[j] = b->host_cloths[j];
+        replay[j].tape = const_cast<float4*>(args[k].tape);
+        replay[j].tape_v = const_cast<float4*>(args[k].tape_v);
+        replay[j].tape_slots = args[k].slots;
         replay[j].yarn_touched = d_touched;
-        }
     }
-    e = cudaMemcpyAsync(d_replay, replay.data(), count * sizeof(DeviceCloth), cudaMemcpyHostToDevice, b->stream);
+    e = cudaMemcpyAsync(arena, host_arena.data(), arena_bytes, cudaMemcpyHostToDevice, b->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(d_replay, replay.data(), count * sizeof(DeviceCloth), cudaMemcpyHostToDevice, b->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_plain, plain.data(), count * sizeof(DeviceCloth), cudaMemcpyHostToDevice, b->stream);
     if (e == cudaSuccess && n_tracked)
         e = cudaMemcpyAsync(d_tracked, tracked, n_tracked * sizeof(uint32_t), cudaMemcpyHostToDevice, b->stream);
