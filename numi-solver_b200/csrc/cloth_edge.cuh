@@ -742,14 +742,14 @@ __device__ void edge_candidates(Ctx& ctx, bool swept, bool rebuilt) {
 // [m] position of each segment, then the build's scratch (two sets of the
 // three lists, the side of each segment, the parent axis of each position).
 #define NC_EDGE_TREE_MAX 4096u
-#define NC_EDGE_TREE_KEY_BYTES (NC_EDGE_TREE_MAX * 8u)
-#define NC_EDGE_TREE_WORDS 14u   /* edge_tree words per segment (13, and one flag word) */
+#define NC_EDGE_TREE_KEY_BYTES (NC_EDGE_TREE_MAX * 20u)   /* the build's shared memory (TreeShared) */
+#define NC_EDGE_TREE_WORDS 14u   /* edge_tree words per segment (the build uses 5, and one flag word) */
 #define NC_EDGE_TREE_WARM 8u     /* odd-even passes tried on the previous order before a full sort */
 __shared__ unsigned char nc_edge_tree_axis[NC_EDGE_TREE_MAX / 8u];
 __shared__ uint32_t nc_edge_scan[3][32];
 
-// The node of position p (or of index j, a path of `level` left/right bits)
-// at depth `level`; false past a leaf.
+// The node of index j, a path of `level` left/right bits, at depth `level`;
+// false past a leaf.
 __device__ __forceinline__ bool tree_node_of_path(uint32_t m, uint32_t level, uint32_t j, uint32_t& b, uint32_t& e) {
     b = 0u;
     e = m;
@@ -762,23 +762,6 @@ __device__ __forceinline__ bool tree_node_of_path(uint32_t m, uint32_t level, ui
             e = mid;
     }
     return true;
-}
-__device__ __forceinline__ uint32_t tree_path_of_position(uint32_t m, uint32_t level, uint32_t p, uint32_t& b,
-                                                          uint32_t& e) {
-    b = 0u;
-    e = m;
-    uint32_t j = 0u;
-    for (uint32_t l = 0; l < level && e - b > 8u; ++l) {
-        const uint32_t mid = b + (e - b) / 2u;
-        j <<= 1;
-        if (p >= mid) {
-            b = mid;
-            j |= 1u;
-        } else {
-            e = mid;
-        }
-    }
-    return j;
 }
 // Float bits in an order of unsigned integers (zeros of either sign equal).
 __device__ __forceinline__ uint32_t ordered_bits(float v) {
@@ -858,60 +841,54 @@ __device__ void block_sort(unsigned long long* keys, uint32_t n) {
     }
 }
 
-// Exclusive prefix counts, for each of the three lists L[a][0..m), of the
-// members that go right (right[segment] = 1), into pre[a][0..m) (shared
-// memory; counts below 65,536): every thread a contiguous run of each list.
-__device__ void tree_prefix3(const uint32_t* L, const uint32_t* right, unsigned short* pre, uint32_t m) {
-    const uint32_t per = (m + blockDim.x - 1u) / blockDim.x;
-    const uint32_t lo = min(threadIdx.x * per, m), hi = min(lo + per, m);
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t sum[3], incl[3];
-#pragma unroll
-    for (uint32_t a = 0; a < 3u; ++a) {
-        sum[a] = 0u;
-        for (uint32_t p = lo; p < hi; ++p) sum[a] += right[L[a * m + p]];
-        incl[a] = sum[a];
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl[a], o);
-            if (lane >= static_cast<uint32_t>(o)) incl[a] += y;
-        }
-        if (lane == 31u) nc_edge_scan[a][warp] = incl[a];
-    }
-    __syncthreads();
-    if (warp < 3u) {
-        const uint32_t warps = blockDim.x >> 5;
-        uint32_t w = lane < warps ? nc_edge_scan[warp][lane] : 0u;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= static_cast<uint32_t>(o)) w += y;
-        }
-        if (lane < warps) nc_edge_scan[warp][lane] = w;
-    }
-    __syncthreads();
-#pragma unroll
-    for (uint32_t a = 0; a < 3u; ++a) {
-        uint32_t run = (warp > 0u ? nc_edge_scan[a][warp - 1u] : 0u) + incl[a] - sum[a];
-        for (uint32_t p = lo; p < hi; ++p) {
-            pre[a * m + p] = static_cast<unsigned short>(run);
-            run += right[L[a * m + p]];
+// The build's arrays in the launch's dynamic shared memory: the sort keys and
+// in their place, once the axes are sorted, the prefix counts of the lists
+// and the side of each segment; two sets of the three lists.
+struct TreeShared {
+    union {
+        unsigned long long keys[NC_EDGE_TREE_MAX];
+        struct {
+            unsigned short pre[3][NC_EDGE_TREE_MAX];
+            unsigned char right[NC_EDGE_TREE_MAX];
+        };
+    };
+    unsigned short list[2][3][NC_EDGE_TREE_MAX];
+};
+static_assert(sizeof(TreeShared) <= NC_EDGE_TREE_KEY_BYTES, "box tree shared memory");
+#define NC_EDGE_TREE_PER (NC_EDGE_TREE_MAX / NC_THREADS)   /* most positions of a thread */
+
+// Axis of a splitting node [b, e): the longest extent of its members' centres
+// (the first of equals).  The lists are in axis order, so the extent along an
+// axis is between the ends of that axis' list; a centre that is no number
+// sorts to an end and has no extent, so then the members are scanned.
+__device__ __forceinline__ unsigned char tree_axis(const float4* centre, const unsigned short (*L)[NC_EDGE_TREE_MAX],
+                                                   uint32_t b, uint32_t e) {
+    V3 lo{centre[L[0][b]].x, centre[L[1][b]].y, centre[L[2][b]].z};
+    V3 hi{centre[L[0][e - 1u]].x, centre[L[1][e - 1u]].y, centre[L[2][e - 1u]].z};
+    if (!(lo.x == lo.x && lo.y == lo.y && lo.z == lo.z && hi.x == hi.x && hi.y == hi.y && hi.z == hi.z)) {
+        lo = V3{INFINITY, INFINITY, INFINITY};
+        hi = V3{-INFINITY, -INFINITY, -INFINITY};
+        for (uint32_t p = b; p < e; ++p) {
+            const float4 c = centre[L[0][p]];
+            lo = V3{fminf(lo.x, c.x), fminf(lo.y, c.y), fminf(lo.z, c.z)};
+            hi = V3{fmaxf(hi.x, c.x), fmaxf(hi.y, c.y), fmaxf(hi.z, c.z)};
         }
     }
-    __syncthreads();
+    const V3 ext = hi - lo;
+    return static_cast<unsigned char>(ext.y > ext.x ? (ext.z > ext.y ? 2u : 1u) : (ext.z > ext.x ? 2u : 0u));
 }
 
 __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
     const DeviceCloth& d = ctx.d;
     // the sort keys, then the prefix counts, in the launch's dynamic shared
     // memory
-    unsigned long long* keys = reinterpret_cast<unsigned long long*>(nc_frame_smem + ctx.s.tree_keys);
-    unsigned short* pre = reinterpret_cast<unsigned short*>(keys);
+    TreeShared& ts = *reinterpret_cast<TreeShared*>(nc_frame_smem + ctx.s.tree_keys);
+    unsigned long long* keys = ts.keys;
+    unsigned short (*pre)[NC_EDGE_TREE_MAX] = ts.pre;
     const uint32_t m = d.y_count;
     const float ex = 0.5f * (2.0f * ctx.c.radius);
     uint32_t* ord = d.edge_tree;
-    uint32_t* lists = d.edge_tree + 2u * m;   // [2][3][m]
-    uint32_t* right = lists + 6u * m;         // per segment: goes to the right child
-    uint32_t* leaf_axis = right + m;          // per position: axis of its deepest split
-    uint32_t* gsort = leaf_axis + m;          // [3][m] the last build's order along each axis
+    uint32_t* gsort = d.edge_tree + 2u * m;   // [3][m] the last build's order along each axis
     uint32_t* valid = gsort + 3u * m;         // 1 once a tree was built
     float4* prev = d.edge_centre + m;         // the last build's centres
     // Every array here is written and read by this CTA alone between CTA
@@ -931,7 +908,6 @@ __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
             changed = changed || __float_as_uint(c.x) != __float_as_uint(q.x) ||
                       __float_as_uint(c.y) != __float_as_uint(q.y) || __float_as_uint(c.z) != __float_as_uint(q.z);
         }
-        leaf_axis[k] = 3u;
     }
     // the same centres as the last build: the same tree
     if (!__syncthreads_or(changed)) return;
@@ -975,79 +951,115 @@ __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
         if (!sorted) block_sort(keys, size);
         for (uint32_t p = threadIdx.x; p < m; p += blockDim.x) {
             const uint32_t sg = static_cast<uint32_t>(keys[p] & 0xfffull);
-            lists[a * m + p] = sg;
+            ts.list[0][a][p] = static_cast<unsigned short>(sg);
             gsort[a * m + p] = sg;
         }
         __syncthreads();
     }
+    // Level by level, every thread a run of `per` positions of all three
+    // lists.  The node a position lies in does not depend on the data, so a
+    // thread keeps its positions' nodes (first | end << 16) from level to
+    // level, and the axis of each one's deepest split (two bits a position).
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, warps = blockDim.x >> 5;
+    const uint32_t per = (m + blockDim.x - 1u) / blockDim.x;
+    const uint32_t own = min(threadIdx.x * per, m), mine = min(per, m - own);
+    uint32_t node[NC_EDGE_TREE_PER];
+#pragma unroll
+    for (uint32_t i = 0; i < NC_EDGE_TREE_PER; ++i) node[i] = m << 16;
+    uint32_t axes = 0xffffffffu;
     uint32_t cur = 0u;
     for (uint32_t level = 0; level < 32u; ++level) {
-        const uint32_t* L = lists + cur * 3u * m;
-        uint32_t* N = lists + (cur ^ 1u) * 3u * m;
-        // centre bounds and axis of every node of the level that splits
+        const unsigned short (*L)[NC_EDGE_TREE_MAX] = ts.list[cur];
+        unsigned short (*N)[NC_EDGE_TREE_MAX] = ts.list[cur ^ 1u];
+        // axis of every node of the level that splits
         const uint32_t nodes = 1u << level;
         bool any = false;
-        for (uint32_t j = warp; j < nodes && j < NC_EDGE_TREE_MAX / 8u; j += warps) {
+        for (uint32_t j = threadIdx.x; j < nodes && j < NC_EDGE_TREE_MAX / 8u; j += blockDim.x) {
             uint32_t b, e;
             if (!tree_node_of_path(m, level, j, b, e) || e - b <= 8u) continue;
-            V3 lo{INFINITY, INFINITY, INFINITY}, hi{-INFINITY, -INFINITY, -INFINITY};
-            for (uint32_t p = b + lane; p < e; p += 32u) {
-                const float4 c = d.edge_centre[L[p]];
-                lo = V3{fminf(lo.x, c.x), fminf(lo.y, c.y), fminf(lo.z, c.z)};
-                hi = V3{fmaxf(hi.x, c.x), fmaxf(hi.y, c.y), fmaxf(hi.z, c.z)};
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o));
-                lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, o));
-                lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, o));
-                hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
-                hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, o));
-                hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, o));
-            }
-            const V3 ext = hi - lo;
-            if (lane == 0)
-                nc_edge_tree_axis[j] = static_cast<unsigned char>(
-                    ext.y > ext.x ? (ext.z > ext.y ? 2u : 1u) : (ext.z > ext.x ? 2u : 0u));
+            nc_edge_tree_axis[b >> 3] = tree_axis(d.edge_centre, L, b, e);
             any = true;
         }
         if (!__syncthreads_or(any)) break;
         // sides: the second half of a splitting node's axis list goes right
-        for (uint32_t p = threadIdx.x; p < m; p += blockDim.x) {
-            uint32_t b, e;
-            const uint32_t j = tree_path_of_position(m, level, p, b, e);
+#pragma unroll
+        for (uint32_t i = 0; i < NC_EDGE_TREE_PER; ++i) {
+            if (i >= mine) break;
+            const uint32_t p = own + i, b = node[i] & 0xffffu, e = node[i] >> 16;
             if (e - b <= 8u) {
-                right[L[p]] = 0u;
+                ts.right[L[0][p]] = 0u;
                 continue;
             }
-            const uint32_t a = nc_edge_tree_axis[j];
-            right[L[a * m + p]] = p - b >= (e - b) / 2u ? 1u : 0u;
-            leaf_axis[p] = a;
+            const uint32_t a = nc_edge_tree_axis[b >> 3];
+            ts.right[L[a][p]] = p - b >= (e - b) / 2u ? 1u : 0u;
+            axes = (axes & ~(3u << (2u * i))) | (a << (2u * i));
+        }
+        __syncthreads();
+        // exclusive prefix counts of the members that go right, list by list
+        uint32_t bits[3], incl[3];
+#pragma unroll
+        for (uint32_t a = 0; a < 3u; ++a) {
+            bits[a] = 0u;
+#pragma unroll
+            for (uint32_t i = 0; i < NC_EDGE_TREE_PER; ++i) {
+                if (i >= mine) break;
+                bits[a] |= static_cast<uint32_t>(ts.right[L[a][own + i]]) << i;
+            }
+            incl[a] = __popc(bits[a]);
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl[a], o);
+                if (lane >= static_cast<uint32_t>(o)) incl[a] += y;
+            }
+            if (lane == 31u) nc_edge_scan[a][warp] = incl[a];
+        }
+        __syncthreads();
+        if (warp < 3u) {
+            uint32_t w = lane < warps ? nc_edge_scan[warp][lane] : 0u;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= static_cast<uint32_t>(o)) w += y;
+            }
+            if (lane < warps) nc_edge_scan[warp][lane] = w;
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t a = 0; a < 3u; ++a) {
+            incl[a] += (warp > 0u ? nc_edge_scan[a][warp - 1u] : 0u) - __popc(bits[a]);
+#pragma unroll
+            for (uint32_t i = 0; i < NC_EDGE_TREE_PER; ++i) {
+                if (i >= mine) break;
+                pre[a][own + i] = static_cast<unsigned short>(incl[a] + __popc(bits[a] & ((1u << i) - 1u)));
+            }
         }
         __syncthreads();
         // every list: stable partition of each splitting node's range
-        tree_prefix3(L, right, pre, m);
-        for (uint32_t q = threadIdx.x; q < 3u * m; q += blockDim.x) {
-            const uint32_t a = q / m, p = q - a * m;
-            uint32_t b, e;
-            tree_path_of_position(m, level, p, b, e);
-            const uint32_t sg = L[q];
-            uint32_t to = p;
-            if (e - b > 8u) {
-                const uint32_t rights = static_cast<uint32_t>(pre[q]) - static_cast<uint32_t>(pre[a * m + b]);
-                to = right[sg] != 0u ? b + (e - b) / 2u + rights : p - rights;
+#pragma unroll
+        for (uint32_t i = 0; i < NC_EDGE_TREE_PER; ++i) {
+            if (i >= mine) break;
+            const uint32_t p = own + i, b = node[i] & 0xffffu, e = node[i] >> 16;
+            const bool split = e - b > 8u;
+            const uint32_t mid = b + (e - b) / 2u;
+#pragma unroll
+            for (uint32_t a = 0; a < 3u; ++a) {
+                uint32_t to = p;
+                if (split) {
+                    const uint32_t rights = incl[a] + __popc(bits[a] & ((1u << i) - 1u)) - pre[a][b];
+                    to = ((bits[a] >> i) & 1u) != 0u ? mid + rights : p - rights;
+                }
+                N[a][to] = L[a][p];
             }
-            N[a * m + to] = sg;
+            if (split) node[i] = p >= mid ? mid | (e << 16) : b | (mid << 16);
         }
         __syncthreads();
         cur ^= 1u;
     }
-    const uint32_t* L = lists + cur * 3u * m;
-    for (uint32_t p = threadIdx.x; p < m; p += blockDim.x) {
-        const uint32_t a = leaf_axis[p];
-        ord[p] = a < 3u ? L[a * m + p] : p;
-        prev[p] = d.edge_centre[p];
+#pragma unroll
+    for (uint32_t i = 0; i < NC_EDGE_TREE_PER; ++i) {
+        if (i >= mine) break;
+        const uint32_t p = own + i, a = (axes >> (2u * i)) & 3u;
+        ord[p] = a < 3u ? ts.list[cur][a][p] : p;
     }
+    for (uint32_t p = threadIdx.x; p < m; p += blockDim.x) prev[p] = d.edge_centre[p];
     __syncthreads();
     for (uint32_t p = threadIdx.x; p < m; p += blockDim.x) ord[m + ord[p]] = p;
     if (threadIdx.x == 0) *valid = 1u;
