@@ -489,18 +489,28 @@ __device__ __forceinline__ bool fruit_near_segment(const float4& fs, const float
 }
 
 // Friction contact records of one yarn segment during a sweep (see
-// DeviceCloth::yarn_slot_a/b): the slot tags are loaded at the segment's
-// first contact and kept in registers; the first record of a substep takes
+// DeviceCloth::yarn_slot_a/b): the slot tags are loaded ahead of the
+// segment's first contact and kept in registers; the first record of a substep takes
 // slot 0 without a search and retires the older ones.
 struct SegRecords {
     uint32_t seg;
     bool loaded, live, was_live, recorded;
+    uint32_t epoch;
     uint32_t rtag[NC_YARN_SLOTS];
 
     __device__ explicit SegRecords(uint32_t s)
-        : seg(s), loaded(false), live(false), was_live(false), recorded(false) {
+        : seg(s), loaded(false), live(false), was_live(false), recorded(false), epoch(0u) {
 #pragma unroll
         for (uint32_t q = 0; q < NC_YARN_SLOTS; ++q) rtag[q] = 0u;
+    }
+
+    // Start the loads of the segment's epoch and slot tags (once it has a
+    // fruit to test: the contact's roots and quotients then hide them).
+    __device__ void preload(const Ctx& ctx) {
+        epoch = __ldcg(ctx.d.yarn_live + seg);
+#pragma unroll
+        for (uint32_t q = 0; q < NC_YARN_SLOTS; ++q)
+            rtag[q] = __float_as_uint(__ldcg(&ctx.d.yarn_slot_b[seg * NC_YARN_SLOTS + q].z));
     }
 
     // Add impulse imp along -n on fruit f with segment weights w0, w1.
@@ -508,12 +518,11 @@ struct SegRecords {
         const DeviceCloth& d = ctx.d;
         if (!loaded) {
             loaded = true;
-            live = __ldcg(d.yarn_live + seg) == ctx.epoch;
+            live = epoch == ctx.epoch;
             was_live = live;
-            if (live) {
+            if (!live) {
 #pragma unroll
-                for (uint32_t q = 0; q < NC_YARN_SLOTS; ++q)
-                    rtag[q] = __float_as_uint(__ldcg(&d.yarn_slot_b[seg * NC_YARN_SLOTS + q].z));
+                for (uint32_t q = 0; q < NC_YARN_SLOTS; ++q) rtag[q] = 0u;
             }
         }
         const uint32_t tag = (ctx.epoch << 6) | f;
@@ -640,6 +649,7 @@ __device__ __forceinline__ bool yarn_warp_contacts(const Ctx& ctx, bool valid, b
     }
     bool changed = false;
     SegRecords rec(seg);
+    if (owner && mask != 0ull) rec.preload(ctx);
     while (mask != 0ull) {
         const uint32_t f = static_cast<uint32_t>(__ffsll(static_cast<long long>(mask)) - 1);
         mask &= mask - 1ull;
@@ -770,7 +780,7 @@ __device__ __forceinline__ void swept_contact_batch(Ctx& ctx, const Batch& bt, b
         const uint2 ij = __ldg(d.d_ij + seg);
         float4 pa = px(ctx, ij.x), pb = px(ctx, ij.y);
         const V3 qa = xyz(ld(d.xp + ij.x)), qb = xyz(ld(d.xp + ij.y));
-        bool changed = false;
+        bool changed = false, tested = false;
         SegRecords rec(seg);
         for (uint32_t f = 0; f < nf; ++f) {
             const float4 fx = s_fx[f], fp = s_fp[f];
@@ -785,6 +795,8 @@ __device__ __forceinline__ void swept_contact_batch(Ctx& ctx, const Batch& bt, b
                 fmaxf(fx.y, fp.y) < slo.y - slack || fminf(fx.y, fp.y) > shi.y + slack ||
                 fmaxf(fx.z, fp.z) < slo.z - slack || fminf(fx.z, fp.z) > shi.z + slack)
                 continue;
+            if (!tested) rec.preload(ctx);
+            tested = true;
             const V3 X = xyz(fx), P = xyz(fp);
             float bound = len3(X - P) + len3(xyz(pa) - qa);
             bound = bound + len3(xyz(pb) - qb);
@@ -2004,6 +2016,16 @@ __device__ void residual_partials(Ctx& ctx, double* out3) {
     const DeviceCloth& d = ctx.d;
     const SubCfg& c = ctx.c;
     double strain = 0.0, ground = 0.0, fruit = 0.0;
+    // the fruits in shared memory (the reductions' array, not in use yet):
+    // read from global memory, every segment waited for five L2 loads of one
+    // fruit after the other, 30 us a pass on the bag's 12
+    float4* s_f = reinterpret_cast<float4*>(&nc_red_smem[0][0]);   // position, radius
+    for (uint32_t f = threadIdx.x; f < d.f_count; f += blockDim.x) {
+        const NumiClothFruit& fr = d.fruits[f];
+        const float4 x = __ldcg(reinterpret_cast<const float4*>(&fr.positionAndInverseMass));
+        s_f[f] = make_float4(x.x, x.y, x.z, __ldcg(&fr.previousAndRadius.w));
+    }
+    __syncthreads();
     for (Range r = item_range(ctx, d.d_count); r.i < r.end; r.i += r.stride) {
         const uint32_t k = r.i;
         const float4 m = __ldg(d.d_mat + k);
@@ -2033,10 +2055,9 @@ __device__ void residual_partials(Ctx& ctx, double* out3) {
                 const float4 pa = px(ctx, ij.x);
                 const float4 pb = px(ctx, ij.y);
                 for (uint32_t f = 0; f < d.f_count; ++f) {
-                    const NumiClothFruit& fr = d.fruits[f];
-                    const double X[3] = {__ldcg(&fr.positionAndInverseMass.x), __ldcg(&fr.positionAndInverseMass.y),
-                                         __ldcg(&fr.positionAndInverseMass.z)};
-                    const double target = static_cast<double>(__ldcg(&fr.previousAndRadius.w)) + c.radius;
+                    const float4 fr = s_f[f];
+                    const double X[3] = {fr.x, fr.y, fr.z};
+                    const double target = static_cast<double>(fr.w) + c.radius;
                     const double A[3] = {pa.x, pa.y, pa.z};
                     const double B[3] = {pb.x, pb.y, pb.z};
                     bool outside = false;
@@ -2058,6 +2079,7 @@ __device__ void residual_partials(Ctx& ctx, double* out3) {
         }
     }
     double (*s_r)[NC_BLOCK_MAX] = nc_red_smem;
+    __syncthreads();   // the staged fruits are read
     s_r[0][threadIdx.x] = strain;
     s_r[1][threadIdx.x] = ground;
     s_r[2][threadIdx.x] = fruit;
