@@ -328,17 +328,18 @@ struct FruitShared {
 
 // The fruit/yarn friction sweep's recorded segments, staged by the fruit CTA
 // in tile mode (friction_stage, after FruitShared in its shared memory):
-// segment, slot tags and records, endpoint particles, for every endpoint
-// the first endpoint slot with the same particle, endpoint positions and
-// velocities.
+// segment, its live records in ascending fruit order with what of their
+// friction no velocity enters (normal and friction limit, segment weights and
+// fruit), endpoint particles, for every endpoint the first endpoint slot with
+// the same particle, endpoint positions and velocities.
 struct FrictionStage {
     uint32_t count;                        // staged segments (NC_FRICTION_STAGE + 1: too many)
     uint32_t seg[NC_FRICTION_STAGE];
-    uint32_t tag[NC_FRICTION_STAGE][NC_YARN_SLOTS];
+    uint32_t records[NC_FRICTION_STAGE];
     uint32_t pid[2 * NC_FRICTION_STAGE];
     unsigned short rep[2 * NC_FRICTION_STAGE];
     float4 x[2 * NC_FRICTION_STAGE];
     float4 v[2 * NC_FRICTION_STAGE];
-    float4 ra[NC_FRICTION_STAGE][NC_YARN_SLOTS];
-    float4 rb[NC_FRICTION_STAGE][NC_YARN_SLOTS];
+    float4 normal[NC_FRICTION_STAGE][NC_YARN_SLOTS];   // xyz, friction limit
+    float4 weight[NC_FRICTION_STAGE][NC_YARN_SLOTS];   // first, second endpoint, fruit (bits)
 };

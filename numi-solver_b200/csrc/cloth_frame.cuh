@@ -2216,14 +2216,10 @@ __device__ __forceinline__ FrictionSeg friction_seg(const DeviceCloth& d, uint32
     return fs;
 }
 
-// The friction of one segment on its loaded endpoints: positions pa, pb,
-// velocities va, vb (updated), slot tags st and the slots' records ra, rb
-// (only the live ones are read).
-__device__ __forceinline__ void yarn_friction_core(const Ctx& ctx, const float4& pa, const float4& pb, float4& va,
-                                                   float4& vb, const uint32_t* st, const float4* ra, const float4* rb,
-                                                   const float4* s_vw, const float4* s_or, unsigned long long* s_sum) {
-    const SubCfg& c = ctx.c;
-    // Live records of this segment, visited in ascending fruit order.
+// The live slots of a segment (tags st) in ascending fruit order: calls
+// visit(slot, fruit) for each.
+template <class F>
+__device__ __forceinline__ void friction_visits(const Ctx& ctx, const uint32_t* st, F&& visit) {
     const uint32_t live = ctx.epoch & 0x3ffffffu;
     uint32_t fruit_of[NC_YARN_SLOTS];
     uint32_t nlive = 0;
@@ -2232,7 +2228,7 @@ __device__ __forceinline__ void yarn_friction_core(const Ctx& ctx, const float4&
         fruit_of[q] = ((st[q] >> 6) == live) ? (st[q] & 63u) : 0xffffffffu;
         nlive += fruit_of[q] != 0xffffffffu ? 1u : 0u;
     }
-    for (uint32_t visit = 0; visit < nlive; ++visit) {
+    for (uint32_t k = 0; k < nlive; ++k) {
         uint32_t slot = 0;
         uint32_t f = 0xffffffffu;
 #pragma unroll
@@ -2244,6 +2240,86 @@ __device__ __forceinline__ void yarn_friction_core(const Ctx& ctx, const float4&
 #pragma unroll
         for (uint32_t q = 0; q < NC_YARN_SLOTS; ++q)
             if (q == slot) fruit_of[q] = 0xffffffffu;
+        visit(slot, f);
+    }
+}
+
+// What of a record's friction no velocity enters: its normal, the segment
+// weights and the friction limit, from the record (sa, sb).  False where the
+// record has no friction.
+__device__ __forceinline__ bool friction_record(const Ctx& ctx, const float4& sa, const float4& sb, V3& normal,
+                                                float wt[2], float& limit) {
+    const float ni = sa.w;
+    const V3 wn{sa.x, sa.y, sa.z};
+    if (ni <= 0.0f || lsq(wn) < 1.0e-20f) return false;
+    normal = normalized3(wn);
+    wt[0] = sb.x / ni;
+    wt[1] = sb.y / ni;
+    const float sum = wt[0] + wt[1];
+    if (sum <= 1.0e-12f) return false;
+    wt[0] = wt[0] / sum;
+    wt[1] = wt[1] / sum;
+    limit = ctx.c.mu_fruit_yarn * ni;
+    return true;
+}
+
+// The friction of one record on its loaded endpoints: positions pa, pb,
+// velocities va, vb (updated).
+__device__ __forceinline__ void friction_apply(const Ctx& ctx, uint32_t f, V3 normal, const float wt[2], float limit,
+                                               const float4& pa, const float4& pb, float4& va, float4& vb,
+                                               const float4* s_vw, const float4* s_or, unsigned long long* s_sum) {
+    const SubCfg& c = ctx.c;
+    FruitState fr;
+    {
+        const float4 vw = s_vw[f];
+        const float4 orr = s_or[f];
+        fr.v = V3{vw.x, vw.y, vw.z};
+        fr.w = vw.w;
+        fr.omega = V3{orr.x, orr.y, orr.z};
+        fr.radius = orr.w;
+    }
+    const V3 yv = (V3{0.0f, 0.0f, 0.0f} + xyz(va) * wt[0]) + xyz(vb) * wt[1];
+    const V3 off = normal * -fr.radius;
+    const V3 bcv = fr.v + cross3(fr.omega, off);
+    const V3 rel = bcv - yv;
+    const V3 tv = rel - normal * dot3(rel, normal);
+    const float slip = len3(tv);
+    if (slip < 1.0e-10f) return;
+    const V3 t = vdiv(tv, slip);
+    const float inv_i = inverse_inertia(fr.w, fr.radius);
+    float den = fr.w + inv_i * lsq(cross3(off, t));
+    V3 resp[2];
+    const float4* pp[2] = {&pa, &pb};
+    for (int s = 0; s < 2; ++s) {
+        resp[s] = t * pp[s]->w;
+        if (c.ground && pp[s]->z <= c.radius + 1.0e-6f && resp[s].z < 0.0f) resp[s].z = 0.0f;
+        den = den + dot3(t, resp[s]) * wt[s] * wt[s];
+    }
+    if (den <= 0.0f) return;
+    const float ti = fminf(slip / den, limit);
+    if (ti <= 0.0f) return;
+    const V3 imp = t * -ti;
+    const V3 dv = imp * fr.w;
+    const V3 dw = cross3(off, imp) * inv_i;
+    cta_sums_add(s_sum + 6u * f + 0u, dv.x);
+    cta_sums_add(s_sum + 6u * f + 1u, dv.y);
+    cta_sums_add(s_sum + 6u * f + 2u, dv.z);
+    cta_sums_add(s_sum + 6u * f + 3u, dw.x);
+    cta_sums_add(s_sum + 6u * f + 4u, dw.y);
+    cta_sums_add(s_sum + 6u * f + 5u, dw.z);
+    const V3 na = xyz(va) + resp[0] * (ti * wt[0]);
+    const V3 nb = xyz(vb) + resp[1] * (ti * wt[1]);
+    va = with_xyz(va, na);
+    vb = with_xyz(vb, nb);
+}
+
+// The friction of one segment on its loaded endpoints: positions pa, pb,
+// velocities va, vb (updated), slot tags st and the slots' records ra, rb
+// (only the live ones are read).
+__device__ __forceinline__ void yarn_friction_core(const Ctx& ctx, const float4& pa, const float4& pb, float4& va,
+                                                   float4& vb, const uint32_t* st, const float4* ra, const float4* rb,
+                                                   const float4* s_vw, const float4* s_or, unsigned long long* s_sum) {
+    friction_visits(ctx, st, [&](uint32_t slot, uint32_t f) {
         float4 sa = ra[0], sb = rb[0];
 #pragma unroll
         for (uint32_t q = 1; q < NC_YARN_SLOTS; ++q)
@@ -2251,59 +2327,11 @@ __device__ __forceinline__ void yarn_friction_core(const Ctx& ctx, const float4&
                 sa = ra[q];
                 sb = rb[q];
             }
-        const float ni = sa.w;
-        const V3 wn{sa.x, sa.y, sa.z};
-        if (ni <= 0.0f || lsq(wn) < 1.0e-20f) continue;
-        FruitState fr;
-        {
-            const float4 vw = s_vw[f];
-            const float4 orr = s_or[f];
-            fr.v = V3{vw.x, vw.y, vw.z};
-            fr.w = vw.w;
-            fr.omega = V3{orr.x, orr.y, orr.z};
-            fr.radius = orr.w;
-        }
-        const V3 normal = normalized3(wn);
-        float wt[2] = {sb.x / ni, sb.y / ni};
-        const float sum = wt[0] + wt[1];
-        if (sum <= 1.0e-12f) continue;
-        wt[0] = wt[0] / sum;
-        wt[1] = wt[1] / sum;
-        const V3 yv = (V3{0.0f, 0.0f, 0.0f} + xyz(va) * wt[0]) + xyz(vb) * wt[1];
-        const V3 off = normal * -fr.radius;
-        const V3 bcv = fr.v + cross3(fr.omega, off);
-        const V3 rel = bcv - yv;
-        const V3 tv = rel - normal * dot3(rel, normal);
-        const float slip = len3(tv);
-        if (slip < 1.0e-10f) continue;
-        const V3 t = vdiv(tv, slip);
-        const float inv_i = inverse_inertia(fr.w, fr.radius);
-        float den = fr.w + inv_i * lsq(cross3(off, t));
-        V3 resp[2];
-        const float4* pp[2] = {&pa, &pb};
-        for (int s = 0; s < 2; ++s) {
-            resp[s] = t * pp[s]->w;
-            if (c.ground && pp[s]->z <= c.radius + 1.0e-6f && resp[s].z < 0.0f) resp[s].z = 0.0f;
-            den = den + dot3(t, resp[s]) * wt[s] * wt[s];
-        }
-        if (den <= 0.0f) continue;
-        const float limit = c.mu_fruit_yarn * ni;
-        const float ti = fminf(slip / den, limit);
-        if (ti <= 0.0f) continue;
-        const V3 imp = t * -ti;
-        const V3 dv = imp * fr.w;
-        const V3 dw = cross3(off, imp) * inv_i;
-        cta_sums_add(s_sum + 6u * f + 0u, dv.x);
-        cta_sums_add(s_sum + 6u * f + 1u, dv.y);
-        cta_sums_add(s_sum + 6u * f + 2u, dv.z);
-        cta_sums_add(s_sum + 6u * f + 3u, dw.x);
-        cta_sums_add(s_sum + 6u * f + 4u, dw.y);
-        cta_sums_add(s_sum + 6u * f + 5u, dw.z);
-        const V3 na = xyz(va) + resp[0] * (ti * wt[0]);
-        const V3 nb = xyz(vb) + resp[1] * (ti * wt[1]);
-        va = with_xyz(va, na);
-        vb = with_xyz(vb, nb);
-    }
+        V3 normal;
+        float wt[2], limit;
+        if (friction_record(ctx, sa, sb, normal, wt, limit))
+            friction_apply(ctx, f, normal, wt, limit, pa, pb, va, vb, s_vw, s_or, s_sum);
+    });
 }
 
 
@@ -2342,8 +2370,10 @@ __shared__ float4 nc_fric_or[NC_MAX_FRUITS];
 
 // Stage the substep's recorded segments for the friction sweep (fruit CTA,
 // tile mode): what the sweep reads that no later phase changes, read as
-// soon as the fruit/yarn sweep has ended: segment, endpoints, slot tags and
-// the live slots' records, and for every endpoint the first endpoint of the
+// soon as the fruit/yarn sweep has ended, while the tiles resolve self
+// contact: segment, endpoints, the live records with the roots and quotients
+// that no velocity enters done (the sweep itself holds up the next
+// substep's fruits), and for every endpoint the first endpoint of the
 // list with the same particle (where a later colour must see an earlier
 // colour's velocity change).  More segments than NC_FRICTION_STAGE are not
 // staged (the sweep reads them from global memory).
@@ -2361,10 +2391,29 @@ __device__ void friction_stage(const Ctx& ctx) {
             fs.seg[k] = seg;
             fs.pid[2u * k] = ij.x;
             fs.pid[2u * k + 1u] = ij.y;
+            uint32_t tag[NC_YARN_SLOTS];
+            float4 ra[NC_YARN_SLOTS], rb[NC_YARN_SLOTS];
 #pragma unroll
             for (uint32_t q = 0; q < NC_YARN_SLOTS; ++q)
-                fs.tag[k][q] = __float_as_uint(__ldcg(&d.yarn_slot_b[seg * NC_YARN_SLOTS + q].z));
-            friction_records(ctx, seg, fs.tag[k], fs.ra[k], fs.rb[k]);
+                tag[q] = __float_as_uint(__ldcg(&d.yarn_slot_b[seg * NC_YARN_SLOTS + q].z));
+            friction_records(ctx, seg, tag, ra, rb);
+            uint32_t records = 0u;
+            friction_visits(ctx, tag, [&](uint32_t slot, uint32_t f) {
+                float4 sa = ra[0], sb = rb[0];
+#pragma unroll
+                for (uint32_t q = 1; q < NC_YARN_SLOTS; ++q)
+                    if (q == slot) {
+                        sa = ra[q];
+                        sb = rb[q];
+                    }
+                V3 normal;
+                float wt[2], limit;
+                if (!friction_record(ctx, sa, sb, normal, wt, limit)) return;
+                fs.normal[k][records] = make_float4(normal.x, normal.y, normal.z, limit);
+                fs.weight[k][records] = make_float4(wt[0], wt[1], __uint_as_float(f), 0.0f);
+                ++records;
+            });
+            fs.records[k] = records;
         }
         __syncthreads();
         for (uint32_t e = threadIdx.x; e < 2u * n; e += blockDim.x) {
@@ -2468,7 +2517,12 @@ __device__ void yarn_friction_sweep(Ctx& ctx) {
             if (seg < bt.first || seg >= bt.first + bt.yarn) continue;
             const uint32_t ea = fs.rep[2u * k], eb = fs.rep[2u * k + 1u];
             float4 va = fs.v[ea], vb = fs.v[eb];
-            yarn_friction_core(ctx, fs.x[ea], fs.x[eb], va, vb, fs.tag[k], fs.ra[k], fs.rb[k], s_vw, s_or, s_sum);
+            const float4 pa = fs.x[ea], pb = fs.x[eb];
+            for (uint32_t r = 0; r < fs.records[k]; ++r) {
+                const float4 nl = fs.normal[k][r], w = fs.weight[k][r];
+                const float wt[2] = {w.x, w.y};
+                friction_apply(ctx, __float_as_uint(w.z), xyz(nl), wt, nl.w, pa, pb, va, vb, s_vw, s_or, s_sum);
+            }
             fs.v[ea] = va;
             fs.v[eb] = vb;
         }
