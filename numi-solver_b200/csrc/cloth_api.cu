@@ -2825,8 +2825,8 @@ std::vector<uint4> adjoint_phases(const DeviceCloth& d, const Schedule& s) {
 // Launch shape of the reverse sweep of `count` cloths: a cluster of `ranks`
 // CTAs per cloth.  More CTAs shorten a phase until each of its items has a
 // thread of its own (256 items a CTA leave half of its threads for the FP64
-// units to switch between), as long as every cloth keeps its own SMs: one
-// 64 x 64 cloth takes 8, sixteen take 8 each, 96 bags one each.
+// units to switch between), as long as all clusters run at once: one
+// 64 x 64 cloth takes 8, 96 bags one each.
 struct AdjointShape {
     uint32_t ranks = 1;
     bool shared = true;
@@ -2881,8 +2881,12 @@ int adjoint_shape(int device, const std::vector<const DeviceCloth*>& cloths, Adj
         cfg.dynamicSmemBytes = out.smem;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
+        // every cloth's cluster at once: sixteen clusters of 8 take two
+        // turns where the GPU's partitions hold fifteen
         int clusters = 0;
-        if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters >= 1) return NUMI_CLOTH_OK;
+        if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess &&
+            static_cast<size_t>(std::max(clusters, 0)) >= cloths.size())
+            return NUMI_CLOTH_OK;
         cudaGetLastError();
     }
 }
