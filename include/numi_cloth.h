@@ -420,6 +420,12 @@ int numi_cloth_step_noalloc(const NumiClothConfig* base, const NumiClothDeviceSt
  *                 the grip orientation) of each substep's Config.
  * The state after the call is the state after the rollout.
  *
+ * The forward is taped as it runs where the tape of the whole rollout fits
+ * 8 GB and a quarter of the free device memory; else, and where a fruit
+ * touches the cloth, segments of checkpoint_every substeps are replayed from
+ * checkpoints with a tape.  The call's device memory stays with the handle
+ * (up to 1 GB) or the batch (up to 9 GB) for the next call.
+ *
  * Supported schedules: iterations = 1, no reconciliation, final or
  * certificate passes, aerodynamics = 0, selfCollision = 0.  Fruit contacts,
  * cloth/ground friction, the swept ground and bend ground active sets are

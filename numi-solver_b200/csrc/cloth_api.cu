@@ -759,9 +759,9 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     h->last_substeps = substeps;
     size_t smem = h->smem;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (h->tiles_wanted && !taped && tile_covers(sc))
+    if (h->tiles_wanted && tile_covers(sc))
         h->tile_substeps = std::min(h->tile_substeps + std::min(substeps, kTilePlanSubsteps), kTilePlanSubsteps);
-    if (h->tiles_wanted && !taped && tile_covers(sc) && h->tile_substeps == kTilePlanSubsteps &&
+    if (h->tiles_wanted && tile_covers(sc) && h->tile_substeps == kTilePlanSubsteps &&
         cudaStreamIsCapturing(h->stream, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone) {
         h->tiles_wanted = false;
         configure_tiles(h, h->tile_grid);
@@ -772,7 +772,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
         d.x_alt = h->d.x_alt;
         d.v_alt = h->d.v_alt;
     }
-    const bool tiled = !taped && tile_schedule(h, sc);
+    const bool tiled = tile_schedule(h, sc);
     if (edge) {
         // the edge/edge phases' box-tree sort keys after the launch's own
         // shared memory, where the device has room
@@ -805,7 +805,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
         e = cudaLaunchKernelExC(&cfg, frame_fn(edge, h->self_exact), args);
     } else if (h->grid == 1 && !tiled) {
         e = cudaLaunchKernel(frame_fn(edge, h->self_exact), dim3(1), dim3(h->block), args, smem, h->stream);
-    } else if (tiled) {   // not a taped launch: the tape follows the colour-by-colour barriers
+    } else if (tiled) {
         if (h->tiles_dirty) {
             if (!rebuild_tiles(h)) return cudaErrorUnknown;
             h->tiles_dirty = false;
@@ -1469,8 +1469,8 @@ int numi_cloth_create(const NumiClothScene* scene, numi_cloth_t** out) {
     // five grid barriers a substep instead of 26 cluster barriers (a frame of
     // a 61 x 61 cloth: 3.6 -> 2.2 ms).  Its plan is built once it has stepped
     // a frame's substeps: a 24 x 24 cloth's takes 0.5 ms, about what it then
-    // saves in as many substeps again, and a cloth that only joins batches or
-    // rollouts never needs one.  The reference-order kernels
+    // saves in as many substeps again, and a cloth that only joins batches
+    // never needs one.  The reference-order kernels
     // stay on the cluster, whose barrier has no bound for the ordered
     // pass's serial fallback to outlast.
     if (want_tiles != 0u && h->cluster > 1u && d.resident != 0u && K == 0u && !h->self_exact && forced == 0u &&
@@ -3268,7 +3268,9 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         h->poisoned = true;
         return NUMI_CLOTH_ECUDA;
     }
-    if (barriers + 1u != slots) return NUMI_CLOTH_ESTATE;   // the phase list does not match the kernel
+    // the phase list does not match the kernel's barriers (tile mode numbers
+    // its slots by phase)
+    if (!h->last_tiles && barriers + 1u != slots) return NUMI_CLOTH_ESTATE;
     std::vector<double> out(ngroups + 2u);
     unsigned int rough = 0;
     e = cudaMemcpyAsync(out.data(), d_out, out.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream);

@@ -738,9 +738,13 @@ __device__ void edge_candidates(Ctx& ctx, bool swept, bool rebuilt) {
 // list to the left child, and a stable partition (one CTA-wide prefix count
 // per list) moves every list's members to their child, in order.  A leaf's
 // order is its parent's axis list.  CTA 0, all threads; at most
-// NC_EDGE_TREE_MAX segments.  edge_tree: [m] segment at each leaf position,
-// [m] position of each segment, then the build's scratch (two sets of the
-// three lists, the side of each segment, the parent axis of each position).
+// NC_EDGE_TREE_MAX segments.  The build is bound by the latency of its
+// dependent gathers, and the cluster's other CTAs wait for it.  So the lists
+// are in shared memory (TreeShared): in global memory every level scattered
+// 9,000 words through the L2, and the top boxes were one warp's scan of all
+// segments (a bag frame's swept pass 236 us, now 92).  edge_tree: [m] segment
+// at each leaf position, [m] position of each segment, then [3][m] the last
+// build's order along each axis.
 #define NC_EDGE_TREE_MAX 4096u
 #define NC_EDGE_TREE_KEY_BYTES (NC_EDGE_TREE_MAX * 20u)   /* the build's shared memory (TreeShared) */
 #define NC_EDGE_TREE_WORDS 14u   /* edge_tree words per segment (the build uses 5, and one flag word) */

@@ -84,7 +84,8 @@ __device__ __forceinline__ bool grid_sync(Ctx& ctx) {
             d.trace_cta[(static_cast<size_t>(ctx.sub) * NC_TRACE_SLOTS + ctx.barriers - 1u) * ctx.ranks + ctx.rank] =
                 globaltimer();
     }
-    for (bool taped = d.tape != nullptr;; taped = false) {
+    // (tile mode writes its own tape: it passes four barriers a substep)
+    for (bool taped = d.tape != nullptr && ctx.s.tiles == 0u;; taped = false) {
         if (d.cluster_barrier)
             cooperative_groups::this_cluster().sync();
         else if (ctx.ranks == 1)

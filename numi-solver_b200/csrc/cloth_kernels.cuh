@@ -782,7 +782,7 @@ __device__ __forceinline__ bool fruit_pair_waves(const DeviceCloth& d, FruitShar
 // took 19.2 us for the walk of 63 colours (0.3 us a colour, its quotients
 // and roots one after the other) and take 6.6 us.  Below NC_PAIR_COLOURS the
 // walk is shorter than building the wavefronts (the bag's 12 fruits have 11
-// colours: 1 % of its frame), and it stays for more than NC_PAIR_NEAR near
+// colours, 3 us), and it stays for more than NC_PAIR_NEAR near
 // pairs and for sweeps that move a fruit too far for the proof.  One warp
 // walks the colours (a colour's pairs are disjoint, so its lanes never touch
 // the same fruit).

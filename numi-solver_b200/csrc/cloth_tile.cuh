@@ -112,6 +112,21 @@ __device__ __forceinline__ void tile_store(const Ctx& ctx, float4* out) {
     for (uint32_t l = threadIdx.x; l < own; l += blockDim.x) out[gi[l]] = ctx.tx[l];
 }
 
+// Adjoint tape: the owned particles into slot `slot` of the substep (the
+// number of the barrier that ends the phase in the colour-by-colour launch:
+// an owned particle has that launch's value after every colour).  Every
+// thread of the CTA, between two CTA barriers of its own.
+__device__ __forceinline__ void tile_tape(const Ctx& ctx, uint32_t slot) {
+    const DeviceCloth& d = ctx.d;
+    if (d.tape == nullptr || slot >= d.tape_slots) return;
+    float4* out = d.tape + (static_cast<size_t>(ctx.s.tape_first + ctx.sub) * d.tape_slots + slot) * d.n;
+    const uint32_t own = ctx.tp[1];
+    const uint32_t* gi = tile_list(ctx);
+    __syncthreads();
+    for (uint32_t l = threadIdx.x; l < own; l += blockDim.x) out[gi[l]] = ctx.tx[l];
+    __syncthreads();
+}
+
 // Substep start of chain 0's particles (predict_particle from the current
 // buffers); the owners keep the substep-start position and publish the
 // predicted velocity (w = predicted vertical velocity) to v_next.
@@ -130,6 +145,11 @@ __device__ void tile_predict(const Ctx& ctx, float4* v_next) {
             const float4 pp = ld(d.xp + i);
             d.xp[i] = make_float4(p.x, p.y, p.z, pp.w);
             v_next[i] = make_float4(vel.x, vel.y, vel.z, vel.z);
+            if (d.tape != nullptr) {
+                const size_t at = ctx.s.tape_first + ctx.sub;
+                d.tape[at * d.tape_slots * d.n + i] = p;
+                d.tape_v[at * d.n + i] = __ldcg(ctx.gv + i);
+            }
         }
     }
     __syncthreads();
@@ -184,8 +204,9 @@ __device__ __forceinline__ void tile_prefetch(const Ctx& ctx, uint32_t chain, ui
         asm volatile("prefetch.global.L1 [%0];" ::"l"(first + k));
 }
 
-// A chain's colours in order, CTA barriers between them.
-__device__ void tile_chain(const Ctx& ctx, uint32_t chain, float dt2) {
+// A chain's colours in order, CTA barriers between them; the first colour's
+// tape slot is `slot`.
+__device__ void tile_chain(const Ctx& ctx, uint32_t chain, float dt2, uint32_t slot) {
     const uint32_t* table = ctx.tp + ctx.tp[8u + 2u * chain];
     const uint32_t colours = ctx.tp[9u + 2u * chain];
     const uint4* staged = reinterpret_cast<const uint4*>(ctx.tp + ctx.tp[3]);
@@ -197,6 +218,7 @@ __device__ void tile_chain(const Ctx& ctx, uint32_t chain, float dt2) {
         for (uint32_t k = threadIdx.x; k < count; k += blockDim.x)
             tile_item(ctx, family, ctx.d.tile_stream != 0u ? __ldg(ctx.ti + first + k) : staged[first + k], dt2);
         __syncthreads();
+        tile_tape(ctx, slot + c);
     }
 }
 
@@ -224,7 +246,7 @@ __device__ void tile_grips(const Ctx& ctx) {
 // The fruit/yarn colours on the closure: a warp takes 32 items of a colour
 // at a time (yarn_warp_contacts); fruits are frozen over the sweep and the
 // owners' displacement sums go to the global sums once.
-__device__ void tile_yarn(const Ctx& ctx) {
+__device__ void tile_yarn(const Ctx& ctx, uint32_t slot) {
     const DeviceCloth& d = ctx.d;
     __shared__ float4 s_fruit[NC_MAX_FRUITS];
     __shared__ float s_fw[NC_MAX_FRUITS];
@@ -262,6 +284,7 @@ __device__ void tile_yarn(const Ctx& ctx) {
             }
         }
         __syncthreads();
+        tile_tape(ctx, slot + c);
     }
     cta_sums_flush(s_sum, reinterpret_cast<unsigned long long*>(d.fruit_partial), 3u * d.f_count);
 }
@@ -429,6 +452,7 @@ __device__ bool substep_tiles(Ctx& ctx, bool last) {
     const float dt2 = ctx.c.dt * ctx.c.dt;
     const bool self = s.self_collision && d.hash_head != nullptr;
     const bool fruits = d.f_count > 0u;
+    uint32_t slot = 1u;   // tape slot of the next phase
     // 1. predict, distance and bend colours, grips
     {
         float4* x_next = other_x(ctx);
@@ -450,10 +474,13 @@ __device__ bool substep_tiles(Ctx& ctx, bool last) {
             tile_mark(ctx, 0u);
             tile_prefetch(ctx, NC_TILE_CONSTRAINTS, 0u);
             tile_predict(ctx, v_next);
+            tile_tape(ctx, slot++);
             tile_mark(ctx, 1u);
-            tile_chain(ctx, NC_TILE_CONSTRAINTS, dt2);
+            tile_chain(ctx, NC_TILE_CONSTRAINTS, dt2, slot);
+            slot += ctx.tp[9u + 2u * NC_TILE_CONSTRAINTS];
             tile_mark(ctx, 2u);
             tile_grips(ctx);
+            tile_tape(ctx, slot++);
             if (self && !fruits) tile_insert(ctx);
             tile_store(ctx, x_next);
             tile_mark(ctx, 3u);
@@ -473,7 +500,8 @@ __device__ bool substep_tiles(Ctx& ctx, bool last) {
             tile_prefetch(ctx, NC_TILE_YARN, 0u);
             tile_load(ctx, NC_TILE_YARN);
             tile_mark(ctx, 5u);
-            tile_yarn(ctx);
+            tile_yarn(ctx, slot);
+            slot += ctx.tp[9u + 2u * NC_TILE_YARN];
             tile_mark(ctx, 6u);
             if (self) tile_insert(ctx);
             tile_mark(ctx, 7u);
@@ -554,10 +582,18 @@ __device__ bool substep_tiles(Ctx& ctx, bool last) {
             tile_load(ctx, NC_TILE_STRAIN);
             if (!split) tile_mark(ctx, 10u);
             if (sw == 0u && !split) tile_self_ground(ctx, false, ctx.tp[4u + NC_TILE_STRAIN]);
+            if (sw == 0u) tile_tape(ctx, slot++);
             tile_mark(ctx, 11u);
-            if (s.strain_sweeps > 0u) tile_chain(ctx, NC_TILE_STRAIN, dt2);
+            if (s.strain_sweeps > 0u) {
+                tile_chain(ctx, NC_TILE_STRAIN, dt2, slot);
+                slot += ctx.tp[9u + 2u * NC_TILE_STRAIN];
+            }
             tile_mark(ctx, 12u);
-            if (final_sweep) tile_finalize(ctx);
+            if (final_sweep) {
+                tile_finalize(ctx);
+                tile_tape(ctx, slot);        // finalize
+                tile_tape(ctx, slot + 1u);   // and the tail, which moves no particle
+            }
             tile_mark(ctx, 13u);
             tile_store(ctx, x_next);
             tile_mark(ctx, 14u);
