@@ -2049,33 +2049,37 @@ __device__ void residual_partials(Ctx& ctx, double* out3) {
                                           static_cast<double>(__ldcg(&d.fruits[f].positionAndInverseMass.z)));
     }
     if (d.f_count > 0u) {
-        for (uint32_t b = 0; b < d.n_dist_batches; ++b) {
-            const Batch bt = d.dist_batches[b];
-            for (Range r = item_range(ctx, bt.yarn); r.i < r.end; r.i += r.stride) {
-                const uint2 ij = __ldg(d.d_ij + bt.first + r.i);
-                const float4 pa = px(ctx, ij.x);
-                const float4 pb = px(ctx, ij.y);
-                for (uint32_t f = 0; f < d.f_count; ++f) {
-                    const float4 fr = s_f[f];
-                    const double X[3] = {fr.x, fr.y, fr.z};
-                    const double target = static_cast<double>(fr.w) + c.radius;
-                    const double A[3] = {pa.x, pa.y, pa.z};
-                    const double B[3] = {pb.x, pb.y, pb.z};
-                    bool outside = false;
-                    for (int e = 0; e < 3; ++e)
-                        outside = outside || X[e] < fmin(A[e], B[e]) - target || X[e] > fmax(A[e], B[e]) + target;
-                    if (outside) continue;
-                    const double dir[3] = {B[0] - A[0], B[1] - A[1], B[2] - A[2]};
-                    const double lb = (dir[0] * dir[0] + dir[1] * dir[1]) + dir[2] * dir[2];
-                    double t = 0.0;
-                    if (lb > 1.0e-20) {
-                        const double proj = (dir[0] * (X[0] - A[0]) + dir[1] * (X[1] - A[1])) + dir[2] * (X[2] - A[2]);
-                        t = fmin(fmax(proj / lb, 0.0), 1.0);
-                    }
-                    const double cx = A[0] + dir[0] * t - X[0], cy = A[1] + dir[1] * t - X[1],
-                                 cz = A[2] + dir[2] * t - X[2];
-                    fruit = fmax(fruit, target - sqrt((cx * cx + cy * cy) + cz * cz));
+        // the yarn prefixes of all colours in one range: no colour's few
+        // segments a CTA wait for another's
+        uint32_t yarn = 0u;
+        for (uint32_t b = 0; b < d.n_dist_batches; ++b) yarn += d.dist_batches[b].yarn;
+        for (Range r = item_range(ctx, yarn); r.i < r.end; r.i += r.stride) {
+            uint32_t b = 0u, k = r.i;
+            while (k >= d.dist_batches[b].yarn) k -= d.dist_batches[b++].yarn;
+            const Batch& bt = d.dist_batches[b];
+            const uint2 ij = __ldg(d.d_ij + bt.first + k);
+            const float4 pa = px(ctx, ij.x);
+            const float4 pb = px(ctx, ij.y);
+            for (uint32_t f = 0; f < d.f_count; ++f) {
+                const float4 fr = s_f[f];
+                const double X[3] = {fr.x, fr.y, fr.z};
+                const double target = static_cast<double>(fr.w) + c.radius;
+                const double A[3] = {pa.x, pa.y, pa.z};
+                const double B[3] = {pb.x, pb.y, pb.z};
+                bool outside = false;
+                for (int e = 0; e < 3; ++e)
+                    outside = outside || X[e] < fmin(A[e], B[e]) - target || X[e] > fmax(A[e], B[e]) + target;
+                if (outside) continue;
+                const double dir[3] = {B[0] - A[0], B[1] - A[1], B[2] - A[2]};
+                const double lb = (dir[0] * dir[0] + dir[1] * dir[1]) + dir[2] * dir[2];
+                double t = 0.0;
+                if (lb > 1.0e-20) {
+                    const double proj = (dir[0] * (X[0] - A[0]) + dir[1] * (X[1] - A[1])) + dir[2] * (X[2] - A[2]);
+                    t = fmin(fmax(proj / lb, 0.0), 1.0);
                 }
+                const double cx = A[0] + dir[0] * t - X[0], cy = A[1] + dir[1] * t - X[1],
+                             cz = A[2] + dir[2] * t - X[2];
+                fruit = fmax(fruit, target - sqrt((cx * cx + cy * cy) + cz * cz));
             }
         }
     }

@@ -806,10 +806,12 @@ __device__ void fruit_pair_sweep(const DeviceCloth& d, FruitShared& fs, float dt
     // sphere; a sphere landing at 4 m/s moves 1.4 mm in a substep).
     bool touching = false;
     const uint32_t lane = threadIdx.x & 31u;
-    float smallest = INFINITY;
-    for (uint32_t f = lane; waves && f < d.f_count; f += 32u) smallest = fminf(smallest, fs.fr[f]);
-    for (int o = 16; o > 0; o >>= 1) smallest = fminf(smallest, __shfl_xor_sync(0xffffffffu, smallest, o));
-    const float margin = 0.4f * smallest;
+    float margin = INFINITY;
+    if (waves) {
+        for (uint32_t f = lane; f < d.f_count; f += 32u) margin = fminf(margin, fs.fr[f]);
+        for (int o = 16; o > 0; o >>= 1) margin = fminf(margin, __shfl_xor_sync(0xffffffffu, margin, o));
+        margin = 0.4f * margin;
+    }
     for (uint32_t base = threadIdx.x - lane; base < d.p_count; base += blockDim.x) {
         const uint32_t k = base + lane;
         bool near = false;
@@ -844,13 +846,19 @@ __device__ void fruit_pair_sweep(const DeviceCloth& d, FruitShared& fs, float dt
             count += total;
         }
         __syncwarp();
-        if (!waves || count > NC_PAIR_NEAR || !fruit_pair_waves(d, fs, dt, count, margin)) {
-            for (uint32_t f = lane; f < d.f_count; f += 32u) {
-                const NumiClothFruit& fr = d.fruits[f];
-                fs.fx[f] = make_float4(fr.positionAndInverseMass.x, fr.positionAndInverseMass.y,
-                                       fr.positionAndInverseMass.z, fr.positionAndInverseMass.w);
+        bool done = false;
+        if (waves && count <= NC_PAIR_NEAR) {
+            done = fruit_pair_waves(d, fs, dt, count, margin);
+            if (!done) {   // back to the sweep's start
+                for (uint32_t f = lane; f < d.f_count; f += 32u) {
+                    const NumiClothFruit& fr = d.fruits[f];
+                    fs.fx[f] = make_float4(fr.positionAndInverseMass.x, fr.positionAndInverseMass.y,
+                                           fr.positionAndInverseMass.z, fr.positionAndInverseMass.w);
+                }
+                __syncwarp();
             }
-            __syncwarp();
+        }
+        if (!done) {
             for (uint32_t b = 0; b < d.n_pair_batches; ++b) {
                 const Batch bt = d.pair_batches[b];
                 bool loaded = false;
