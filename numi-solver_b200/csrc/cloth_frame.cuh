@@ -921,8 +921,9 @@ __device__ __forceinline__ uint32_t cell_bucket(int x, int y, int z, uint32_t ma
 // tile's 443 particles met some 1,600 lines of a head or a slot each, twice
 // what the L1 holds beside the tile's shared memory, and a warp's 32 loads as
 // many lines.  A row of the cloth now shares its lines among neighbours: on
-// the 256 x 256 cloth the query takes 9.4 us instead of 11.8 and the insert
-// 2.0 instead of 3.2, on the 512 x 512 cloth the query 21 instead of 38.  The
+// the 256 x 256 cloth the query takes 9.4 us instead of 11.8 (8.6 with the
+// tests of a batch without branches) and the insert 2.0 instead of 3.2, on
+// the 512 x 512 cloth the query 21 (18.4) instead of 38.  The
 // hash of a group is a sum of odd multiples of its coordinates through the
 // 32-bit finalizer lowbias32 (Wellons, hash-prospector).
 #define NC_HASH_GROUP 8u
@@ -1054,20 +1055,22 @@ __device__ __forceinline__ void self_heads(const Ctx& ctx, const float4& p, Self
     }
 }
 
-// Candidates per bucket of this pass (a bucket met twice counts once).
+// Candidates of cell c of a query (a bucket met twice counts once).  Cells
+// that differ in x or y are different cells of their groups, so only the two
+// cells of a z pair, c and c - 4, can share a bucket.
+__device__ __forceinline__ uint32_t self_cell_count(uint32_t tag, const SelfQuery& q, const unsigned long long hd[8],
+                                                    const bool near[8], uint32_t c) {
+    const bool repeat = c >= 4u && near[c & 3u] && q.bk[c & 3u] == q.bk[c];
+    return (near[c] && !repeat && static_cast<uint32_t>(hd[c] >> 32) == tag) ? min(static_cast<uint32_t>(hd[c]), NC_HASH_CAP)
+                                                                            : 0u;
+}
+
+// Candidates per bucket of this pass as prefix counts.
 __device__ __forceinline__ uint32_t self_counts(uint32_t tag, SelfQuery& q, const unsigned long long hd[8],
                                                 const bool near[8]) {
     q.pre[0] = 0u;
 #pragma unroll
-    for (uint32_t c = 0; c < 8u; ++c) {
-        bool repeat = false;
-#pragma unroll
-        for (uint32_t e = 0; e < c; ++e) repeat = repeat || (near[e] && q.bk[e] == q.bk[c]);
-        const uint32_t cnt = (near[c] && !repeat && static_cast<uint32_t>(hd[c] >> 32) == tag)
-                                 ? min(static_cast<uint32_t>(hd[c]), NC_HASH_CAP)
-                                 : 0u;
-        q.pre[c + 1u] = q.pre[c] + cnt;
-    }
+    for (uint32_t c = 0; c < 8u; ++c) q.pre[c + 1u] = q.pre[c] + self_cell_count(tag, q, hd, near, c);
     return q.pre[8];
 }
 
@@ -1164,6 +1167,8 @@ __device__ __forceinline__ bool self_solve_one(const Ctx& ctx, uint32_t tag, uin
     bool near[8];
     self_heads(ctx, p, q, hd, near);
     const uint32_t total = self_counts(tag, q, hd, near);
+    const float target = 2.0f * ctx.c.radius;
+    const float far2 = target * target * 1.00001f;   // as in self_pair
     long long sum[3] = {0, 0, 0};
     bool touched = false;
     for (uint32_t t0 = 0; t0 < total; t0 += NC_SELF_BATCH) {
@@ -1173,9 +1178,19 @@ __device__ __forceinline__ bool self_solve_one(const Ctx& ctx, uint32_t tag, uin
             const uint32_t slot = self_slot(q, t0 + j, total);
             e[j] = l1 ? __ldca(&d.hash[slot].pos) : __ldcg(&d.hash[slot].pos);
         }
+        // nearly all candidates are the particle's neighbours on the cloth,
+        // out of reach: the batch is tested without branches, the few in
+        // reach are read again
+        uint32_t hits = 0u;
 #pragma unroll
-        for (uint32_t j = 0; j < NC_SELF_BATCH; ++j)
-            if (t0 + j < total) self_pair(ctx, a, p, e[j], sum, touched, contacts, max_pen);
+        for (uint32_t j = 0; j < NC_SELF_BATCH; ++j) {
+            const bool in = t0 + j < total && !(lsq(xyz(e[j]) - xyz(p)) > far2) && __float_as_uint(e[j].w) != a;
+            hits |= (in ? 1u : 0u) << j;
+        }
+        for (; hits != 0u; hits &= hits - 1u) {
+            const uint32_t j = static_cast<uint32_t>(__ffs(static_cast<int>(hits)) - 1);
+            self_pair(ctx, a, p, __ldcg(&d.hash[self_slot(q, t0 + j, total)].pos), sum, touched, contacts, max_pen);
+        }
     }
     return self_finish(ctx, tag, a, p, sum, touched, moved, contacts, max_pen);
 }
