@@ -466,7 +466,7 @@ bool prepare_neighbours(numi_cloth* h, const NumiClothScene* scene) {
 // particles would not fit the shared memory of one CTA per SM or a closure
 // holds 65,536 particles or more.
 struct TileColour {
-    uint32_t family, first, count;
+    uint32_t family, first, count, batch;
 };
 
 bool build_tiles(numi_cloth* h, uint32_t grid_width, const std::vector<uint2>& dij, const std::vector<float4>& dmat,
@@ -504,32 +504,27 @@ bool build_tiles(numi_cloth* h, uint32_t grid_width, const std::vector<uint2>& d
     std::vector<std::vector<TileColour>> chains(NC_TILE_CHAINS);
     for (uint32_t b = 0; b < d.n_dist_batches; ++b) {
         const Batch& bt = d.dist_batches[b];
-        chains[NC_TILE_CONSTRAINTS].push_back({NC_TILE_DISTANCE, bt.first, bt.count});
-        if (bt.yarn) chains[NC_TILE_YARN].push_back({NC_TILE_SEGMENT, bt.first, bt.yarn});
-        if (bt.limited) chains[NC_TILE_STRAIN].push_back({NC_TILE_LIMIT, bt.first, bt.limited});
+        chains[NC_TILE_CONSTRAINTS].push_back({NC_TILE_DISTANCE, bt.first, bt.count, b});
+        if (bt.yarn) chains[NC_TILE_YARN].push_back({NC_TILE_SEGMENT, bt.first, bt.yarn, b});
+        if (bt.limited) chains[NC_TILE_STRAIN].push_back({NC_TILE_LIMIT, bt.first, bt.limited, b});
     }
     for (uint32_t b = 0; b < d.n_bend_batches; ++b)
-        chains[NC_TILE_CONSTRAINTS].push_back({NC_TILE_BEND, d.bend_batches[b].first, d.bend_batches[b].count});
-    // particle -> records (CSR), distances and bends
-    auto csr = [&](uint32_t records, auto ends, std::vector<uint32_t>& off, std::vector<uint32_t>& idx) {
-        off.assign(n + 1u, 0u);
-        for (uint32_t k = 0; k < records; ++k) {
-            const uint2 e = ends(k);
-            ++off[e.x + 1u];
-            ++off[e.y + 1u];
+        chains[NC_TILE_CONSTRAINTS].push_back({NC_TILE_BEND, d.bend_batches[b].first, d.bend_batches[b].count, b});
+    // the record of every particle in each colour (a colour's records share
+    // none)
+    constexpr uint32_t kNone = ~0u;
+    std::vector<uint32_t> dist_of(static_cast<size_t>(d.n_dist_batches) * n, kNone);
+    std::vector<uint32_t> bend_of(static_cast<size_t>(d.n_bend_batches) * n, kNone);
+    for (uint32_t b = 0; b < d.n_dist_batches; ++b)
+        for (uint32_t k = 0; k < d.dist_batches[b].count; ++k) {
+            const uint32_t rec = d.dist_batches[b].first + k;
+            dist_of[static_cast<size_t>(b) * n + dij[rec].x] = dist_of[static_cast<size_t>(b) * n + dij[rec].y] = rec;
         }
-        for (uint32_t i = 0; i < n; ++i) off[i + 1u] += off[i];
-        idx.assign(off[n], 0u);
-        std::vector<uint32_t> at(off.begin(), off.end() - 1);
-        for (uint32_t k = 0; k < records; ++k) {
-            const uint2 e = ends(k);
-            idx[at[e.x]++] = k;
-            idx[at[e.y]++] = k;
+    for (uint32_t b = 0; b < d.n_bend_batches; ++b)
+        for (uint32_t k = 0; k < d.bend_batches[b].count; ++k) {
+            const uint32_t rec = d.bend_batches[b].first + k;
+            bend_of[static_cast<size_t>(b) * n + bij[rec].x] = bend_of[static_cast<size_t>(b) * n + bij[rec].z] = rec;
         }
-    };
-    std::vector<uint32_t> doff, didx, boff, bidx;
-    csr(d.d_count, [&](uint32_t k) { return dij[k]; }, doff, didx);
-    csr(d.b_count, [&](uint32_t k) { return make_uint2(bij[k].x, bij[k].z); }, boff, bidx);
     auto ends = [&](uint32_t family, uint32_t rec) {
         return family == NC_TILE_BEND ? make_uint2(bij[rec].x, bij[rec].z) : dij[rec];
     };
@@ -556,25 +551,22 @@ bool build_tiles(numi_cloth* h, uint32_t grid_width, const std::vector<uint2>& d
                 const TileColour& col = chains[k][c];
                 const uint32_t cs = ++stamp;
                 std::vector<uint32_t>& its = items[k][c];
+                const uint32_t* record_of =
+                    (col.family == NC_TILE_BEND ? bend_of.data() : dist_of.data()) + static_cast<size_t>(col.batch) * n;
+                std::vector<uint32_t>& ist = col.family == NC_TILE_BEND ? item_stamp_b : item_stamp_d;
                 const size_t upto = cur.size();
                 for (size_t q = 0; q < upto; ++q) {
                     const uint32_t p = cur[q];
-                    const bool bend = col.family == NC_TILE_BEND;
-                    const std::vector<uint32_t>& off = bend ? boff : doff;
-                    const std::vector<uint32_t>& idx = bend ? bidx : didx;
-                    std::vector<uint32_t>& ist = bend ? item_stamp_b : item_stamp_d;
-                    for (uint32_t e = off[p]; e < off[p + 1u]; ++e) {
-                        const uint32_t rec = idx[e];
-                        if (rec < col.first || rec >= col.first + col.count || ist[rec] == cs) continue;
-                        ist[rec] = cs;
-                        its.push_back(rec);
-                        const uint2 pe = ends(col.family, rec);
-                        for (uint32_t v : {pe.x, pe.y})
-                            if (need_stamp[v] != g) {
-                                need_stamp[v] = g;
-                                cur.push_back(v);
-                            }
-                    }
+                    const uint32_t rec = record_of[p];
+                    if (rec >= col.first + col.count || ist[rec] == cs) continue;   // (kNone is past any colour)
+                    ist[rec] = cs;
+                    its.push_back(rec);
+                    const uint2 pe = ends(col.family, rec);
+                    for (uint32_t v : {pe.x, pe.y})
+                        if (need_stamp[v] != g) {
+                            need_stamp[v] = g;
+                            cur.push_back(v);
+                        }
                 }
                 std::sort(its.begin(), its.end());
             }
@@ -722,7 +714,7 @@ bool tile_covers(const Schedule& s) {
 }
 bool tile_schedule(const numi_cloth* h, const Schedule& s) { return h->tiles && tile_covers(s); }
 bool configure_tiles(numi_cloth* h, uint32_t grid);
-constexpr uint32_t kTilePlanSubsteps = 48;
+constexpr uint32_t kTilePlanSubsteps = 128;
 
 // Adjoint tape of a launch: [substep][slots][n] positions, [substep][n]
 // velocities.
@@ -1467,12 +1459,11 @@ int numi_cloth_create(const NumiClothScene* scene, numi_cloth_t** out) {
     // tile mode too, on as many CTAs as the cluster has and one for the
     // fruits (the same share of the GPU when several cloths step at once):
     // five grid barriers a substep instead of 26 cluster barriers (a frame of
-    // a 61 x 61 cloth: 3.6 -> 2.2 ms).  Its plan is built once it has stepped
-    // a frame's substeps: a 24 x 24 cloth's takes 0.5 ms, about what it then
-    // saves in as many substeps again, and a cloth that only joins batches
-    // never needs one.  The reference-order kernels
-    // stay on the cluster, whose barrier has no bound for the ordered
-    // pass's serial fallback to outlast.
+    // a 61 x 61 cloth: 3.6 -> 2.1 ms).  Its plan is built once it has stepped
+    // kTilePlanSubsteps: building costs about what as many substeps again
+    // save, and a cloth that only joins batches never needs one.  The
+    // reference-order kernels stay on the cluster, whose barrier has no bound
+    // for the ordered pass's serial fallback to outlast.
     if (want_tiles != 0u && h->cluster > 1u && d.resident != 0u && K == 0u && !h->self_exact && forced == 0u &&
         !forced_block && std::getenv("NUMI_CLOTH_CLUSTER") == nullptr && std::getenv("NUMI_CLOTH_RESIDENT") == nullptr &&
         std::getenv("NUMI_CLOTH_RESIDENT_CHUNK") == nullptr) {
