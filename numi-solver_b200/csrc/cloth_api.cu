@@ -233,6 +233,8 @@ const void* batch_fn(bool edge) {
                 : reinterpret_cast<const void*>(numi_cloth_batch_kernel);
 }
 
+const void* batch_cluster_fn() { return reinterpret_cast<const void*>(numi_cloth_batch_cluster_kernel); }
+
 cudaError_t raise_smem(const void* fn, size_t bytes) {
     cudaFuncAttributes fa{};
     cudaError_t e = cudaFuncGetAttributes(&fa, fn);
@@ -2325,7 +2327,7 @@ size_t batch_room(const numi_cloth_batch* b, bool edge) {
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, batch_fn(edge)) != cudaSuccess) return 0;
-    const size_t fixed = nc_resident_offset() + fa.sharedSizeBytes + (edge ? NC_EDGE_TREE_KEY_BYTES + 256u : 0u);
+    const size_t fixed = nc_resident_offset() + fa.sharedSizeBytes + 256u + (edge ? NC_EDGE_TREE_KEY_BYTES : 0u);
     return static_cast<size_t>(optin) > fixed ? static_cast<size_t>(optin) - fixed : 0u;
 }
 
@@ -2359,7 +2361,8 @@ int batch_fit(numi_cloth_batch* b) {
             }
             const size_t smem = nc_resident_offset() + bytes;
             const size_t launch = edge ? nc_round256(smem) + NC_EDGE_TREE_KEY_BYTES : smem;
-            if (raise_smem(batch_fn(edge), launch) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+            const void* fn = r > 1u ? batch_cluster_fn() : batch_fn(edge);
+            if (raise_smem(fn, launch) != cudaSuccess) return NUMI_CLOTH_ECUDA;
             int fit = 0;
             if (r > 1u) {
                 cudaLaunchAttribute attr{};
@@ -2373,7 +2376,7 @@ int batch_fit(numi_cloth_batch* b) {
                 cfg.dynamicSmemBytes = launch;
                 cfg.attrs = &attr;
                 cfg.numAttrs = 1;
-                if (cudaOccupancyMaxActiveClusters(&fit, batch_fn(edge), &cfg) != cudaSuccess ||
+                if (cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) != cudaSuccess ||
                     static_cast<uint32_t>(std::max(fit, 0)) < count) {
                     // not every cloth would have a cluster: fewer CTAs each
                     cudaGetLastError();
@@ -2382,7 +2385,7 @@ int batch_fit(numi_cloth_batch* b) {
                 }
             } else {
                 int k = 0;
-                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, batch_fn(edge), static_cast<int>(b->block), launch) !=
+                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, fn, static_cast<int>(b->block), launch) !=
                         cudaSuccess ||
                     k < 1)
                     return NUMI_CLOTH_EINVAL;
@@ -2435,7 +2438,7 @@ cudaError_t batch_kernel(numi_cloth_batch* b, const DeviceCloth* cloths, const S
     cfg.numAttrs = ranks > 1u ? 1u : 0u;
     unsigned int* queue = b->queue;
     void* args[] = {&cloths, &count, &sc, &queue, &ranks};
-    return cudaLaunchKernelExC(&cfg, batch_fn(edge), args);
+    return cudaLaunchKernelExC(&cfg, ranks > 1u ? batch_cluster_fn() : batch_fn(edge), args);
 }
 
 // Descriptors of every cloth for a launch of `substeps` Configs each.

@@ -12,7 +12,6 @@ __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_frame_edge_kernel(
 }
 
 __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_batch_edge_kernel(const DeviceCloth* cloths, uint32_t count,
-                                                                              Schedule s, unsigned int* queue,
-                                                                              uint32_t ranks) {
+                                                                              Schedule s, unsigned int* queue) {
     NC_BATCH_BODY(true)
 }
