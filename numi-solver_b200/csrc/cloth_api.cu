@@ -2248,6 +2248,7 @@ struct numi_cloth_batch {
     bool rollout_touched = false;   // a fruit touched a cloth in the last rollout
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    void* graph_mem = nullptr;   // the captured launch's own descriptors and Configs
     const NumiClothConfig* graph_cfg = nullptr;
     uint32_t graph_substeps = 0;
 };
@@ -2517,14 +2518,16 @@ int batch_prepare(numi_cloth_batch* b, const NumiClothConfig* configs, uint32_t 
     return batch_layout(b, substeps, sched.primitiveSelf != 0u);
 }
 
-cudaError_t batch_launch(numi_cloth_batch* b, const NumiClothConfig* configs, uint32_t substeps, const Schedule& s) {
+// One step over `cloths` (launch order), whose Configs are d_cfg.
+cudaError_t batch_launch(numi_cloth_batch* b, const DeviceCloth* cloths, NumiClothConfig* d_cfg,
+                         const NumiClothConfig* configs, uint32_t substeps, const Schedule& s) {
     const uint32_t count = static_cast<uint32_t>(b->cloths.size());
-    cudaError_t e = cudaMemcpyAsync(b->d_cfg, configs, static_cast<size_t>(count) * substeps * sizeof(NumiClothConfig),
+    cudaError_t e = cudaMemcpyAsync(d_cfg, configs, static_cast<size_t>(count) * substeps * sizeof(NumiClothConfig),
                                     cudaMemcpyHostToDevice, b->stream);
     Schedule sc = s;
     sc.substeps = substeps;
     sc.epoch_ptr = b->epoch;
-    if (e == cudaSuccess) e = batch_kernel(b, b->d_cloths, sc);
+    if (e == cudaSuccess) e = batch_kernel(b, cloths, sc);
     if (e != cudaSuccess) return e;
     numi_cloth_epoch_kernel<<<1, 1, 0, b->stream>>>(b->epoch, substeps);
     return cudaGetLastError();
@@ -2542,8 +2545,10 @@ void batch_advance(numi_cloth_batch* b, uint32_t substeps) {
 void batch_drop_graph(numi_cloth_batch* b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
+    cudaFree(b->graph_mem);   // (a launch in flight ends first)
     b->exec = nullptr;
     b->graph = nullptr;
+    b->graph_mem = nullptr;
     b->graph_cfg = nullptr;
 }
 
@@ -2634,7 +2639,7 @@ int numi_cloth_batch_step(numi_cloth_batch_t* b, const NumiClothConfig* configs,
     const int rc = batch_prepare(b, configs, substeps, *schedule);
     if (rc > 0) return NUMI_CLOTH_OK;   // a rejected Config: its cloth's failure word reports it
     if (rc != NUMI_CLOTH_OK) return rc;
-    const cudaError_t e = batch_launch(b, configs, substeps, device_schedule(*schedule));
+    const cudaError_t e = batch_launch(b, b->d_cloths, b->d_cfg, configs, substeps, device_schedule(*schedule));
     batch_advance(b, substeps);
     if (e != cudaSuccess) {
         for (numi_cloth* h : b->cloths) h->poisoned = true;
@@ -2677,7 +2682,7 @@ int numi_cloth_batch_tune(numi_cloth_batch_t* b, const NumiClothConfig* configs,
             rc = batch_prepare(b, configs, substeps, *schedule);
             if (rc != NUMI_CLOTH_OK) break;
             cudaEventRecord(t0, b->stream);
-            const cudaError_t e = batch_launch(b, configs, substeps, s);
+            const cudaError_t e = batch_launch(b, b->d_cloths, b->d_cfg, configs, substeps, s);
             cudaEventRecord(t1, b->stream);
             if (e != cudaSuccess || cudaEventSynchronize(t1) != cudaSuccess) {
                 rc = NUMI_CLOTH_ECUDA;
@@ -2715,13 +2720,41 @@ int numi_cloth_batch_capture(numi_cloth_batch_t* b, const NumiClothConfig* confi
     int rc = batch_prepare(b, configs, substeps, *schedule);
     if (rc > 0) return NUMI_CLOTH_EINVAL;
     if (rc != NUMI_CLOTH_OK) return rc;
+    // the graph has descriptors and Configs of its own: a step with the other
+    // kernel family (another residency and barrier) or another substep count
+    // lays the batch's out anew in place
+    const size_t count = b->cloths.size();
+    DeviceCloth* cloths = nullptr;
+    NumiClothConfig* d_cfg = nullptr;
+    auto pieces = [&](Carver& c) {
+        cloths = c.get<DeviceCloth>(count);
+        d_cfg = c.get<NumiClothConfig>(count * substeps);
+    };
+    Carver measure{nullptr};
+    pieces(measure);
+    if (cudaMalloc(&b->graph_mem, measure.used) != cudaSuccess) {
+        cudaGetLastError();
+        b->graph_mem = nullptr;
+        return NUMI_CLOTH_ENOMEM;
+    }
+    Carver carver{static_cast<char*>(b->graph_mem)};
+    pieces(carver);
+    std::vector<DeviceCloth> host = b->host_cloths;
+    for (size_t j = 0; j < count; ++j) host[j].cfg = d_cfg + static_cast<size_t>(b->order[j]) * substeps;
+    if (cudaMemcpy(cloths, host.data(), count * sizeof(DeviceCloth), cudaMemcpyHostToDevice) != cudaSuccess) {
+        batch_drop_graph(b);
+        return NUMI_CLOTH_ECUDA;
+    }
     cudaStream_t cap = nullptr;
-    if (cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+    if (cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) != cudaSuccess) {
+        batch_drop_graph(b);
+        return NUMI_CLOTH_ECUDA;
+    }
     cudaStream_t saved = b->stream;
     b->stream = cap;
     cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        const cudaError_t le = batch_launch(b, configs, substeps, device_schedule(*schedule));
+        const cudaError_t le = batch_launch(b, cloths, d_cfg, configs, substeps, device_schedule(*schedule));
         e = cudaStreamEndCapture(cap, &b->graph);
         if (le != cudaSuccess) e = le;
     }
