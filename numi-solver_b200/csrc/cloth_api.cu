@@ -3295,9 +3295,9 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         h->poisoned = true;
         return NUMI_CLOTH_ECUDA;
     }
-    // the phase list does not match the kernel's barriers (tile mode numbers
-    // its slots by phase)
-    if (!h->last_tiles && barriers + 1u != slots) return NUMI_CLOTH_ESTATE;
+    // the phase list does not match the kernel's barriers (the last launch
+    // was taped; in tile mode it counts its slots)
+    if (barriers + 1u != slots) return NUMI_CLOTH_ESTATE;
     std::vector<double> out(ngroups + 2u);
     unsigned int rough = 0;
     e = cudaMemcpyAsync(out.data(), d_out, out.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream);

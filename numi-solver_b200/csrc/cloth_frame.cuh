@@ -3088,9 +3088,12 @@ __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule
         ctx.c = nc::load_cfg(d.cfg + s.cfg_offset + sub);
         ctx.epoch = epoch_base + sub;
         ctx.barriers = 0;
-        if (d.tape != nullptr) {
+        if (d.tape != nullptr && s.tiles == 0u) {
             // adjoint tape: state at the start of the substep (its first
-            // phase moves a CTA's own particles, thread by thread as here)
+            // phase moves a CTA's own particles, thread by thread as here).
+            // Not in tile mode, where the previous substep's friction sweep
+            // may still be moving velocities: tile_predict writes its own
+            // after the wait for it
             nc::tape_store(ctx);
             for (nc::Range r = nc::particle_range(ctx); r.i < r.end; r.i += r.stride)
                 d.tape_v[static_cast<size_t>(s.tape_first + sub) * d.n + r.i] = pv(ctx, r.i);

@@ -591,8 +591,8 @@ __device__ bool substep_tiles(Ctx& ctx, bool last) {
             tile_mark(ctx, 12u);
             if (final_sweep) {
                 tile_finalize(ctx);
-                tile_tape(ctx, slot);        // finalize
-                tile_tape(ctx, slot + 1u);   // and the tail, which moves no particle
+                tile_tape(ctx, slot++);   // finalize
+                tile_tape(ctx, slot);     // and the tail, which moves no particle
             }
             tile_mark(ctx, 13u);
             tile_store(ctx, x_next);
@@ -628,6 +628,9 @@ __device__ bool substep_tiles(Ctx& ctx, bool last) {
         ctx.fruit_wait = false;
         NC_SYNC(ctx);
     }
+    // a taped launch counts its slots, as the colour-by-colour launch's
+    // barriers number them (the host compares them with the phase list)
+    if (d.tape != nullptr) ctx.barriers = slot;
     return true;
 }
 
