@@ -3,8 +3,8 @@
 // docs/CLOTH_SPECIMEN_CALIBRATION.md:52-82).
 //
 // The forward records a tape: the positions at the start of every substep
-// and after every phase barrier, and the velocities at the start of every
-// substep.  This kernel walks the taped substeps and each substep's phases in
+// and after every phase barrier, the velocities at the start of every
+// substep, and the grips of every substep.  This kernel walks the taped substeps and each substep's phases in
 // reverse and applies the vector-Jacobian product of every projection.  Branch decisions are
 // recomputed in FP32 from the tape exactly as the forward made them; the
 // derivatives are evaluated in FP64 at the FP32 state, and adjoints and
@@ -47,6 +47,7 @@ struct AdjointArgs {
     const NumiClothConfig* cfg;      // the segment's Configs
     const float4* tape;              // [substeps][slots][n]
     const float4* tape_v;            // [substeps][n]
+    const NumiClothGrip* tape_grip;  // [substeps][grips], where the grip is active
     const uint4* phases;             // [slots - 1] (type, first record, records, 0) per barrier
     uint32_t slots;
     uint32_t shift;                  // log2 of the particles each CTA of the cluster owns
@@ -632,7 +633,7 @@ __device__ __forceinline__ void adjoint_segment(const AdjointArgs& A, uint32_t r
                 const uint32_t g = threadIdx.x;
                 double gg[6] = {0, 0, 0, 0, 0, 0};
                 if (g < d.g_count) {
-                    const NumiClothGrip grip = d.grips[g];
+                    const NumiClothGrip grip = A.tape_grip[static_cast<size_t>(si) * d.g_count + g];
                     if (grip.particle.y == cf.gripControl.x) {
                         const uint32_t i = grip.particle.x;
                         const float4 p = pre[i];

@@ -719,10 +719,11 @@ bool configure_tiles(numi_cloth* h, uint32_t grid);
 constexpr uint32_t kTilePlanSubsteps = 128;
 
 // Adjoint tape of a launch: [substep][slots][n] positions, [substep][n]
-// velocities.
+// velocities, [substep][grips] grips.
 struct Tape {
     float4* x = nullptr;      // null: the launch is not taped
     float4* v = nullptr;
+    NumiClothGrip* grip = nullptr;
     uint32_t slots = 0;
     uint32_t first = 0;       // substep of the tape the launch starts at
     uint32_t* touched = nullptr;   // set where a fruit touched the cloth
@@ -738,6 +739,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     if (taped) {
         d.tape = tape.x;
         d.tape_v = tape.v;
+        d.tape_grip = tape.grip;
         d.tape_slots = tape.slots;
         d.trace = nullptr;
     }
@@ -3122,13 +3124,14 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
     for (const auto& r : h->dynamic) state_bytes += (r.bytes + 255u) & ~size_t(255u);
     // the taped segment, and without a tape of the whole rollout the
     // checkpoints of the segments before it
-    const size_t tape_step = static_cast<size_t>(slots + 1u) * n * sizeof(float4);
+    const size_t tape_step = static_cast<size_t>(slots + 1u) * n * sizeof(float4) + h->d.g_count * sizeof(NumiClothGrip);
     uint32_t every = taped_substeps(substeps, checkpoint_every, tape_step);   // substeps on the tape
     const bool fruits = h->d.f_count > 0u;
     const uint32_t interval = std::min(checkpoint_every, substeps);
     if (fruits && (h->rollout_touched || every < substeps)) every = interval;
     uint32_t seg = 0, segs = 0;   // substeps of a forward launch, their number
     float4 *tape_x = nullptr, *tape_v = nullptr;
+    NumiClothGrip* tape_grip = nullptr;
     char* ckpt = nullptr;
     uint4* d_phases = nullptr;
     DeviceCloth* d_cloth = nullptr;
@@ -3165,6 +3168,7 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         gg = c.get<uint8_t>(groups.g.size());
         tape_x = c.get<float4>(static_cast<size_t>(every) * slots * n);
         tape_v = c.get<float4>(static_cast<size_t>(every) * n);
+        tape_grip = c.get<NumiClothGrip>(static_cast<size_t>(every) * h->d.g_count);
         if (fruits || segs > 1u) ckpt = c.get<char>((segs + 1u) * state_bytes);
     };
     Workspace::Lease mem(h->grad, h->stream);
@@ -3205,7 +3209,7 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         seg_epoch[g] = h->epoch;
         if ((fruits || g + 1u < segs) && !save(g)) return NUMI_CLOTH_ECUDA;
         Tape tape;
-        if (last_taped(g)) tape = Tape{tape_x, tape_v, slots, whole ? first : 0u};
+        if (last_taped(g)) tape = Tape{tape_x, tape_v, tape_grip, slots, whole ? first : 0u};
         tape.touched = d_touched;
         e = launch(h, count, s, first, tape);
         h->epoch += count;
@@ -3243,7 +3247,7 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
             replayed = true;
             if (!load(g)) return NUMI_CLOTH_ECUDA;
             h->epoch = seg_epoch[g];
-            e = launch(h, count, s, first, Tape{tape_x, tape_v, slots});
+            e = launch(h, count, s, first, Tape{tape_x, tape_v, tape_grip, slots});
             h->epoch = end_epoch;
             if (e != cudaSuccess) {
                 h->poisoned = true;
@@ -3255,6 +3259,7 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         A.cfg = h->d_cfg + first;
         A.tape = tape_x;
         A.tape_v = tape_v;
+        A.tape_grip = tape_grip;
         A.phases = d_phases;
         A.slots = slots;
         A.shift = adjoint_shift(n, shape.ranks);
@@ -3322,6 +3327,8 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
 // launch per segment, and the adjoint of every cloth's segment in one grid
 // (a cluster per cloth).  Checkpoints are moved by one copy kernel per segment.
 
+constexpr size_t kGripFloat4s = sizeof(NumiClothGrip) / sizeof(float4);   // a grip's room on the tape
+
 extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiClothConfig* configs, uint32_t substeps,
                                              const NumiClothSchedule* schedule, uint32_t checkpoint_every,
                                              const uint32_t* tracked, uint32_t n_tracked, const double* targets,
@@ -3372,7 +3379,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         const int rc = compliance_groups(h, groups[k]);
         if (rc != NUMI_CLOTH_OK) return rc;
         phases[k] = adjoint_phases(h->d, s);
-        tape_step += (phases[k].size() + 2u) * h->d.n;   // positions + velocities
+        tape_step += (phases[k].size() + 2u) * h->d.n + kGripFloat4s * h->d.g_count;   // positions, velocities, grips
         for (const auto& r : h->dynamic) state_bytes[k] += (r.bytes + 255u) & ~size_t(255u);
         state_total += state_bytes[k];
         regions += static_cast<uint32_t>(h->dynamic.size());
@@ -3464,6 +3471,8 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         A.tape = tape_at;
         A.tape_v = A.tape + static_cast<size_t>(every) * slots * n;
         tape_at += static_cast<size_t>(every) * (slots + 1u) * n;
+        A.tape_grip = reinterpret_cast<const NumiClothGrip*>(tape_at);
+        tape_at += static_cast<size_t>(every) * kGripFloat4s * h->d.g_count;
         A.phases = ph;
         A.slots = slots;
         A.shift = adjoint_shift(n, shape.ranks);
@@ -3492,6 +3501,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         replay[j] = b->host_cloths[j];
         replay[j].tape = const_cast<float4*>(args[k].tape);
         replay[j].tape_v = const_cast<float4*>(args[k].tape_v);
+        replay[j].tape_grip = const_cast<NumiClothGrip*>(args[k].tape_grip);
         replay[j].tape_slots = args[k].slots;
         replay[j].yarn_touched = d_touched;
     }

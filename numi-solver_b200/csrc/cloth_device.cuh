@@ -257,6 +257,9 @@ struct DeviceCloth {
     float4* tape;
     float4* tape_v;
     uint32_t tape_slots;
+    // and the grips as the substep's grip phase met them, [substep][g_count]
+    // (written where the grip is active)
+    NumiClothGrip* tape_grip;
     // set to 1 by a segment that records a fruit/yarn contact (null: not asked)
     uint32_t* yarn_touched;
     // tile mode of the cooperative grid (cloth_tile.cuh): CTA r's plan is

@@ -306,12 +306,19 @@ __device__ __forceinline__ bool grip_core(const DeviceCloth& d, const SubCfg& c,
     return true;
 }
 
+// Adjoint tape: grip g of the substep (a later re-attach rewrites its
+// particle, offset and generation).
+__device__ __forceinline__ void tape_grip(const Ctx& ctx, uint32_t g, const NumiClothGrip& grip) {
+    ctx.d.tape_grip[static_cast<size_t>(ctx.s.tape_first + ctx.sub) * ctx.d.g_count + g] = grip;
+}
+
 __device__ void solve_grips(const Ctx& ctx) {
     const DeviceCloth& d = ctx.d;
     const SubCfg& c = ctx.c;
     const uint32_t g = threadIdx.x;
     if (g >= d.g_count || !c.grip_active) return;
     NumiClothGrip grip = d.grips[g];
+    if (d.tape != nullptr) tape_grip(ctx, g, grip);
     if (grip.particle.y != c.grip_gen) return;
     const uint32_t i = grip.particle.x;
     float4 p = px(ctx, i);

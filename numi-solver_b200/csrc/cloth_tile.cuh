@@ -234,6 +234,7 @@ __device__ void tile_grips(const Ctx& ctx) {
         grip.lambda.x = 0.0f;
         grip.lambda.y = 0.0f;
         grip.lambda.z = 0.0f;
+        if (d.tape != nullptr && c.grip_active) tape_grip(ctx, g, grip);
         if (c.grip_active && grip.particle.y == c.grip_gen) {
             float4 p = ctx.tx[own & 0xffffu];
             if (grip_core(d, c, grip, p)) ctx.tx[own & 0xffffu] = p;

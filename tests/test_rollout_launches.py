@@ -84,3 +84,54 @@ def test_tape_of_a_large_cloth(contact):
     assert one["info"]["grid"] == 1
     _same_gradients(tiled, plain)
     _same_gradients(tiled, one)
+
+
+def _regrab(scene, substeps=24):
+    """The grip lets go half way and takes hold again elsewhere (a later
+    generation); the second loss' targets are what the rollout reaches, so
+    only the first, before the re-grab, has gradients."""
+    cfg, tracked, targets = _rollout(scene, substeps)
+    half = substeps // 2
+    cfg["gripControl"][half:, 0] += 1
+    cfg["gripTargetAndActive"][half:, 0] += np.float32(0.003)
+    cfg["gripTargetAndActive"][half:half + 2, 3] = 0.0   # open for two substeps
+    sched = nc.Schedule.make(**dict(PLAIN, damping=0.5))
+    sv = nc.ClothSolver(scene)
+    sv.step(cfg, sched)
+    x = sv.particles()["positionAndInverseMass"][tracked, :3].astype(np.float64)
+    assert sv.failure() == 0 and int(sv.grips()["particle"][0, 1]) == int(cfg["gripControl"][-1, 0])
+    sv.close()
+    return cfg, sched, tracked, np.stack([targets[0], x])
+
+
+@pytest.mark.parametrize("every", [5, 12, 24])
+@pytest.mark.parametrize("side", [12, 40, 72], ids=["one-cta", "cluster", "tiles"])
+def test_gradients_before_a_regrab(side, every):
+    """The reverse sweep meets every substep's own grips, not the last
+    generation's: gradients up to a re-grab are those of the rollout that
+    ends there (sums in other segments: 1e-10)."""
+    scene = _scene(side, False)
+    cfg, sched, tracked, targets = _regrab(scene)
+    sv = nc.ClothSolver(scene)
+    sv.snapshot(0)
+    half = sv.rollout_grad(cfg[:12], sched, tracked, targets[:1], 12, checkpoint_every=12)
+    sv.restore(0)
+    full = sv.rollout_grad(cfg, sched, tracked, targets, 12, checkpoint_every=every)
+    sv.close()
+    batched = []
+    for c, t in ((cfg[:12], targets[:1]), (cfg, targets)):
+        solvers = [nc.ClothSolver(scene) for _ in range(2)]
+        batch = nc.ClothBatch(solvers)
+        r = batch.rollout_grad(np.stack([c, c]), sched, tracked, np.stack([t, t]), 12, checkpoint_every=every)
+        batched.append((r["loss"][1], r["grads"][1], r["damping"][1]))
+        batch.close()
+    assert np.abs(half["grip"]).max() > 0.0 and half["loss"] > 0.0
+    scale = np.abs(half["grip"]).max()
+    assert np.allclose(full["grip"][:12], half["grip"], rtol=1e-10, atol=1e-10 * scale)
+    assert np.array_equal(full["grip"][12:], np.zeros((12, 6)))
+    for a, b in ((full, half),):
+        assert np.allclose(a["loss"], b["loss"], rtol=1e-12)
+        assert np.allclose(a["grads"], b["grads"], rtol=1e-10, atol=1e-10 * np.abs(b["grads"]).max())
+        assert np.allclose(a["damping"], b["damping"], rtol=1e-10)
+    for a, b in zip(batched[1], (half["loss"], half["grads"], half["damping"])):
+        assert np.allclose(a, b, rtol=1e-10, atol=1e-10 * np.abs(b).max())
