@@ -234,6 +234,15 @@ const void* batch_fn(bool edge) {
 }
 
 const void* batch_cluster_fn() { return reinterpret_cast<const void*>(numi_cloth_batch_cluster_kernel); }
+// The kernels of rollout gradients (for handles of either self-contact order:
+// their schedules have none).
+const void* frame_tape_fn() { return reinterpret_cast<const void*>(numi_cloth_frame_tape_kernel); }
+const void* batch_tape_fn(bool cluster) {
+    return cluster ? reinterpret_cast<const void*>(numi_cloth_batch_cluster_tape_kernel)
+                   : reinterpret_cast<const void*>(numi_cloth_batch_tape_kernel);
+}
+const std::initializer_list<const void*> kFrameKernels = {frame_fn(false), frame_fn(true), frame_fn(false, true),
+                                                          frame_fn(true, true), frame_tape_fn()};
 
 cudaError_t raise_smem(const void* fn, size_t bytes) {
     cudaFuncAttributes fa{};
@@ -244,26 +253,41 @@ cudaError_t raise_smem(const void* fn, size_t bytes) {
 }
 cudaError_t raise_frame_smem(size_t bytes) {
     cudaError_t e = cudaSuccess;
-    for (bool exact : {false, true})
-        for (bool edge : {false, true})
-            if (e == cudaSuccess) e = raise_smem(frame_fn(edge, exact), bytes);
+    for (const void* fn : kFrameKernels)
+        if (e == cudaSuccess) e = raise_smem(fn, bytes);
     return e;
 }
 void allow_large_clusters() {
-    for (bool exact : {false, true})
-        for (bool edge : {false, true})
-            cudaFuncSetAttribute(frame_fn(edge, exact), cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (const void* fn : kFrameKernels) cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 // Clusters of cfg's shape that every frame kernel can place at once.
 int frame_clusters(const cudaLaunchConfig_t& cfg) {
     int lo = 1 << 30;
-    for (bool exact : {false, true})
-        for (bool edge : {false, true}) {
-            int clusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&clusters, frame_fn(edge, exact), &cfg) != cudaSuccess) return 0;
-            lo = std::min(lo, clusters);
-        }
+    for (const void* fn : kFrameKernels) {
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) return 0;
+        lo = std::min(lo, clusters);
+    }
     return lo;
+}
+// Shared memory of its own the larger of a handle's tile-mode kernels has.
+size_t tile_static_smem(const numi_cloth* h) {
+    cudaFuncAttributes fa{}, ft{};
+    cudaFuncGetAttributes(&fa, frame_fn(false, h->self_exact));
+    cudaFuncGetAttributes(&ft, frame_tape_fn());
+    return std::max(fa.sharedSizeBytes, ft.sharedSizeBytes);
+}
+// Whether the device holds the handle's tile launch co-resident.
+bool tiles_fit(const numi_cloth* h) {
+    int sms = 0, lo = 1 << 30;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
+    if (raise_frame_smem(h->tile_smem) != cudaSuccess) return false;
+    for (const void* fn : {frame_fn(false, h->self_exact), frame_tape_fn()}) {
+        int k = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, fn, NC_BLOCK_MAX, h->tile_smem) != cudaSuccess) return false;
+        lo = std::min(lo, k);
+    }
+    return static_cast<uint64_t>(lo) * static_cast<uint64_t>(sms) >= h->tile_grid;
 }
 
 bool finite4(const numi_float4& v) {
@@ -703,9 +727,7 @@ bool rebuild_tiles(numi_cloth* h) {
         return false;
     int max_optin = 0;
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
-    cudaFuncAttributes fa{};
-    cudaFuncGetAttributes(&fa, frame_fn(false, h->self_exact));
-    return build_tiles(h, d.grid_width, dij, dmat, bij, bmat, static_cast<size_t>(max_optin) - fa.sharedSizeBytes);
+    return build_tiles(h, d.grid_width, dij, dmat, bij, bmat, static_cast<size_t>(max_optin) - tile_static_smem(h));
 }
 
 // A launch runs in tile mode when the cloth has tile plans and the
@@ -735,6 +757,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     d.cfg = h->d_cfg + cfg_offset;
     d.epoch_base = h->epoch;
     const bool taped = tape.x != nullptr;
+    const bool rollout = taped || tape.touched != nullptr;
     d.yarn_touched = tape.touched;
     if (taped) {
         d.tape = tape.x;
@@ -748,6 +771,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     sc.tape_first = tape.first;
     void* args[] = {&d, &sc};
     const bool edge = sc.primitive_self != 0u && d.edge_count != nullptr;
+    const void* fn = rollout ? frame_tape_fn() : frame_fn(edge, h->self_exact);
     if (d.trace != nullptr && substeps > h->trace_capacity) d.trace = nullptr;
     if (d.trace == nullptr) d.trace_cta = nullptr;
     cudaError_t e = cudaMemsetAsync(h->d.bar_count, 0, kBarrierWords * sizeof(unsigned long long), h->stream);
@@ -798,9 +822,9 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         d.cluster_barrier = 1u;
-        e = cudaLaunchKernelExC(&cfg, frame_fn(edge, h->self_exact), args);
+        e = cudaLaunchKernelExC(&cfg, fn, args);
     } else if (h->grid == 1 && !tiled) {
-        e = cudaLaunchKernel(frame_fn(edge, h->self_exact), dim3(1), dim3(h->block), args, smem, h->stream);
+        e = cudaLaunchKernel(fn, dim3(1), dim3(h->block), args, smem, h->stream);
     } else if (tiled) {
         if (h->tiles_dirty) {
             if (!rebuild_tiles(h)) return cudaErrorUnknown;
@@ -813,8 +837,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
         if (h->tile_grid > h->grid) d.trace_cta = nullptr;
         e = raise_frame_smem(h->tile_smem);
         if (e == cudaSuccess)
-            e = cudaLaunchCooperativeKernel(frame_fn(false, h->self_exact), dim3(h->tile_grid), dim3(h->tile_block), args,
-                                            h->tile_smem, h->stream);
+            e = cudaLaunchCooperativeKernel(fn, dim3(h->tile_grid), dim3(h->tile_block), args, h->tile_smem, h->stream);
         h->last_grid = h->tile_grid;
         h->last_block = h->tile_block;
         h->last_tiles = true;
@@ -823,13 +846,12 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     } else {
         // neighbour syncs between colours (the kernel without the edge/edge
         // phases; its flags start at zero in every launch)
-        if (h->neighbours && !edge && !taped) {
+        if (h->neighbours && !edge && !rollout) {
             d.nbr_on = 1u;
             e = cudaMemsetAsync(d.nbr_flag, 0, NC_NBR_FLAG_STRIDE * h->grid * sizeof(unsigned int), h->stream);
             if (e != cudaSuccess) return e;
         }
-        e = cudaLaunchCooperativeKernel(frame_fn(edge, h->self_exact), dim3(h->grid), dim3(h->block), args,
-                                        d.nbr_on ? h->nbr_smem : smem, h->stream);
+        e = cudaLaunchCooperativeKernel(fn, dim3(h->grid), dim3(h->block), args, d.nbr_on ? h->nbr_smem : smem, h->stream);
     }
     h->last_grid = h->cluster > 0 ? h->cluster : h->grid;
     h->last_block = h->block;
@@ -1215,11 +1237,11 @@ int numi_cloth_create(const NumiClothScene* scene, numi_cloth_t** out) {
     const bool forced_block = env_u32("NUMI_CLOTH_BLOCK", block);
     if (forced_block && block != NC_BLOCK_MAX) block = NC_THREADS;
     h->block = block;
-    for (bool edge : {false, true}) {
+    per_sm = 1 << 30;
+    for (const void* fn : {frame_fn(false, h->self_exact), frame_fn(true, h->self_exact), frame_tape_fn()}) {
         int k = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, frame_fn(edge, h->self_exact), static_cast<int>(block),
-                                                      nc_resident_offset());
-        per_sm = edge ? std::min(per_sm, k) : k;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, fn, static_cast<int>(block), nc_resident_offset());
+        per_sm = std::min(per_sm, k);
     }
     uint32_t work = std::max({n, D, K, B});
     uint32_t grid = (work <= 8192u) ? 1u : std::min<uint32_t>(sms * std::max(per_sm, 1), (work + block - 1u) / block);
@@ -1478,21 +1500,13 @@ int numi_cloth_create(const NumiClothScene* scene, numi_cloth_t** out) {
     if (want_tiles != 0u && h->grid > 1u && h->cluster == 0u && d.resident == 0u && K == 0u) {
         int max_optin = 0;
         cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
-        cudaFuncAttributes fa{};
-        cudaFuncGetAttributes(&fa, frame_fn(false, h->self_exact));
         uint32_t tgrid = static_cast<uint32_t>(sms);
         env_u32("NUMI_CLOTH_TILE_GRID", tgrid);
         h->tile_grid = std::max(tgrid, 3u);
         h->tile_block = NC_BLOCK_MAX;
         h->tiles = build_tiles(h, scene->gridWidth, hij, hdm, hbij, hbm,
-                               static_cast<size_t>(max_optin) - fa.sharedSizeBytes);
-        if (h->tiles) {
-            int k = 0;
-            h->tiles = raise_frame_smem(h->tile_smem) == cudaSuccess &&
-                       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, frame_fn(false, h->self_exact), NC_BLOCK_MAX,
-                                                                     h->tile_smem) == cudaSuccess &&
-                       static_cast<uint64_t>(k) * static_cast<uint64_t>(sms) >= h->tile_grid;
-        }
+                               static_cast<size_t>(max_optin) - tile_static_smem(h)) &&
+                   tiles_fit(h);
         cudaGetLastError();
     }
     for (uint32_t g = 0; g < G; ++g) h->grip_compliance.push_back(scene->grips[g].targetOffsetAndCompliance.w);
@@ -1874,18 +1888,9 @@ namespace {
 // Tile plans for a tile launch of `grid` CTAs, and whether the device holds
 // that grid co-resident with their shared memory.
 bool configure_tiles(numi_cloth* h, uint32_t grid) {
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
     h->tile_grid = grid;
-    h->tiles = rebuild_tiles(h);
+    h->tiles = rebuild_tiles(h) && tiles_fit(h);
     h->tiles_dirty = false;
-    if (h->tiles) {
-        int k = 0;
-        h->tiles = raise_frame_smem(h->tile_smem) == cudaSuccess &&
-                   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, frame_fn(false, h->self_exact), NC_BLOCK_MAX, h->tile_smem) ==
-                       cudaSuccess &&
-                   static_cast<uint64_t>(k) * static_cast<uint64_t>(sms) >= h->tile_grid;
-    }
     cudaGetLastError();
     return h->tiles;
 }
@@ -2330,7 +2335,10 @@ size_t batch_room(const numi_cloth_batch* b, bool edge) {
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, batch_fn(edge)) != cudaSuccess) return 0;
-    const size_t fixed = nc_resident_offset() + fa.sharedSizeBytes + 256u + (edge ? NC_EDGE_TREE_KEY_BYTES : 0u);
+    cudaFuncAttributes ft = fa;
+    if (!edge && cudaFuncGetAttributes(&ft, batch_tape_fn(false)) != cudaSuccess) return 0;
+    const size_t fixed = nc_resident_offset() + std::max(fa.sharedSizeBytes, ft.sharedSizeBytes) + 256u +
+                         (edge ? NC_EDGE_TREE_KEY_BYTES : 0u);
     return static_cast<size_t>(optin) > fixed ? static_cast<size_t>(optin) - fixed : 0u;
 }
 
@@ -2412,9 +2420,10 @@ int batch_fit(numi_cloth_batch* b) {
     return NUMI_CLOTH_OK;
 }
 
-// Launch of the batch kernel over `cloths` (launch order) in the batch's
-// shape; the work queue starts at zero.
-cudaError_t batch_kernel(numi_cloth_batch* b, const DeviceCloth* cloths, const Schedule& s) {
+// Launch of the batch kernel (of rollout gradients with `rollout`) over
+// `cloths` (launch order) in the batch's shape; the work queue starts at
+// zero.
+cudaError_t batch_kernel(numi_cloth_batch* b, const DeviceCloth* cloths, const Schedule& s, bool rollout = false) {
     const bool edge = s.primitive_self != 0u;
     const bool fit_edge = b->fitted && edge;
     uint32_t ranks = fit_edge ? 1u : b->ranks;
@@ -2441,7 +2450,9 @@ cudaError_t batch_kernel(numi_cloth_batch* b, const DeviceCloth* cloths, const S
     cfg.numAttrs = ranks > 1u ? 1u : 0u;
     unsigned int* queue = b->queue;
     void* args[] = {&cloths, &count, &sc, &queue, &ranks};
-    return cudaLaunchKernelExC(&cfg, ranks > 1u ? batch_cluster_fn() : batch_fn(edge), args);
+    const void* fn = rollout ? batch_tape_fn(ranks > 1u) : ranks > 1u ? batch_cluster_fn() : batch_fn(edge);
+    if (rollout) e = raise_smem(fn, smem);
+    return e == cudaSuccess ? cudaLaunchKernelExC(&cfg, fn, args) : e;
 }
 
 // Descriptors of every cloth for a launch of `substeps` Configs each.
@@ -3551,7 +3562,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         st.cfg_offset = first;
         st.epoch_ptr = b->epoch;
         st.tape_first = tape_first;
-        return batch_kernel(b, taped ? d_replay : b->d_cloths, st) == cudaSuccess;
+        return batch_kernel(b, taped ? d_replay : b->d_cloths, st, true) == cudaSuccess;
     };
     // forward: taped where the tape holds it, else checkpointed (the last
     // segment of cloths without fruits is taped as it runs)

@@ -85,7 +85,7 @@ __device__ __forceinline__ bool grid_sync(Ctx& ctx) {
                 globaltimer();
     }
     // (tile mode writes its own tape: it passes four barriers a substep)
-    for (bool taped = d.tape != nullptr && ctx.s.tiles == 0u;; taped = false) {
+    for (bool taped = kTaped && d.tape != nullptr && ctx.s.tiles == 0u;; taped = false) {
         if (d.cluster_barrier)
             cooperative_groups::this_cluster().sync();
         else if (ctx.ranks == 1)
@@ -577,7 +577,7 @@ struct SegRecords {
 
     __device__ void finish(const Ctx& ctx) const {
         if (!recorded) return;
-        if (ctx.d.yarn_touched != nullptr) *ctx.d.yarn_touched = 1u;
+        if (kTaped && ctx.d.yarn_touched != nullptr) *ctx.d.yarn_touched = 1u;
         ctx.d.yarn_live[seg] = ctx.epoch;
         // first record of the substep: the segment joins the friction list
         if (!was_live) ctx.d.yarn_list[atomicAdd(ctx.d.yarn_list_n, 1u)] = seg;
@@ -3088,7 +3088,7 @@ __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule
         ctx.c = nc::load_cfg(d.cfg + s.cfg_offset + sub);
         ctx.epoch = epoch_base + sub;
         ctx.barriers = 0;
-        if (d.tape != nullptr && s.tiles == 0u) {
+        if (nc::kTaped && d.tape != nullptr && s.tiles == 0u) {
             // adjoint tape: state at the start of the substep (its first
             // phase moves a CTA's own particles, thread by thread as here).
             // Not in tile mode, where the previous substep's friction sweep
@@ -3139,6 +3139,12 @@ __global__ void numi_cloth_batch_edge_kernel(const DeviceCloth* cloths, uint32_t
 // registers in every phase.
 __global__ void numi_cloth_frame_exact_kernel(DeviceCloth d, Schedule s);
 __global__ void numi_cloth_frame_edge_exact_kernel(DeviceCloth d, Schedule s);
+// And the kernels of rollout gradients in cloth_tape_kernels.cu.
+__global__ void numi_cloth_frame_tape_kernel(DeviceCloth d, Schedule s);
+__global__ void numi_cloth_batch_tape_kernel(const DeviceCloth* cloths, uint32_t count, Schedule s,
+                                             unsigned int* queue);
+__global__ void numi_cloth_batch_cluster_tape_kernel(const DeviceCloth* cloths, uint32_t count, Schedule s,
+                                                     unsigned int* queue, uint32_t ranks);
 
 // Many independent cloths in one persistent launch: every CTA, or every
 // cluster of `ranks` CTAs, takes the next cloth from a device work queue
@@ -3158,6 +3164,28 @@ __global__ void numi_cloth_frame_edge_exact_kernel(DeviceCloth d, Schedule s);
         __syncthreads();                                                      \
     }
 
+// The cluster's first CTA draws for all of its CTAs; the barrier after a frame
+// keeps a CTA from staging the next cloth over particles another CTA of the
+// cluster still reads.
+#define NC_BATCH_CLUSTER_BODY                                                                  \
+    extern __shared__ __align__(16) unsigned char nc_dynamic_smem[];                           \
+    __shared__ uint32_t s_next;                                                                \
+    const uint32_t rank = blockIdx.x % ranks;                                                  \
+    cooperative_groups::this_cluster().sync(); /* every CTA's shared memory is up */           \
+    for (;;) {                                                                                 \
+        if (rank == 0u && threadIdx.x == 0) {                                                  \
+            const uint32_t drawn = atomicAdd(queue, 1u);                                       \
+            s_next = drawn;                                                                    \
+            for (uint32_t r = 1; r < ranks; ++r)                                               \
+                *static_cast<uint32_t*>(__cluster_map_shared_rank(&s_next, r)) = drawn;        \
+        }                                                                                      \
+        cooperative_groups::this_cluster().sync();                                             \
+        const uint32_t k = s_next;                                                             \
+        if (k >= count) break;                                                                 \
+        run_frame<false, true>(cloths[k], s, rank, ranks, nc_dynamic_smem);                    \
+        cooperative_groups::this_cluster().sync();                                             \
+    }
+
 #ifndef NC_EDGE_KERNELS
 // One cloth on the whole grid (one CTA, a cooperative grid or a cluster).
 __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_frame_kernel(DeviceCloth d, Schedule s) {
@@ -3169,29 +3197,10 @@ __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_batch_kernel(const
     NC_BATCH_BODY(false)
 }
 
-// The cluster's first CTA draws for all of its CTAs; the barrier after a frame
-// keeps a CTA from staging the next cloth over particles another CTA of the
-// cluster still reads.
 __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_batch_cluster_kernel(const DeviceCloth* cloths,
                                                                                  uint32_t count, Schedule s,
                                                                                  unsigned int* queue, uint32_t ranks) {
-    extern __shared__ __align__(16) unsigned char nc_dynamic_smem[];
-    __shared__ uint32_t s_next;
-    const uint32_t rank = blockIdx.x % ranks;
-    cooperative_groups::this_cluster().sync();   // every CTA's shared memory is up
-    for (;;) {
-        if (rank == 0u && threadIdx.x == 0) {
-            const uint32_t drawn = atomicAdd(queue, 1u);
-            s_next = drawn;
-            for (uint32_t r = 1; r < ranks; ++r)
-                *static_cast<uint32_t*>(__cluster_map_shared_rank(&s_next, r)) = drawn;
-        }
-        cooperative_groups::this_cluster().sync();
-        const uint32_t k = s_next;
-        if (k >= count) break;
-        run_frame<false, true>(cloths[k], s, rank, ranks, nc_dynamic_smem);
-        cooperative_groups::this_cluster().sync();
-    }
+    NC_BATCH_CLUSTER_BODY
 }
 
 // Advance the batch substep counter after a batch launch.

@@ -306,6 +306,14 @@ __device__ __forceinline__ bool grip_core(const DeviceCloth& d, const SubCfg& c,
     return true;
 }
 
+// The adjoint tape is written, and fruit contact recorded, by kernels of their
+// own (cloth_tape_kernels.cu).
+#ifdef NC_TAPE_KERNELS
+constexpr bool kTaped = true;
+#else
+constexpr bool kTaped = false;
+#endif
+
 // Adjoint tape: grip g of the substep (a later re-attach rewrites its
 // particle, offset and generation).
 __device__ __forceinline__ void tape_grip(const Ctx& ctx, uint32_t g, const NumiClothGrip& grip) {
@@ -318,7 +326,7 @@ __device__ void solve_grips(const Ctx& ctx) {
     const uint32_t g = threadIdx.x;
     if (g >= d.g_count || !c.grip_active) return;
     NumiClothGrip grip = d.grips[g];
-    if (d.tape != nullptr) tape_grip(ctx, g, grip);
+    if (kTaped && d.tape != nullptr) tape_grip(ctx, g, grip);
     if (grip.particle.y != c.grip_gen) return;
     const uint32_t i = grip.particle.x;
     float4 p = px(ctx, i);

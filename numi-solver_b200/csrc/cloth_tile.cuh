@@ -118,7 +118,7 @@ __device__ __forceinline__ void tile_store(const Ctx& ctx, float4* out) {
 // thread of the CTA, between two CTA barriers of its own.
 __device__ __forceinline__ void tile_tape(const Ctx& ctx, uint32_t slot) {
     const DeviceCloth& d = ctx.d;
-    if (d.tape == nullptr || slot >= d.tape_slots) return;
+    if (!kTaped || d.tape == nullptr || slot >= d.tape_slots) return;
     float4* out = d.tape + (static_cast<size_t>(ctx.s.tape_first + ctx.sub) * d.tape_slots + slot) * d.n;
     const uint32_t own = ctx.tp[1];
     const uint32_t* gi = tile_list(ctx);
@@ -145,7 +145,7 @@ __device__ void tile_predict(const Ctx& ctx, float4* v_next) {
             const float4 pp = ld(d.xp + i);
             d.xp[i] = make_float4(p.x, p.y, p.z, pp.w);
             v_next[i] = make_float4(vel.x, vel.y, vel.z, vel.z);
-            if (d.tape != nullptr) {
+            if (kTaped && d.tape != nullptr) {
                 const size_t at = ctx.s.tape_first + ctx.sub;
                 d.tape[at * d.tape_slots * d.n + i] = p;
                 d.tape_v[at * d.n + i] = __ldcg(ctx.gv + i);
@@ -234,7 +234,7 @@ __device__ void tile_grips(const Ctx& ctx) {
         grip.lambda.x = 0.0f;
         grip.lambda.y = 0.0f;
         grip.lambda.z = 0.0f;
-        if (d.tape != nullptr && c.grip_active) tape_grip(ctx, g, grip);
+        if (kTaped && d.tape != nullptr && c.grip_active) tape_grip(ctx, g, grip);
         if (c.grip_active && grip.particle.y == c.grip_gen) {
             float4 p = ctx.tx[own & 0xffffu];
             if (grip_core(d, c, grip, p)) ctx.tx[own & 0xffffu] = p;
@@ -631,7 +631,7 @@ __device__ bool substep_tiles(Ctx& ctx, bool last) {
     }
     // a taped launch counts its slots, as the colour-by-colour launch's
     // barriers number them (the host compares them with the phase list)
-    if (d.tape != nullptr) ctx.barriers = slot;
+    if (kTaped && d.tape != nullptr) ctx.barriers = slot;
     return true;
 }
 
