@@ -167,6 +167,7 @@ struct Ctx {
     // shared memory
     const uint32_t* tp;
     const uint4* ti;          // its items: in shared memory too, or streamed from global memory
+    bool stream;              // the latter
     float4* tx;
     FrictionStage* fst;       // tile mode, fruit CTA: the staged friction sweep
     bool hold_tail;           // tile mode: a grid barrier follows the fruit-CTA tail
