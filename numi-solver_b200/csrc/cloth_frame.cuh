@@ -3008,7 +3008,8 @@ __device__ bool validate_records(const DeviceCloth& d, const SubCfg& c0) {
 // shared memory.
 // The descriptor is copied into shared memory first, so both kernels run
 // the phases on the same (shared-memory) view of it.
-template <bool kEdge, bool kIlp>
+// kBatch: one of many cloths in a launch, whose residency is its own.
+template <bool kEdge, bool kIlp, bool kBatch>
 __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule& s, uint32_t rank, uint32_t ranks,
                                           unsigned char* dynamic_smem) {
     {
@@ -3033,7 +3034,10 @@ __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule
     ctx.seq = 0;
     ctx.nseq = 0;
     ctx.resident = d.resident != 0u;
-    ctx.resident_v = d.resident == 1u;
+    // velocities live with the positions except in a batch.  Known to be one
+    // switch, a phase that reads both issues its loads together (a 96 x 96
+    // cloth on one CTA: predict 18.9 us with two, finalize 11.8)
+    ctx.resident_v = kBatch ? d.resident == 1u : ctx.resident;
     ctx.rank = rank;
     ctx.ranks = ranks;
     ctx.shift = d.resident_shift;
@@ -3160,7 +3164,7 @@ __global__ void numi_cloth_batch_cluster_tape_kernel(const DeviceCloth* cloths, 
         __syncthreads();                                                      \
         const uint32_t k = s_next;                                            \
         if (k >= count) break;                                                \
-        run_frame<kEdge, true>(cloths[k], s, 0u, 1u, nc_dynamic_smem);        \
+        run_frame<kEdge, true, true>(cloths[k], s, 0u, 1u, nc_dynamic_smem);  \
         __syncthreads();                                                      \
     }
 
@@ -3182,7 +3186,7 @@ __global__ void numi_cloth_batch_cluster_tape_kernel(const DeviceCloth* cloths, 
         cooperative_groups::this_cluster().sync();                                             \
         const uint32_t k = s_next;                                                             \
         if (k >= count) break;                                                                 \
-        run_frame<false, true>(cloths[k], s, rank, ranks, nc_dynamic_smem);                    \
+        run_frame<false, true, true>(cloths[k], s, rank, ranks, nc_dynamic_smem);              \
         cooperative_groups::this_cluster().sync();                                             \
     }
 
@@ -3190,7 +3194,7 @@ __global__ void numi_cloth_batch_cluster_tape_kernel(const DeviceCloth* cloths, 
 // One cloth on the whole grid (one CTA, a cooperative grid or a cluster).
 __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_frame_kernel(DeviceCloth d, Schedule s) {
     extern __shared__ __align__(16) unsigned char nc_dynamic_smem[];
-    run_frame<false, false>(d, s, blockIdx.x, gridDim.x, nc_dynamic_smem);
+    run_frame<false, false, false>(d, s, blockIdx.x, gridDim.x, nc_dynamic_smem);
 }
 __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_batch_kernel(const DeviceCloth* cloths, uint32_t count,
                                                                          Schedule s, unsigned int* queue) {

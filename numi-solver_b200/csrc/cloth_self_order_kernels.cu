@@ -11,10 +11,10 @@
 
 __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_frame_exact_kernel(DeviceCloth d, Schedule s) {
     extern __shared__ __align__(16) unsigned char nc_dynamic_smem[];
-    run_frame<false, false>(d, s, blockIdx.x, gridDim.x, nc_dynamic_smem);
+    run_frame<false, false, false>(d, s, blockIdx.x, gridDim.x, nc_dynamic_smem);
 }
 
 __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_frame_edge_exact_kernel(DeviceCloth d, Schedule s) {
     extern __shared__ __align__(16) unsigned char nc_dynamic_smem[];
-    run_frame<true, true>(d, s, blockIdx.x, gridDim.x, nc_dynamic_smem);
+    run_frame<true, true, false>(d, s, blockIdx.x, gridDim.x, nc_dynamic_smem);
 }

@@ -8,7 +8,7 @@
 
 __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_frame_tape_kernel(DeviceCloth d, Schedule s) {
     extern __shared__ __align__(16) unsigned char nc_dynamic_smem[];
-    run_frame<false, false>(d, s, blockIdx.x, gridDim.x, nc_dynamic_smem);
+    run_frame<false, false, false>(d, s, blockIdx.x, gridDim.x, nc_dynamic_smem);
 }
 
 __global__ void __launch_bounds__(NC_BLOCK_MAX, 1) numi_cloth_batch_tape_kernel(const DeviceCloth* cloths,
