@@ -879,13 +879,13 @@ Schedule device_schedule(const NumiClothSchedule& schedule) {
     return s;
 }
 
-// Point self-contact grid of a cloth, allocated on first use (about two
-// buckets per particle); the bucket heads are cleared when the 26-bit
+// Point self-contact grid of a cloth, allocated on first use (about four
+// buckets per particle, of which a cloth in an axis plane uses half); the bucket heads are cleared when the 26-bit
 // substep part of their tags wraps within the next `substeps`.
 int prepare_self_grid(numi_cloth* h, bool self_collision, uint32_t substeps) {
     if (self_collision && h->d.hash_head == nullptr) {
         uint32_t buckets = 1024u;
-        while (buckets < 2u * h->d.n) buckets <<= 1;
+        while (buckets < 4u * h->d.n) buckets <<= 1;
         DeviceCloth& d = h->d;
         d.hash_head = h->buf.alloc<unsigned long long>(buckets);
         d.hash_over_head = h->buf.alloc<unsigned long long>(1);

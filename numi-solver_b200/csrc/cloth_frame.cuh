@@ -915,25 +915,31 @@ __device__ __forceinline__ uint32_t cell_bucket(int x, int y, int z, uint32_t ma
 }
 
 // The point self-contact grid's buckets come in groups of NC_HASH_GROUP
-// neighbouring cells (4 x 2 x 1), and a group's storage is slot by slot, each
+// neighbouring cells (2 x 2 x 2), and a group's storage is slot by slot, each
 // slot's eight cells in one 128-byte line, its heads in half of one.  The
 // query is bound by the lines it touches: with every cell hashed on its own a
 // tile's 443 particles met some 1,600 lines of a head or a slot each, twice
 // what the L1 holds beside the tile's shared memory, and a warp's 32 loads as
-// many lines.  A row of the cloth now shares its lines among neighbours: on
-// the 256 x 256 cloth the query takes 9.4 us instead of 11.8 (8.6 with the
-// tests of a batch without branches) and the insert 2.0 instead of 3.2, on
-// the 512 x 512 cloth the query 21 (18.4) instead of 38.  The
-// hash of a group is a sum of odd multiples of its coordinates through the
-// 32-bit finalizer lowbias32 (Wellons, hash-prospector).
+// many lines.  Neighbours on the cloth now share their lines.  A cloth lies
+// in any plane, and a group's section by each axis plane is four cells, so
+// half of the table is used and it has four buckets a particle.  Insert and
+// query of a 256 x 256 cloth in the planes z, y and x = const: 10.4, 10.9 and
+// 10.7 us a substep, 15.3 to 15.8 with cells hashed on their own (9.7, 10.4
+// and 22 with groups of 4 x 2 x 1 and two buckets, where a cloth at x = const
+// is left with a quarter of the table); 512 x 512: 30.8, 30.8 and 29.9, 53 to
+// 55 (29.2, 29.3 and 104).  The hash of a group is a sum of odd multiples of
+// its coordinates through the 32-bit finalizer lowbias32 (Wellons,
+// hash-prospector).
 #define NC_HASH_GROUP 8u
 __device__ __forceinline__ uint32_t self_bucket(int x, int y, int z, uint32_t mask) {
-    uint32_t k = static_cast<uint32_t>(x >> 2) * 0x9e3779b1u + static_cast<uint32_t>(y >> 1) * 0x85ebca77u +
-                 static_cast<uint32_t>(z) * 0xc2b2ae3du;
+    uint32_t k = static_cast<uint32_t>(x >> 1) * 0x9e3779b1u + static_cast<uint32_t>(y >> 1) * 0x85ebca77u +
+                 static_cast<uint32_t>(z >> 1) * 0xc2b2ae3du;
     k = (k ^ (k >> 16)) * 0x7feb352du;
     k = (k ^ (k >> 15)) * 0x846ca68bu;
     k ^= k >> 16;
-    return (k * NC_HASH_GROUP + (static_cast<uint32_t>(x) & 3u) + 4u * (static_cast<uint32_t>(y) & 1u)) & mask;
+    return (k * NC_HASH_GROUP + (static_cast<uint32_t>(x) & 1u) + 2u * (static_cast<uint32_t>(y) & 1u) +
+            4u * (static_cast<uint32_t>(z) & 1u)) &
+           mask;
 }
 __device__ __forceinline__ uint32_t hash_slot(uint32_t bucket, uint32_t j) {
     return ((bucket / NC_HASH_GROUP) * NC_HASH_CAP + j) * NC_HASH_GROUP + bucket % NC_HASH_GROUP;
@@ -1055,22 +1061,16 @@ __device__ __forceinline__ void self_heads(const Ctx& ctx, const float4& p, Self
     }
 }
 
-// Candidates of cell c of a query (a bucket met twice counts once).  Cells
-// that differ in x or y are different cells of their groups, so only the two
-// cells of a z pair, c and c - 4, can share a bucket.
-__device__ __forceinline__ uint32_t self_cell_count(uint32_t tag, const SelfQuery& q, const unsigned long long hd[8],
-                                                    const bool near[8], uint32_t c) {
-    const bool repeat = c >= 4u && near[c & 3u] && q.bk[c & 3u] == q.bk[c];
-    return (near[c] && !repeat && static_cast<uint32_t>(hd[c] >> 32) == tag) ? min(static_cast<uint32_t>(hd[c]), NC_HASH_CAP)
-                                                                            : 0u;
-}
-
-// Candidates per bucket of this pass as prefix counts.
+// Candidates per bucket of this pass as prefix counts.  A query's eight cells
+// differ by one in some coordinate, so they are different cells of their
+// groups and no two share a bucket.
 __device__ __forceinline__ uint32_t self_counts(uint32_t tag, SelfQuery& q, const unsigned long long hd[8],
                                                 const bool near[8]) {
     q.pre[0] = 0u;
 #pragma unroll
-    for (uint32_t c = 0; c < 8u; ++c) q.pre[c + 1u] = q.pre[c] + self_cell_count(tag, q, hd, near, c);
+    for (uint32_t c = 0; c < 8u; ++c) q.pre[c + 1u] = q.pre[c] + (near[c] && static_cast<uint32_t>(hd[c] >> 32) == tag
+                                        ? min(static_cast<uint32_t>(hd[c]), NC_HASH_CAP)
+                                        : 0u);
     return q.pre[8];
 }
 
@@ -3035,8 +3035,8 @@ __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule
     ctx.nseq = 0;
     ctx.resident = d.resident != 0u;
     // velocities live with the positions except in a batch.  Known to be one
-    // switch, a phase that reads both issues its loads together (a 96 x 96
-    // cloth on one CTA: predict 18.9 us with two, finalize 11.8)
+    // switch, a phase that reads both issues its loads together (finalize of
+    // a 96 x 96 cloth on one CTA: 11.8 us with two, 10.1)
     ctx.resident_v = kBatch ? d.resident == 1u : ctx.resident;
     ctx.rank = rank;
     ctx.ranks = ranks;
