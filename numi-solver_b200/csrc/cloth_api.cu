@@ -9,11 +9,18 @@
 
 #include <algorithm>
 #include <cmath>
+#include <condition_variable>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <new>
+#include <deque>
+#include <initializer_list>
+#include <memory>
 #include <mutex>
+#include <new>
+#include <system_error>
+#include <thread>
+#include <utility>
 #include <vector>
 
 #include "cloth_frame.cuh"
@@ -153,6 +160,52 @@ struct Workspace {
     };
 };
 
+// What the tile plans of a cloth are made from: its colours, grid width and
+// particles, the ends of its records, and the shape of the tile launch.
+struct TileSource {
+    DeviceCloth d;
+    uint32_t grid = 0;   // CTAs of the tile launch
+    size_t smem_budget = 0;
+    std::vector<uint2> distances, bends;
+};
+
+// A plan on the device, with the buffers that a tile launch alternates to;
+// one allocation.
+struct TileBlock {
+    void* mem = nullptr;
+    uint32_t* words = nullptr;
+    uint32_t* off = nullptr;
+    uint32_t* owner = nullptr;
+    float4 *x_alt = nullptr, *v_alt = nullptr;
+    bool stream = false;
+    size_t smem = 0;
+    TileBlock() = default;
+    TileBlock(const TileBlock&) = delete;
+    TileBlock& operator=(const TileBlock&) = delete;
+    TileBlock& operator=(TileBlock&& o) noexcept {
+        if (mem != nullptr) cudaFree(mem);
+        mem = std::exchange(o.mem, nullptr);
+        words = o.words;
+        off = o.off;
+        owner = o.owner;
+        x_alt = o.x_alt;
+        v_alt = o.v_alt;
+        stream = o.stream;
+        smem = o.smem;
+        return *this;
+    }
+    ~TileBlock() {
+        if (mem != nullptr) cudaFree(mem);
+    }
+};
+
+struct TileJob {
+    TileSource source;
+    int device = 0;
+    TileBlock block;   // no memory where the plan did not fit
+    enum { kQueued, kRunning, kDone } state = kQueued;
+};
+
 struct numi_cloth {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -175,15 +228,18 @@ struct numi_cloth {
     float yarn_rest_median = 0.0f;   // median yarn segment rest length
     bool neighbours = false;         // neighbour-sync tables built for the cooperative grid
     size_t nbr_smem = 0;             // dynamic shared memory of a frame launch with them
-    // tile mode (cloth_tile.cuh): launch shape and shared memory of a tile
-    // launch; the plan is rebuilt before the next launch when a material
-    // changed (its items carry the materials)
+    // tile mode (cloth_tile.cuh): plan, launch shape and shared memory of a
+    // tile launch
     bool tiles = false;
-    bool tiles_dirty = false;
-    bool tiles_wanted = false;   // small cloth: its plan is built once it has stepped kTilePlanSubsteps
-    uint32_t tile_substeps = 0;  // substeps it has stepped (or is about to) that a plan covers
+    TileBlock plan;
     uint32_t tile_grid = 0, tile_block = 0;
     size_t tile_smem = 0;
+    // a small cloth that will have a plan: what it is made from until the
+    // build is under way, and the substeps it has stepped (or is about to)
+    // that a plan covers
+    std::unique_ptr<TileSource> tile_source;
+    std::shared_ptr<TileJob> tile_job;
+    uint32_t tile_substeps = 0;
     uint32_t last_grid = 0, last_block = 0;
     bool last_tiles = false;
     // host copies for the edge/edge local lists, built with the edge buffers
@@ -495,10 +551,15 @@ struct TileColour {
     uint32_t family, first, count, batch;
 };
 
-bool build_tiles(numi_cloth* h, uint32_t grid_width, const std::vector<uint2>& dij, const std::vector<float4>& dmat,
-                 const std::vector<uint4>& bij, const std::vector<float2>& bmat, size_t smem_budget) {
-    const DeviceCloth& d = h->d;
-    const uint32_t n = d.n, R = h->tile_grid, T = R - 1u;
+struct TilePlan {
+    std::vector<uint32_t> words, off, owner;
+    bool stream = false;
+    size_t smem = 0;
+};
+
+bool build_tiles(const TileSource& src, TilePlan& plan) {
+    const DeviceCloth& d = src.d;
+    const uint32_t n = d.n, grid_width = d.grid_width, R = src.grid, T = R - 1u;
     if (R < 3u || n == 0u) return false;
     // tiles
     std::vector<uint32_t> tile_of(n);
@@ -544,15 +605,17 @@ bool build_tiles(numi_cloth* h, uint32_t grid_width, const std::vector<uint2>& d
     for (uint32_t b = 0; b < d.n_dist_batches; ++b)
         for (uint32_t k = 0; k < d.dist_batches[b].count; ++k) {
             const uint32_t rec = d.dist_batches[b].first + k;
-            dist_of[static_cast<size_t>(b) * n + dij[rec].x] = dist_of[static_cast<size_t>(b) * n + dij[rec].y] = rec;
+            const uint2 e = src.distances[rec];
+            dist_of[static_cast<size_t>(b) * n + e.x] = dist_of[static_cast<size_t>(b) * n + e.y] = rec;
         }
     for (uint32_t b = 0; b < d.n_bend_batches; ++b)
         for (uint32_t k = 0; k < d.bend_batches[b].count; ++k) {
             const uint32_t rec = d.bend_batches[b].first + k;
-            bend_of[static_cast<size_t>(b) * n + bij[rec].x] = bend_of[static_cast<size_t>(b) * n + bij[rec].z] = rec;
+            const uint2 e = src.bends[rec];
+            bend_of[static_cast<size_t>(b) * n + e.x] = bend_of[static_cast<size_t>(b) * n + e.y] = rec;
         }
     auto ends = [&](uint32_t family, uint32_t rec) {
-        return family == NC_TILE_BEND ? make_uint2(bij[rec].x, bij[rec].z) : dij[rec];
+        return family == NC_TILE_BEND ? src.bends[rec] : src.distances[rec];
     };
     std::vector<uint32_t> owner(n, 0u), local_of(n, 0u);
     std::vector<uint32_t> need_stamp(n, 0u), item_stamp_d(d.d_count, 0u), item_stamp_b(d.b_count, 0u);
@@ -654,19 +717,6 @@ bool build_tiles(numi_cloth* h, uint32_t grid_width, const std::vector<uint2>& d
                     uint32_t* o = w.data() + items_at + 4u * item++;
                     o[0] = static_cast<uint32_t>(lidx[pe.x]) | (static_cast<uint32_t>(lidx[pe.y]) << 16);
                     o[1] = rec | ((t < tiles && tile_of[pe.x] == t) ? 0x80000000u : 0u);
-                    float m0 = 0.0f, m1 = 0.0f;
-                    if (col.family == NC_TILE_DISTANCE) {
-                        m0 = dmat[rec].x;
-                        m1 = dmat[rec].y;
-                    } else if (col.family == NC_TILE_BEND) {
-                        m0 = bmat[rec].x;
-                        m1 = bmat[rec].y;
-                    } else if (col.family == NC_TILE_LIMIT) {
-                        m0 = dmat[rec].x;
-                        m1 = dmat[rec].w;
-                    }
-                    std::memcpy(o + 2, &m0, 4);
-                    std::memcpy(o + 3, &m1, 4);
                 }
             }
         }
@@ -680,55 +730,208 @@ bool build_tiles(numi_cloth* h, uint32_t grid_width, const std::vector<uint2>& d
     // 512 x 512 cloth's are 25,000 items a CTA, 59 MB in all, which the L2
     // holds (a substep 158 us colour by colour, 101 with streamed items).
     const size_t fruit = nc_resident_offset() + sizeof(FrictionStage);
-    const bool stream = std::max(fruit, nc_fruit_offset() + widest) > smem_budget;
+    const bool stream = std::max(fruit, nc_fruit_offset() + widest) > src.smem_budget;
     const size_t smem = std::max(fruit, nc_fruit_offset() + (stream ? widest_stream : widest));
-    if (smem > smem_budget) return false;
-    std::vector<uint32_t> off(R + 1u, 0u), words;
+    if (smem > src.smem_budget) return false;
+    plan.off.assign(R + 1u, 0u);
     for (uint32_t t = 0; t < R; ++t) {
-        words.insert(words.end(), plans[t].begin(), plans[t].end());
-        off[t + 1u] = static_cast<uint32_t>(words.size());
+        plan.words.insert(plan.words.end(), plans[t].begin(), plans[t].end());
+        plan.off[t + 1u] = static_cast<uint32_t>(plan.words.size());
     }
-    std::vector<uint32_t> owner_word(n);
-    for (uint32_t i = 0; i < n; ++i) owner_word[i] = (owner[i] << 16) | local_of[i];
-    DeviceCloth& dd = h->d;
-    if (dd.x_alt == nullptr) {
-        dd.x_alt = h->buf.alloc<float4>(n);
-        dd.v_alt = h->buf.alloc<float4>(n);
-        dd.tile_owner = h->buf.alloc<uint32_t>(n);
-        dd.tile_off = h->buf.alloc<uint32_t>(R + 1u);
-    }
-    // the words are replaced on a rebuild (their size can change)
-    uint32_t* dw = h->buf.alloc<uint32_t>(words.size());
-    if (!dd.x_alt || !dd.v_alt || !dd.tile_owner || !dd.tile_off || !dw) return false;
-    if (cudaMemcpy(const_cast<uint32_t*>(dd.tile_owner), owner_word.data(), n * sizeof(uint32_t),
-                   cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(const_cast<uint32_t*>(dd.tile_off), off.data(), off.size() * sizeof(uint32_t),
-                   cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(dw, words.data(), words.size() * sizeof(uint32_t), cudaMemcpyHostToDevice) != cudaSuccess)
-        return false;
-    dd.tile_words = dw;
-    dd.tile_stream = stream ? 1u : 0u;
-    h->tile_smem = smem;
+    plan.owner.resize(n);
+    for (uint32_t i = 0; i < n; ++i) plan.owner[i] = (owner[i] << 16) | local_of[i];
+    plan.stream = stream;
+    plan.smem = smem;
     return true;
 }
 
-// Rebuild the tile plan from the device records (after a material change).
-bool rebuild_tiles(numi_cloth* h) {
-    const DeviceCloth& d = h->d;
-    std::vector<uint2> dij(d.d_count);
-    std::vector<float4> dmat(d.d_count);
-    std::vector<uint4> bij(d.b_count);
-    std::vector<float2> bmat(d.b_count);
-    if (cudaStreamSynchronize(h->stream) != cudaSuccess ||
-        (d.d_count && (cudaMemcpy(dij.data(), d.d_ij, d.d_count * sizeof(uint2), cudaMemcpyDeviceToHost) != cudaSuccess ||
-                       cudaMemcpy(dmat.data(), d.d_mat, d.d_count * sizeof(float4), cudaMemcpyDeviceToHost) != cudaSuccess)) ||
-        (d.b_count && (cudaMemcpy(bij.data(), d.b_ij, d.b_count * sizeof(uint4), cudaMemcpyDeviceToHost) != cudaSuccess ||
-                       cudaMemcpy(bmat.data(), d.b_mat, d.b_count * sizeof(float2), cudaMemcpyDeviceToHost) != cudaSuccess)))
+// While one lives, the calls of this thread are none that another stream's
+// capture forbids.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// A plan of `src` on the current device, on a stream of its own: no other
+// stream is waited for.  False where it does not fit.
+bool make_tiles(const TileSource& src, TileBlock& out) {
+    TilePlan plan;
+    if (!build_tiles(src, plan)) return false;
+    RelaxedCapture relaxed;
+    TileBlock block;
+    auto pieces = [&](Carver& c) {
+        block.words = c.get<uint32_t>(plan.words.size());
+        block.off = c.get<uint32_t>(plan.off.size());
+        block.owner = c.get<uint32_t>(plan.owner.size());
+        block.x_alt = c.get<float4>(src.d.n);
+        block.v_alt = c.get<float4>(src.d.n);
+    };
+    Carver measure{nullptr};
+    pieces(measure);
+    cudaStream_t stream = nullptr;
+    cudaError_t e = cudaMalloc(&block.mem, measure.used);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+    Carver carver{static_cast<char*>(block.mem)};
+    pieces(carver);
+    auto up = [&](uint32_t* dst, const std::vector<uint32_t>& v) {
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, stream);
+    };
+    up(block.words, plan.words);
+    up(block.off, plan.off);
+    up(block.owner, plan.owner);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (stream != nullptr) cudaStreamDestroy(stream);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
         return false;
+    }
+    block.stream = plan.stream;
+    block.smem = plan.smem;
+    out = std::move(block);
+    return true;
+}
+
+// The materials of a plan's items from the records (a plan is built without
+// them, and written again where they change).  A CTA per CTA of the plan.
+__global__ void numi_cloth_tile_materials_kernel(DeviceCloth d) {
+    uint32_t* plan = const_cast<uint32_t*>(d.tile_words) + d.tile_off[blockIdx.x];
+    for (uint32_t chain = 0; chain < NC_TILE_CHAINS; ++chain) {
+        const uint32_t* table = plan + plan[8u + 2u * chain];
+        for (uint32_t c = 0; c < plan[9u + 2u * chain]; ++c) {
+            uint4* items = reinterpret_cast<uint4*>(plan + plan[3]) + table[2u * c];
+            const uint32_t count = table[2u * c + 1u] & 0x0fffffffu, family = table[2u * c + 1u] >> 28;
+            if (family == NC_TILE_SEGMENT) continue;
+            for (uint32_t k = threadIdx.x; k < count; k += blockDim.x) {
+                const uint32_t rec = items[k].y & 0x7fffffffu;
+                float2 m;
+                if (family == NC_TILE_BEND) {
+                    m = d.b_mat[rec];
+                } else {
+                    const float4 v = d.d_mat[rec];
+                    m = make_float2(v.x, family == NC_TILE_DISTANCE ? v.y : v.w);
+                }
+                items[k].z = __float_as_uint(m.x);
+                items[k].w = __float_as_uint(m.y);
+            }
+        }
+    }
+}
+
+cudaError_t tile_materials(numi_cloth* h) {
+    numi_cloth_tile_materials_kernel<<<h->tile_grid, 256, 0, h->stream>>>(h->d);
+    return cudaGetLastError();
+}
+
+// Tile mode with this plan from the next launch on, where the device holds
+// the tile launch.  The plan it replaces is no longer in use.
+void adopt_tiles(numi_cloth* h, TileBlock&& block) {
+    h->plan = std::move(block);
+    DeviceCloth& d = h->d;
+    d.tile_words = h->plan.words;
+    d.tile_off = h->plan.off;
+    d.tile_owner = h->plan.owner;
+    d.tile_stream = h->plan.stream ? 1u : 0u;
+    d.x_alt = h->plan.x_alt;
+    d.v_alt = h->plan.v_alt;
+    h->tile_smem = h->plan.smem;
+    h->tiles = h->plan.mem != nullptr && tiles_fit(h) && tile_materials(h) == cudaSuccess;
+    cudaGetLastError();
+}
+
+// Source of a handle's plans, without the ends of its records.
+TileSource tile_source(const numi_cloth* h) {
     int max_optin = 0;
     cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
-    return build_tiles(h, d.grid_width, dij, dmat, bij, bmat, static_cast<size_t>(max_optin) - tile_static_smem(h));
+    TileSource src;
+    src.d = h->d;
+    src.grid = h->tile_grid;
+    src.smem_budget = static_cast<size_t>(max_optin) - tile_static_smem(h);
+    return src;
 }
+
+// One thread of the process that builds small cloths' plans beside the
+// threads that step them: started with the first build, ended with the
+// process.  A build is a few milliseconds of host work at most.
+class TileBuilder {
+  public:
+    static TileBuilder& get() {
+        static TileBuilder builder;
+        return builder;
+    }
+    void submit(const std::shared_ptr<TileJob>& job) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        queue_.push_back(job);
+        if (!thread_.joinable()) {
+            try {
+                thread_ = std::thread([this] { run(); });
+            } catch (const std::system_error&) {   // no thread: finish() builds
+            }
+        }
+        wake_.notify_all();
+    }
+    // The job done: by the thread, or here where it had not begun.
+    void finish(const std::shared_ptr<TileJob>& job) {
+        std::unique_lock<std::mutex> lock(mutex_);
+        if (take(job)) {
+            lock.unlock();
+            build(*job);
+            lock.lock();
+            job->state = TileJob::kDone;
+        }
+        wake_.wait(lock, [&] { return job->state == TileJob::kDone; });
+    }
+    // The job not done, or over.
+    void abandon(const std::shared_ptr<TileJob>& job) {
+        std::unique_lock<std::mutex> lock(mutex_);
+        if (take(job)) return;
+        wake_.wait(lock, [&] { return job->state != TileJob::kRunning; });
+    }
+
+  private:
+    ~TileBuilder() {
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            stop_ = true;
+        }
+        wake_.notify_all();
+        if (thread_.joinable()) thread_.join();
+    }
+    bool take(const std::shared_ptr<TileJob>& job) {
+        const auto at = std::find(queue_.begin(), queue_.end(), job);
+        if (at == queue_.end()) return false;
+        queue_.erase(at);
+        return true;
+    }
+    static void build(TileJob& job) {
+        cudaSetDevice(job.device);
+        try {
+            make_tiles(job.source, job.block);
+        } catch (const std::bad_alloc&) {   // no plan: the cloth stays on its cluster
+        }
+    }
+    void run() {
+        std::unique_lock<std::mutex> lock(mutex_);
+        for (;;) {
+            wake_.wait(lock, [&] { return stop_ || !queue_.empty(); });
+            if (stop_) return;
+            const std::shared_ptr<TileJob> job = queue_.front();
+            queue_.pop_front();
+            job->state = TileJob::kRunning;
+            lock.unlock();
+            build(*job);
+            lock.lock();
+            job->state = TileJob::kDone;
+            wake_.notify_all();
+        }
+    }
+    std::mutex mutex_;
+    std::condition_variable wake_;
+    std::deque<std::shared_ptr<TileJob>> queue_;
+    std::thread thread_;
+    bool stop_ = false;
+};
 
 // A launch runs in tile mode when the cloth has tile plans and the
 // schedule is one the tile substep covers.
@@ -737,8 +940,33 @@ bool tile_covers(const Schedule& s) {
            s.primitive_self == 0u && s.reconcile_passes == 0u && s.final_passes == 0u && s.certificate_passes == 0u;
 }
 bool tile_schedule(const numi_cloth* h, const Schedule& s) { return h->tiles && tile_covers(s); }
-bool configure_tiles(numi_cloth* h, uint32_t grid);
-constexpr uint32_t kTilePlanSubsteps = 128;
+
+// A small cloth's plan is built from its kTileBuildSubsteps'th covered
+// substep on, beside the stepping thread, and taken up at its
+// kTilePlanSubsteps'th: a build takes 0.5 to 2 ms of another core and as
+// many substeps are 5 ms of the GPU's time, so the launch that takes it up
+// finds it done unless launches are issued far ahead of the GPU.  A cloth
+// that only joins batches never needs one.
+constexpr uint32_t kTileBuildSubsteps = 32, kTilePlanSubsteps = 128;
+void prepare_small_tiles(numi_cloth* h, uint32_t substeps) {
+    h->tile_substeps += std::min(substeps, kTilePlanSubsteps - std::min(h->tile_substeps, kTilePlanSubsteps));
+    if (h->tile_source != nullptr) {
+        if (h->tile_substeps < kTileBuildSubsteps) return;
+        h->tile_job = std::make_shared<TileJob>();
+        h->tile_job->source = std::move(*h->tile_source);
+        h->tile_job->device = h->device;
+        h->tile_source.reset();
+        TileBuilder::get().submit(h->tile_job);
+        return;   // for a later launch
+    }
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (h->tile_substeps < kTilePlanSubsteps || cudaStreamIsCapturing(h->stream, &capturing) != cudaSuccess ||
+        capturing != cudaStreamCaptureStatusNone)
+        return;
+    TileBuilder::get().finish(h->tile_job);
+    adopt_tiles(h, std::move(h->tile_job->block));
+    h->tile_job.reset();
+}
 
 // Adjoint tape of a launch: [substep][slots][n] positions, [substep][n]
 // velocities, [substep][grips] grips.
@@ -753,6 +981,7 @@ struct Tape {
 
 cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t cfg_offset = 0,
                    const Tape& tape = {}) {
+    if ((h->tile_source != nullptr || h->tile_job != nullptr) && tile_covers(s)) prepare_small_tiles(h, substeps);
     DeviceCloth d = h->d;
     d.cfg = h->d_cfg + cfg_offset;
     d.epoch_base = h->epoch;
@@ -778,20 +1007,6 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     if (e != cudaSuccess) return e;
     h->last_substeps = substeps;
     size_t smem = h->smem;
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (h->tiles_wanted && tile_covers(sc))
-        h->tile_substeps = std::min(h->tile_substeps + std::min(substeps, kTilePlanSubsteps), kTilePlanSubsteps);
-    if (h->tiles_wanted && tile_covers(sc) && h->tile_substeps == kTilePlanSubsteps &&
-        cudaStreamIsCapturing(h->stream, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone) {
-        h->tiles_wanted = false;
-        configure_tiles(h, h->tile_grid);
-        d.tile_off = h->d.tile_off;
-        d.tile_words = h->d.tile_words;
-        d.tile_owner = h->d.tile_owner;
-        d.tile_stream = h->d.tile_stream;
-        d.x_alt = h->d.x_alt;
-        d.v_alt = h->d.v_alt;
-    }
     const bool tiled = tile_schedule(h, sc);
     if (edge) {
         // the edge/edge phases' box-tree sort keys after the launch's own
@@ -826,12 +1041,6 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     } else if (h->grid == 1 && !tiled) {
         e = cudaLaunchKernel(fn, dim3(1), dim3(h->block), args, smem, h->stream);
     } else if (tiled) {
-        if (h->tiles_dirty) {
-            if (!rebuild_tiles(h)) return cudaErrorUnknown;
-            h->tiles_dirty = false;
-            d.tile_words = h->d.tile_words;
-            d.tile_stream = h->d.tile_stream;
-        }
         sc.tiles = 1u;
         d.resident = 0u;   // a small cloth's other launches keep it in a cluster's shared memory
         if (h->tile_grid > h->grid) d.trace_cta = nullptr;
@@ -1485,9 +1694,8 @@ int numi_cloth_create(const NumiClothScene* scene, numi_cloth_t** out) {
     // tile mode too, on as many CTAs as the cluster has and one for the
     // fruits (the same share of the GPU when several cloths step at once):
     // five grid barriers a substep instead of 26 cluster barriers (a frame of
-    // a 61 x 61 cloth: 3.6 -> 2.1 ms).  Its plan is built once it has stepped
-    // kTilePlanSubsteps: building costs about what as many substeps again
-    // save, and a cloth that only joins batches never needs one.  The
+    // a 61 x 61 cloth: 3.6 -> 2.1 ms), once it has stepped a little
+    // (prepare_small_tiles).  The
     // reference-order kernels stay on the cluster, whose barrier has no bound
     // for the ordered pass's serial fallback to outlast.
     if (want_tiles != 0u && h->cluster > 1u && d.resident != 0u && K == 0u && !h->self_exact && forced == 0u &&
@@ -1495,19 +1703,20 @@ int numi_cloth_create(const NumiClothScene* scene, numi_cloth_t** out) {
         std::getenv("NUMI_CLOTH_RESIDENT_CHUNK") == nullptr) {
         h->tile_grid = std::max(h->cluster + 1u, 3u);
         h->tile_block = NC_BLOCK_MAX;
-        h->tiles_wanted = true;
+        h->tile_source = std::make_unique<TileSource>(tile_source(h));
+        h->tile_source->distances = hij;
+        for (const uint4& q : hbij) h->tile_source->bends.push_back(make_uint2(q.x, q.z));
     }
     if (want_tiles != 0u && h->grid > 1u && h->cluster == 0u && d.resident == 0u && K == 0u) {
-        int max_optin = 0;
-        cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
         uint32_t tgrid = static_cast<uint32_t>(sms);
         env_u32("NUMI_CLOTH_TILE_GRID", tgrid);
         h->tile_grid = std::max(tgrid, 3u);
         h->tile_block = NC_BLOCK_MAX;
-        h->tiles = build_tiles(h, scene->gridWidth, hij, hdm, hbij, hbm,
-                               static_cast<size_t>(max_optin) - tile_static_smem(h)) &&
-                   tiles_fit(h);
-        cudaGetLastError();
+        TileSource src = tile_source(h);
+        src.distances = hij;
+        for (const uint4& q : hbij) src.bends.push_back(make_uint2(q.x, q.z));
+        TileBlock block;
+        if (make_tiles(src, block)) adopt_tiles(h, std::move(block));
     }
     for (uint32_t g = 0; g < G; ++g) h->grip_compliance.push_back(scene->grips[g].targetOffsetAndCompliance.w);
     h->dynamic = {{d.x, n * sizeof(float4)},
@@ -1527,6 +1736,7 @@ int numi_cloth_create(const NumiClothScene* scene, numi_cloth_t** out) {
 void numi_cloth_destroy(numi_cloth_t* h) {
     if (h == nullptr) return;
     cudaSetDevice(h->device);
+    if (h->tile_job) TileBuilder::get().abandon(h->tile_job);
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (auto& s : h->snaps)
         if (s.mem) cudaFree(s.mem);
@@ -1885,13 +2095,23 @@ int numi_cloth_pass_counts(numi_cloth_t* h, uint32_t out[3]) {
 
 namespace {
 
-// Tile plans for a tile launch of `grid` CTAs, and whether the device holds
-// that grid co-resident with their shared memory.
+// Tile plans for a tile launch of `grid` CTAs; false where the device does
+// not hold that grid co-resident with their shared memory.
 bool configure_tiles(numi_cloth* h, uint32_t grid) {
+    const DeviceCloth& d = h->d;
     h->tile_grid = grid;
-    h->tiles = rebuild_tiles(h) && tiles_fit(h);
-    h->tiles_dirty = false;
-    cudaGetLastError();
+    h->tiles = false;
+    TileSource src = tile_source(h);
+    src.distances.resize(d.d_count);
+    std::vector<uint4> bends(d.b_count);
+    if (cudaStreamSynchronize(h->stream) != cudaSuccess ||
+        (d.d_count &&
+         cudaMemcpy(src.distances.data(), d.d_ij, d.d_count * sizeof(uint2), cudaMemcpyDeviceToHost) != cudaSuccess) ||
+        (d.b_count && cudaMemcpy(bends.data(), d.b_ij, d.b_count * sizeof(uint4), cudaMemcpyDeviceToHost) != cudaSuccess))
+        return false;
+    for (const uint4& q : bends) src.bends.push_back(make_uint2(q.x, q.z));
+    TileBlock block;
+    if (make_tiles(src, block)) adopt_tiles(h, std::move(block));
     return h->tiles;
 }
 
@@ -3079,9 +3299,10 @@ extern "C" int numi_cloth_compliance_groups(numi_cloth_t* h, uint32_t family[NUM
 extern "C" int numi_cloth_replace_compliance(numi_cloth_t* h, uint32_t family, float from, float to) {
     if (h == nullptr || family > 3u || !(to >= 0.0f) || !std::isfinite(to)) return NUMI_CLOTH_EINVAL;
     cudaSetDevice(h->device);
-    h->tiles_dirty = h->tiles;   // the tile plan's items carry the materials
     numi_cloth_replace_compliance_kernel<<<64, 256, 0, h->stream>>>(h->d, family, from, to);
     if (cudaGetLastError() != cudaSuccess) return NUMI_CLOTH_ECUDA;
+    // a tile plan's items carry the materials
+    if (h->tiles && (family == 0u || family == 2u) && tile_materials(h) != cudaSuccess) return NUMI_CLOTH_ECUDA;
     replaced_compliance(h, family, from, to);
     return NUMI_CLOTH_OK;
 }
