@@ -478,6 +478,9 @@ int numi_cloth_batch_shape(numi_cloth_batch_t* batch, uint32_t out[3]);
  * family's box tree (80 KB) serves only schedules with
  * primitiveSelf = 0: a step or capture with primitiveSelf on returns EINVAL
  * on it, and the tuner skips it for such schedules. */
+/* resident_chunk: 0, a power of two up to 4096, or the chunk that
+ * numi_cloth_batch_shape or numi_cloth_batch_tune gave for a batch of the
+ * same cloths; threads: 256 or 512. */
 int numi_cloth_batch_set_shape(numi_cloth_batch_t* batch, uint32_t resident_chunk, uint32_t threads);
 
 /* Autotuner: times one step of every candidate shape (the fitted one;

@@ -2467,6 +2467,7 @@ struct numi_cloth_batch {
     // `ranks` CTAs per cloth; its launches with the edge/edge family run one
     // CTA per cloth
     bool fitted = false;
+    uint32_t fit_chunk = 0;            // the chunk that shape reports
     uint32_t ranks = 1;
     uint32_t edge_ctas = 0;
     size_t edge_smem = 0;
@@ -2635,6 +2636,7 @@ int batch_fit(numi_cloth_batch* b) {
     }
     b->ranks = ranks;
     b->fitted = true;
+    b->fit_chunk = b->chunk;
     b->edge_room = true;
     b->layout_valid = false;
     return NUMI_CLOTH_OK;
@@ -2849,12 +2851,14 @@ int numi_cloth_batch_set_stream(numi_cloth_batch_t* b, void* stream) {
 }
 
 int numi_cloth_batch_set_shape(numi_cloth_batch_t* b, uint32_t resident_chunk, uint32_t threads) {
-    if (b == nullptr || (threads != NC_THREADS && threads != NC_BLOCK_MAX) ||
-        (resident_chunk != 0u && (resident_chunk & (resident_chunk - 1u)) != 0u) || resident_chunk > 4096u)
-        return NUMI_CLOTH_EINVAL;
+    if (b == nullptr || (threads != NC_THREADS && threads != NC_BLOCK_MAX)) return NUMI_CLOTH_EINVAL;
+    const bool power = (resident_chunk & (resident_chunk - 1u)) == 0u && resident_chunk <= 4096u;
+    // what batch_shape or the tuner reported of the default shape
+    const bool fit = !power && resident_chunk == b->fit_chunk && threads == NC_BLOCK_MAX;
+    if (!power && !fit) return NUMI_CLOTH_EINVAL;
     cudaSetDevice(b->device);
     batch_drop_graph(b);
-    return batch_shape(b, resident_chunk, threads);
+    return fit ? batch_fit(b) : batch_shape(b, resident_chunk, threads);
 }
 
 int numi_cloth_batch_shape(numi_cloth_batch_t* b, uint32_t out[3]) {

@@ -174,3 +174,29 @@ def test_compliance_groups_follow_replacements_and_restores():
     fresh.replace_compliance("distance", float(stretch), float(shear))
     fresh.replace_compliance("bend", float(bend), 2e-3)
     assert fresh.compliance_groups() == sv.compliance_groups()
+
+
+@pytest.mark.parametrize("sides", [(17,), (40, 64, 9), (64, 65, 96, 110) + (7,) * 72], ids=["one", "clusters", "one-cta"])
+def test_reported_batch_shape_is_accepted(sides):
+    """A program that keeps the shape a batch or its tuner reported can set it
+    again; chunks of no kind stay refused."""
+    scenes = [nc.square_scene(side=s, fruitCount=2, seed=s, **RESTING) for s in sides]
+    cfg = np.stack([nc.substep_configs(s, 4) for s in scenes])
+    sched = nc.Schedule.make(**PLAIN)
+    out = []
+    for again in (False, True):
+        solvers = [nc.ClothSolver(s) for s in scenes]
+        batch = nc.ClothBatch(solvers)
+        if again:
+            for s in (batch.shape(), batch.tune(cfg, sched)):
+                batch.set_shape(4096, 256)
+                batch.set_shape(s["resident_chunk"], s["threads"])
+                assert batch.shape()["threads"] == s["threads"]
+            for bad in (3, 4097, 8192, max(s * s for s in sides) + 1):
+                with pytest.raises(nc.ClothError):
+                    batch.set_shape(bad, 512)
+        batch.step(cfg, sched)
+        out.append([sv.particles() for sv in solvers])
+        batch.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
