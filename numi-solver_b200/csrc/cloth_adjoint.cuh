@@ -53,6 +53,7 @@ struct AdjointArgs {
     uint32_t shift;                  // log2 of the particles each CTA of the cluster owns
     uint32_t substeps;               // substeps of the segment
     uint32_t first_substep;          // rollout index of the segment's first substep
+    uint32_t interval;               // substeps whose gradients are summed before they join the totals
     float damping;                   // the schedule's (or the cloth's) damping
     uint32_t frictions;              // the schedule's frictions switch
     const uint32_t* tracked;         // [n_tracked]
@@ -435,6 +436,44 @@ __device__ __forceinline__ void adjoint_segment(const AdjointArgs& A, uint32_t r
             apply(it);
         }
     };
+    // The sums since the last flush, in a fixed order: lanes, warps, then the
+    // cluster's CTAs.  Called at the same substeps of the rollout however its
+    // segments are taped, so that one call's bits depend on its arguments
+    // alone.  The first CTA adds a flush's parts to the totals at the next
+    // one (a cluster has colour phases between, whose barriers order them), so
+    // a flush costs none of the cluster's barriers.
+    __shared__ double s_red[ADJ_MAX_GROUPS + 2u][ADJ_THREADS / 32u];
+    __shared__ double s_part[2][ADJ_CLUSTER_MAX][ADJ_MAX_GROUPS + 2u];
+    __shared__ double s_total[ADJ_MAX_GROUPS + 2u];
+    if (threadIdx.x <= A.groups + 1u)   // later segments' sums
+        s_total[threadIdx.x] = threadIdx.x <= A.groups ? A.grads[threadIdx.x] : *A.loss;
+    uint32_t flushes = 0u;
+    auto add_parts = [&]() {
+        if (rank != 0u || flushes == 0u || threadIdx.x > A.groups + 1u) return;
+        double sum = 0.0;
+        for (uint32_t r = 0; r < ranks; ++r) sum += s_part[(flushes - 1u) & 1u][r][threadIdx.x];
+        s_total[threadIdx.x] += sum;
+    };
+    auto flush = [&]() {
+        __syncthreads();   // s_red is read (a cloth may have no colour phase)
+        add_parts();
+        for (uint32_t e = 0; e <= A.groups + 1u; ++e) {
+            double v = e <= A.groups ? acc[e] : loss;
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (threadIdx.x % 32u == 0u) s_red[e][threadIdx.x / 32u] = v;
+            if (e <= A.groups) acc[e] = 0.0;
+        }
+        loss = 0.0;
+        __syncthreads();
+        if (threadIdx.x <= A.groups + 1u) {
+            double sum = 0.0;
+            for (uint32_t w = 0; w < blockDim.x / 32u; ++w) sum += s_red[threadIdx.x][w];
+            double* part = &s_part[flushes & 1u][rank][threadIdx.x];
+            if (ranks > 1u) part = static_cast<double*>(__cluster_map_shared_rank(part, 0u));
+            *part = sum;
+        }
+        ++flushes;
+    };
     sync();
     fetch(A.substeps, 0u);
     bool loose = false;   // own-particle phases ran since the last barrier
@@ -726,33 +765,18 @@ __device__ __forceinline__ void adjoint_segment(const AdjointArgs& A, uint32_t r
                 loose = true;
             }
         }
+        if (si == 0u || step % A.interval == 0u) flush();
     }
     if constexpr (kShared)
         for (uint32_t i = own + threadIdx.x; i < own_end; i += blockDim.x) put(A.gx, i, gx.get(i));
-    // fixed-order reductions: each CTA's threads, then the cluster's CTAs
-    __shared__ double s_red[ADJ_THREADS];
-    __shared__ double s_part[ADJ_CLUSTER_MAX][ADJ_MAX_GROUPS + 2u];
-    double* parts = &s_part[rank][0];
-    if (ranks > 1u) parts = static_cast<double*>(__cluster_map_shared_rank(parts, 0u));
-    for (uint32_t e = 0; e <= A.groups + 1u; ++e) {
-        __syncthreads();
-        s_red[threadIdx.x] = e <= A.groups ? acc[e] : loss;
-        __syncthreads();
-        for (uint32_t st = blockDim.x / 2u; st > 0u; st >>= 1u) {
-            if (threadIdx.x < st) s_red[threadIdx.x] += s_red[threadIdx.x + st];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) parts[e] = s_red[0];
-    }
     if (rough) atomicAdd(A.nonsmooth, rough);
     sync();
+    add_parts();
     if (rank == 0u && threadIdx.x <= A.groups + 1u) {
-        double sum = 0.0;
-        for (uint32_t r = 0; r < ranks; ++r) sum += s_part[r][threadIdx.x];
         if (threadIdx.x <= A.groups)
-            A.grads[threadIdx.x] += sum;
+            A.grads[threadIdx.x] = s_total[threadIdx.x];
         else
-            *A.loss += sum;
+            *A.loss = s_total[threadIdx.x];
     }
 }
 

@@ -3053,9 +3053,16 @@ namespace {
 // runs.  So a cloth with fruits is taped and checkpointed, and the tape is
 // used where nothing was recorded; a rollout after one that did record does
 // not tape.
+//
+// However it is taped, a rollout's gradients are summed checkpoint interval
+// by interval (AdjointArgs::interval): equal calls give equal bits.
+// NUMI_CLOTH_TAPE_BYTES is a test hook: a smaller limit gives small rollouts
+// several segments.
 constexpr size_t kTapeBytes = size_t(8) << 30;
 uint32_t taped_substeps(uint32_t substeps, uint32_t checkpoint_every, size_t bytes_per_substep) {
-    const size_t fit = kTapeBytes / std::max<size_t>(bytes_per_substep, 1u);
+    uint32_t limit = 0;
+    const size_t bytes = env_u32("NUMI_CLOTH_TAPE_BYTES", limit) ? limit : kTapeBytes;
+    const size_t fit = bytes / std::max<size_t>(bytes_per_substep, 1u);
     if (substeps <= fit) return substeps;
     const size_t whole = std::max<size_t>(fit / checkpoint_every, 1u) * checkpoint_every;
     return static_cast<uint32_t>(std::min<size_t>(whole, substeps));
@@ -3501,6 +3508,7 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
         A.shift = adjoint_shift(n, shape.ranks);
         A.substeps = count;
         A.first_substep = first;
+        A.interval = checkpoint_every;
         A.damping = damping;
         A.frictions = s.frictions;
         A.tracked = d_tracked;
@@ -3712,6 +3720,7 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
         A.phases = ph;
         A.slots = slots;
         A.shift = adjoint_shift(n, shape.ranks);
+        A.interval = checkpoint_every;
         A.damping = h->d.damping >= 0.0f ? h->d.damping : s.damping;
         A.frictions = s.frictions;
         A.tracked = d_tracked;

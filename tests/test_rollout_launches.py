@@ -135,3 +135,68 @@ def test_gradients_before_a_regrab(side, every):
         assert np.allclose(a["damping"], b["damping"], rtol=1e-10)
     for a, b in zip(batched[1], (half["loss"], half["grads"], half["damping"])):
         assert np.allclose(a, b, rtol=1e-10, atol=1e-10 * np.abs(b).max())
+
+
+def _tape_limit(monkeypatch, scene, substeps):
+    """Limits the tape to about `substeps` substeps (at least one interval is
+    always taped)."""
+    phases = 2 * len(np.unique(scene.distances["particlesAndColor"][:, 2])) + 12
+    monkeypatch.setenv("NUMI_CLOTH_TAPE_BYTES", str(int(substeps * phases * scene.n * 16)))
+
+
+@pytest.mark.parametrize("side, spheres", [(9, 0), (40, 0), (40, 2), (72, 0)])
+@pytest.mark.parametrize("every", [1, 5, 8, 24])
+def test_equal_bits_however_the_rollout_is_taped(monkeypatch, side, spheres, every):
+    """The whole rollout on one tape, in segments of several intervals or of
+    one: the same bits (spheres far above, which never touch)."""
+    scene = small_square(side=side, fruits=spheres, gripCorners=1, stretchCompliance=1e-4, shearCompliance=2e-4,
+                         bendCompliance=1e-3, fruitHeightMin=2.0, fruitHeightMax=3.0)
+    sched = nc.Schedule.make(**dict(PLAIN, damping=0.5))
+    whole = _run(scene, sched, every=every)
+    for substeps in (1, 13):
+        _tape_limit(monkeypatch, scene, substeps)
+        _same_gradients(_run(scene, sched, every=every), whole)
+    monkeypatch.delenv("NUMI_CLOTH_TAPE_BYTES")
+    _same_gradients(_run(scene, sched, every=every, repeats=3), whole)
+
+
+@pytest.mark.parametrize("every", [5, 24])
+def test_equal_bits_however_a_batch_is_taped(monkeypatch, every):
+    scenes = [_scene(side, False) for side in (12, 33, 40)]
+    sched = nc.Schedule.make(**dict(PLAIN, damping=0.5))
+    cfg, tracked, targets = _rollout(scenes[0])
+    out = []
+    for limit in (None, 1, 13):
+        if limit is not None:
+            _tape_limit(monkeypatch, scenes[2], 1.7 * limit)
+        solvers = [nc.ClothSolver(s) for s in scenes]
+        batch = nc.ClothBatch(solvers)
+        cfgs = np.stack([_rollout(s)[0] for s in scenes])
+        r = batch.rollout_grad(cfgs, sched, tracked, np.stack([targets] * 3), 12, checkpoint_every=every)
+        out.append((r["loss"], np.concatenate(r["grads"]), r["damping"], r["nonsmooth"],
+                    *[sv.particles() for sv in solvers]))
+        batch.close()
+    for other in out[1:]:
+        for a, b in zip(out[0], other):
+            assert np.array_equal(a, b)
+
+
+def test_equal_bits_after_a_rollout_with_contact():
+    """What a handle's earlier rollout met changes no bit of the next."""
+    scene = _scene(24, True)
+    free = scene.fruits.copy()
+    free["positionAndInverseMass"][:, 2] += 5.0
+    free["previousAndRadius"][:, 2] += 5.0
+    sched = nc.Schedule.make(**dict(PLAIN, damping=0.5))
+    cfg, tracked, targets = _rollout(scene)
+    sv = nc.ClothSolver(scene)
+    sv.snapshot(0)
+    runs = []
+    for fruits in (scene.fruits, free, free, scene.fruits, free):
+        sv.restore(0)
+        sv.write_fruits(fruits)
+        runs.append(sv.rollout_grad(cfg, sched, tracked, targets, 12, checkpoint_every=8))
+    assert [r["nonsmooth"] > 0 for r in runs] == [True, False, False, True, False]
+    for a, b in ((0, 3), (1, 2), (1, 4)):
+        for name in ("loss", "grads", "damping", "grip"):
+            assert np.array_equal(runs[a][name], runs[b][name]), (a, b, name)
