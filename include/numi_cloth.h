@@ -423,8 +423,12 @@ int numi_cloth_step_noalloc(const NumiClothConfig* base, const NumiClothDeviceSt
  * The forward is taped as it runs where the tape of the whole rollout fits
  * 8 GB and a quarter of the free device memory; else, and where a fruit
  * touches the cloth, segments of checkpoint_every substeps are replayed from
- * checkpoints with a tape.  The call's device memory stays with the handle
- * (up to 1 GB) or the batch (up to 9 GB) for the next call.
+ * checkpoints with a tape.  However it is taped, the gradients are summed
+ * checkpoint interval by interval, so equal calls give equal bits.  The call's
+ * device memory stays with the handle or batch for the next call as long as
+ * all that the process keeps so takes at most a sixteenth of the device's
+ * memory; it is given back with its owner, and when another allocation of the
+ * library finds no room.
  *
  * Supported schedules: iterations = 1, no reconciliation, final or
  * certificate passes, aerodynamics = 0, selfCollision = 0.  Fruit contacts,

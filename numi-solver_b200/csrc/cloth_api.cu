@@ -68,22 +68,6 @@ struct Snapshot {
     std::vector<float> grip_compliance;   // the grips' at the snapshot
 };
 
-struct DeviceBuffers {
-    std::vector<void*> owned;
-    template <class T>
-    T* alloc(size_t count) {
-        if (count == 0) count = 1;
-        void* p = nullptr;
-        if (cudaMalloc(&p, count * sizeof(T)) != cudaSuccess) return nullptr;
-        cudaMemset(p, 0, count * sizeof(T));
-        owned.push_back(p);
-        return static_cast<T*>(p);
-    }
-    ~DeviceBuffers() {
-        for (void* p : owned) cudaFree(p);
-    }
-};
-
 bool env_u32(const char* name, uint32_t& out) {
     const char* v = std::getenv(name);
     if (v == nullptr || *v == 0) return false;
@@ -106,32 +90,82 @@ struct Carver {
     }
 };
 
+cudaError_t device_malloc(void** p, size_t bytes);
+
 // Device memory of the rollout gradients of one handle or batch: kept from
-// call to call up to `keep` bytes (an allocation and its release cost more
-// than a small rollout), and freed with its owner; a call that needs more
-// gives it back at its end.
+// call to call (an allocation and its release cost more than a small
+// rollout) as long as all that the process keeps so takes no more than a
+// sixteenth of the device's memory, else given back at the call's end.  It is
+// freed with its owner, and when another allocation of the library finds no
+// room.
 struct Workspace {
-    size_t keep = size_t(1) << 30;
     void* mem = nullptr;
-    size_t bytes = 0;
-    Workspace() = default;
+    size_t bytes = 0, most = 0;   // most: what may be kept on its device
+    int device = -1;
+    bool busy = false;   // a call uses it
+    Workspace() {
+        std::lock_guard<std::mutex> lock(mutex());
+        all().push_back(this);
+    }
     Workspace(const Workspace&) = delete;
     Workspace& operator=(const Workspace&) = delete;
-    ~Workspace() { release(); }
+    ~Workspace() {
+        std::lock_guard<std::mutex> lock(mutex());
+        all().erase(std::find(all().begin(), all().end(), this));
+        release();
+    }
     void release() {
         if (mem != nullptr) cudaFree(mem);
         mem = nullptr;
         bytes = 0;
     }
-    // One call's use of it.
+    static std::mutex& mutex() {
+        static std::mutex m;
+        return m;
+    }
+    static std::vector<Workspace*>& all() {
+        static std::vector<Workspace*> list;
+        return list;
+    }
+    // Gives back what no call uses on the device; false where that is nothing.
+    static bool reclaim(int device) {
+        std::lock_guard<std::mutex> lock(mutex());
+        bool any = false;
+        for (Workspace* w : all())
+            if (!w->busy && w->mem != nullptr && w->device == device) {
+                w->release();
+                any = true;
+            }
+        return any;
+    }
+    // One call's use of it, on the current device.
     struct Lease {
         Workspace& w;
         cudaStream_t stream;
-        Lease(Workspace& space, cudaStream_t s) : w(space), stream(s) {}
+        Lease(Workspace& space, cudaStream_t s) : w(space), stream(s) {
+            std::lock_guard<std::mutex> lock(mutex());
+            w.busy = true;
+            cudaGetDevice(&w.device);
+        }
         ~Lease() {
-            if (w.bytes <= w.keep) return;
-            cudaStreamSynchronize(stream);
+            std::unique_lock<std::mutex> lock(mutex());
+            size_t kept = 0;
+            for (const Workspace* o : all())
+                if (o->device == w.device) kept += o->bytes;
+            if (kept > w.most) {
+                lock.unlock();
+                cudaStreamSynchronize(stream);
+                lock.lock();
+                w.release();
+            }
+            w.busy = false;
+        }
+        void hold(void* p, size_t bytes, size_t most) {
+            std::lock_guard<std::mutex> lock(mutex());
             w.release();
+            w.mem = p;
+            w.bytes = bytes;
+            w.most = most;
         }
         // False where the device has no room for the pieces; with `quarter`
         // also where they would take more than a quarter of what is free.
@@ -141,23 +175,50 @@ struct Workspace {
             pieces(measure);
             if (measure.used > w.bytes) {
                 size_t room = 0, total = 0;
-                if (quarter && cudaMemGetInfo(&room, &total) == cudaSuccess && measure.used > (room + w.bytes) / 4u)
-                    return false;
+                if (cudaMemGetInfo(&room, &total) != cudaSuccess) return false;
+                if (quarter && measure.used > (room + w.bytes) / 4u) return false;
                 // whatever ran on the old memory has ended
                 if (w.mem != nullptr && cudaStreamSynchronize(stream) != cudaSuccess) return false;
-                w.release();
-                if (cudaMalloc(&w.mem, measure.used) != cudaSuccess) {
-                    cudaGetLastError();
-                    w.mem = nullptr;
-                    return false;
-                }
-                w.bytes = measure.used;
+                hold(nullptr, 0, 0);
+                void* p = nullptr;
+                if (device_malloc(&p, measure.used) != cudaSuccess) return false;
+                hold(p, measure.used, total / 16u);
             }
             Carver c{static_cast<char*>(w.mem)};
             pieces(c);
             return true;
         }
     };
+};
+
+// cudaMalloc on the current device, which takes back idle workspaces where
+// there is no room.
+cudaError_t device_malloc(void** p, size_t bytes) {
+    int device = 0;
+    cudaGetDevice(&device);
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && Workspace::reclaim(device)) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
+struct DeviceBuffers {
+    std::vector<void*> owned;
+    template <class T>
+    T* alloc(size_t count) {
+        if (count == 0) count = 1;
+        void* p = nullptr;
+        if (device_malloc(&p, count * sizeof(T)) != cudaSuccess) return nullptr;
+        cudaMemset(p, 0, count * sizeof(T));
+        owned.push_back(p);
+        return static_cast<T*>(p);
+    }
+    ~DeviceBuffers() {
+        for (void* p : owned) cudaFree(p);
+    }
 };
 
 // What the tile plans of a cloth are made from: its colours, grid width and
@@ -770,7 +831,7 @@ bool make_tiles(const TileSource& src, TileBlock& out) {
     Carver measure{nullptr};
     pieces(measure);
     cudaStream_t stream = nullptr;
-    cudaError_t e = cudaMalloc(&block.mem, measure.used);
+    cudaError_t e = device_malloc(&block.mem, measure.used);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
     Carver carver{static_cast<char*>(block.mem)};
     pieces(carver);
@@ -1771,7 +1832,7 @@ int numi_cloth_step(numi_cloth_t* h, const NumiClothConfig* configs, uint32_t co
     if (count > h->cfg_capacity) {
         cudaFree(h->d_cfg);
         h->d_cfg = nullptr;
-        if (cudaMalloc(&h->d_cfg, count * sizeof(NumiClothConfig)) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+        if (device_malloc(reinterpret_cast<void**>(&h->d_cfg), count * sizeof(NumiClothConfig)) != cudaSuccess) return NUMI_CLOTH_ECUDA;
         h->cfg_capacity = count;
     }
     if (cudaMemcpyAsync(h->d_cfg, configs, count * sizeof(NumiClothConfig), cudaMemcpyHostToDevice, h->stream) !=
@@ -2033,7 +2094,7 @@ int snapshot_slot(numi_cloth_t* h, uint32_t slot) {
     for (const auto& r : h->dynamic) total += (r.bytes + 255u) & ~size_t(255u);
     Snapshot& s = h->snaps[slot];
     if (s.mem == nullptr) {
-        if (cudaMalloc(&s.mem, total) != cudaSuccess) return NUMI_CLOTH_ENOMEM;
+        if (device_malloc(&s.mem, total) != cudaSuccess) return NUMI_CLOTH_ENOMEM;
         s.bytes = total;
     }
     if (copy_state(h, static_cast<char*>(s.mem), true) != cudaSuccess) return NUMI_CLOTH_ECUDA;
@@ -2969,8 +3030,7 @@ int numi_cloth_batch_capture(numi_cloth_batch_t* b, const NumiClothConfig* confi
     };
     Carver measure{nullptr};
     pieces(measure);
-    if (cudaMalloc(&b->graph_mem, measure.used) != cudaSuccess) {
-        cudaGetLastError();
+    if (device_malloc(&b->graph_mem, measure.used) != cudaSuccess) {
         b->graph_mem = nullptr;
         return NUMI_CLOTH_ENOMEM;
     }
@@ -3345,7 +3405,7 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
     if (substeps > h->cfg_capacity) {
         cudaFree(h->d_cfg);
         h->d_cfg = nullptr;
-        if (cudaMalloc(&h->d_cfg, substeps * sizeof(NumiClothConfig)) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+        if (device_malloc(reinterpret_cast<void**>(&h->d_cfg), substeps * sizeof(NumiClothConfig)) != cudaSuccess) return NUMI_CLOTH_ECUDA;
         h->cfg_capacity = substeps;
     }
     if (cudaMemcpyAsync(h->d_cfg, configs, substeps * sizeof(NumiClothConfig), cudaMemcpyHostToDevice, h->stream) !=
@@ -3674,7 +3734,6 @@ extern "C" int numi_cloth_batch_rollout_grad(numi_cloth_batch_t* b, const NumiCl
             ckpt = c.get<char>((segs + 1u) * state_total);
         }
     };
-    b->grad.keep = kTapeBytes + (kTapeBytes >> 3);
     Workspace::Lease mem(b->grad, b->stream);
     if (!mem.layout(layout, every > checkpoint_every)) {
         every = interval;
