@@ -434,7 +434,12 @@ int numi_cloth_step_noalloc(const NumiClothConfig* base, const NumiClothDeviceSt
  * certificate passes, aerodynamics = 0, selfCollision = 0.  Fruit contacts,
  * cloth/ground friction, the swept ground and bend ground active sets are
  * not differentiated: the number of such events met is returned in
- * *nonsmooth (0 = the gradient is exact for the discrete forward).  Returns
+ * *nonsmooth (0 = the gradient is exact for the discrete forward).  Where a
+ * fruit touches the cloth, the replayed segments meet the forward's contact
+ * records of the same substeps and resolve the fruits' friction by them, so
+ * the trajectory that loss and gradients are taken on is not quite the
+ * forward's that the handle's state follows (1 % of the loss on the produce
+ * bag's first frame).  Returns
  * NUMI_CLOTH_EINVAL for unsupported schedules. */
 #define NUMI_CLOTH_MAX_GROUPS 16u
 int numi_cloth_compliance_groups(numi_cloth_t* handle, uint32_t family[NUMI_CLOTH_MAX_GROUPS],
