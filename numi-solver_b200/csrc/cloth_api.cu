@@ -207,12 +207,14 @@ cudaError_t device_malloc(void** p, size_t bytes) {
 
 struct DeviceBuffers {
     std::vector<void*> owned;
+    // Zeroed on the stream that uses it first (the default stream does not
+    // order a non-blocking one's work).
     template <class T>
-    T* alloc(size_t count) {
+    T* alloc(size_t count, cudaStream_t stream = nullptr) {
         if (count == 0) count = 1;
         void* p = nullptr;
         if (device_malloc(&p, count * sizeof(T)) != cudaSuccess) return nullptr;
-        cudaMemset(p, 0, count * sizeof(T));
+        cudaMemsetAsync(p, 0, count * sizeof(T), stream);
         owned.push_back(p);
         return static_cast<T*>(p);
     }
@@ -1152,16 +1154,16 @@ Schedule device_schedule(const NumiClothSchedule& schedule) {
 // Point self-contact grid of a cloth, allocated on first use (about four
 // buckets per particle, of which a cloth in an axis plane uses half); the bucket heads are cleared when the 26-bit
 // substep part of their tags wraps within the next `substeps`.
-int prepare_self_grid(numi_cloth* h, bool self_collision, uint32_t substeps) {
+int prepare_self_grid(numi_cloth* h, bool self_collision, uint32_t substeps, cudaStream_t stream) {
     if (self_collision && h->d.hash_head == nullptr) {
         uint32_t buckets = 1024u;
         while (buckets < 4u * h->d.n) buckets <<= 1;
         DeviceCloth& d = h->d;
-        d.hash_head = h->buf.alloc<unsigned long long>(buckets);
-        d.hash_over_head = h->buf.alloc<unsigned long long>(1);
-        d.hash_over = h->buf.alloc<HashSlot>(h->d.n);
-        d.hash = h->buf.alloc<HashSlot>(static_cast<size_t>(buckets) * NC_HASH_CAP);
-        d.self_stats = h->buf.alloc<unsigned long long>(8);
+        d.hash_head = h->buf.alloc<unsigned long long>(buckets, stream);
+        d.hash_over_head = h->buf.alloc<unsigned long long>(1, stream);
+        d.hash_over = h->buf.alloc<HashSlot>(h->d.n, stream);
+        d.hash = h->buf.alloc<HashSlot>(static_cast<size_t>(buckets) * NC_HASH_CAP, stream);
+        d.self_stats = h->buf.alloc<unsigned long long>(8, stream);
         // the ordered pass's list: room for three pairs per particle (a
         // power of two, at least 4,096); scratch of three words per listed
         // pair (sort keys, or the wavefront form's keys, predecessors and
@@ -1170,13 +1172,13 @@ int prepare_self_grid(numi_cloth* h, bool self_collision, uint32_t substeps) {
         while (list_cap < 3u * h->d.n) list_cap <<= 1;
         bool order_ok = true;
         if (h->self_exact) {
-            d.self_list = h->buf.alloc<float4>(2u * static_cast<size_t>(list_cap));
-            d.self_list_head = h->buf.alloc<unsigned long long>(1);
-            d.self_pass_stats = h->buf.alloc<unsigned long long>(2);
-            d.self_keys = h->buf.alloc<unsigned long long>(3u * static_cast<size_t>(list_cap) + NC_SELF_GROUP);
-            d.self_mark = h->buf.alloc<unsigned long long>(h->d.n);
-            d.self_x0 = h->buf.alloc<float4>(h->d.n);
-            d.self_disp = h->buf.alloc<float>(h->d.n);
+            d.self_list = h->buf.alloc<float4>(2u * static_cast<size_t>(list_cap), stream);
+            d.self_list_head = h->buf.alloc<unsigned long long>(1, stream);
+            d.self_pass_stats = h->buf.alloc<unsigned long long>(2, stream);
+            d.self_keys = h->buf.alloc<unsigned long long>(3u * static_cast<size_t>(list_cap) + NC_SELF_GROUP, stream);
+            d.self_mark = h->buf.alloc<unsigned long long>(h->d.n, stream);
+            d.self_x0 = h->buf.alloc<float4>(h->d.n, stream);
+            d.self_disp = h->buf.alloc<float>(h->d.n, stream);
             order_ok = d.self_list != nullptr && d.self_list_head != nullptr && d.self_pass_stats != nullptr &&
                        d.self_keys != nullptr && d.self_mark != nullptr && d.self_x0 != nullptr &&
                        d.self_disp != nullptr;
@@ -1192,12 +1194,12 @@ int prepare_self_grid(numi_cloth* h, bool self_collision, uint32_t substeps) {
     }
     if (h->d.hash_head != nullptr && ((h->epoch + substeps) >> 26) != (h->epoch >> 26)) {
         if (cudaMemsetAsync(h->d.hash_head, 0, (static_cast<size_t>(h->d.hash_mask) + 1u) * sizeof(unsigned long long),
-                            h->stream) != cudaSuccess ||
-            cudaMemsetAsync(h->d.hash_over_head, 0, sizeof(unsigned long long), h->stream) != cudaSuccess ||
+                            stream) != cudaSuccess ||
+            cudaMemsetAsync(h->d.hash_over_head, 0, sizeof(unsigned long long), stream) != cudaSuccess ||
             (h->self_exact &&
-             (cudaMemsetAsync(h->d.self_list_head, 0, sizeof(unsigned long long), h->stream) != cudaSuccess ||
+             (cudaMemsetAsync(h->d.self_list_head, 0, sizeof(unsigned long long), stream) != cudaSuccess ||
               cudaMemsetAsync(h->d.self_mark, 0, static_cast<size_t>(h->d.n) * sizeof(unsigned long long),
-                              h->stream) != cudaSuccess)))
+                              stream) != cudaSuccess)))
             return NUMI_CLOTH_ECUDA;
     }
     return NUMI_CLOTH_OK;
@@ -1277,7 +1279,7 @@ bool build_local_lists(const numi_cloth* h, std::vector<uint32_t>& off, std::vec
     return true;
 }
 
-int prepare_edge_grid(numi_cloth* h, bool primitive, uint32_t substeps, float radius) {
+int prepare_edge_grid(numi_cloth* h, bool primitive, uint32_t substeps, float radius, cudaStream_t stream) {
     (void)substeps;
     DeviceCloth& d = h->d;
     if (primitive && d.edge_count == nullptr && d.y_count > 0u) {
@@ -1287,12 +1289,12 @@ int prepare_edge_grid(numi_cloth* h, bool primitive, uint32_t substeps, float ra
         const uint32_t list_cap = std::max(2048u, 32u * d.y_count);
         const uint32_t ctas = std::max<uint32_t>(h->grid, 1u);
         DeviceCloth e = d;
-        e.edge_count = h->buf.alloc<uint32_t>(buckets);
-        e.edge_offs = h->buf.alloc<uint32_t>(buckets);
-        e.edge_chunk_total = h->buf.alloc<uint32_t>(ctas);
-        e.edge_entries = h->buf.alloc<float4>(static_cast<size_t>(54u) * d.y_count);
-        e.edge_giant = h->buf.alloc<uint32_t>(d.y_count);
-        e.edge_bbox = h->buf.alloc<float4>(2u * d.y_count);
+        e.edge_count = h->buf.alloc<uint32_t>(buckets, stream);
+        e.edge_offs = h->buf.alloc<uint32_t>(buckets, stream);
+        e.edge_chunk_total = h->buf.alloc<uint32_t>(ctas, stream);
+        e.edge_entries = h->buf.alloc<float4>(static_cast<size_t>(54u) * d.y_count, stream);
+        e.edge_giant = h->buf.alloc<uint32_t>(d.y_count, stream);
+        e.edge_bbox = h->buf.alloc<float4>(2u * d.y_count, stream);
         std::vector<uint32_t> loc_off, loc_idx;
         build_local_lists(h, loc_off, loc_idx);
         uint32_t* d_loc_off = h->buf.alloc<uint32_t>(loc_off.size());
@@ -1305,27 +1307,27 @@ int prepare_edge_grid(numi_cloth* h, bool primitive, uint32_t substeps, float ra
             d_loc_off = nullptr;
         e.edge_loc_off = d_loc_off;
         e.edge_loc_idx = d_loc_idx;
-        e.edge_pairs = h->buf.alloc<uint2>(list_cap);
-        e.edge_xb = h->buf.alloc<float4>(d.n);
-        e.edge_pb = h->buf.alloc<float4>(d.n);
-        e.edge_built_radius = h->buf.alloc<float>(1);
-        e.edge_sph = h->buf.alloc<float4>(d.y_count);
-        e.edge_x0 = h->buf.alloc<float4>(d.n);
-        e.edge_path = h->buf.alloc<float>(d.n);
-        e.edge_cand = h->buf.alloc<uint4>(cap);
-        e.edge_order = h->buf.alloc<unsigned long long>(cap);
-        e.edge_sorted = h->buf.alloc<unsigned long long>(cap);
-        e.edge_new = h->buf.alloc<EdgeRecord>(cap);
-        e.edge_done = h->buf.alloc<uint32_t>(cap);
-        e.edge_lv = h->buf.alloc<uint32_t>(cap);
-        e.edge_level = h->buf.alloc<uint32_t>(d.n);
-        e.edge_qbox_raw = h->buf.alloc<float>(6u * d.y_count);
-        e.edge_tree = h->buf.alloc<uint32_t>(static_cast<size_t>(NC_EDGE_TREE_WORDS) * d.y_count);
-        e.edge_centre = h->buf.alloc<float4>(2u * static_cast<size_t>(d.y_count));   // centres, last build's
-        e.edge_rec = h->buf.alloc<EdgeRecord>(cap);
-        e.edge_ctl = h->buf.alloc<uint32_t>(8);
-        e.edge_stats = h->buf.alloc<unsigned long long>(2);
-        e.edge_red = h->buf.alloc<double>(3u * ctas);
+        e.edge_pairs = h->buf.alloc<uint2>(list_cap, stream);
+        e.edge_xb = h->buf.alloc<float4>(d.n, stream);
+        e.edge_pb = h->buf.alloc<float4>(d.n, stream);
+        e.edge_built_radius = h->buf.alloc<float>(1, stream);
+        e.edge_sph = h->buf.alloc<float4>(d.y_count, stream);
+        e.edge_x0 = h->buf.alloc<float4>(d.n, stream);
+        e.edge_path = h->buf.alloc<float>(d.n, stream);
+        e.edge_cand = h->buf.alloc<uint4>(cap, stream);
+        e.edge_order = h->buf.alloc<unsigned long long>(cap, stream);
+        e.edge_sorted = h->buf.alloc<unsigned long long>(cap, stream);
+        e.edge_new = h->buf.alloc<EdgeRecord>(cap, stream);
+        e.edge_done = h->buf.alloc<uint32_t>(cap, stream);
+        e.edge_lv = h->buf.alloc<uint32_t>(cap, stream);
+        e.edge_level = h->buf.alloc<uint32_t>(d.n, stream);
+        e.edge_qbox_raw = h->buf.alloc<float>(6u * d.y_count, stream);
+        e.edge_tree = h->buf.alloc<uint32_t>(static_cast<size_t>(NC_EDGE_TREE_WORDS) * d.y_count, stream);
+        e.edge_centre = h->buf.alloc<float4>(2u * static_cast<size_t>(d.y_count), stream);   // centres, last build's
+        e.edge_rec = h->buf.alloc<EdgeRecord>(cap, stream);
+        e.edge_ctl = h->buf.alloc<uint32_t>(8, stream);
+        e.edge_stats = h->buf.alloc<unsigned long long>(2, stream);
+        e.edge_red = h->buf.alloc<double>(3u * ctas, stream);
         if (!e.edge_count || !e.edge_offs || !e.edge_chunk_total || !e.edge_entries || !e.edge_giant ||
             !e.edge_pairs || !e.edge_xb || !e.edge_pb || !e.edge_built_radius || !e.edge_sph || !e.edge_x0 ||
             !e.edge_path || !e.edge_cand || !e.edge_order || !e.edge_sorted || !e.edge_new || !e.edge_done || !e.edge_rec ||
@@ -1839,8 +1841,8 @@ int numi_cloth_step(numi_cloth_t* h, const NumiClothConfig* configs, uint32_t co
         cudaSuccess)
         return NUMI_CLOTH_ECUDA;
     const Schedule s = device_schedule(*schedule);
-    int rc = prepare_self_grid(h, s.self_collision != 0u, count);
-    if (rc == NUMI_CLOTH_OK) rc = prepare_edge_grid(h, s.primitive_self != 0u, count, configs[0].clothMaterial.x);
+    int rc = prepare_self_grid(h, s.self_collision != 0u, count, h->stream);
+    if (rc == NUMI_CLOTH_OK) rc = prepare_edge_grid(h, s.primitive_self != 0u, count, configs[0].clothMaterial.x, h->stream);
     if (rc != NUMI_CLOTH_OK) return rc;
     const cudaError_t e = launch(h, count, s);
     h->epoch += count;
@@ -1889,7 +1891,7 @@ static_assert(sizeof(NumiClothParticle) == 3u * sizeof(float4), "particle record
 
 // The handle's staging buffer for particle records, allocated on first use.
 static NumiClothParticle* particle_io(numi_cloth_t* h) {
-    if (h->io == nullptr) h->io = h->buf.alloc<NumiClothParticle>(h->d.n);
+    if (h->io == nullptr) h->io = h->buf.alloc<NumiClothParticle>(h->d.n, h->stream);
     return h->io;
 }
 
@@ -2801,10 +2803,10 @@ int batch_prepare(numi_cloth_batch* b, const NumiClothConfig* configs, uint32_t 
         void* edge_before = h->d.edge_count;
         const float cell_before = h->d.edge_cell;
         h->epoch = b->epoch_host;
-        int rc = prepare_self_grid(h, sched.selfCollision != 0u, substeps);
+        int rc = prepare_self_grid(h, sched.selfCollision != 0u, substeps, b->stream);
         if (rc == NUMI_CLOTH_OK)
             rc = prepare_edge_grid(h, sched.primitiveSelf != 0u, substeps,
-                                   configs[k * substeps].clothMaterial.x);
+                                   configs[k * substeps].clothMaterial.x, b->stream);
         if (rc != NUMI_CLOTH_OK) return rc;
         if (h->d.hash_head != before || h->d.edge_count != edge_before || h->d.edge_cell != cell_before)
             b->layout_valid = false;
