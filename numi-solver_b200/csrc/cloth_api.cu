@@ -287,6 +287,7 @@ struct numi_cloth {
     size_t smem = nc_resident_offset();   // dynamic shared memory of a frame launch
     uint32_t launches = 0;
     uint32_t trace_capacity = 0;   // substeps the trace buffer holds
+    uint32_t trace_ctas = 0;       // CTAs its per-CTA part holds
     uint32_t last_substeps = 0;
     float yarn_rest_median = 0.0f;   // median yarn segment rest length
     bool neighbours = false;         // neighbour-sync tables built for the cooperative grid
@@ -1106,7 +1107,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     } else if (tiled) {
         sc.tiles = 1u;
         d.resident = 0u;   // a small cloth's other launches keep it in a cluster's shared memory
-        if (h->tile_grid > h->grid) d.trace_cta = nullptr;
+        if (h->tile_grid > h->trace_ctas) d.trace_cta = nullptr;
         e = raise_frame_smem(h->tile_smem);
         if (e == cudaSuccess)
             e = cudaLaunchCooperativeKernel(fn, dim3(h->tile_grid), dim3(h->tile_block), args, h->tile_smem, h->stream);
@@ -1628,9 +1629,11 @@ int numi_cloth_create(const NumiClothScene* scene, numi_cloth_t** out) {
         d.trace = h->buf.alloc<unsigned long long>(static_cast<size_t>(trace_substeps) * NC_TRACE_SLOTS);
         h->trace_capacity = d.trace ? trace_substeps : 0u;
         uint32_t per_cta = 0;
-        if (env_u32("NUMI_CLOTH_TRACE_CTA", per_cta) && per_cta > 0)
+        if (env_u32("NUMI_CLOTH_TRACE_CTA", per_cta) && per_cta > 0) {
+            h->trace_ctas = h->grid + 1u;   // a small cloth's tile launch has one more than its cluster
             d.trace_cta = h->buf.alloc<unsigned long long>(static_cast<size_t>(trace_substeps) * NC_TRACE_SLOTS *
-                                                           std::max<uint32_t>(h->grid, 1u));
+                                                           h->trace_ctas);
+        }
     }
     const uint32_t chunks = (n + NC_THREADS - 1u) / NC_THREADS;
     d.red = h->buf.alloc<double>(std::max<size_t>(3u * 4096u, 2u * chunks + 8u));
@@ -2132,7 +2135,7 @@ int numi_cloth_trace_cta(numi_cloth_t* h, unsigned long long* out, uint32_t subs
     cudaSetDevice(h->device);
     // the last launch's CTAs (a tile launch may use fewer than the grid)
     const uint32_t grid = h->last_grid != 0u ? h->last_grid : h->grid;
-    if (grid > h->grid) return NUMI_CLOTH_ESTATE;   // not traced per CTA
+    if (grid > h->trace_ctas) return NUMI_CLOTH_ESTATE;   // not traced per CTA
     if (cudaStreamSynchronize(h->stream) != cudaSuccess ||
         cudaMemcpy(out, h->d.trace_cta,
                    static_cast<size_t>(substeps) * NC_TRACE_SLOTS * grid * sizeof(unsigned long long),

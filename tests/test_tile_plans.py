@@ -135,3 +135,18 @@ def test_handles_closed_while_their_plans_are_built():
         assert all(np.array_equal(sv.particles(), first) for sv in solvers[3::2])
         for sv in solvers[1::2]:
             sv.close()
+
+
+def test_per_cta_trace_of_a_small_cloth():
+    """The per-CTA stamps stay available once a small cloth takes tile mode,
+    one CTA more than its cluster."""
+    scene = _scene()
+    sv = make_solver(scene, env={"NUMI_CLOTH_TRACE": "48", "NUMI_CLOTH_TRACE_CTA": "1"})
+    cfg = nc.substep_configs(scene, 48)
+    for frame in range(4):
+        sv.step(cfg, SCHED)
+        t = sv.trace_cta(48)
+        info = sv.launch_info()
+        assert t.shape[2] == info["grid"] and sv.failure() == 0
+        assert info["last_tiles"] == (frame >= 2)
+        assert (t[:, 0, :] > 0).all() and (np.diff(t[:, 0, :].astype(np.int64), axis=0) > 0).all()
