@@ -315,7 +315,10 @@ struct numi_cloth {
     // record's index among them (read from the device when first asked for,
     // then kept in step by numi_cloth_replace_compliance, the only writer);
     // and every grip's compliance, which a restore brings back with the grips.
+    // What a graph replays the host does not see: once a change was captured,
+    // both are read from the device every time.
     bool compliance_known = false;
+    bool compliance_captured = false;
     std::vector<float> compliance[3];
     std::vector<uint8_t> compliance_id[3];
     std::vector<float> grip_compliance;
@@ -2054,6 +2057,12 @@ int numi_cloth_restore(numi_cloth_t* h, uint32_t slot) {
 
 namespace {
 
+void note_capture(numi_cloth* h) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &capturing) == cudaSuccess && capturing != cudaStreamCaptureStatusNone)
+        h->compliance_captured = true;
+}
+
 // The dynamic state's regions (each a whole number of 4-byte words, 16-byte
 // aligned) to or from one block, every region at a multiple of 256 bytes:
 // one launch in place of ten copies of 2 us of host time each.
@@ -2104,6 +2113,7 @@ int snapshot_slot(numi_cloth_t* h, uint32_t slot) {
     }
     if (copy_state(h, static_cast<char*>(s.mem), true) != cudaSuccess) return NUMI_CLOTH_ECUDA;
     s.grip_compliance = h->grip_compliance;
+    note_capture(h);
     s.valid = true;
     return NUMI_CLOTH_OK;
 }
@@ -2112,6 +2122,7 @@ int restore_slot(numi_cloth_t* h, uint32_t slot) {
     cudaSetDevice(h->device);
     if (copy_state(h, static_cast<char*>(h->snaps[slot].mem), false) != cudaSuccess) return NUMI_CLOTH_ECUDA;
     h->grip_compliance = h->snaps[slot].grip_compliance;
+    note_capture(h);
     return NUMI_CLOTH_OK;
 }
 }  // namespace
@@ -3263,7 +3274,7 @@ void distinct_values(const std::vector<float>& values, std::vector<float>& disti
 }
 
 int read_compliance(numi_cloth* h) {
-    if (h->compliance_known) return NUMI_CLOTH_OK;
+    if (h->compliance_known && !h->compliance_captured) return NUMI_CLOTH_OK;
     const DeviceCloth& d = h->d;
     std::vector<float4> dm(d.d_count);
     std::vector<float2> km(d.k_count), bm(d.b_count);
@@ -3271,7 +3282,11 @@ int read_compliance(numi_cloth* h) {
     if (e == cudaSuccess && d.d_count) e = cudaMemcpy(dm.data(), d.d_mat, d.d_count * sizeof(float4), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && d.k_count) e = cudaMemcpy(km.data(), d.k_mat, d.k_count * sizeof(float2), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && d.b_count) e = cudaMemcpy(bm.data(), d.b_mat, d.b_count * sizeof(float2), cudaMemcpyDeviceToHost);
+    std::vector<NumiClothGrip> grips(h->compliance_captured ? d.g_count : 0u);
+    if (e == cudaSuccess && !grips.empty())
+        e = cudaMemcpy(grips.data(), d.grips, grips.size() * sizeof(NumiClothGrip), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return NUMI_CLOTH_ECUDA;
+    for (size_t g = 0; g < grips.size(); ++g) h->grip_compliance[g] = grips[g].targetOffsetAndCompliance.w;
     std::vector<float> v;
     for (const float4& m : dm) v.push_back(m.y);
     distinct_values(v, h->compliance[0], h->compliance_id[0]);
@@ -3380,6 +3395,7 @@ extern "C" int numi_cloth_replace_compliance(numi_cloth_t* h, uint32_t family, f
     // a tile plan's items carry the materials
     if (h->tiles && (family == 0u || family == 2u) && tile_materials(h) != cudaSuccess) return NUMI_CLOTH_ECUDA;
     replaced_compliance(h, family, from, to);
+    note_capture(h);
     return NUMI_CLOTH_OK;
 }
 

@@ -200,3 +200,32 @@ def test_reported_batch_shape_is_accepted(sides):
         batch.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def test_compliance_groups_after_captured_changes():
+    """A captured change takes place when its graph is replayed, and a captured
+    restore brings the grips' compliances back then."""
+    import torch
+    scene = small_square(side=9, fruits=0, gripCorners=2, stretchCompliance=1e-4, shearCompliance=2e-4,
+                         bendCompliance=1e-3)
+    stretch, shear, bend, grip = (float(np.float32(v)) for v in (1e-4, 2e-4, 1e-3, 2e-4))
+    before = [("distance", stretch), ("distance", shear), ("bend", bend), ("grip", grip)]
+    f = lambda v: float(np.float32(v))   # noqa: E731
+    stream = torch.cuda.Stream()
+    sv = nc.ClothSolver(scene)
+    sv.set_stream(stream.cuda_stream)
+    sv.snapshot(0)
+    assert sv.compliance_groups() == before
+    change, restore = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(change, stream=stream):
+        sv.replace_compliance("bend", bend, 2e-3)
+        sv.replace_compliance("grip", grip, 7e-4)
+    with torch.cuda.graph(restore, stream=stream):
+        sv.restore(0)
+    assert sv.compliance_groups() == before
+    change.replay()
+    torch.cuda.synchronize()
+    assert sv.compliance_groups() == before[:2] + [("bend", f(2e-3)), ("grip", f(7e-4))]
+    restore.replay()
+    torch.cuda.synchronize()
+    assert sv.compliance_groups() == before[:2] + [("bend", f(2e-3)), ("grip", grip)]
