@@ -14,10 +14,12 @@
 #include <cstdlib>
 #include <cstring>
 #include <deque>
+#include <functional>
 #include <initializer_list>
 #include <memory>
 #include <mutex>
 #include <new>
+#include <queue>
 #include <system_error>
 #include <thread>
 #include <utility>
@@ -2544,7 +2546,9 @@ struct numi_cloth_batch {
     // `ranks` CTAs per cloth; its launches with the edge/edge family run one
     // CTA per cloth
     bool fitted = false;
-    uint32_t fit_chunk = 0;            // the chunk that shape reports
+    uint32_t per_sm = 1;               // CTAs per SM of its launches without the edge/edge family
+    size_t room = 0;                   // shared memory a CTA of those has for particles
+    uint32_t fit_chunk = 0, fit_block = 0;   // the chunk and threads that shape reports
     uint32_t ranks = 1;
     uint32_t edge_ctas = 0;
     size_t edge_smem = 0;
@@ -2627,10 +2631,17 @@ Residency batch_residency(uint32_t n, uint32_t ranks, size_t room) {
     return r;
 }
 
-// Shared memory a CTA of the batch kernel has left for particles.
-size_t batch_room(const numi_cloth_batch* b, bool edge) {
+// Shared memory a CTA of the batch kernel has left for particles, where an
+// SM holds `per_sm` of them.
+size_t batch_room(const numi_cloth_batch* b, bool edge, uint32_t per_sm) {
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
+    if (per_sm > 1u) {
+        int sm = 0, reserved = 0;
+        cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, b->device);
+        cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, b->device);
+        optin = std::min(optin, sm / static_cast<int>(per_sm) - reserved);
+    }
     cudaFuncAttributes fa{};
     if (cudaFuncGetAttributes(&fa, batch_fn(edge)) != cudaSuccess) return 0;
     cudaFuncAttributes ft = fa;
@@ -2640,25 +2651,75 @@ size_t batch_room(const numi_cloth_batch* b, bool edge) {
     return static_cast<size_t>(optin) > fixed ? static_cast<size_t>(optin) - fixed : 0u;
 }
 
-// The default launch shape: 512 threads (a cloth's frame is latency-bound on
-// its SM: 192 square cloths of 16 to 96 particles a side take 10.6 ms a frame,
-// 15.6 with 256 threads and global particles), particles in shared memory as
-// far as they fit, and where there are
-// SMs to spare a cluster of up to 8 CTAs per cloth, until each CTA holds 256
-// particles (the single cloth's resident cluster).
+// Time until a queue of cloths (largest first) is empty, `workers` taking the
+// next one when they are free.
+template <class F>
+double queue_time(const std::vector<uint32_t>& particles, size_t workers, F&& time) {
+    std::priority_queue<double, std::vector<double>, std::greater<double>> free;
+    double end = 0.0;
+    for (uint32_t n : particles) {
+        double at = 0.0;
+        if (free.size() == workers) {
+            at = free.top();
+            free.pop();
+        }
+        at += time(n);
+        free.push(at);
+        end = std::max(end, at);
+    }
+    return end;
+}
+
+// CTAs per SM of a batch with a CTA per cloth: one of 512 threads, which
+// ends a cloth's frame soonest (a frame is latency-bound on its SM), or two
+// of 256, which end two cloths in less than twice that time.  24 substeps of
+// cloths of 100, 576, 1,024, 1,600, 3,136 and 5,184 particles take 970, 1,130,
+// 1,360, 1,630, 2,270 and 3,760 us alone on an SM with 512 threads, two of
+// them with 256 threads each 990, 1,450, 1,640, 2,070, 4,050 and 6,210 (from some
+// 2,700 on nothing of a cloth fits in half an SM's shared memory).  It is
+// the queue that decides: 160 cloths of 576 take 2,117 us by ones and 1,446 by
+// twos, 148 take 1,133 and 1,279, 300 cloths of 3,136 take 6,169 and 7,250,
+// 400 square cloths of 24 to 64 particles a side 5.14 ms and 4.85, and 512 of
+// 16 to 96, whose largest have 9,216 particles, 9.5 and 10.8.  The lines below
+// are these times, which are off by some per cent.
+uint32_t batch_per_sm(const numi_cloth_batch* b, size_t sms) {
+    if (b->cloths.size() <= sms) return 1u;
+    std::vector<uint32_t> particles;
+    for (numi_cloth* h : b->cloths) particles.push_back(h->d.n);
+    std::sort(particles.begin(), particles.end(), std::greater<uint32_t>());
+    const double ones =
+        queue_time(particles, sms, [](double n) { return n <= 4400.0 ? 900.0 + 0.46 * n : 900.0 + 0.55 * n; });
+    const double twos =
+        queue_time(particles, 2u * sms, [](double n) { return n <= 2700.0 ? 1000.0 + 0.68 * n : 430.0 + 1.13 * n; });
+    return twos < 0.98 * ones ? 2u : 1u;
+}
+
+// The default launch shape: one or two CTAs per SM, particles in shared
+// memory as far as they fit, and where there are SMs to spare a cluster of up
+// to 8 CTAs per cloth, until each CTA holds 256 particles (the single cloth's
+// resident cluster).  Launches with the edge/edge family, whose box tree takes
+// most of an SM's shared memory, run one CTA of 512 threads per cloth.
 int batch_fit(numi_cloth_batch* b) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
     const uint32_t count = static_cast<uint32_t>(b->cloths.size());
     uint32_t largest = 0;
     for (numi_cloth* h : b->cloths) largest = std::max(largest, h->d.n);
-    b->block = NC_BLOCK_MAX;
+    b->per_sm = batch_per_sm(b, static_cast<size_t>(std::max(sms, 1)));
+    b->block = NC_BLOCK_MAX / b->per_sm;
     uint32_t ranks = 1;
     while (ranks < 8u && static_cast<uint64_t>(count) * 2u * ranks <= static_cast<uint64_t>(std::max(sms, 1)) &&
            256u * ranks < largest)
         ranks *= 2u;
     for (bool edge : {false, true}) {
-        const size_t room = batch_room(b, edge);
+        size_t room = batch_room(b, edge, edge ? 1u : b->per_sm);
+        // two to an SM, particles in shared memory only where every cloth's
+        // are: the others read theirs through the L1, which has what shared
+        // memory leaves (400 cloths of 24 to 64 a side: 4.84 ms, 5.48 with
+        // those in shared memory that fit)
+        if (!edge && b->per_sm > 1u && batch_residency(largest, 1u, room).mode == 0u) room = 0u;
+        if (!edge) b->room = room;
+        const uint32_t block = edge ? NC_BLOCK_MAX : b->block;
         for (;;) {
             const uint32_t r = edge ? 1u : ranks;
             size_t bytes = 0;
@@ -2681,7 +2742,7 @@ int batch_fit(numi_cloth_batch* b) {
                 attr.val.clusterDim.z = 1;
                 cudaLaunchConfig_t cfg{};
                 cfg.gridDim = dim3(r);
-                cfg.blockDim = dim3(b->block);
+                cfg.blockDim = dim3(block);
                 cfg.dynamicSmemBytes = launch;
                 cfg.attrs = &attr;
                 cfg.numAttrs = 1;
@@ -2694,7 +2755,7 @@ int batch_fit(numi_cloth_batch* b) {
                 }
             } else {
                 int k = 0;
-                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, fn, static_cast<int>(b->block), launch) !=
+                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, fn, static_cast<int>(block), launch) !=
                         cudaSuccess ||
                     k < 1)
                     return NUMI_CLOTH_EINVAL;
@@ -2714,6 +2775,7 @@ int batch_fit(numi_cloth_batch* b) {
     b->ranks = ranks;
     b->fitted = true;
     b->fit_chunk = b->chunk;
+    b->fit_block = b->block;
     b->edge_room = true;
     b->layout_valid = false;
     return NUMI_CLOTH_OK;
@@ -2742,7 +2804,7 @@ cudaError_t batch_kernel(numi_cloth_batch* b, const DeviceCloth* cloths, const S
     attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(fit_edge ? b->edge_ctas : b->ctas);
-    cfg.blockDim = dim3(b->block);
+    cfg.blockDim = dim3(fit_edge ? NC_BLOCK_MAX : b->block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = b->stream;
     cfg.attrs = &attr;
@@ -2759,7 +2821,7 @@ int batch_layout(numi_cloth_batch* b, uint32_t substeps, bool edge) {
     if (b->layout_valid && b->layout_substeps == substeps && (!b->fitted || b->layout_edge == edge))
         return NUMI_CLOTH_OK;
     const uint32_t ranks = b->fitted && !edge ? b->ranks : 1u;
-    const size_t room = b->fitted ? batch_room(b, edge) : 0u;
+    const size_t room = !b->fitted ? 0u : edge ? batch_room(b, true, 1u) : b->room;
     const uint32_t count = static_cast<uint32_t>(b->cloths.size());
     std::vector<DeviceCloth>& host = b->host_cloths;
     host.resize(count);
@@ -2931,7 +2993,7 @@ int numi_cloth_batch_set_shape(numi_cloth_batch_t* b, uint32_t resident_chunk, u
     if (b == nullptr || (threads != NC_THREADS && threads != NC_BLOCK_MAX)) return NUMI_CLOTH_EINVAL;
     const bool power = (resident_chunk & (resident_chunk - 1u)) == 0u && resident_chunk <= 4096u;
     // what batch_shape or the tuner reported of the default shape
-    const bool fit = !power && resident_chunk == b->fit_chunk && threads == NC_BLOCK_MAX;
+    const bool fit = !power && resident_chunk == b->fit_chunk && threads == b->fit_block;
     if (!power && !fit) return NUMI_CLOTH_EINVAL;
     cudaSetDevice(b->device);
     batch_drop_graph(b);

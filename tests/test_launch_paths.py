@@ -229,3 +229,32 @@ def test_compliance_groups_after_captured_changes():
     restore.replay()
     torch.cuda.synchronize()
     assert sv.compliance_groups() == before[:2] + [("bend", f(2e-3)), ("grip", grip)]
+
+
+@pytest.mark.parametrize("sides", [(40, 33, 24, 9) + (32,) * 300, (53, 40, 33, 24, 9) + (32,) * 300],
+                         ids=["resident", "global"])
+def test_fitted_batch_by_twos_equals_alone(sides):
+    """More small cloths than SMs run two to an SM, on 256 threads each, with
+    positions and velocities or positions alone (40 x 40) in half of its shared
+    memory, or nothing where the largest does not fit (53 x 53); with the
+    edge/edge family one to an SM.  (By ones they would take three turns.)"""
+    scenes = {s: nc.square_scene(side=s, fruitCount=2, seed=s, **RESTING) for s in set(sides)}
+    for extra in ({}, {"selfCollision": 1}, {"primitiveSelf": 1}):
+        sched = nc.Schedule.make(**dict(PLAIN, **extra))
+        solvers = [nc.ClothSolver(scenes[s]) for s in sides]
+        batch = nc.ClothBatch(solvers)
+        shape = batch.shape()
+        assert shape["threads"] == 256 and shape["ctas"] > 148
+        assert (shape["resident_chunk"] > 0) == (max(sides) <= 40)
+        batch.set_shape(shape["resident_chunk"], shape["threads"])
+        assert batch.shape() == shape
+        cfg = np.stack([nc.substep_configs(scenes[s], 6) for s in sides])
+        batch.step(cfg, sched)
+        for k in (0, 1, 2, 3, 4, 5, len(sides) - 1):
+            alone = run_gpu(scenes[sides[k]], cfg[k], sched)
+            assert solvers[k].failure() == 0 and alone["failure"] == 0
+            assert np.array_equal(solvers[k].particles(), alone["particles"]), (extra, k)
+            assert np.array_equal(solvers[k].fruits(), alone["fruits"]), (extra, k)
+        batch.close()
+        for sv in solvers:
+            sv.close()
