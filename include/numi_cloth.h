@@ -484,8 +484,8 @@ int numi_cloth_batch_step(numi_cloth_batch_t* batch, const NumiClothConfig* conf
  * tune replace it. */
 int numi_cloth_batch_shape(numi_cloth_batch_t* batch, uint32_t out[3]);
 /* A shape whose resident chunk leaves no shared memory for the edge/edge
- * family's box tree (80 KB) serves only schedules with
- * primitiveSelf = 0: a step or capture with primitiveSelf on returns EINVAL
+ * family's box tree (4 to 32 KB by the largest cloth's yarn segments) serves
+ * only schedules with primitiveSelf = 0: a step or capture with primitiveSelf on returns EINVAL
  * on it, and the tuner skips it for such schedules. */
 /* resident_chunk: 0, a power of two up to 4096, or the chunk that
  * numi_cloth_batch_shape or numi_cloth_batch_tune gave for a batch of the

@@ -1078,17 +1078,19 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     size_t smem = h->smem;
     const bool tiled = tile_schedule(h, sc);
     if (edge) {
-        // the edge/edge phases' box-tree sort keys after the launch's own
-        // shared memory, where the device has room
+        // the edge/edge phases' box tree after the launch's own shared memory,
+        // where the device has room and the cloth is of a size that has one
         int max_optin = 0;
         cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
         cudaFuncAttributes fe{};
         cudaFuncGetAttributes(&fe, frame_fn(true, h->self_exact));
         const size_t at = nc_round256(smem);
-        if (at + NC_EDGE_TREE_KEY_BYTES + fe.sharedSizeBytes <= static_cast<size_t>(max_optin) &&
-            raise_smem(frame_fn(true, h->self_exact), at + NC_EDGE_TREE_KEY_BYTES) == cudaSuccess) {
+        const size_t bytes = at + edge_tree_bytes(d.y_count, true);
+        if (d.y_count <= NC_EDGE_TREE_MAX && bytes + fe.sharedSizeBytes <= static_cast<size_t>(max_optin) &&
+            raise_smem(frame_fn(true, h->self_exact), bytes) == cudaSuccess) {
             sc.tree_keys = static_cast<uint32_t>(at);
-            smem = at + NC_EDGE_TREE_KEY_BYTES;
+            sc.tree_lists = 1u;
+            smem = bytes;
         }
         cudaGetLastError();
     }
@@ -1328,7 +1330,7 @@ int prepare_edge_grid(numi_cloth* h, bool primitive, uint32_t substeps, float ra
         e.edge_lv = h->buf.alloc<uint32_t>(cap, stream);
         e.edge_level = h->buf.alloc<uint32_t>(d.n, stream);
         e.edge_qbox_raw = h->buf.alloc<float>(6u * d.y_count, stream);
-        e.edge_tree = h->buf.alloc<uint32_t>(static_cast<size_t>(NC_EDGE_TREE_WORDS) * d.y_count, stream);
+        e.edge_tree = h->buf.alloc<uint32_t>(static_cast<size_t>(NC_EDGE_TREE_WORDS) * d.y_count + NC_EDGE_TREE_HEAD, stream);
         e.edge_centre = h->buf.alloc<float4>(2u * static_cast<size_t>(d.y_count), stream);   // centres, last build's
         e.edge_rec = h->buf.alloc<EdgeRecord>(cap, stream);
         e.edge_ctl = h->buf.alloc<uint32_t>(8, stream);
@@ -2539,7 +2541,9 @@ struct numi_cloth_batch {
     uint32_t epoch_host = 1;
     uint32_t block = NC_THREADS;
     uint32_t chunk = 0;                // resident particle chunk (0: none)
-    bool edge_room = true;             // the shape leaves room for the box tree's sort keys
+    bool edge_room = true;             // the shape leaves room for the box tree
+    bool edge_lists = true;            // and for its lists
+    uint32_t tree_segments = 0;        // of the largest member that has one
     uint32_t ctas = 0;
     size_t smem = 0;
     // the default shape (batch_fit): residency cloth by cloth, a cluster of
@@ -2570,6 +2574,11 @@ uint32_t log2_pow2(uint32_t v) {
     return s;
 }
 
+// Shared memory of an edge/edge launch whose particles and fruits take `smem`.
+size_t batch_edge_smem(const numi_cloth_batch* b, size_t smem, bool lists) {
+    return nc_round256(smem) + edge_tree_bytes(b->tree_segments, lists);
+}
+
 // Launch shape: resident chunk (0 or a power of two), threads per CTA, and
 // as many CTAs as fit on the device (never more than the cloths).
 int batch_shape(numi_cloth_batch* b, uint32_t chunk, uint32_t block) {
@@ -2578,30 +2587,35 @@ int batch_shape(numi_cloth_batch* b, uint32_t chunk, uint32_t block) {
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, b->device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
     int per_sm = 1 << 30;
-    bool edge_room = false;
+    bool edge_room = false, edge_lists = false;
     for (bool edge : {false, true}) {
-        // the edge/edge kernel also holds the box tree's sort keys; a shape
-        // without room for them serves only schedules without that family
-        const size_t bytes = edge ? nc_round256(smem) + NC_EDGE_TREE_KEY_BYTES : smem;
+        // the edge/edge kernel also holds the box tree's sort keys, and its
+        // lists where an SM then holds as many CTAs as without; a shape
+        // without room for the keys serves only schedules without that family
         cudaFuncAttributes fa{};
         if (cudaFuncGetAttributes(&fa, batch_fn(edge)) != cudaSuccess) return NUMI_CLOTH_ECUDA;
-        if (bytes + fa.sharedSizeBytes > static_cast<size_t>(optin)) {
-            if (edge) continue;
-            return NUMI_CLOTH_EINVAL;
+        int most = 0;
+        for (bool lists : {false, true}) {
+            if (lists && !edge) break;
+            const size_t bytes = edge ? batch_edge_smem(b, smem, lists) : smem;
+            int k = 0;
+            if (bytes + fa.sharedSizeBytes > static_cast<size_t>(optin)) break;
+            if (raise_smem(batch_fn(edge), bytes) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, batch_fn(edge), static_cast<int>(block), bytes) !=
+                cudaSuccess)
+                return NUMI_CLOTH_EINVAL;
+            if (edge) {
+                edge_room = true;
+                edge_lists = lists && k >= most;
+            } else {
+                per_sm = k;
+            }
+            most = k;
         }
-        if (raise_smem(batch_fn(edge), bytes) != cudaSuccess) return NUMI_CLOTH_ECUDA;
-        if (edge) {
-            edge_room = true;
-            continue;   // launched without co-residence
-        }
-        int k = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, batch_fn(edge), static_cast<int>(block), bytes) !=
-            cudaSuccess)
-            return NUMI_CLOTH_EINVAL;
-        per_sm = std::min(per_sm, k);
+        if (!edge && most == 0) return NUMI_CLOTH_EINVAL;
     }
-    if (per_sm < 1) return NUMI_CLOTH_EINVAL;
     b->edge_room = edge_room;
+    b->edge_lists = edge_lists;
     b->chunk = chunk;
     b->block = block;
     b->smem = smem;
@@ -2647,7 +2661,7 @@ size_t batch_room(const numi_cloth_batch* b, bool edge, uint32_t per_sm) {
     cudaFuncAttributes ft = fa;
     if (!edge && cudaFuncGetAttributes(&ft, batch_tape_fn(false)) != cudaSuccess) return 0;
     const size_t fixed = nc_resident_offset() + std::max(fa.sharedSizeBytes, ft.sharedSizeBytes) + 256u +
-                         (edge ? NC_EDGE_TREE_KEY_BYTES : 0u);
+                         (edge ? edge_tree_bytes(b->tree_segments, true) : 0u);
     return static_cast<size_t>(optin) > fixed ? static_cast<size_t>(optin) - fixed : 0u;
 }
 
@@ -2730,7 +2744,7 @@ int batch_fit(numi_cloth_batch* b) {
                 if (!edge && res.mode != 0u) b->chunk = std::max(b->chunk, h->d.n);
             }
             const size_t smem = nc_resident_offset() + bytes;
-            const size_t launch = edge ? nc_round256(smem) + NC_EDGE_TREE_KEY_BYTES : smem;
+            const size_t launch = edge ? batch_edge_smem(b, smem, true) : smem;
             const void* fn = r > 1u ? batch_cluster_fn() : batch_fn(edge);
             if (raise_smem(fn, launch) != cudaSuccess) return NUMI_CLOTH_ECUDA;
             int fit = 0;
@@ -2776,7 +2790,7 @@ int batch_fit(numi_cloth_batch* b) {
     b->fitted = true;
     b->fit_chunk = b->chunk;
     b->fit_block = b->block;
-    b->edge_room = true;
+    b->edge_room = b->edge_lists = true;
     b->layout_valid = false;
     return NUMI_CLOTH_OK;
 }
@@ -2791,9 +2805,10 @@ cudaError_t batch_kernel(numi_cloth_batch* b, const DeviceCloth* cloths, const S
     uint32_t count = static_cast<uint32_t>(b->cloths.size());
     Schedule sc = s;
     size_t smem = fit_edge ? b->edge_smem : b->smem;
-    if (edge) {   // the box tree's sort keys (the shape has room for them)
+    if (edge) {   // the box tree (the shape has room for it)
         sc.tree_keys = static_cast<uint32_t>(nc_round256(smem));
-        smem = nc_round256(smem) + NC_EDGE_TREE_KEY_BYTES;
+        sc.tree_lists = b->edge_lists ? 1u : 0u;
+        smem = batch_edge_smem(b, smem, b->edge_lists);
     }
     cudaError_t e = cudaMemsetAsync(b->queue, 0, sizeof(unsigned int), b->stream);
     if (e != cudaSuccess) return e;
@@ -2946,6 +2961,8 @@ int numi_cloth_batch_create(numi_cloth_t* const* cloths, uint32_t count, numi_cl
                 return NUMI_CLOTH_EINVAL;
             }
         b->cloths.push_back(cloths[k]);
+        if (cloths[k]->d.y_count <= NC_EDGE_TREE_MAX)
+            b->tree_segments = std::max(b->tree_segments, cloths[k]->d.y_count);
         b->epoch_host = std::max(b->epoch_host, cloths[k]->epoch);
     }
     cudaSetDevice(b->device);

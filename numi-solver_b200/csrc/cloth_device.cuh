@@ -22,6 +22,7 @@
 
 #define NC_MAX_FRUITS 64u
 #define NC_MAX_GRIPS 32u
+#define NC_BLOCK_MAX 512    /* largest CTA (cluster launch) */
 #define NC_MAX_BATCHES 64u
 #define NC_YARN_SLOTS 4u
 #define NC_MAX_PAIRS 2016u
@@ -305,9 +306,25 @@ struct Schedule {
     // 1: the launch runs in tile mode (cloth_tile.cuh)
     uint32_t tiles;
     // edge/edge launches: byte offset in dynamic shared memory of the box
-    // tree's sort keys (edge_tree_order), 0 when the launch has none
+    // tree's sort keys (edge_tree_order), 0 when the launch has none; and 1
+    // where its lists follow them
     uint32_t tree_keys;
+    uint32_t tree_lists;
 };
+
+// The box tree's build (edge_tree_order) of a cloth of at most
+// NC_EDGE_TREE_MAX yarn segments: sort keys (a power of two, at least one a
+// thread), and bytes of dynamic shared memory without and with its lists.
+#define NC_EDGE_TREE_MAX 4096u
+__host__ __device__ inline uint32_t edge_tree_keys(uint32_t segments) {
+    uint32_t keys = NC_BLOCK_MAX;
+    while (keys < segments) keys <<= 1;
+    return keys;
+}
+__host__ __device__ inline size_t edge_tree_bytes(uint32_t segments, bool lists) {
+    return edge_tree_keys(segments) * sizeof(unsigned long long) +
+           (lists ? 6u * static_cast<size_t>(segments) * sizeof(unsigned short) : 0u);
+}
 
 // Fruit-side state kept in the shared memory of the fruit CTA for a whole
 // launch: compact pair indices (loaded once) and the pair contact impulses

@@ -740,14 +740,15 @@ __device__ void edge_candidates(Ctx& ctx, bool swept, bool rebuilt) {
 // order is its parent's axis list.  CTA 0, all threads; at most
 // NC_EDGE_TREE_MAX segments.  The build is bound by the latency of its
 // dependent gathers, and the cluster's other CTAs wait for it.  So the lists
-// are in shared memory (TreeShared): in global memory every level scattered
-// 9,000 words through the L2, and the top boxes were one warp's scan of all
-// segments (a bag frame's swept pass 236 us, now 92).  edge_tree: [m] segment
-// at each leaf position, [m] position of each segment, then [3][m] the last
-// build's order along each axis.
-#define NC_EDGE_TREE_MAX 4096u
-#define NC_EDGE_TREE_KEY_BYTES (NC_EDGE_TREE_MAX * 20u)   /* the build's shared memory (TreeShared) */
-#define NC_EDGE_TREE_WORDS 14u   /* edge_tree words per segment (the build uses 5, and one flag word) */
+// are in shared memory where the launch has room (Schedule::tree_lists): in
+// global memory every level scattered 9,000 words through the L2, and the top
+// boxes were one warp's scan of all segments (a bag frame's swept pass 236
+// us, now 92).  A batch shape that holds two CTAs an SM only without them
+// keeps them in edge_tree.  edge_tree: [m] segment at each leaf position, [m]
+// position of each segment, [3][m] the last build's order along each axis, a
+// flag, and room for the lists.
+#define NC_EDGE_TREE_WORDS 9u    /* edge_tree words per segment */
+#define NC_EDGE_TREE_HEAD 8u     /* and words of the flag */
 #define NC_EDGE_TREE_WARM 8u     /* odd-even passes tried on the previous order before a full sort */
 __shared__ unsigned char nc_edge_tree_axis[NC_EDGE_TREE_MAX / 8u];
 __shared__ uint32_t nc_edge_scan[3][32];
@@ -845,35 +846,21 @@ __device__ void block_sort(unsigned long long* keys, uint32_t n) {
     }
 }
 
-// The build's arrays in the launch's dynamic shared memory: the sort keys and
-// in their place, once the axes are sorted, the prefix counts of the lists
-// and the side of each segment; two sets of the three lists.
-struct TreeShared {
-    union {
-        unsigned long long keys[NC_EDGE_TREE_MAX];
-        struct {
-            unsigned short pre[3][NC_EDGE_TREE_MAX];
-            unsigned char right[NC_EDGE_TREE_MAX];
-        };
-    };
-    unsigned short list[2][3][NC_EDGE_TREE_MAX];
-};
-static_assert(sizeof(TreeShared) <= NC_EDGE_TREE_KEY_BYTES, "box tree shared memory");
 #define NC_EDGE_TREE_PER (NC_EDGE_TREE_MAX / NC_THREADS)   /* most positions of a thread */
 
 // Axis of a splitting node [b, e): the longest extent of its members' centres
 // (the first of equals).  The lists are in axis order, so the extent along an
 // axis is between the ends of that axis' list; a centre that is no number
 // sorts to an end and has no extent, so then the members are scanned.
-__device__ __forceinline__ unsigned char tree_axis(const float4* centre, const unsigned short (*L)[NC_EDGE_TREE_MAX],
+__device__ __forceinline__ unsigned char tree_axis(const float4* centre, const unsigned short* L, uint32_t m,
                                                    uint32_t b, uint32_t e) {
-    V3 lo{centre[L[0][b]].x, centre[L[1][b]].y, centre[L[2][b]].z};
-    V3 hi{centre[L[0][e - 1u]].x, centre[L[1][e - 1u]].y, centre[L[2][e - 1u]].z};
+    V3 lo{centre[L[b]].x, centre[L[m + b]].y, centre[L[2u * m + b]].z};
+    V3 hi{centre[L[e - 1u]].x, centre[L[m + e - 1u]].y, centre[L[2u * m + e - 1u]].z};
     if (!(lo.x == lo.x && lo.y == lo.y && lo.z == lo.z && hi.x == hi.x && hi.y == hi.y && hi.z == hi.z)) {
         lo = V3{INFINITY, INFINITY, INFINITY};
         hi = V3{-INFINITY, -INFINITY, -INFINITY};
         for (uint32_t p = b; p < e; ++p) {
-            const float4 c = centre[L[0][p]];
+            const float4 c = centre[L[p]];
             lo = V3{fminf(lo.x, c.x), fminf(lo.y, c.y), fminf(lo.z, c.z)};
             hi = V3{fmaxf(hi.x, c.x), fmaxf(hi.y, c.y), fmaxf(hi.z, c.z)};
         }
@@ -882,15 +869,23 @@ __device__ __forceinline__ unsigned char tree_axis(const float4* centre, const u
     return static_cast<unsigned char>(ext.y > ext.x ? (ext.z > ext.y ? 2u : 1u) : (ext.z > ext.x ? 2u : 0u));
 }
 
-__device__ void edge_tree_order(const Ctx& ctx, bool swept) {
-    const DeviceCloth& d = ctx.d;
-    // the sort keys, then the prefix counts, in the launch's dynamic shared
-    // memory
-    TreeShared& ts = *reinterpret_cast<TreeShared*>(nc_frame_smem + ctx.s.tree_keys);
-    unsigned long long* keys = ts.keys;
-    unsigned short (*pre)[NC_EDGE_TREE_MAX] = ts.pre;
+// kShared: the lists are in shared memory (known where the build is compiled:
+// a pointer to either costs the registers of both).
+template <bool kShared>
+__device__ __forceinline__ void edge_tree_order(const DeviceCloth& d, float radius, uint32_t tree_keys, bool swept) {
     const uint32_t m = d.y_count;
-    const float ex = 0.5f * (2.0f * ctx.c.radius);
+    // in the launch's dynamic shared memory the sort keys, and in their place
+    // once the axes are sorted the prefix counts of the lists, [3][m], and
+    // the side of each segment; two sets of the three lists, [2][3][m]
+    unsigned long long* keys = reinterpret_cast<unsigned long long*>(nc_frame_smem + tree_keys);
+    unsigned short* pre = reinterpret_cast<unsigned short*>(keys);
+    unsigned char* right = reinterpret_cast<unsigned char*>(pre + 3u * m);
+    unsigned short* lists;
+    if constexpr (kShared)
+        lists = reinterpret_cast<unsigned short*>(keys + edge_tree_keys(m));
+    else
+        lists = reinterpret_cast<unsigned short*>(d.edge_tree + 5u * m + NC_EDGE_TREE_HEAD);
+    const float ex = 0.5f * (2.0f * radius);
     uint32_t* ord = d.edge_tree;
     uint32_t* gsort = d.edge_tree + 2u * m;   // [3][m] the last build's order along each axis
     uint32_t* valid = gsort + 3u * m;         // 1 once a tree was built
@@ -915,8 +910,7 @@ __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
     }
     // the same centres as the last build: the same tree
     if (!__syncthreads_or(changed)) return;
-    uint32_t size = blockDim.x;
-    while (size < m) size <<= 1;
+    const uint32_t size = edge_tree_keys(m);
     // the three axis lists, (centre, index) order: from the last build's
     // order, a few odd-even transposition passes while it is not sorted
     // (the centres move little from pass to pass), else a full sort
@@ -955,7 +949,7 @@ __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
         if (!sorted) block_sort(keys, size);
         for (uint32_t p = threadIdx.x; p < m; p += blockDim.x) {
             const uint32_t sg = static_cast<uint32_t>(keys[p] & 0xfffull);
-            ts.list[0][a][p] = static_cast<unsigned short>(sg);
+            lists[a * m + p] = static_cast<unsigned short>(sg);
             gsort[a * m + p] = sg;
         }
         __syncthreads();
@@ -973,15 +967,15 @@ __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
     uint32_t axes = 0xffffffffu;
     uint32_t cur = 0u;
     for (uint32_t level = 0; level < 32u; ++level) {
-        const unsigned short (*L)[NC_EDGE_TREE_MAX] = ts.list[cur];
-        unsigned short (*N)[NC_EDGE_TREE_MAX] = ts.list[cur ^ 1u];
+        const unsigned short* L = lists + cur * 3u * m;
+        unsigned short* N = lists + (cur ^ 1u) * 3u * m;
         // axis of every node of the level that splits
         const uint32_t nodes = 1u << level;
         bool any = false;
         for (uint32_t j = threadIdx.x; j < nodes && j < NC_EDGE_TREE_MAX / 8u; j += blockDim.x) {
             uint32_t b, e;
             if (!tree_node_of_path(m, level, j, b, e) || e - b <= 8u) continue;
-            nc_edge_tree_axis[b >> 3] = tree_axis(d.edge_centre, L, b, e);
+            nc_edge_tree_axis[b >> 3] = tree_axis(d.edge_centre, L, m, b, e);
             any = true;
         }
         if (!__syncthreads_or(any)) break;
@@ -991,11 +985,11 @@ __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
             if (i >= mine) break;
             const uint32_t p = own + i, b = node[i] & 0xffffu, e = node[i] >> 16;
             if (e - b <= 8u) {
-                ts.right[L[0][p]] = 0u;
+                right[L[p]] = 0u;
                 continue;
             }
             const uint32_t a = nc_edge_tree_axis[b >> 3];
-            ts.right[L[a][p]] = p - b >= (e - b) / 2u ? 1u : 0u;
+            right[L[a * m + p]] = p - b >= (e - b) / 2u ? 1u : 0u;
             axes = (axes & ~(3u << (2u * i))) | (a << (2u * i));
         }
         __syncthreads();
@@ -1007,7 +1001,7 @@ __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
 #pragma unroll
             for (uint32_t i = 0; i < NC_EDGE_TREE_PER; ++i) {
                 if (i >= mine) break;
-                bits[a] |= static_cast<uint32_t>(ts.right[L[a][own + i]]) << i;
+                bits[a] |= static_cast<uint32_t>(right[L[a * m + own + i]]) << i;
             }
             incl[a] = __popc(bits[a]);
             for (int o = 1; o < 32; o <<= 1) {
@@ -1032,7 +1026,7 @@ __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
 #pragma unroll
             for (uint32_t i = 0; i < NC_EDGE_TREE_PER; ++i) {
                 if (i >= mine) break;
-                pre[a][own + i] = static_cast<unsigned short>(incl[a] + __popc(bits[a] & ((1u << i) - 1u)));
+                pre[a * m + own + i] = static_cast<unsigned short>(incl[a] + __popc(bits[a] & ((1u << i) - 1u)));
             }
         }
         __syncthreads();
@@ -1047,10 +1041,10 @@ __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
             for (uint32_t a = 0; a < 3u; ++a) {
                 uint32_t to = p;
                 if (split) {
-                    const uint32_t rights = incl[a] + __popc(bits[a] & ((1u << i) - 1u)) - pre[a][b];
+                    const uint32_t rights = incl[a] + __popc(bits[a] & ((1u << i) - 1u)) - pre[a * m + b];
                     to = ((bits[a] >> i) & 1u) != 0u ? mid + rights : p - rights;
                 }
-                N[a][to] = L[a][p];
+                N[a * m + to] = L[a * m + p];
             }
             if (split) node[i] = p >= mid ? mid | (e << 16) : b | (mid << 16);
         }
@@ -1061,7 +1055,7 @@ __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
     for (uint32_t i = 0; i < NC_EDGE_TREE_PER; ++i) {
         if (i >= mine) break;
         const uint32_t p = own + i, a = (axes >> (2u * i)) & 3u;
-        ord[p] = a < 3u ? ts.list[cur][a][p] : p;
+        ord[p] = a < 3u ? lists[(3u * cur + a) * m + p] : p;
     }
     for (uint32_t p = threadIdx.x; p < m; p += blockDim.x) prev[p] = d.edge_centre[p];
     __syncthreads();
@@ -1069,6 +1063,12 @@ __device__ void edge_tree_order(const Ctx& ctx, bool swept) {
     if (threadIdx.x == 0) *valid = 1u;
     __syncthreads();
 }
+
+#ifdef NC_EDGE_BATCH_KERNELS
+__device__ __noinline__ void edge_tree_global(const DeviceCloth& d, float radius, uint32_t tree_keys, bool swept) {
+    edge_tree_order<false>(d, radius, tree_keys, swept);
+}
+#endif
 
 // Phase 3 (CTA 0): sort the ordered pairs, undo the previous round, then
 // resolve them in the reference's order as wavefronts: a pair's level is one
@@ -1132,7 +1132,13 @@ __device__ void edge_resolve(Ctx& ctx, bool swept, bool redo) {
         }
     }
     const bool tree = __syncthreads_or(mine) != 0 && d.y_count <= NC_EDGE_TREE_MAX && ctx.s.tree_keys != 0u;
-    if (tree) edge_tree_order(ctx, swept);
+#ifdef NC_EDGE_BATCH_KERNELS
+    if (tree && ctx.s.tree_lists == 0u)
+        edge_tree_global(d, ctx.c.radius, ctx.s.tree_keys, swept);
+    else
+#endif
+    if (tree)
+        edge_tree_order<true>(d, ctx.c.radius, ctx.s.tree_keys, swept);
     const uint32_t* tpos = d.edge_tree + d.y_count;
     auto sort_key = [&](unsigned long long key) {
         return tree ? ((key & 0xffffffff00000000ull) | __ldcg(tpos + static_cast<uint32_t>(key))) : key;

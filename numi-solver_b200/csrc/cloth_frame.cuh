@@ -3131,9 +3131,9 @@ __device__ __forceinline__ void run_frame(const DeviceCloth& src, const Schedule
 }
 
 // The frame and batch kernels with the edge/edge yarn self-collision phases
-// are defined in cloth_edge_kernels.cu, a translation unit of their own: with
-// them in the same unit the compiler inlines the shared phases differently
-// and the default kernels grow a call frame.
+// are defined in cloth_edge_kernels.cu and cloth_edge_batch_kernels.cu, units
+// of their own: with them in the same unit the compiler inlines the shared
+// phases differently and the default kernels grow a call frame.
 __global__ void numi_cloth_frame_edge_kernel(DeviceCloth d, Schedule s);
 __global__ void numi_cloth_batch_edge_kernel(const DeviceCloth* cloths, uint32_t count, Schedule s,
                                              unsigned int* queue);

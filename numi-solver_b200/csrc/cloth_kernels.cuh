@@ -30,7 +30,6 @@
 #include <cooperative_groups.h>
 
 #define NC_THREADS 256      /* threads of a CTA in the cooperative-grid launch; width of the fixed reduction trees */
-#define NC_BLOCK_MAX 512    /* largest CTA (cluster launch) */
 #define NC_FIXED_SCALE 1099511627776.0   /* 2^40 */
 #define NC_BARRIER_SPIN_LIMIT (1u << 22)
 

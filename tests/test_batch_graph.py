@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import numi_cloth as nc
-from helpers import PLAIN, small_square
+from helpers import PLAIN, lift_trajectory_path, small_square
 
 pytestmark = pytest.mark.gpu
 
@@ -50,3 +50,27 @@ def test_replay_after_another_launch(sides, captured, between, substeps):
         assert np.array_equal(sv.fruits(), rv.fruits())
     batch.close()
     plain.close()
+
+
+@pytest.mark.parametrize("shape", [(0, 256), (0, 512), (1024, 256)], ids=["two-an-sm", "one-an-sm", "resident"])
+def test_edge_family_on_bags_equals_alone(shape):
+    """The produce bag's edge/edge contacts in a batch: the box tree's lists in
+    global memory (two CTAs an SM, for whose bags' some 2,600 segments half an
+    SM has no room) and in shared memory."""
+    scene = nc.bag_scene(scenario="recorded", timestep=1.0 / 2880.0)
+    motion = nc.GripTrajectory(lift_trajectory_path())
+    cfg = motion.configs(scene.config, scene.handle_base, 0, 6, 1.0 / 2880.0)
+    sched = nc.Schedule.make(**dict(EDGES, strainSweeps=3, finalPasses=2, selfCollision=1))
+    alone = nc.ClothSolver(scene)
+    alone.step(cfg, sched)
+    assert alone.failure() == 0 and alone.edge_contacts()[0] > 0
+    small = small_square(side=14, fruits=1)
+    scenes = [scene, small, scene]
+    solvers = [nc.ClothSolver(s) for s in scenes]
+    batch = nc.ClothBatch(solvers)
+    batch.set_shape(*shape)
+    batch.step(np.stack([cfg, nc.substep_configs(small, 6), cfg]), sched)
+    for k in (0, 2):
+        assert solvers[k].failure() == 0 and solvers[k].edge_contacts() == alone.edge_contacts()
+        assert np.array_equal(solvers[k].particles(), alone.particles())
+    batch.close()
