@@ -480,8 +480,8 @@ int numi_cloth_batch_step(numi_cloth_batch_t* batch, const NumiClothConfig* conf
  * many particles keep them in shared memory; 0 = none), out[1] threads per
  * CTA, out[2] CTAs of the persistent launch.  The shape of a new batch is
  * fitted to its cloths (particles in shared memory as far as they fit, a
- * cluster of CTAs per cloth where there are SMs to spare); set_shape and
- * tune replace it. */
+ * cluster of CTAs per cloth where there are SMs to spare, two CTAs an SM for
+ * more small cloths than SMs); set_shape and tune replace it. */
 int numi_cloth_batch_shape(numi_cloth_batch_t* batch, uint32_t out[3]);
 /* A shape whose resident chunk leaves no shared memory for the edge/edge
  * family's box tree (4 to 32 KB by the largest cloth's yarn segments) serves

@@ -795,10 +795,13 @@ __device__ __forceinline__ bool fruit_pair_waves(const DeviceCloth& d, FruitShar
 // has few near pairs, so the near pairs in dependence order (a handful of
 // rounds) replace the walk of every colour: 64 spheres resting on a cloth
 // took 19.2 us for the walk of 63 colours (0.3 us a colour, its quotients
-// and roots one after the other) and take 6.6 us.  Below NC_PAIR_COLOURS the
-// walk is shorter than building the wavefronts (the bag's 12 fruits have 11
-// colours, 3 us), and it stays for more than NC_PAIR_NEAR near
-// pairs and for sweeps that move a fruit too far for the proof.  One warp
+// and roots one after the other) and take 6.6 us.  Colours come as 7, 15, 31 or
+// 63 (11 on the bag): frames of resting cloths take the same either way with
+// 15 (12 or 15 spheres: within 0.3 %), up to 9 % less by wavefronts with 31 (18
+// to 30 spheres: 2,234 us against 2,403, 2,126 against 2,331, never more), and
+// the bag 1 % less by the walk.  The walk also stays for more than
+// NC_PAIR_NEAR near pairs and for sweeps that move a fruit too far for the
+// proof.  One warp
 // walks the colours (a colour's pairs are disjoint, so its lanes never touch
 // the same fruit).
 __device__ void fruit_pair_sweep(const DeviceCloth& d, FruitShared& fs, float dt) {
