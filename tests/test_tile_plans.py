@@ -150,3 +150,52 @@ def test_per_cta_trace_of_a_small_cloth():
         assert t.shape[2] == info["grid"] and sv.failure() == 0
         assert info["last_tiles"] == (frame >= 2)
         assert (t[:, 0, :] > 0).all() and (np.diff(t[:, 0, :].astype(np.int64), axis=0) > 0).all()
+
+
+def test_plans_of_handles_on_several_threads():
+    """Threads with handles and streams of their own, whose plans are built and
+    taken up, materials changed and gradients taken side by side."""
+    import threading
+
+    import torch
+    scene = _scene(30)
+    cfg = nc.substep_configs(scene, 16)
+    tracked = np.arange(4, dtype=np.uint32)
+    target = scene.particles["positionAndInverseMass"][None, :4, :3].astype(np.float64) + 1e-3
+    smooth = nc.Schedule.make(**dict(PLAIN, damping=0.5))
+    out, errors = {}, []
+
+    def work(name):
+        try:
+            stream = torch.cuda.Stream()
+            solvers = [make_solver(scene) for _ in range(4)]
+            for sv in solvers:
+                sv.set_stream(stream.cuda_stream)
+            for k in range(10):
+                for sv in solvers:
+                    sv.step(cfg, SCHED)
+                if k == 8:
+                    for sv in solvers:
+                        sv.replace_compliance("distance", 1e-6, 3e-6)
+            grads = [sv.rollout_grad(cfg, smooth, tracked, target, 16) for sv in solvers]
+            out[name] = [(sv.failure(), sv.launch_info()["last_tiles"], sv.particles(), g["loss"], g["grads"])
+                         for sv, g in zip(solvers, grads)]
+            for sv in solvers:
+                sv.close()
+        except Exception as e:   # noqa: BLE001
+            errors.append(e)
+
+    work("alone")
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    ref = out["alone"][0]
+    assert ref[0] == 0 and ref[1]
+    for rows in out.values():
+        for failure, tiles, particles, loss, grads in rows:
+            assert failure == 0 and tiles
+            assert np.array_equal(particles, ref[2])
+            assert loss == ref[3] and np.array_equal(grads, ref[4])
