@@ -1076,6 +1076,7 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
     if (e != cudaSuccess) return e;
     h->last_substeps = substeps;
     size_t smem = h->smem;
+    uint32_t grid = h->grid;
     const bool tiled = tile_schedule(h, sc);
     if (edge) {
         // the edge/edge phases' box tree after the launch's own shared memory,
@@ -1092,6 +1093,13 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
             sc.tree_lists = 1u;
             smem = bytes;
         }
+        // the tree can cost a cooperative grid its second CTA on an SM: as
+        // many as are co-resident (the bits are those of any grid)
+        int k = 0, sms = 0;
+        if (h->cluster == 0u && grid > 1u &&
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, fn, static_cast<int>(h->block), smem) == cudaSuccess &&
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) == cudaSuccess && k > 0)
+            grid = std::min(grid, static_cast<uint32_t>(k * sms));
         cudaGetLastError();
     }
     if (h->cluster > 0 && !tiled) {
@@ -1131,9 +1139,9 @@ cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t
             e = cudaMemsetAsync(d.nbr_flag, 0, NC_NBR_FLAG_STRIDE * h->grid * sizeof(unsigned int), h->stream);
             if (e != cudaSuccess) return e;
         }
-        e = cudaLaunchCooperativeKernel(fn, dim3(h->grid), dim3(h->block), args, d.nbr_on ? h->nbr_smem : smem, h->stream);
+        e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(h->block), args, d.nbr_on ? h->nbr_smem : smem, h->stream);
     }
-    h->last_grid = h->cluster > 0 ? h->cluster : h->grid;
+    h->last_grid = h->cluster > 0 ? h->cluster : grid;
     h->last_block = h->block;
     h->last_tiles = false;
     if (e == cudaSuccess) ++h->launches;
