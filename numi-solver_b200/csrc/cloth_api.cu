@@ -105,15 +105,18 @@ struct Workspace {
     size_t bytes = 0, most = 0;   // most: what may be kept on its device
     int device = -1;
     bool busy = false;   // a call uses it
+    Workspace* next = nullptr;   // every workspace of the process
     Workspace() {
         std::lock_guard<std::mutex> lock(mutex());
-        all().push_back(this);
+        next = std::exchange(first(), this);
     }
     Workspace(const Workspace&) = delete;
     Workspace& operator=(const Workspace&) = delete;
     ~Workspace() {
         std::lock_guard<std::mutex> lock(mutex());
-        all().erase(std::find(all().begin(), all().end(), this));
+        Workspace** at = &first();
+        while (*at != this) at = &(*at)->next;
+        *at = next;
         release();
     }
     void release() {
@@ -125,15 +128,15 @@ struct Workspace {
         static std::mutex m;
         return m;
     }
-    static std::vector<Workspace*>& all() {
-        static std::vector<Workspace*> list;
-        return list;
+    static Workspace*& first() {
+        static Workspace* head = nullptr;
+        return head;
     }
     // Gives back what no call uses on the device; false where that is nothing.
     static bool reclaim(int device) {
         std::lock_guard<std::mutex> lock(mutex());
         bool any = false;
-        for (Workspace* w : all())
+        for (Workspace* w = first(); w != nullptr; w = w->next)
             if (!w->busy && w->mem != nullptr && w->device == device) {
                 w->release();
                 any = true;
@@ -152,7 +155,7 @@ struct Workspace {
         ~Lease() {
             std::unique_lock<std::mutex> lock(mutex());
             size_t kept = 0;
-            for (const Workspace* o : all())
+            for (const Workspace* o = first(); o != nullptr; o = o->next)
                 if (o->device == w.device) kept += o->bytes;
             if (kept > w.most) {
                 lock.unlock();
@@ -1012,10 +1015,10 @@ bool tile_schedule(const numi_cloth* h, const Schedule& s) { return h->tiles && 
 
 // A small cloth's plan is built from its kTileBuildSubsteps'th covered
 // substep on, beside the stepping thread, and taken up at its
-// kTilePlanSubsteps'th: a build takes 0.5 to 2 ms of another core and as
-// many substeps are 5 ms of the GPU's time, so the launch that takes it up
-// finds it done unless launches are issued far ahead of the GPU.  A cloth
-// that only joins batches never needs one.
+// kTilePlanSubsteps'th: a build takes 0.4 (24 x 24) to 3 ms (61 x 61) of
+// another core, and the substeps between are 5 to 7 ms of the GPU's time, so
+// the launch that takes it up finds it done unless launches are issued far
+// ahead of the GPU.  A cloth that only joins batches never needs one.
 constexpr uint32_t kTileBuildSubsteps = 32, kTilePlanSubsteps = 128;
 void prepare_small_tiles(numi_cloth* h, uint32_t substeps) {
     h->tile_substeps += std::min(substeps, kTilePlanSubsteps - std::min(h->tile_substeps, kTilePlanSubsteps));
@@ -1050,7 +1053,15 @@ struct Tape {
 
 cudaError_t launch(numi_cloth* h, uint32_t substeps, const Schedule& s, uint32_t cfg_offset = 0,
                    const Tape& tape = {}) {
-    if ((h->tile_source != nullptr || h->tile_job != nullptr) && tile_covers(s)) prepare_small_tiles(h, substeps);
+    if ((h->tile_source != nullptr || h->tile_job != nullptr) && tile_covers(s)) {
+        try {
+            prepare_small_tiles(h, substeps);
+        } catch (const std::bad_alloc&) {   // it stays on its cluster
+            h->tile_source.reset();
+            if (h->tile_job) TileBuilder::get().abandon(h->tile_job);
+            h->tile_job.reset();
+        }
+    }
     DeviceCloth d = h->d;
     d.cfg = h->d_cfg + cfg_offset;
     d.epoch_base = h->epoch;
@@ -1852,7 +1863,9 @@ int numi_cloth_step(numi_cloth_t* h, const NumiClothConfig* configs, uint32_t co
     if (count > h->cfg_capacity) {
         cudaFree(h->d_cfg);
         h->d_cfg = nullptr;
-        if (device_malloc(reinterpret_cast<void**>(&h->d_cfg), count * sizeof(NumiClothConfig)) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+        h->cfg_capacity = 0;
+        if (device_malloc(reinterpret_cast<void**>(&h->d_cfg), count * sizeof(NumiClothConfig)) != cudaSuccess)
+            return NUMI_CLOTH_ECUDA;
         h->cfg_capacity = count;
     }
     if (cudaMemcpyAsync(h->d_cfg, configs, count * sizeof(NumiClothConfig), cudaMemcpyHostToDevice, h->stream) !=
@@ -3513,7 +3526,9 @@ extern "C" int numi_cloth_rollout_grad(numi_cloth_t* h, const NumiClothConfig* c
     if (substeps > h->cfg_capacity) {
         cudaFree(h->d_cfg);
         h->d_cfg = nullptr;
-        if (device_malloc(reinterpret_cast<void**>(&h->d_cfg), substeps * sizeof(NumiClothConfig)) != cudaSuccess) return NUMI_CLOTH_ECUDA;
+        h->cfg_capacity = 0;
+        if (device_malloc(reinterpret_cast<void**>(&h->d_cfg), substeps * sizeof(NumiClothConfig)) != cudaSuccess)
+            return NUMI_CLOTH_ECUDA;
         h->cfg_capacity = substeps;
     }
     if (cudaMemcpyAsync(h->d_cfg, configs, substeps * sizeof(NumiClothConfig), cudaMemcpyHostToDevice, h->stream) !=
