@@ -984,6 +984,7 @@ class TileBuilder {
         }
     }
     void run() {
+        RelaxedCapture relaxed;   // also where the thread is the last to drop a job
         std::unique_lock<std::mutex> lock(mutex_);
         for (;;) {
             wake_.wait(lock, [&] { return stop_ || !queue_.empty(); });
